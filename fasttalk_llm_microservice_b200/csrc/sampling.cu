@@ -1,25 +1,41 @@
 // K7 — fused temperature / top-k / top-p / argmax sampling over fp32 logits [B, V].
 //
-// One 1024-thread CTA per sequence.  Greedy (temperature <= 0) is an argmax with
-// lowest-index tie-break (torch.argmax semantics).  Otherwise e_i = exp((x_i - max)/T) and the
-// kept set is found WITHOUT sorting: a 3-level radix select over the (monotone) float bit
-// pattern of e_i finds first the k-th largest value (counts), then the nucleus threshold
-// (masses) in 3 passes each; the draw walks the kept set in index order.  The row (513 KB for
-// V = 128256) stays L2-resident between passes.
+// One cluster of up to eight CTAs per sequence, each with one contiguous share of the row.  Greedy (temperature <= 0) is an
+// argmax with lowest-index tie-break (torch.argmax semantics).  Otherwise every CTA keeps the weights e_i = exp((x_i - max)/T) of
+// its share in shared memory, so the row is read from memory once, and the kept set is found WITHOUT sorting: a radix select over
+// the (monotone) bit pattern of e_i finds first the k-th largest value (counts), then the nucleus threshold (masses), in at most
+// three passes of 11 / 11 / 9 bits each — a pass ends the search as soon as its bin holds one element.  Histograms are whole
+// numbers: a bin's mass is count * (smallest value of the bin) + (sum of the elements' offsets in it) * (their unit), which the
+// native integer atomics of shared memory add up exactly and in any order, where adding the floats themselves would loop on
+// compare-and-swap and depend on the order.  CTA r of the cluster sums bins [r, r + 1) * 2048 / C over the cluster's histograms.
+// The draw walks the kept set in index order.
+//
+// What bounds it: a chain of short passes over data in shared memory and of cluster barriers (3 per radix pass).  One CTA per row
+// with every pass reading the row again took 148 us for one row of 128256 and 202 us for 64 (greedy and sampled rows mixed);
+// the cluster takes 25 and 69 us.
 #include "common.cuh"
 #include "ft_internal.h"
 
 namespace ft {
 
-constexpr int SAMPLE_THREADS = 1024;
+constexpr int SAMPLE_THREADS = 512;
 constexpr int SAMPLE_WARPS = SAMPLE_THREADS / 32;
+constexpr int SAMPLE_BINS = 2048, SAMPLE_GROUPS = SAMPLE_BINS / 64;
+constexpr int SAMPLE_MAX_CTAS = 8;          // portable cluster size
+constexpr int SAMPLE_PARTS = 32;            // runs of a row whose sums the draw adds up
+constexpr int SAMPLE_CACHE = 40960;         // weights a CTA keeps (160 KB); a longer share's rest is formed again in every pass
 
 struct SampleSmem {
-    float hist[2048];
-    float warp_val[SAMPLE_WARPS];
-    int warp_idx[SAMPLE_WARPS];
-    float bc_f[4];
-    int bc_i[4];
+    unsigned cnt[SAMPLE_BINS], hi[SAMPLE_BINS], lo[SAMPLE_BINS];      // a bin's elements, and their offsets in two parts
+    float bins[SAMPLE_GROUPS][64];                                    // weights of the bins this CTA sums over the cluster
+    bool single_in[SAMPLE_GROUPS][64];
+    double total[SAMPLE_GROUPS];                                      // from here to `single`: written by every CTA of the cluster
+    float group[SAMPLE_GROUPS], mass[SAMPLE_PARTS];
+    float val[SAMPLE_MAX_CTAS], above, target;
+    int idx[SAMPLE_MAX_CTAS];
+    int bin, single;
+    float warp_f[SAMPLE_WARPS];
+    int warp_i[SAMPLE_WARPS];
 };
 
 __device__ __forceinline__ unsigned long long splitmix64(unsigned long long x) {
@@ -29,124 +45,202 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long x) {
     return x ^ (x >> 31);
 }
 
-__device__ __forceinline__ float block_max(float v, SampleSmem& sm) {
-    v = warp_max(v);
-    if ((threadIdx.x & 31) == 0) sm.warp_val[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float r = sm.warp_val[0];
-#pragma unroll
-    for (int w = 1; w < SAMPLE_WARPS; ++w) r = fmaxf(r, sm.warp_val[w]);
-    __syncthreads();
+// The same shared-memory variable in another CTA of the cluster.
+__device__ __forceinline__ uint32_t peer_addr(const void* p, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
     return r;
 }
-
-__device__ __forceinline__ float weight_of(float x, float maxv, float inv_t) {
-    return __expf((x - maxv) * inv_t);
+__device__ __forceinline__ unsigned peer_ld(const unsigned* p, int rank) {
+    unsigned v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_addr(p, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void peer_st(int* p, int rank, int v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer_addr(p, rank)), "r"(v) : "memory");
+}
+__device__ __forceinline__ void peer_st(float* p, int rank, float v) { peer_st(reinterpret_cast<int*>(p), rank, __float_as_int(v)); }
+__device__ __forceinline__ void peer_st(double* p, int rank, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(peer_addr(p, rank)), "d"(v) : "memory");
 }
 
-// Largest key K such that weight{key >= K, key >= min_key} >= target (weight = count or mass).
-// Returns K; *w_ge = weight{key >= K}.  All threads must call; result is uniform.
-__device__ uint32_t radix_threshold(const float* __restrict__ x, int V, float maxv, float inv_t,
-                                    uint32_t min_key, float target, bool by_mass, SampleSmem& sm,
-                                    float* w_ge) {
+// e = exp((x - max) / T) as its bit pattern; 0 where the difference has no value (NaN logits, infinity minus infinity)
+__device__ __forceinline__ uint32_t weight_key(float x, float maxv, float inv_t) {
+    const float e = __expf((x - maxv) * inv_t);
+    return e > 0.f ? __float_as_uint(e) : 0u;
+}
+
+// A CTA's share of the row: the cached weights, and the logits of what did not fit.
+struct SampleShare {
+    const uint32_t* key;
+    const float* x;
+    int n, cached;
+    float maxv, inv_t;
+    __device__ __forceinline__ uint32_t at(int i) const { return i < cached ? key[i] : weight_key(x[i], maxv, inv_t); }
+};
+
+// Largest key K such that weight{key >= K, key >= min_key} >= target, or a smaller one that keeps the same elements.  MASS: the
+// weight is the sum of the elements, and the target `part` of the sum of all elements with key >= min_key; otherwise the weight is
+// their number and the target `part` itself.  The bins are walked from the top in 32-bit sums, 64 at a time and then one by one,
+// whatever C is.  Every thread of the cluster calls; the result is the same for all.
+template <bool MASS>
+__device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, float part, int rank, int C, SampleSmem& sm) {
+    const int shifts[3] = {20, 9, 0}, bits[3] = {11, 11, 9};
+    const int groups = SAMPLE_GROUPS / C, w = threadIdx.x >> 5, l = threadIdx.x & 31;      // this CTA's groups of 64 bins
     uint32_t prefix = 0, mask = 0;
-    float above = 0.f, at = 0.f;
-    const int shifts[3] = {20, 9, 0};
-    const int bits[3] = {11, 11, 9};
+    float above = 0.f, target = part;
     for (int lvl = 0; lvl < 3; ++lvl) {
         const int shift = shifts[lvl], nb = 1 << bits[lvl];
-        for (int i = threadIdx.x; i < 2048; i += SAMPLE_THREADS) sm.hist[i] = 0.f;
-        __syncthreads();
-        for (int i = threadIdx.x; i < V; i += SAMPLE_THREADS) {
-            const float e = weight_of(x[i], maxv, inv_t);
-            const uint32_t key = __float_as_uint(e);
-            if (key >= min_key && (key & mask) == prefix)
-                atomicAdd(&sm.hist[(key >> shift) & (nb - 1)], by_mass ? e : 1.f);
+        for (int i = threadIdx.x; i < SAMPLE_BINS; i += SAMPLE_THREADS) {
+            sm.cnt[i] = 0;
+            if (MASS) sm.hi[i] = sm.lo[i] = 0;
         }
         __syncthreads();
-        // warp w sums bins [64w, 64w+64)
-        {
-            const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-            float s = sm.hist[w * 64 + l] + sm.hist[w * 64 + 32 + l];
-            s = warp_sum(s);
-            if (l == 0) sm.warp_val[w] = s;
+        for (int i = threadIdx.x; i < s.n; i += SAMPLE_THREADS) {
+            const uint32_t key = s.at(i);
+            if (key >= min_key && (key & mask) == prefix) {
+                const uint32_t b = (key >> shift) & (nb - 1), off = key & ((1u << shift) - 1);
+                atomicAdd(&sm.cnt[b], 1u);
+                if (MASS && (off >> 10)) atomicAdd(&sm.hi[b], off >> 10);
+                if (MASS && (off & 1023u)) atomicAdd(&sm.lo[b], off & 1023u);
+            }
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float acc = above;
-            int bin = 0;
-            float acc_above = above, at_bin = 0.f;
-            bool found = false;
-            for (int w = SAMPLE_WARPS - 1; w >= 0 && !found; --w) {
-                if (acc + sm.warp_val[w] >= target) {
-                    for (int b = w * 64 + 63; b >= w * 64; --b) {
-                        if (acc + sm.hist[b] >= target) {
-                            bin = b; acc_above = acc; at_bin = sm.hist[b]; found = true;
-                            break;
-                        }
-                        acc += sm.hist[b];
+        cluster_sync_all();                          // every histogram of the cluster is complete
+        for (int g = w; g < groups; g += SAMPLE_WARPS) {      // a warp per group: bins l and l + 32 of it
+            float wt[2];
+            double all = 0.0;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int b = (rank * groups + g) * 64 + 32 * j + l;
+                unsigned c = 0;
+                unsigned long long off = 0;
+                for (int p = 0; p < C; ++p) {
+                    c += peer_ld(&sm.cnt[b], p);
+                    if (MASS) off += ((unsigned long long)peer_ld(&sm.hi[b], p) << 10) + peer_ld(&sm.lo[b], p);
+                }
+                double m = (double)c;
+                if (MASS && c) {
+                    const uint32_t k0 = prefix | ((uint32_t)b << shift);
+                    const double base = (double)__uint_as_float(k0);
+                    m = m * base + (double)off * ((double)__uint_as_float(k0 + 1) - base);
+                }
+                wt[j] = (float)m;
+                sm.bins[g][32 * j + l] = wt[j];
+                sm.single_in[g][32 * j + l] = c == 1u;
+                all += m;
+            }
+            const float sum = warp_sum(wt[0] + wt[1]);
+            if (MASS && lvl == 0)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+            if (l == 0)
+                for (int p = 0; p < C; ++p) {
+                    peer_st(&sm.group[rank * groups + g], p, sum);
+                    if (MASS && lvl == 0) peer_st(&sm.total[rank * groups + g], p, all);
+                }
+        }
+        cluster_sync_all();                          // the groups' sums are everywhere; the histograms have been read
+        if (w == 0) {
+            if (MASS && lvl == 0) {
+                double z = sm.total[l];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+                target = part * (float)z;
+            }
+            // every lane walks the same way: the group, then the bin in it
+            const float gs = sm.group[l];
+            float acc = above, stop = above;
+            int in = -1;
+#pragma unroll
+            for (int g = SAMPLE_GROUPS - 1; g >= 0; --g) {
+                const float v = __shfl_sync(0xffffffffu, gs, g);
+                if (in < 0 && acc + v >= target) { in = g; stop = acc; }
+                acc += v;
+            }
+            if (in / groups == rank || (in < 0 && rank == 0)) {
+                const float v0 = sm.bins[max(in, 0) % groups][l], v1 = sm.bins[max(in, 0) % groups][l + 32];
+                float over = stop, at = 0.f;
+                int bin = -1;
+                if (in >= 0) {
+                    float run = stop;
+#pragma unroll
+                    for (int j = 63; j >= 0; --j) {
+                        const float v = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, j & 31);
+                        if (bin < 0 && run + v >= target) { bin = j; over = run; }
+                        run += v;
+                        if (j == 0) at = v;
                     }
-                    if (!found) {      // rounding: the warp total said yes, the walk said no
-                        bin = w * 64; acc_above = acc - sm.hist[bin]; at_bin = sm.hist[bin]; found = true;
-                    }
-                } else {
-                    acc += sm.warp_val[w];
+                    if (bin < 0) { bin = 0; over = run - at - at; }      // rounding: the group's sum said yes, the walk said no
+                } else {                              // more than there is: keep everything
+                    bin = 0;
+                    over = acc - __shfl_sync(0xffffffffu, v0, 0);
+                    in = 0;
+                }
+                if (l < C) {
+                    peer_st(&sm.bin, l, in * 64 + bin);
+                    peer_st(&sm.single, l, sm.single_in[in % groups][bin] ? 1 : 0);
+                    peer_st(&sm.above, l, over);
+                    peer_st(&sm.target, l, target);
                 }
             }
-            if (!found) {              // target above the total weight: keep everything
-                bin = 0; acc_above = acc - sm.hist[0]; at_bin = sm.hist[0];
-            }
-            sm.bc_i[0] = bin;
-            sm.bc_f[0] = acc_above;
-            sm.bc_f[1] = at_bin;
         }
-        __syncthreads();
-        prefix |= (uint32_t)sm.bc_i[0] << shift;
+        cluster_sync_all();
+        prefix |= (uint32_t)sm.bin << shift;
         mask |= (uint32_t)(nb - 1) << shift;
-        above = sm.bc_f[0];
-        at = sm.bc_f[1];
-        __syncthreads();
+        above = sm.above;
+        target = sm.target;
+        if (sm.single) break;                        // the bin's only element is the one: its lower edge keeps the same set
     }
-    *w_ge = above + at;
     return prefix < min_key ? min_key : prefix;
 }
 
-__global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__ temperature,
+__global__ void __launch_bounds__(SAMPLE_THREADS, 2)
+sample_kernel(const float* __restrict__ logits, int V, int span, int cache, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
-              const unsigned long long* __restrict__ seeds, int* __restrict__ out_tokens) {
+              const unsigned long long* __restrict__ seeds, int* __restrict__ out_tokens, int C) {
     __shared__ SampleSmem sm;
+    extern __shared__ __align__(16) uint32_t keys[];
+    const int b = blockIdx.x / C, rank = blockIdx.x % C;      // clusters are runs of C consecutive blocks
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     pdl_wait();
     pdl_launch_dependents();
-    const int b = blockIdx.x;
-    const float* x = logits + (size_t)b * V;
+    const int lo = min(rank * span, V), hi = min(lo + span, V);
+    const float* x = logits + (size_t)b * V + lo;
+    SampleShare s;
+    s.key = keys; s.x = x; s.n = hi - lo;
     const float temp = temperature ? temperature[b] : 0.f;
+    const bool greedy = temp <= 1e-6f;
+    s.cached = greedy ? 0 : min(s.n, cache);
 
-    // ---- max (+ argmax, lowest index on ties)
+    // ---- max (+ argmax, lowest index on ties); the logits of a sampled row stay in shared memory
     float best = -INFINITY;
     int best_i = 0x7fffffff;
-    if ((V & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-        // 16-byte loads, four in flight per thread: the row is 513 KB behind ONE CTA, so it is the
-        // number of outstanding loads, not arithmetic, that sets this pass's time
+    auto take = [&](float v, int i) {                // ascending index order inside the thread
+        if (v > best) { best = v; best_i = lo + i; }
+    };
+    if ((s.n & 3) == 0 && (s.cached & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+        // 16-byte loads, four in flight per thread
         const float4* x4 = reinterpret_cast<const float4*>(x);
-        const int n4 = V >> 2;
-        auto take = [&](const float4& v, int i4) {      // ascending index order inside the thread
-            if (v.x > best) { best = v.x; best_i = 4 * i4; }
-            if (v.y > best) { best = v.y; best_i = 4 * i4 + 1; }
-            if (v.z > best) { best = v.z; best_i = 4 * i4 + 2; }
-            if (v.w > best) { best = v.w; best_i = 4 * i4 + 3; }
-        };
-        int i = threadIdx.x;
-        for (; i + 3 * SAMPLE_THREADS < n4; i += 4 * SAMPLE_THREADS) {
-            const float4 a = __ldcg(x4 + i), b4 = __ldcg(x4 + i + SAMPLE_THREADS),
-                         c4 = __ldcg(x4 + i + 2 * SAMPLE_THREADS), d4 = __ldcg(x4 + i + 3 * SAMPLE_THREADS);
-            take(a, i); take(b4, i + SAMPLE_THREADS); take(c4, i + 2 * SAMPLE_THREADS); take(d4, i + 3 * SAMPLE_THREADS);
+        const int n4 = s.n >> 2;
+        for (int i = threadIdx.x; i < n4; i += 4 * SAMPLE_THREADS) {
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i + u * SAMPLE_THREADS < n4) v[u] = __ldcg(x4 + i + u * SAMPLE_THREADS);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int c = 4 * (i + u * SAMPLE_THREADS);
+                if (c >= s.n) break;
+                take(v[u].x, c); take(v[u].y, c + 1); take(v[u].z, c + 2); take(v[u].w, c + 3);
+                if (c < s.cached) *reinterpret_cast<float4*>(keys + c) = v[u];
+            }
         }
-        for (; i < n4; i += SAMPLE_THREADS) take(__ldcg(x4 + i), i);
     } else {
-        for (int i = threadIdx.x; i < V; i += SAMPLE_THREADS) {
+        for (int i = threadIdx.x; i < s.n; i += SAMPLE_THREADS) {
             const float v = x[i];
-            if (v > best) { best = v; best_i = i; }      // ascending i per thread: first max wins
+            take(v, i);
+            if (i < s.cached) keys[i] = __float_as_uint(v);
         }
     }
 #pragma unroll
@@ -155,128 +249,131 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
         const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
         if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
     }
-    if ((threadIdx.x & 31) == 0) { sm.warp_val[threadIdx.x >> 5] = best; sm.warp_idx[threadIdx.x >> 5] = best_i; }
+    if (l == 0) { sm.warp_f[w] = best; sm.warp_i[w] = best_i; }
     __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // every CTA of the cluster has started
     if (threadIdx.x == 0) {
-        float bv = sm.warp_val[0];
-        int bi = sm.warp_idx[0];
-        for (int w = 1; w < SAMPLE_WARPS; ++w)
-            if (sm.warp_val[w] > bv || (sm.warp_val[w] == bv && sm.warp_idx[w] < bi)) {
-                bv = sm.warp_val[w]; bi = sm.warp_idx[w];
-            }
-        sm.bc_f[2] = bv;
-        sm.bc_i[2] = bi;
+        for (int i = 1; i < SAMPLE_WARPS; ++i)
+            if (sm.warp_f[i] > best || (sm.warp_f[i] == best && sm.warp_i[i] < best_i)) { best = sm.warp_f[i]; best_i = sm.warp_i[i]; }
+        for (int p = 0; p < C; ++p) {
+            peer_st(&sm.val[rank], p, best);
+            peer_st(&sm.idx[rank], p, best_i);
+        }
     }
-    __syncthreads();
-    const float maxv = sm.bc_f[2];
-    const int argmax = sm.bc_i[2];
-    __syncthreads();
-    if (temp <= 1e-6f) {
-        if (threadIdx.x == 0) out_tokens[b] = argmax;
+    cluster_sync_all();
+    float maxv = sm.val[0];
+    int argmax = sm.idx[0];
+    for (int p = 1; p < C; ++p)
+        if (sm.val[p] > maxv) { maxv = sm.val[p]; argmax = sm.idx[p]; }      // shares are in index order: the first maximum wins
+    if (greedy) {
+        if (rank == 0 && threadIdx.x == 0) out_tokens[b] = argmax;
         return;
     }
-    const float inv_t = 1.f / temp;
+    s.maxv = maxv;
+    s.inv_t = 1.f / temp;
+    for (int i = threadIdx.x; i < s.cached; i += SAMPLE_THREADS) keys[i] = weight_key(__uint_as_float(keys[i]), maxv, s.inv_t);
+    __syncthreads();
     const int k = top_k ? top_k[b] : 0;
     const float p = top_p ? top_p[b] : 1.f;
 
     uint32_t thr = 0;           // keep keys >= thr
-    float kept = 0.f;           // mass of the kept set
-    bool have_mass = false;
-    if (k > 0 && k < V) {
-        float cnt;
-        thr = radix_threshold(x, V, maxv, inv_t, 0u, (float)k, false, sm, &cnt);
-    }
+    if (k > 0 && k < V) thr = radix_threshold<false>(s, 0u, (float)k, rank, C, sm);
     if (p < 1.f) {
-        // mass of the top-k survivors (or of everything)
-        float z = 0.f;
-        for (int i = threadIdx.x; i < V; i += SAMPLE_THREADS) {
-            const float e = weight_of(x[i], maxv, inv_t);
-            if (__float_as_uint(e) >= thr) z += e;
-        }
-        z = warp_sum(z);
-        if ((threadIdx.x & 31) == 0) sm.warp_val[threadIdx.x >> 5] = z;
-        __syncthreads();
-        float Z = 0.f;
-        for (int w = 0; w < SAMPLE_WARPS; ++w) Z += sm.warp_val[w];
-        __syncthreads();
-        thr = radix_threshold(x, V, maxv, inv_t, thr, p * Z, true, sm, &kept);
-        have_mass = false;      // recompute exactly below (histogram sums are order-dependent)
+        if (p > 0.f) thr = radix_threshold<true>(s, thr, p, rank, C, sm);
+        else thr = 0xffffffffu;                      // an empty nucleus: the most likely token
     }
-    (void)have_mass;
 
-    // ---- draw: warp w owns the contiguous index range [w*span, (w+1)*span)
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int span = (V + SAMPLE_WARPS - 1) / SAMPLE_WARPS;
-    const int lo = w * span, hi = lo + span < V ? lo + span : V;
-    float mine = 0.f;
-    for (int i = lo + l; i < hi; i += 32) {
-        const float e = weight_of(x[i], maxv, inv_t);
-        if (__float_as_uint(e) >= thr) mine += e;
-    }
-    mine = warp_sum(mine);
-    if (l == 0) sm.warp_val[w] = mine;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float tot = 0.f;
-        for (int i = 0; i < SAMPLE_WARPS; ++i) tot += sm.warp_val[i];
-        const unsigned long long r = splitmix64(seeds ? seeds[b] : 0x1234ull + b);
-        const float u = (float)(r >> 40) * (1.0f / 16777216.0f) * tot;      // [0, tot)
-        float acc = 0.f;
-        int ww = SAMPLE_WARPS - 1;
-        for (int i = 0; i < SAMPLE_WARPS; ++i) {
-            if (acc + sm.warp_val[i] > u) { ww = i; break; }
-            acc += sm.warp_val[i];
-        }
-        // if rounding pushed u past the total, fall back to the last warp that holds mass
-        while (ww > 0 && sm.warp_val[ww] == 0.f) --ww;
-        sm.bc_i[0] = ww;
-        sm.bc_f[0] = u - acc;
-        sm.bc_i[1] = argmax;       // final fallback
-    }
-    __syncthreads();
-    if (w == sm.bc_i[0]) {
-        float need = sm.bc_f[0];
-        int chosen = -1, last_kept = -1;
-        float run = 0.f;
-        for (int i0 = lo; i0 < hi && chosen < 0; i0 += 32) {
-            const int i = i0 + l;
-            float e = 0.f;
-            if (i < hi) {
-                e = weight_of(x[i], maxv, inv_t);
-                if (__float_as_uint(e) < thr) e = 0.f;
-            }
-            float inc = e;          // inclusive warp scan
+    // ---- draw: the row as SAMPLE_PARTS runs of `part` elements, 1 / C of them in this CTA's share.  A run is summed by one warp and
+    // the runs' sums are added in order whatever C is, so that a token does not depend on how the row was shared out.
+    auto kept = [&](int i) {
+        const uint32_t key = s.at(i);
+        return key >= thr ? __uint_as_float(key) : 0.f;
+    };
+    const int part = span / (SAMPLE_PARTS / C);
+    for (int q = w; q < SAMPLE_PARTS / C; q += SAMPLE_WARPS) {
+        const int qhi = min((q + 1) * part, s.n);
+        float mine = 0.f;
+        int i = q * part + l;
+        for (; i + 7 * 32 < qhi; i += 8 * 32) {       // eight reads in flight, added one by one
+            float e[8];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const float n = __shfl_up_sync(0xffffffffu, inc, o);
-                if (l >= o) inc += n;
-            }
-            const bool hit = e > 0.f && run + inc > need;
-            const unsigned ballot = __ballot_sync(0xffffffffu, hit);
-            const unsigned kept_mask = __ballot_sync(0xffffffffu, e > 0.f);
-            if (kept_mask) last_kept = i0 + 31 - __clz(kept_mask);
-            if (ballot) chosen = i0 + __ffs(ballot) - 1;
-            run += __shfl_sync(0xffffffffu, inc, 31);
+            for (int u = 0; u < 8; ++u) e[u] = kept(i + u * 32);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) mine += e[u];
         }
-        if (l == 0) out_tokens[b] = chosen >= 0 ? chosen : (last_kept >= 0 ? last_kept : sm.bc_i[1]);
+        for (; i < qhi; i += 32) mine += kept(i);
+        mine = warp_sum(mine);
+        if (l == 0)
+            for (int peer = 0; peer < C; ++peer) peer_st(&sm.mass[rank * (SAMPLE_PARTS / C) + q], peer, mine);
     }
+    cluster_sync_all();                              // nothing is read from or written to another CTA after this
+    float tot = 0.f;
+    for (int q = 0; q < SAMPLE_PARTS; ++q) tot += sm.mass[q];
+    if (!(tot > 0.f)) {
+        if (rank == 0 && threadIdx.x == 0) out_tokens[b] = argmax;
+        return;
+    }
+    const unsigned long long r = splitmix64(seeds ? seeds[b] : 0x1234ull + b);
+    const float u = (float)(r >> 40) * (1.0f / 16777216.0f) * tot;      // [0, tot)
+    float before = 0.f;
+    int in = SAMPLE_PARTS - 1;
+    for (int q = 0; q < SAMPLE_PARTS; ++q) {
+        if (before + sm.mass[q] > u) { in = q; break; }
+        before += sm.mass[q];
+    }
+    while (in > 0 && sm.mass[in] == 0.f) --in;        // rounding pushed u past the total: the last run that holds mass
+    if (in / (SAMPLE_PARTS / C) != rank || w != 0) return;
+    const float need = u - before;
+    const int wlo = in % (SAMPLE_PARTS / C) * part, whi = min(wlo + part, s.n);
+    int chosen = -1, last_kept = -1;
+    float run = 0.f;
+    for (int b0 = wlo; b0 < whi && chosen < 0; b0 += 32) {
+        const int i = b0 + l;
+        const float e = i < whi ? kept(i) : 0.f;
+        float inc = e;          // inclusive warp scan
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float n = __shfl_up_sync(0xffffffffu, inc, o);
+            if (l >= o) inc += n;
+        }
+        const unsigned ballot = __ballot_sync(0xffffffffu, e > 0.f && run + inc > need);
+        const unsigned kept_mask = __ballot_sync(0xffffffffu, e > 0.f);
+        if (kept_mask) last_kept = b0 + 31 - __clz(kept_mask);
+        if (ballot) chosen = b0 + __ffs(ballot) - 1;
+        run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (l == 0) out_tokens[b] = chosen >= 0 ? lo + chosen : last_kept >= 0 ? lo + last_kept : argmax;
 }
 
 int launch_sample(const float* logits, int B, int V, const float* temperature, const int* top_k,
                   const float* top_p, const unsigned long long* seeds, int* out_tokens, bool pdl,
                   cudaStream_t stream) {
     FT_REQUIRE(B >= 1 && V >= 1, "sample: B=%d V=%d", B, V);
+    // CTAs per row: a share of 4096 logits keeps 512 threads busy for longer than a cluster barrier takes
+    int C = 1;
+    while (C < SAMPLE_MAX_CTAS && V > 4096 * C) C *= 2;
+    while (C > 1 && (long long)B * C > 0x7fffffffll) C /= 2;
+    const int span = (V + SAMPLE_PARTS - 1) / SAMPLE_PARTS * (SAMPLE_PARTS / C);      // a multiple of 4: shares start on 16 bytes where the rows do
+    const int cache = span < SAMPLE_CACHE ? span : SAMPLE_CACHE;
+    static PerDeviceFlag attr_set;
+    if (!attr_set.done()) {
+        FT_CHECK_CUDA(cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_CACHE * 4));
+        attr_set.mark();
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(B);
+    cfg.gridDim = dim3(B * C);
     cfg.blockDim = dim3(SAMPLE_THREADS);
+    cfg.dynamicSmemBytes = temperature ? (size_t)cache * 4 : 0;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, sample_kernel, logits, V, temperature, top_k, top_p, seeds,
-                                     out_tokens));
+    cfg.numAttrs = pdl ? 2 : 1;
+    FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, sample_kernel, logits, V, span, cache, temperature, top_k, top_p, seeds,
+                                     out_tokens, C));
     return 0;
 }
 

@@ -564,6 +564,57 @@ def test_sample_full_vocab_row(K):
         assert ref[tok[b].item()] > 0
 
 
+def _draw_point(seed):
+    """The 24-bit point of [0, 1) that a row's seed stands for (splitmix64)."""
+    m = (1 << 64) - 1
+    x = (int(seed) + 0x9E3779B97F4A7C15) & m
+    x = ((x ^ (x >> 30)) * 0xBF58476D1CE4E5B9) & m
+    x = ((x ^ (x >> 27)) * 0x94D049BB133111EB) & m
+    return ((x ^ (x >> 31)) >> 40) / 16777216.0
+
+
+@pytest.mark.parametrize("B,V", [(3, 1), (5, 3), (2, 4096), (3, 4097), (2, 32767), (7, 50257), (3, 128256), (2, 8 * 40960 + 37)])
+def test_sample_against_the_sorted_row(K, B, V):
+    """Shares of one, two, four and eight CTAs, rows that do not start on 16 bytes, a share beyond the cached weights: the token is
+    the one whose stretch of the kept probabilities (index order, 64 bits) holds the row's point, give or take the rounding of
+    32-bit sums, and it is in the kept set, whose edge may move by one token for the same reason."""
+    g = torch.Generator(device=DEV).manual_seed(V)
+    logits = torch.randn(B, V, device=DEV, generator=g) * 2.5
+    for temp, k, p in [(0.7, 0, 0.9), (0.7, 40, 0.9), (1.3, 5, 1.0), (1.0, 0, 1.0), (0.4, 1, 0.5), (0.9, 0, 1e-6), (1.0, 0, 0.0)]:
+        seeds = torch.randint(1 << 62, (B,), device=DEV, generator=g, dtype=torch.int64)
+        tok = K.sample(logits, torch.full((B,), temp, device=DEV), torch.full((B,), k, device=DEV, dtype=torch.int32),
+                       torch.full((B,), p, device=DEV), seeds)
+        for b in range(B):
+            t = int(tok[b])
+            if p <= 0.0:
+                assert t == int(logits[b].argmax())
+                continue
+            prob = O.sampling_support(logits[b].cpu(), temp, k, p)
+            cum = torch.cumsum(prob, 0)
+            u = _draw_point(seeds[b])
+            # 32-bit sums of up to V terms and exp to a few ulp; one token more or less at the nucleus' edge moves every stretch
+            slack = 1e-5 + (float(prob[prob > 0].min()) if p < 1.0 else 0.0)
+            assert prob[t] > 0, (temp, k, p, b)
+            assert float(cum[t] - prob[t]) - slack <= u <= float(cum[t]) + slack, (temp, k, p, b)
+
+
+def test_sample_rows_without_numbers(K):
+    """Infinities and NaN: minus infinity is never drawn, an infinite logit wins, a NaN is never drawn, the index stays inside."""
+    V = 32768
+    logits = torch.randn(6, V, device=DEV, generator=torch.Generator(device=DEV).manual_seed(4))
+    logits[0, : V - 5] = -float("inf")
+    logits[1, 777] = float("inf")
+    logits[2, 3] = float("nan")
+    logits[3] = -float("inf")
+    logits[4] = float("nan")
+    logits[5, ::2] = -float("inf")
+    n = torch.full((6,), 0.8, device=DEV)
+    for top_k, top_p in [(0, 1.0), (20, 0.9), (0, 0.9)]:
+        tok = K.sample(logits, n, torch.full((6,), top_k, device=DEV, dtype=torch.int32), torch.full((6,), top_p, device=DEV),
+                       torch.arange(6, device=DEV, dtype=torch.int64)).tolist()
+        assert tok[0] >= V - 5 and tok[1] == 777 and 0 <= tok[2] < V and tok[2] != 3 and tok[5] % 2 == 1
+
+
 def test_gemm_split_k_alternating_arrival_words(K):
     """ft_gemm_epilogue.sync_mode 1 / 2 (what the engine uses): launches that share one `sync` buffer alternate
     between the two words of each counter pair and clear the other for ALL slots, whatever their tile counts —
