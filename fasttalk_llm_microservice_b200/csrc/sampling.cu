@@ -27,8 +27,6 @@ constexpr int SAMPLE_CACHE = 40960;         // weights a CTA keeps (160 KB); a l
 
 struct SampleSmem {
     unsigned cnt[SAMPLE_BINS], hi[SAMPLE_BINS], lo[SAMPLE_BINS];      // a bin's elements, and their offsets in two parts
-    float bins[SAMPLE_GROUPS][64];                                    // weights of the bins this CTA sums over the cluster
-    bool single_in[SAMPLE_GROUPS][64];
     double total[SAMPLE_GROUPS];                                      // from here to `single`: written by every CTA of the cluster
     float group[SAMPLE_GROUPS], mass[SAMPLE_PARTS];
     float val[SAMPLE_MAX_CTAS], above, target;
@@ -79,6 +77,21 @@ struct SampleShare {
     __device__ __forceinline__ uint32_t at(int i) const { return i < cached ? key[i] : weight_key(x[i], maxv, inv_t); }
 };
 
+// Adds the n lanes' values to acc one by one from the last lane down and stops at the first that would reach the target; -1: none does.
+__device__ __forceinline__ int walk_down(float v, int n, float& acc, float target) {
+    for (int top = n - 8; top >= 0; top -= 8) {
+        float x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = __shfl_sync(0xffffffffu, v, top + 7 - u);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (acc + x[u] >= target) return top + 7 - u;
+            acc += x[u];
+        }
+    }
+    return -1;
+}
+
 // Largest key K such that weight{key >= K, key >= min_key} >= target, or a smaller one that keeps the same elements.  MASS: the
 // weight is the sum of the elements, and the target `part` of the sum of all elements with key >= min_key; otherwise the weight is
 // their number and the target `part` itself.  The bins are walked from the top in 32-bit sums, 64 at a time and then one by one,
@@ -106,17 +119,30 @@ __device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, floa
             }
         }
         cluster_sync_all();                          // every histogram of the cluster is complete
-        for (int g = w; g < groups; g += SAMPLE_WARPS) {      // a warp per group: bins l and l + 32 of it
-            float wt[2];
+        // warp w sums groups w and w + 16 of this CTA over the cluster, two bins of each per lane
+        float wt[2][2];
+        unsigned ct[2][2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int g = w + SAMPLE_WARPS * x;
+            if (g >= groups) break;
             double all = 0.0;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const int b = (rank * groups + g) * 64 + 32 * j + l;
+                unsigned pc[SAMPLE_MAX_CTAS], ph[SAMPLE_MAX_CTAS], pl[SAMPLE_MAX_CTAS];      // all reads in flight before the first sum
+#pragma unroll
+                for (int p = 0; p < SAMPLE_MAX_CTAS; ++p) {
+                    pc[p] = p < C ? peer_ld(&sm.cnt[b], p) : 0u;
+                    ph[p] = MASS && p < C ? peer_ld(&sm.hi[b], p) : 0u;
+                    pl[p] = MASS && p < C ? peer_ld(&sm.lo[b], p) : 0u;
+                }
                 unsigned c = 0;
                 unsigned long long off = 0;
-                for (int p = 0; p < C; ++p) {
-                    c += peer_ld(&sm.cnt[b], p);
-                    if (MASS) off += ((unsigned long long)peer_ld(&sm.hi[b], p) << 10) + peer_ld(&sm.lo[b], p);
+#pragma unroll
+                for (int p = 0; p < SAMPLE_MAX_CTAS; ++p) {
+                    c += pc[p];
+                    off += ((unsigned long long)ph[p] << 10) + pl[p];
                 }
                 double m = (double)c;
                 if (MASS && c) {
@@ -124,65 +150,53 @@ __device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, floa
                     const double base = (double)__uint_as_float(k0);
                     m = m * base + (double)off * ((double)__uint_as_float(k0 + 1) - base);
                 }
-                wt[j] = (float)m;
-                sm.bins[g][32 * j + l] = wt[j];
-                sm.single_in[g][32 * j + l] = c == 1u;
+                wt[x][j] = (float)m;
+                ct[x][j] = c;
                 all += m;
             }
-            const float sum = warp_sum(wt[0] + wt[1]);
+            const float sum = warp_sum(wt[x][0] + wt[x][1]);
             if (MASS && lvl == 0)
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
-            if (l == 0)
-                for (int p = 0; p < C; ++p) {
-                    peer_st(&sm.group[rank * groups + g], p, sum);
-                    if (MASS && lvl == 0) peer_st(&sm.total[rank * groups + g], p, all);
-                }
+            if (l < C) {
+                peer_st(&sm.group[rank * groups + g], l, sum);
+                if (MASS && lvl == 0) peer_st(&sm.total[rank * groups + g], l, all);
+            }
         }
         cluster_sync_all();                          // the groups' sums are everywhere; the histograms have been read
-        if (w == 0) {
+        if (w < groups) {
             if (MASS && lvl == 0) {
                 double z = sm.total[l];
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
                 target = part * (float)z;
             }
-            // every lane walks the same way: the group, then the bin in it
+            // every lane walks the same way: the group, and in the warp that summed it the bin
             const float gs = sm.group[l];
-            float acc = above, stop = above;
-            int in = -1;
+            float acc = above;
+            const int in = walk_down(gs, SAMPLE_GROUPS, acc, target);
+            const int at = max(in, 0) - rank * groups;
 #pragma unroll
-            for (int g = SAMPLE_GROUPS - 1; g >= 0; --g) {
-                const float v = __shfl_sync(0xffffffffu, gs, g);
-                if (in < 0 && acc + v >= target) { in = g; stop = acc; }
-                acc += v;
-            }
-            if (in / groups == rank || (in < 0 && rank == 0)) {
-                const float v0 = sm.bins[max(in, 0) % groups][l], v1 = sm.bins[max(in, 0) % groups][l + 32];
-                float over = stop, at = 0.f;
-                int bin = -1;
-                if (in >= 0) {
-                    float run = stop;
-#pragma unroll
-                    for (int j = 63; j >= 0; --j) {
-                        const float v = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, j & 31);
-                        if (bin < 0 && run + v >= target) { bin = j; over = run; }
-                        run += v;
-                        if (j == 0) at = v;
+            for (int x = 0; x < 2; ++x)
+                if (at == w + SAMPLE_WARPS * x && at < groups) {
+                    int bin = 0;
+                    float over = acc;
+                    if (in >= 0) {
+                        bin = walk_down(wt[x][1], 32, over, target);
+                        bin = bin >= 0 ? bin + 32 : walk_down(wt[x][0], 32, over, target);
+                        // rounding: the group's sum said yes, the walk said no
+                        if (bin < 0) bin = 0, over -= __shfl_sync(0xffffffffu, wt[x][0], 0);
+                    } else {                          // more than there is: keep everything
+                        over -= __shfl_sync(0xffffffffu, wt[x][0], 0);
                     }
-                    if (bin < 0) { bin = 0; over = run - at - at; }      // rounding: the group's sum said yes, the walk said no
-                } else {                              // more than there is: keep everything
-                    bin = 0;
-                    over = acc - __shfl_sync(0xffffffffu, v0, 0);
-                    in = 0;
+                    const unsigned c = bin < 32 ? __shfl_sync(0xffffffffu, ct[x][0], bin) : __shfl_sync(0xffffffffu, ct[x][1], bin - 32);
+                    if (l < C) {
+                        peer_st(&sm.bin, l, max(in, 0) * 64 + bin);
+                        peer_st(&sm.single, l, c == 1u);
+                        peer_st(&sm.above, l, over);
+                        peer_st(&sm.target, l, target);
+                    }
                 }
-                if (l < C) {
-                    peer_st(&sm.bin, l, in * 64 + bin);
-                    peer_st(&sm.single, l, sm.single_in[in % groups][bin] ? 1 : 0);
-                    peer_st(&sm.above, l, over);
-                    peer_st(&sm.target, l, target);
-                }
-            }
         }
         cluster_sync_all();
         prefix |= (uint32_t)sm.bin << shift;
@@ -322,27 +336,68 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
         before += sm.mass[q];
     }
     while (in > 0 && sm.mass[in] == 0.f) --in;        // rounding pushed u past the total: the last run that holds mass
-    if (in / (SAMPLE_PARTS / C) != rank || w != 0) return;
+    if (in / (SAMPLE_PARTS / C) != rank) return;
+    // Inside the run: blocks of 32 elements, an inclusive scan in each.  All warps scan blocks and leave every block's sum and the
+    // largest kept prefix in it; the running sum over the blocks then stops at the first one with a prefix beyond the point.
     const float need = u - before;
     const int wlo = in % (SAMPLE_PARTS / C) * part, whi = min(wlo + part, s.n);
-    int chosen = -1, last_kept = -1;
-    float run = 0.f;
-    for (int b0 = wlo; b0 < whi && chosen < 0; b0 += 32) {
+    float* bsum = reinterpret_cast<float*>(sm.cnt);
+    float* bmax = reinterpret_cast<float*>(sm.hi);
+    auto scan = [&](int b0, float& e) {
         const int i = b0 + l;
-        const float e = i < whi ? kept(i) : 0.f;
-        float inc = e;          // inclusive warp scan
+        e = i < whi ? kept(i) : 0.f;
+        float inc = e;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const float n = __shfl_up_sync(0xffffffffu, inc, o);
             if (l >= o) inc += n;
         }
-        const unsigned ballot = __ballot_sync(0xffffffffu, e > 0.f && run + inc > need);
-        const unsigned kept_mask = __ballot_sync(0xffffffffu, e > 0.f);
-        if (kept_mask) last_kept = b0 + 31 - __clz(kept_mask);
-        if (ballot) chosen = b0 + __ffs(ballot) - 1;
-        run += __shfl_sync(0xffffffffu, inc, 31);
+        return inc;
+    };
+    int last_kept = -1;
+    float run = 0.f;
+    for (int c0 = wlo; c0 < whi; c0 += 32 * SAMPLE_BINS) {      // (one round, except for rows of more than two million)
+        const int blocks = (min(c0 + 32 * SAMPLE_BINS, whi) - c0 + 31) / 32;
+        __syncthreads();
+        for (int q = w; q < blocks; q += SAMPLE_WARPS) {
+            float e;
+            const float inc = scan(c0 + 32 * q, e);
+            const float most = warp_max(e > 0.f ? inc : -1.f);
+            if (l == 31) { bsum[q] = inc; bmax[q] = most; }
+        }
+        __syncthreads();
+        int q = blocks;
+        for (int q8 = 0; q8 < blocks && q == blocks; q8 += 8) {      // every thread walks the same way, eight blocks read at a time
+            float bs[8], bm[8];
+#pragma unroll
+            for (int x = 0; x < 8; ++x) { bs[x] = bsum[q8 + x]; bm[x] = bmax[q8 + x]; }
+#pragma unroll
+            for (int x = 0; x < 8; ++x)
+                if (q8 + x < blocks && q == blocks) {
+                    if (bm[x] >= 0.f && run + bm[x] > need) q = q8 + x;
+                    else {
+                        if (bm[x] >= 0.f) last_kept = q8 + x;
+                        run += bs[x];
+                    }
+                }
+        }
+        if (q < blocks || last_kept >= 0) {
+            if (w != 0) {
+                if (q < blocks) return;
+            } else {
+                float e;
+                const int at = c0 + 32 * (q < blocks ? q : last_kept);
+                const float inc = scan(at, e);
+                const unsigned hit = __ballot_sync(0xffffffffu, e > 0.f && run + inc > need), any = __ballot_sync(0xffffffffu, e > 0.f);
+                if (q < blocks) {
+                    if (l == 0) out_tokens[b] = lo + at + __ffs(hit) - 1;
+                    return;
+                }
+                if (l == 0) out_tokens[b] = lo + at + 31 - __clz(any);      // rounding: the last kept one, unless a later round holds it
+                last_kept = -1;
+            }
+        }
     }
-    if (l == 0) out_tokens[b] = chosen >= 0 ? lo + chosen : last_kept >= 0 ? lo + last_kept : argmax;
 }
 
 int launch_sample(const float* logits, int B, int V, const float* temperature, const int* top_k,
