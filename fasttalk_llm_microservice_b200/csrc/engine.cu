@@ -592,10 +592,7 @@ static int dense(Engine* e, const float* A, const void* hi, const void* lo, cons
             hi = L.pl_hi;
             lo = L.pl_lo;
         }
-        ft_gemm_epilogue ep = {};
-        ep.mode = FT_EPI_PARTIAL;
-        ep.out = C;
-        FT_TRY(ft_gemm_fused(W, hi, lo, N, T, K, 1, &ep, e->stream));
+        FT_TRY(launch_gemm_plain(W, hi, lo, C, N, T, K, false, e->stream));
         e->st.kernel_launches++;
         if (softcap > 0.f) {
             FT_TRY(launch_softcap(C, (size_t)T * N, softcap, e->stream));

@@ -45,6 +45,10 @@ int launch_gemm(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap*
                 int T, int K, int splits, const ft_gemm_epilogue& epi, bool pdl, cudaStream_t stream,
                 const CUtensorMap* mx_half = nullptr, const CUtensorMap* mx_lo_half = nullptr);
 
+// ---- gemm_plain.cu: out[t][n] = sum_k (hi + lo)[t][k] W[n][k], fp32 results without a fused layer step
+bool gemm_plain_ok(int n_out, int T, int K);
+int launch_gemm_plain(const void* w, const void* hi, const void* lo, float* out, int n_out, int T, int K, bool pdl, cudaStream_t stream);
+
 // ---- elementwise.cu
 int launch_add_rmsnorm(float* resid, const float* partials, int n_splits, size_t split_stride,
                        const int* embed_tokens, const void* embed_table, const void* norm_w,

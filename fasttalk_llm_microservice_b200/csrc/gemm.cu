@@ -1384,6 +1384,8 @@ extern "C" int ft_gemm_fused(const void* w, const void* x, const void* x_lo, int
     const int bn = gemm_pick_bn(T, hilo);
     if (n_splits <= 0)
         n_splits = epi->mode == FT_EPI_PARTIAL || staged ? gemm_pick_splits(n_out, T, K, sms, hilo) : 1;
+    if (hilo && epi->mode == FT_EPI_PARTIAL && n_splits == 1)      // one unsplit fp32 result: the kernels made for it
+        return launch_gemm_plain(w, x, x_lo, reinterpret_cast<float*>(epi->out), n_out, T, K, false, static_cast<cudaStream_t>(stream));
     CUtensorMap mw, mx, mxl;
     if (int r = make_tmap_bf16_k64(&mw, w, n_out, K, GEMM_BM)) return r;
     if (int r = make_tmap_bf16_k64(&mx, x, T, K, bn)) return r;

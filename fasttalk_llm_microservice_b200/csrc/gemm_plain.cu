@@ -1,0 +1,403 @@
+// Plain projections on tcgen05: out[t][n] = sum_k (hi + lo)[t][k] W[n][k] in fp32, no fused layer step — every projection of the
+// layered models, and ft_gemm_bf16 / ft_gemm_fused with unsplit fp32 results.  Operands as in gemm.cu (W rows are the UMMA A operand,
+// the activation's two bf16 planes the B operand, both products into one fp32 accumulator in TMEM); two kernels:
+//
+//   many tokens   CTA pairs (cta_group::2) that walk units of 256 weight rows x `bn` tokens, two accumulators, as gemm_pair_kernel
+//                 does, with a token tile whose width is a run-time value.  A projection of 2313 tokens and 2048 rows is 152 units of
+//                 128 tokens for 74 pairs: three rounds, the last one nearly empty; 160 tokens wide it is 120 units in two.  The
+//                 width that the launcher takes is the one with the least time over all rounds (plain_token_tile).
+//                 Measured (2313 tokens, hi + lo): 2048 x 2048 45 -> 31 us, 2048 -> 10752 182 -> 150 us against one CTA per tile.
+//   few tokens    one token tile; K is shared by the up to eight CTAs of a cluster, which add their partial tiles through distributed
+//                 shared memory in rank order: no slabs, no arrival words, no second launch.  Bound by latency (launch, first load,
+//                 one pass over at most 32 chunks): 16 tokens, 2048 x 2048 by one CTA per 128 rows took 12.5 us.
+#include "common.cuh"
+#include "ft_internal.h"
+
+namespace ft {
+namespace {
+
+constexpr int PL_BM = 128, PL_BK = 64, PL_A = PL_BM * PL_BK * 2;      // weight rows per CTA, K chunk, bytes of a weight tile
+constexpr int PL_THREADS = 320;                                       // many tokens: TMA warp, MMA warp, eight epilogue warps
+constexpr int PL_MAX_STAGES = 8;
+
+// ------------------------------------------------------------------ many tokens
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PL_THREADS, 1)
+gemm_plain_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_hi,
+                       const __grid_constant__ CUtensorMap map_lo, float* __restrict__ out, int n_out, int T, int k_chunks, int stages, int bn) {
+    extern __shared__ uint8_t pl_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(pl_raw) + 1023) & ~uintptr_t(1023));
+    __shared__ uint64_t full[PL_MAX_STAGES], empty[PL_MAX_STAGES], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_slot;
+    const int plane = bn / 2 * PL_BK * 2;                 // bytes of this CTA's half of one plane's tile
+    const int stage_bytes = PL_A + 2 * plane;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)cluster_ctarank();
+    const int row_pairs = (n_out / PL_BM + 1) / 2;        // the last pair's second tile may lie beyond the matrix: zero rows, not stored
+    const int units = row_pairs * ((T + bn - 1) / bn);
+    const int cl = (int)cluster_id_x(), n_cl = (int)gridDim.x / 2;
+    if (warp == 0 && lane == 0) {
+        tma_prefetch_desc(&map_w);
+        tma_prefetch_desc(&map_hi);
+        tma_prefetch_desc(&map_lo);
+        for (int s = 0; s < stages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int a = 0; a < 2; ++a) {
+            mbar_init(&acc_full[a], 1);
+            mbar_init(&acc_empty[a], 2);                  // both CTAs' epilogues, on the leader's copy
+        }
+        fence_mbar_init();
+    }
+    if (warp == 1) {
+        tmem_alloc_pair(&tmem_slot, 512);
+        tmem_relinquish_pair();
+    }
+    tc_fence_before();
+    cluster_sync_all();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();
+    if (warp == 0) {
+        if (elect_one()) {
+            // weights are read again by every token tile; a launch of one token tile streams them
+            const bool multi = T > bn;
+            const uint64_t pol_w = multi ? policy_evict_last() : policy_evict_first(), pol_x = multi ? policy_evict_first() : policy_evict_last();
+            pdl_wait();
+            int it = 0;
+            for (int u = cl; u < units; u += n_cl) {
+                const int row0 = (2 * (u % row_pairs) + rank) * PL_BM, tok0 = u / row_pairs * bn + rank * (bn / 2);
+                for (int i = 0; i < k_chunks; ++i, ++it) {
+                    const int s = it % stages;
+                    if (it >= stages) mbar_wait(&empty[s], ((it / stages) - 1) & 1);
+                    if (rank == 0) mbar_expect_tx(&full[s], 2 * stage_bytes);
+                    uint8_t* st = smem + (size_t)s * stage_bytes;
+                    tma_tile_2d_pair(st, &map_w, i * PL_BK, row0, &full[s], pol_w);
+                    tma_tile_2d_pair(st + PL_A, &map_hi, i * PL_BK, tok0, &full[s], pol_x);
+                    tma_tile_2d_pair(st + PL_A + plane, &map_lo, i * PL_BK, tok0, &full[s], pol_x);
+                }
+            }
+        }
+    } else if (warp == 1 && rank == 0) {
+        if (elect_one()) {
+            const uint32_t idesc = umma_idesc_bf16(2 * PL_BM, bn);
+            int it = 0;
+            uint32_t use = 0;
+            for (int u = cl; u < units; u += n_cl, ++use) {
+                const uint32_t acc = use & 1;
+                if (use >= 2) {
+                    mbar_wait(&acc_empty[acc], ((use >> 1) - 1) & 1);
+                    tc_fence_after();
+                }
+                const uint32_t d = tmem + acc * 256;
+                for (int i = 0; i < k_chunks; ++i, ++it) {
+                    const int s = it % stages;
+                    mbar_wait(&full[s], (it / stages) & 1);
+                    tc_fence_after();
+                    const uint32_t base = smem_u32(smem + (size_t)s * stage_bytes);
+                    const uint64_t wd = umma_desc_k128(base), hd = umma_desc_k128(base + PL_A), ld = umma_desc_k128(base + PL_A + plane);
+#pragma unroll
+                    for (int k = 0; k < PL_BK / 16; ++k) umma_bf16_pair(d, wd + 2 * k, hd + 2 * k, idesc, (i | k) != 0);
+#pragma unroll
+                    for (int k = 0; k < PL_BK / 16; ++k) umma_bf16_pair(d, wd + 2 * k, ld + 2 * k, idesc, 1u);
+                    umma_commit_pair(&empty[s]);
+                }
+                umma_commit_pair(&acc_full[acc]);
+            }
+        }
+    } else if (warp >= 2) {
+        pdl_wait();
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        uint32_t use = 0;
+        for (int u = cl; u < units; u += n_cl, ++use) {
+            const uint32_t acc = use & 1;
+            const int row0 = (2 * (u % row_pairs) + rank) * PL_BM, tok0 = u / row_pairs * bn;
+            const int n_tok = min(bn, T - tok0);
+            mbar_wait(&acc_full[acc], (use >> 1) & 1);
+            tc_fence_after();
+            if (row0 < n_out) {
+                float* p = out + (size_t)tok0 * n_out + row0 + quarter * 32 + lane;
+                for (int c = 16 * half; c < n_tok; c += 32) {      // a row per lane: 128 consecutive bytes per warp and token
+                    float v[16];
+                    tmem_ld16(tmem + acc * 256 + ((uint32_t)(quarter * 32) << 16) + c, v);
+                    float* q = p + (size_t)c * n_out;
+                    if (c + 16 <= n_tok) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) q[(size_t)j * n_out] = v[j];
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (c + j < n_tok) q[(size_t)j * n_out] = v[j];
+                    }
+                }
+            }
+            tc_fence_before();
+            asm volatile("bar.sync 2, 256;" ::: "memory");      // all eight warps have read the accumulator
+            if (threadIdx.x == 64) mbar_arrive_leader(&acc_empty[acc]);
+        }
+    }
+    tc_fence_before();
+    cluster_sync_all();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem, 512);
+    }
+}
+
+// ------------------------------------------------------------------ few tokens
+constexpr int PF_THREADS = 192;                           // TMA warp, MMA warp, four epilogue warps
+
+__device__ __forceinline__ float peer_f32(uint32_t addr, int rank) {
+    uint32_t r;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(r) : "memory");
+    return v;
+}
+
+// grid (row tiles, S), clusters of (1, S): CTA (x, s) takes the s-th share of K of weight rows 128 x .. 128 x + 127.
+template <int BN>
+__global__ void __launch_bounds__(PF_THREADS)
+gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_hi,
+                      const __grid_constant__ CUtensorMap map_lo, float* __restrict__ out, int n_out, int T, int k_chunks, int stages) {
+    constexpr int PLANE = BN * PL_BK * 2, STAGE = PL_A + 2 * PLANE;
+    constexpr uint32_t COLS = BN < 32 ? 32 : BN;
+    extern __shared__ uint8_t pf_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(pf_raw) + 1023) & ~uintptr_t(1023));
+    __shared__ uint64_t full[PL_MAX_STAGES], empty[PL_MAX_STAGES], acc_full;
+    __shared__ uint32_t tmem_slot;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int S = (int)gridDim.y, rank = blockIdx.y, row0 = blockIdx.x * PL_BM;
+    const int kc0 = k_chunks * rank / S, n_iter = k_chunks * (rank + 1) / S - kc0;      // at least one chunk each
+    if (warp == 0 && lane == 0) {
+        tma_prefetch_desc(&map_w);
+        tma_prefetch_desc(&map_hi);
+        tma_prefetch_desc(&map_lo);
+        for (int s = 0; s < stages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(&acc_full, 1);
+        fence_mbar_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(&tmem_slot, COLS);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();
+    if (warp == 0) {
+        if (elect_one()) {
+            const uint64_t pol_w = policy_evict_first(), pol_x = policy_evict_last();
+            const int pre = min(n_iter, stages);
+            for (int i = 0; i < pre; ++i) {               // the weights do not depend on the kernel before
+                mbar_expect_tx(&full[i], STAGE);
+                tma_tile_2d(smem + (size_t)i * STAGE, &map_w, (kc0 + i) * PL_BK, row0, &full[i], pol_w);
+            }
+            pdl_wait();
+            for (int i = 0; i < n_iter; ++i) {
+                const int s = i % stages;
+                uint8_t* st = smem + (size_t)s * STAGE;
+                if (i >= pre) {
+                    mbar_wait(&empty[s], ((i / stages) - 1) & 1);
+                    mbar_expect_tx(&full[s], STAGE);
+                    tma_tile_2d(st, &map_w, (kc0 + i) * PL_BK, row0, &full[s], pol_w);
+                }
+                tma_tile_2d(st + PL_A, &map_hi, (kc0 + i) * PL_BK, 0, &full[s], pol_x);
+                tma_tile_2d(st + PL_A + PLANE, &map_lo, (kc0 + i) * PL_BK, 0, &full[s], pol_x);
+            }
+        }
+    } else if (warp == 1) {
+        if (elect_one()) {
+            constexpr uint32_t idesc = umma_idesc_bf16(PL_BM, BN);
+            for (int i = 0; i < n_iter; ++i) {
+                const int s = i % stages;
+                mbar_wait(&full[s], (i / stages) & 1);
+                tc_fence_after();
+                const uint32_t base = smem_u32(smem + (size_t)s * STAGE);
+                const uint64_t wd = umma_desc_k128(base), hd = umma_desc_k128(base + PL_A), ld = umma_desc_k128(base + PL_A + PLANE);
+#pragma unroll
+                for (int k = 0; k < PL_BK / 16; ++k) umma_bf16(tmem, wd + 2 * k, hd + 2 * k, idesc, (i | k) != 0);
+#pragma unroll
+                for (int k = 0; k < PL_BK / 16; ++k) umma_bf16(tmem, wd + 2 * k, ld + 2 * k, idesc, 1u);
+                umma_commit(&empty[s]);
+            }
+            umma_commit(&acc_full);
+        }
+    } else {
+        pdl_wait();                                       // out may still be read by the kernel before
+        mbar_wait(&acc_full, 0);
+        tc_fence_after();
+        const int quarter = warp & 3, f = quarter * 32 + lane;
+        float* tile = reinterpret_cast<float*>(smem);     // [BN][128]: the stages are idle once the products have retired
+#pragma unroll 1
+        for (int c = 0; c < BN && c < T; c += 16) {
+            float v[16];
+            tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + c, v);
+            if (S == 1) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (c + j < T) out[(size_t)(c + j) * n_out + row0 + f] = v[j];
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) tile[(c + j) * PL_BM + f] = v[j];
+            }
+        }
+    }
+    tc_fence_before();
+    if (S > 1) {
+        cluster_sync_all();                               // every share of the row tile lies in its CTA's shared memory
+        if (warp >= 2) {
+            const int f = threadIdx.x - 64;
+            const uint32_t at = smem_u32(smem) + (uint32_t)f * 4;
+            for (int t = rank; t < T; t += S) {
+                float v[8];
+#pragma unroll
+                for (int p = 0; p < 8; ++p) v[p] = p < S ? peer_f32(at + (uint32_t)t * (PL_BM * 4), p) : 0.f;
+                float sum = v[0];
+#pragma unroll
+                for (int p = 1; p < 8; ++p) sum += v[p];
+                out[(size_t)t * n_out + row0 + f] = sum;
+            }
+        }
+        cluster_sync_all();                               // nobody leaves while its tile is being read
+    } else {
+        __syncthreads();
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, COLS);
+    }
+}
+
+int sm_count() {
+    static int sms[kMaxDevices] = {};
+    int& n = sms[current_device_slot()];
+    if (!n) {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
+        n = v;
+    }
+    return n;
+}
+
+constexpr int PL_RING = 222 * 1024;                       // shared memory for the stages (+ 1 KB to align them)
+
+void fill(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, dim3 grid, int threads, size_t smem, bool pdl, cudaStream_t stream) {
+    cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+}
+
+template <int BN>
+int launch_few(const CUtensorMap& mw, const CUtensorMap& mh, const CUtensorMap& ml, float* out, int n_out, int T, int K, bool pdl, cudaStream_t stream) {
+    constexpr int STAGE = PL_A + 2 * BN * PL_BK * 2;
+    const int kc = K / PL_BK, tiles = n_out / PL_BM;
+    // CTAs per row tile: as many as leave each three chunks and the grid at most two CTAs per SM
+    int S = 8;
+    while (S > 1 && (kc / S < 3 || tiles * S > 2 * sm_count())) S /= 2;
+    // a deep ring where a CTA has an SM for itself, half of one otherwise
+    const int budget = tiles * S <= sm_count() ? 200 * 1024 : 104 * 1024;
+    int stages = budget / STAGE;
+    if (stages > PL_MAX_STAGES) stages = PL_MAX_STAGES;
+    if (stages > (kc + S - 1) / S) stages = (kc + S - 1) / S;
+    if (stages < 1) stages = 1;
+    size_t smem = (size_t)stages * STAGE;
+    if (smem < (size_t)BN * PL_BM * 4) smem = (size_t)BN * PL_BM * 4;      // the partial tile
+    smem += 1024;
+    static PerDeviceFlag attr_set;
+    if (!attr_set.done()) {
+        FT_CHECK_CUDA(cudaFuncSetAttribute(gemm_plain_few_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 201 * 1024));
+        FT_CHECK_CUDA(cudaFuncSetAttribute(gemm_plain_few_kernel<BN>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        attr_set.mark();
+    }
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    fill(cfg, attr, dim3(tiles, S), PF_THREADS, smem, pdl, stream);
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = 1; attr[cfg.numAttrs].val.clusterDim.y = S; attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+    FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_plain_few_kernel<BN>, mw, mh, ml, out, n_out, T, kc, stages));
+    return 0;
+}
+
+// Pairs that can be resident at once.
+int plain_clusters() {
+    static int n_dev[kMaxDevices] = {};
+    int& n = n_dev[current_device_slot()];
+    if (!n) {
+        FT_CHECK_CUDA(cudaFuncSetAttribute(gemm_plain_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PL_RING + 1024));
+        cudaLaunchConfig_t q = {};
+        q.gridDim = dim3(sm_count() & ~1);
+        q.blockDim = dim3(PL_THREADS);
+        q.dynamicSmemBytes = PL_RING + 1024;
+        cudaLaunchAttribute qa[1];
+        qa[0].id = cudaLaunchAttributeClusterDimension;
+        qa[0].val.clusterDim.x = 2; qa[0].val.clusterDim.y = 1; qa[0].val.clusterDim.z = 1;
+        q.attrs = qa;
+        q.numAttrs = 1;
+        int v = 0;
+        if (cudaOccupancyMaxActiveClusters(&v, gemm_plain_pair_kernel, &q) != cudaSuccess || v <= 0) v = sm_count() / 2;
+        n = v;
+    }
+    return n;
+}
+
+// Tokens per tile.  A unit takes about as long as it is wide, but not less than 96 tokens' time (below that the products wait for the
+// weight tile in shared memory) and a fixed part for its first loads; the last round's results leave after its products.  Multiples of
+// 32: the widths a 256-row product has, and half of one, a CTA's share, is then whole 8-row swizzle groups.
+int plain_token_tile(int row_pairs, int T, int clusters) {
+    int best = 128;
+    double least = 1e30;
+    for (int bn = 32; bn <= 256; bn += 32) {
+        const long long units = (long long)row_pairs * ((T + bn - 1) / bn), rounds = (units + clusters - 1) / clusters;
+        const double t = (double)rounds * ((bn > 96 ? bn : 96) + 12) + 0.5 * bn;
+        if (t < least) { least = t; best = bn; }
+    }
+    return best;
+}
+
+}  // namespace
+
+bool gemm_plain_ok(int n_out, int T, int K) { return n_out >= PL_BM && n_out % PL_BM == 0 && K >= PL_BK && K % PL_BK == 0 && T >= 1; }
+
+int launch_gemm_plain(const void* w, const void* hi, const void* lo, float* out, int n_out, int T, int K, bool pdl, cudaStream_t stream) {
+    FT_REQUIRE(w && hi && lo && out && gemm_plain_ok(n_out, T, K), "gemm (plain): bad sizes or operands (n_out %d, T %d, K %d)", n_out, T, K);
+    CUtensorMap mw, mh, ml;
+    if (int r = make_tmap_bf16_k64(&mw, w, n_out, K, PL_BM)) return r;
+    if (T <= 128) {
+        const int bn = gemm_pick_bn(T, true);
+        if (int r = make_tmap_bf16_k64(&mh, hi, T, K, bn)) return r;
+        if (int r = make_tmap_bf16_k64(&ml, lo, T, K, bn)) return r;
+        switch (bn) {
+            case 16: return launch_few<16>(mw, mh, ml, out, n_out, T, K, pdl, stream);
+            case 32: return launch_few<32>(mw, mh, ml, out, n_out, T, K, pdl, stream);
+            case 64: return launch_few<64>(mw, mh, ml, out, n_out, T, K, pdl, stream);
+            default: return launch_few<128>(mw, mh, ml, out, n_out, T, K, pdl, stream);
+        }
+    }
+    const int clusters = plain_clusters();
+    if (clusters <= 0) return clusters;
+    const int row_pairs = (n_out / PL_BM + 1) / 2, bn = plain_token_tile(row_pairs, T, clusters);
+    if (int r = make_tmap_bf16_k64(&mh, hi, T, K, bn / 2)) return r;
+    if (int r = make_tmap_bf16_k64(&ml, lo, T, K, bn / 2)) return r;
+    const int units = row_pairs * ((T + bn - 1) / bn), stage = PL_A + bn * PL_BK * 2;
+    int stages = PL_RING / stage;
+    if (stages > PL_MAX_STAGES) stages = PL_MAX_STAGES;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    fill(cfg, attr, dim3(2 * (units < clusters ? units : clusters)), PL_THREADS, (size_t)stages * stage + 1024, pdl, stream);
+    FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_plain_pair_kernel, mw, mh, ml, out, n_out, T, K / PL_BK, stages, bn));
+    return 0;
+}
+
+}  // namespace ft

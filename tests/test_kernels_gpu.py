@@ -564,6 +564,25 @@ def test_sample_full_vocab_row(K):
         assert ref[tok[b].item()] > 0
 
 
+@pytest.mark.parametrize("T", [1, 16, 17, 33, 128, 129, 161, 600, 2313])
+@pytest.mark.parametrize("n_out,Kd", [(128, 64), (384, 192), (2048, 2048), (4352, 1024), (640, 8192)])
+def test_gemm_plain_fp32(K, T, n_out, Kd):
+    """Unsplit fp32 results of both planes: K shared by a cluster (up to 128 tokens) and CTA pairs with token tiles of every width,
+    odd row tile counts, ragged last tiles.  Both planes are exact inputs of the reference; what is left is the rounding of fp32
+    sums of Kd products in another order, at most Kd * 2^-24 of the sum of magnitudes and in practice its square root."""
+    g = torch.Generator(device=DEV).manual_seed(T * 7 + n_out)
+    w = (torch.randn(n_out, Kd, device=DEV, generator=g) * 0.05).bfloat16()
+    x, x_lo = K.split_hi_lo(torch.randn(T, Kd, device=DEV, generator=g))
+    guard = torch.full((T + 1, n_out), 7.0, device=DEV)
+    from fasttalk_llm_microservice_b200 import native as N
+    N.check(N.load().ft_gemm_bf16(N.ptr(w), N.ptr(x), N.ptr(x_lo), N.ptr(guard), 0, n_out, T, Kd, 1, 0, N.cur_stream()), "ft_gemm_bf16")
+    xs = x.double() + x_lo.double()
+    ref = xs @ w.double().T
+    bound = (xs.abs() @ w.double().abs().T) * (4.0 * Kd ** 0.5 * 2.0 ** -24)
+    assert bool(((guard[:T].double() - ref).abs() <= bound + 1e-30).all())
+    assert bool((guard[T] == 7.0).all())
+
+
 def _draw_point(seed):
     """The 24-bit point of [0, 1) that a row's seed stands for (splitmix64)."""
     m = (1 << 64) - 1
