@@ -6,10 +6,11 @@
 //                 does, with a token tile whose width is a run-time value.  A projection of 2313 tokens and 2048 rows is 152 units of
 //                 128 tokens for 74 pairs: three rounds, the last one nearly empty; 160 tokens wide it is 120 units in two.  The
 //                 width that the launcher takes is the one with the least time over all rounds (plain_token_tile).
-//                 Measured (2313 tokens, hi + lo): 2048 x 2048 45 -> 31 us, 2048 -> 10752 182 -> 150 us against one CTA per tile.
+//                 Measured (2313 tokens, hi + lo, one CTA per tile before): 2048 -> 2048 45 -> 40 us, 2048 -> 10752 182 -> 143 us.
 //   few tokens    one token tile; K is shared by the up to eight CTAs of a cluster, which add their partial tiles through distributed
 //                 shared memory in rank order: no slabs, no arrival words, no second launch.  Bound by latency (launch, first load,
-//                 one pass over at most 32 chunks): 16 tokens, 2048 x 2048 by one CTA per 128 rows took 12.5 us.
+//                 one pass over a few chunks), and per chunk by the tensor core's reads of the weight tile, which both planes share
+//                 (16 tokens, 2048 x 2048: one CTA per 128 rows 13.1 us, K shared by eight 6.6, one product for both planes 5.9).
 #include "common.cuh"
 #include "ft_internal.h"
 
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(PF_THREADS)
 gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_hi,
                       const __grid_constant__ CUtensorMap map_lo, float* __restrict__ out, int n_out, int T, int k_chunks, int stages) {
     constexpr int PLANE = BN * PL_BK * 2, STAGE = PL_A + 2 * PLANE;
-    constexpr uint32_t COLS = BN < 32 ? 32 : BN;
+    constexpr uint32_t COLS = 2 * BN;                     // the hi plane's products, then the lo plane's
     extern __shared__ uint8_t pf_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(pf_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint64_t full[PL_MAX_STAGES], empty[PL_MAX_STAGES], acc_full;
@@ -212,17 +213,16 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         }
     } else if (warp == 1) {
         if (elect_one()) {
-            constexpr uint32_t idesc = umma_idesc_bf16(PL_BM, BN);
+            // the two planes' tiles lie one after the other: ONE operand of 2 BN rows, so the weight tile is read once for both
+            constexpr uint32_t idesc = umma_idesc_bf16(PL_BM, 2 * BN);
             for (int i = 0; i < n_iter; ++i) {
                 const int s = i % stages;
                 mbar_wait(&full[s], (i / stages) & 1);
                 tc_fence_after();
                 const uint32_t base = smem_u32(smem + (size_t)s * STAGE);
-                const uint64_t wd = umma_desc_k128(base), hd = umma_desc_k128(base + PL_A), ld = umma_desc_k128(base + PL_A + PLANE);
+                const uint64_t wd = umma_desc_k128(base), xd = umma_desc_k128(base + PL_A);
 #pragma unroll
-                for (int k = 0; k < PL_BK / 16; ++k) umma_bf16(tmem, wd + 2 * k, hd + 2 * k, idesc, (i | k) != 0);
-#pragma unroll
-                for (int k = 0; k < PL_BK / 16; ++k) umma_bf16(tmem, wd + 2 * k, ld + 2 * k, idesc, 1u);
+                for (int k = 0; k < PL_BK / 16; ++k) umma_bf16(tmem, wd + 2 * k, xd + 2 * k, idesc, (i | k) != 0);
                 umma_commit(&empty[s]);
             }
             umma_commit(&acc_full);
@@ -235,8 +235,11 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         float* tile = reinterpret_cast<float*>(smem);     // [BN][128]: the stages are idle once the products have retired
 #pragma unroll 1
         for (int c = 0; c < BN && c < T; c += 16) {
-            float v[16];
+            float v[16], low[16];
             tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + c, v);
+            tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + BN + c, low);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] += low[j];
             if (S == 1) {
 #pragma unroll
                 for (int j = 0; j < 16; ++j)
@@ -302,11 +305,14 @@ template <int BN>
 int launch_few(const CUtensorMap& mw, const CUtensorMap& mh, const CUtensorMap& ml, float* out, int n_out, int T, int K, bool pdl, cudaStream_t stream) {
     constexpr int STAGE = PL_A + 2 * BN * PL_BK * 2;
     const int kc = K / PL_BK, tiles = n_out / PL_BM;
-    // CTAs per row tile: as many as leave each three chunks and the grid at most two CTAs per SM
+    // CTAs per row tile: as many as leave each three chunks and the grid one CTA per SM, two from four CTAs per tile on (weights of
+    // 10752 x 2048 and 64 tokens: 12.8 us with S = 1, 16.1 with 2; 8576 x 2048 and 16 tokens: 8.5 us with S = 2, 7.9 with 4)
     int S = 8;
-    while (S > 1 && (kc / S < 3 || tiles * S > 2 * sm_count())) S /= 2;
-    // a deep ring where a CTA has an SM for itself, half of one otherwise
-    const int budget = tiles * S <= sm_count() ? 200 * 1024 : 104 * 1024;
+    while (S > 1 && (kc / S < 3 || tiles * S > (S >= 4 ? 2 : 1) * sm_count())) S /= 2;
+    // A deep ring where a CTA has an SM for itself, half of one otherwise.  Clusters of four or eight always leave room for a second CTA:
+    // they must lie within one GPC, and with one CTA per SM sixteen clusters of eight do not all find one (2048 x 4096, 16 tokens:
+    // 12.9 us with 160 KB per CTA, more than with half the CTAs).
+    const int budget = tiles * S <= sm_count() && S <= 2 ? 200 * 1024 : 104 * 1024;
     int stages = budget / STAGE;
     if (stages > PL_MAX_STAGES) stages = PL_MAX_STAGES;
     if (stages > (kc + S - 1) / S) stages = (kc + S - 1) / S;
@@ -352,15 +358,16 @@ int plain_clusters() {
     return n;
 }
 
-// Tokens per tile.  A unit takes about as long as it is wide, but not less than 96 tokens' time (below that the products wait for the
-// weight tile in shared memory) and a fixed part for its first loads; the last round's results leave after its products.  Multiples of
-// 32: the widths a 256-row product has, and half of one, a CTA's share, is then whole 8-row swizzle groups.
+// Tokens per tile.  A round of units takes as long as its tile is wide, but not less than the weight tiles need to come out of L2
+// (92 + bn / 3 tokens' time), and the last round's results leave after its products.  The constants are fitted to 2313 tokens of
+// 2048 columns (us per round of K = 2048): 10.0 / 11.5 / 12.5 / 12.9 / 16.2 / 19.9 / 24.8 for 32 / 64 / 96 / 128 / 160 / 192 / 256 tokens.
+// Multiples of 32: the widths a 256-row product has, and half of one, a CTA's share, is then whole 8-row swizzle groups.
 int plain_token_tile(int row_pairs, int T, int clusters) {
     int best = 128;
     double least = 1e30;
     for (int bn = 32; bn <= 256; bn += 32) {
         const long long units = (long long)row_pairs * ((T + bn - 1) / bn), rounds = (units + clusters - 1) / clusters;
-        const double t = (double)rounds * ((bn > 96 ? bn : 96) + 12) + 0.5 * bn;
+        const double round = bn > 92 + bn / 3.0 ? bn : 92 + bn / 3.0, t = rounds * round + 0.25 * bn;
         if (t < least) { least = t; best = bn; }
     }
     return best;
