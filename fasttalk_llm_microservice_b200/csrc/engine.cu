@@ -193,7 +193,7 @@ struct Layered {
     size_t slot_stride = 0;            // floats per state slot
     int n_stateful = 0;                // layers whose mixer carries state from token to token
     int ld_proj = 0, top_max = 0, scan_ws_rows = 0;
-    float *hn = nullptr, *proj = nullptr, *b1 = nullptr, *b2 = nullptr, *b3 = nullptr, *b4 = nullptr, *beta = nullptr, *scan_ws = nullptr,
+    float *hn = nullptr, *proj = nullptr, *b1 = nullptr, *b2 = nullptr, *b3 = nullptr, *b4 = nullptr, *beta = nullptr, *kq = nullptr, *scan_ws = nullptr,
           *attn_part = nullptr, *mix = nullptr, *act = nullptr, *eout = nullptr, *wts = nullptr, *xlast = nullptr;
     // branch mixers and sandwich layers: queries, prepared values, rule outputs, read-out, (decay, input) pairs, log gates,
     // denominator floors, the second branch's projection, feed-forward halves, router logits
@@ -1091,7 +1091,7 @@ static int forward_layered(Engine* e, const Batch& b) {
             }
             da.proj = L.proj; da.ldp = ld; da.o_q = c.o_q; da.o_beta = c.o_beta;
             da.conv = c.conv_w; da.dt_bias = c.dt_bias; da.a_log = c.a_log;
-            da.qkv = L.b3; da.decay = L.b1; da.beta = L.beta; da.o = L.b4;
+            da.qkv = L.b3; da.decay = L.b1; da.beta = L.beta; da.kq = L.kq; da.o = L.b4;
             da.state = L.state; da.slot_stride = (long long)L.slot_stride; da.s_off = (long long)ll.s_off;
             da.tail_off = (long long)ll.tail_off;
             da.seq_rows = d + m.o_rows; da.req_start = d + m.o_xstart; da.req_pos0 = d + m.o_xpos0;
@@ -2102,7 +2102,8 @@ static int engine_init_layered(Engine* e) {
     }
     FT_TRY(alloc(&L.b3, T * buf * 4));
     FT_TRY(alloc(&L.b4, T * buf * 4));
-    FT_TRY(alloc(&L.beta, T * heads_max * 4));
+    FT_TRY(alloc(&L.beta, 2 * T * heads_max * 4));      // betas, then the delta rule's products of keys and queries
+    L.kq = L.beta + T * heads_max;
     part_cols = std::max(part_cols, rank_max);
     if (part_cols > 0) FT_TRY(alloc(&L.attn_part, (size_t)kAttnSplitPairs * kAttnMaxSplits * (part_cols + 2) * 4));
     FT_TRY(alloc(&L.mix, T * W * 4));

@@ -219,8 +219,9 @@ struct DeltaArgs {
     const float* dt_bias = nullptr;   // [heads*dim]
     const float* a_log = nullptr;     // [heads]
     float* qkv = nullptr;             // out [T][channels]
-    float* decay = nullptr;           // out [T][heads*dim] (may alias araw)
+    float* decay = nullptr;           // out [T][heads*dim] (may alias araw), or [T][heads] with head_decay
     float* beta = nullptr;            // out [T][heads]
+    float* kq = nullptr;              // out [T][kvh]: products of the normed keys and queries
     float* o = nullptr;               // out [T][heads*vdim]
     float* state = nullptr;           // slots of slot_stride floats; this layer's S at s_off, its tails at tail_off
     long long slot_stride = 0, s_off = 0, tail_off = 0;
@@ -229,7 +230,7 @@ struct DeltaArgs {
     const int* req_pos0 = nullptr;    // [n_req] position of that row in its sequence
     const int* req_slot = nullptr;    // [n_req] state slot
     int heads = 0, kvh = 0, dim = 0, vdim = 0, taps = 0;
-    int head_decay = 0;               // 1: araw holds one value per head (row stride ld_araw), dt_bias is [heads]
+    int head_decay = 0;               // 1: araw holds one value per head (row stride ld_araw), dt_bias is [heads], one decay per head
     int ld_araw = 0;
 };
 // prep (convolutions, norms, decays) -> tails -> recurrence -> output norm and gate (in place in a.o)

@@ -45,6 +45,9 @@ __device__ __forceinline__ float block_sum(float v, float* red) {      // red: >
 __device__ __forceinline__ void cp_async4(float* dst_smem, const float* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async16(float* dst_smem, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
@@ -702,54 +705,138 @@ int launch_latent_attn(const LatentArgs& a, int T, cudaStream_t stream) {
 
 // ------------------------------------------------------------------ channel delta
 // Per token: the three short convolutions over time + SiLU (inputs before the step's first token come from the session's
-// tail of raw inputs; zeros before position 0), unit norms of q and k per head (q also times dim^-1/2), the decay
-// exp(-exp(A_log_h) * softplus(a + dt_bias)) per head and key channel, beta = sigmoid.
+// tail of raw inputs; zeros before position 0), unit norms of q and k per head (q also times dim^-1/2), the product k q of a head's
+// normed rows, the decay exp(-exp(A_log_h) * softplus(a + dt_bias)) per head and key channel (or per head), beta = sigmoid.
 // qkv out: [T][channels] with channels = 2 * kvh * dim + heads * vdim in the order q | k | v.
-__global__ void __launch_bounds__(256)
-delta_prep_kernel(DeltaArgs a) {
-    extern __shared__ float sh[];
-    const int t = blockIdx.x;
-    const int req = a.seq_rows[t];
-    const int r = t - a.req_start[req];              // index inside this step's portion
-    const int pos0 = a.req_pos0[req];
-    const int qk = a.kvh * a.dim, ch = 2 * qk + a.heads * a.vdim;
-    const float* tail = a.state + (size_t)a.req_slot[req] * a.slot_stride + a.tail_off;
-    const int taps = a.taps;
-    for (int c = threadIdx.x; c < ch; c += blockDim.x) {
-        float s = 0.f;
-        for (int i = 0; i < taps; ++i) {
-            const int back = taps - 1 - i;
-            float v;
-            if (r - back >= 0) v = a.proj[(size_t)(t - back) * a.ldp + a.o_q + c];
-            else if (pos0 + r - back >= 0) v = tail[(size_t)c * (taps - 1) + (taps - 1 + r - back)];
-            else v = 0.f;
-            s = fmaf(a.conv[(size_t)c * taps + i], v, s);
+// CTA (tokens x .. + TB - 1, group y): group y < kvh is a q and a k head, then come 128 value channels each, then decays and betas.  A thread keeps its channels over the TB tokens, so that the rows the taps share come out of L1 (one CTA per
+// token, all channels after one another: 121 us for 2313 tokens of 6144 channels).
+template <int TB>
+__global__ void __launch_bounds__(128)
+delta_prep_kernel(DeltaArgs a, int T) {
+    __shared__ float red[3][TB][4];
+    const int t0 = blockIdx.x * TB, nt = min(TB, T - t0), g = blockIdx.y;
+    const int qk = a.kvh * a.dim, ch = 2 * qk + a.heads * a.vdim, hd = a.heads * a.dim;
+    const int v_groups = (a.heads * a.vdim + 127) / 128, taps = a.taps;
+    if (g >= a.kvh + v_groups) {
+        // decays: one per head (one group for all of them), or per head and key channel (a group per head); the first group also betas
+        const int dg = g - a.kvh - v_groups, per = a.head_decay ? a.heads : a.dim;
+        for (int i = threadIdx.x; i < nt * per; i += 128) {
+            const int t = t0 + i / per, c = dg * per + i % per, h = a.head_decay ? c : dg;
+            const float z = (a.head_decay ? a.araw[(size_t)t * a.ld_araw + c] : a.araw[(size_t)t * hd + c]) + a.dt_bias[c];
+            const float sp = z > 20.f ? z : log1pf(expf(z));
+            a.decay[(size_t)t * (a.head_decay ? a.heads : hd) + c] = expf(-expf(a.a_log[h]) * sp);
         }
-        sh[c] = s / (1.f + expf(-s));
+        for (int i = threadIdx.x; dg == 0 && i < nt * a.heads; i += 128)
+            a.beta[(size_t)(t0 + i / a.heads) * a.heads + i % a.heads] = sigmoid_exact(a.proj[(size_t)(t0 + i / a.heads) * a.ldp + a.o_beta + i % a.heads]);
+        return;
+    }
+    auto conv = [&](int t, int c) {
+        const int req = a.seq_rows[t], r = t - a.req_start[req], pos0 = a.req_pos0[req];
+        const float* tail = a.state + (size_t)a.req_slot[req] * a.slot_stride + a.tail_off;
+        const float* w = a.conv + (size_t)c * taps;
+        const float* row = a.proj + (size_t)t * a.ldp + a.o_q + c;
+        float s = 0.f;
+        if (r >= taps - 1) {                          // every input is a row of this step: four reads in flight at a time
+            int i = 0;
+            for (; i + 4 <= taps; i += 4) {
+                float v[4];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) v[x] = row[(long long)(i + x - (taps - 1)) * a.ldp];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) s = fmaf(w[i + x], v[x], s);
+            }
+            for (; i < taps; ++i) s = fmaf(w[i], row[(long long)(i - (taps - 1)) * a.ldp], s);
+        } else {
+            for (int i = 0; i < taps; ++i) {
+                const int back = taps - 1 - i;
+                float v;
+                if (r - back >= 0) v = row[-(long long)back * a.ldp];
+                else if (pos0 + r - back >= 0) v = tail[(size_t)c * (taps - 1) + (taps - 1 + r - back)];
+                else v = 0.f;
+                s = fmaf(w[i], v, s);
+            }
+        }
+        return s / (1.f + expf(-s));
+    };
+    // The block's tokens of one channel.  Up to four taps whose inputs are all rows of this step and of one request: each row is read once.
+    bool inside = nt == TB && taps <= 4;
+    if (inside) {
+        const int req = a.seq_rows[t0];
+        inside = a.seq_rows[t0 + TB - 1] == req && t0 - a.req_start[req] >= 3;
+    }
+    auto block = [&](int c, float* y) {
+        if (inside) {
+            float w[4], v[TB + 3];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) w[x] = x >= 4 - taps ? a.conv[(size_t)c * taps + x - (4 - taps)] : 0.f;
+            const float* row = a.proj + (size_t)(t0 - 3) * a.ldp + a.o_q + c;
+#pragma unroll
+            for (int x = 0; x < TB + 3; ++x) v[x] = row[(size_t)x * (unsigned)a.ldp];
+#pragma unroll
+            for (int i = 0; i < TB; ++i) {
+                float s = 0.f;
+#pragma unroll
+                for (int x = 0; x < 4; ++x) s = fmaf(w[x], v[i + x], s);
+                y[i] = s / (1.f + expf(-s));
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < TB; ++i) y[i] = i < nt ? conv(t0 + i, c) : 0.f;
+        }
+    };
+    if (g >= a.kvh) {
+        const int c = 2 * qk + (g - a.kvh) * 128 + threadIdx.x;
+        if (c >= ch) return;
+        float y[TB];
+        block(c, y);
+#pragma unroll
+        for (int i = 0; i < TB; ++i)
+            if (i < nt) a.qkv[(size_t)(t0 + i) * ch + c] = y[i];
+        return;
+    }
+    float q[2][TB], k[2][TB];                        // head sizes up to 256: two channels per thread
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        const int d = threadIdx.x + 128 * x;
+        if (d < a.dim) {
+            block(g * a.dim + d, q[x]);
+            block(qk + g * a.dim + d, k[x]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < TB; ++i) q[x][i] = k[x][i] = 0.f;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < TB; ++i) {
+        float s[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            s[0] = fmaf(q[x][i], q[x][i], s[0]);
+            s[1] = fmaf(k[x][i], k[x][i], s[1]);
+            s[2] = fmaf(q[x][i], k[x][i], s[2]);
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            s[j] = warp_sum(s[j]);
+            if ((threadIdx.x & 31) == 0) red[j][i][threadIdx.x >> 5] = s[j];
+        }
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    float* dst = a.qkv + (size_t)t * ch;
-    for (int hh = wid; hh < 2 * a.kvh; hh += nw) {          // q heads, then k heads
-        const float* v = sh + (size_t)hh * a.dim;
-        float ss = 0.f;
-        for (int d = lane; d < a.dim; d += 32) ss += v[d] * v[d];
-        ss = warp_sum(ss);
-        float sc = 1.f / sqrtf(ss + 1e-6f);
-        if (hh < a.kvh) sc *= 1.f / sqrtf((float)a.dim);
-        for (int d = lane; d < a.dim; d += 32) dst[(size_t)hh * a.dim + d] = v[d] * sc;
-    }
-    for (int c = 2 * qk + threadIdx.x; c < ch; c += blockDim.x) dst[c] = sh[c];
-    const int hd = a.heads * a.dim;
-    for (int i = threadIdx.x; i < hd; i += blockDim.x) {
-        // one decay per head and key channel, or (head_decay) one per head, written to all of the head's channels
-        const float z = a.head_decay ? a.araw[(size_t)t * a.ld_araw + i / a.dim] + a.dt_bias[i / a.dim]
-                                     : a.araw[(size_t)t * hd + i] + a.dt_bias[i];
-        const float sp = z > 20.f ? z : log1pf(expf(z));
-        a.decay[(size_t)t * hd + i] = expf(-expf(a.a_log[i / a.dim]) * sp);
-    }
-    for (int h = threadIdx.x; h < a.heads; h += blockDim.x)
-        a.beta[(size_t)t * a.heads + h] = sigmoid_exact(a.proj[(size_t)t * a.ldp + a.o_beta + h]);
+#pragma unroll
+    for (int i = 0; i < TB; ++i)
+        if (i < nt) {
+            float s[3];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) s[j] = (red[j][i][0] + red[j][i][1]) + (red[j][i][2] + red[j][i][3]);
+            const float sq = 1.f / sqrtf(s[0] + 1e-6f) * (1.f / sqrtf((float)a.dim)), sk = 1.f / sqrtf(s[1] + 1e-6f);
+            float* dst = a.qkv + (size_t)(t0 + i) * ch + (size_t)g * a.dim;
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int d = threadIdx.x + 128 * x;
+                if (d < a.dim) { dst[d] = q[x][i] * sq; dst[qk + d] = k[x][i] * sk; }
+            }
+            if (threadIdx.x == 0) a.kq[(size_t)(t0 + i) * a.kvh + g] = s[2] * sq * sk;
+        }
 }
 
 // New tail of raw convolution inputs per (request, channel): the last taps-1 entries of (old tail ++ this step's inputs).
@@ -769,60 +856,159 @@ __global__ void delta_tail_kernel(DeltaArgs a, int n_req) {
     for (int i = 0; i < keep; ++i) tail[i] = v[i];
 }
 
-// The recurrence, one CTA per (request, head, block of DCOLS state columns).  Per token
+// The recurrence, one CTA per (request, head, block of state columns).  Per token
 //   S <- diag(g) S;  u = beta (v - S^T k);  S <- S + k u^T;  o = S^T q
-// is local to a column of the state S [dim][vdim].  Four neighbouring lanes share a column, each holding a run of DPT key
-// channels of it in registers, so the two sums over key channels are two short chains plus two shuffles.
-// q, k, g, v, beta of DCHUNK tokens at a time are copied into shared memory asynchronously (cp.async), one chunk ahead
-// of the one being computed.
-constexpr int DCHUNK = 8, DCOLS = 32;
+// is local to a column of the state S [dim][vdim].  Sixteen neighbouring lanes share two columns, lane s holding channels
+// 64 i + 4 s .. + 3 of them, two to a packed multiply-add.  The read-out of the new state is formed from the old one,
+//   o = S^T q + u (k q)     (S after its decay, k q from the preparation),
+// so that both sums over key channels are taken in one pass and only one of them, S^T k, lies on the chain from token to token:
+// a few multiply-adds, four shuffles, u, the update.  q, k, g, v of DCHUNK tokens at a time are copied into shared memory one
+// chunk ahead; channels beyond dim are zeros.
+// Bound by that chain (one or two warps per scheduler).  Four lanes per column with one column per thread, unpacked, both sums one
+// after the other: 515 us for three requests of 771 tokens, 16 heads of 128 x 128.
+constexpr int DCHUNK = 16, DLANES = 16, DCPT = 2;
 
-// Shared-memory layout of one staged token: q, k, g each as four runs of DPT channels (one per lane of a column's quad)
-// with four floats of padding between runs, so that the quad's 16-byte reads fall into different banks; then v, then beta.
-template <int DPT>
-__host__ __device__ constexpr int delta_run() { return DPT + 4; }
-__host__ __device__ inline int delta_token_floats(int dpt, int vdim) { return (12 * (dpt + 4) + vdim + 1 + 3) & ~3; }
-
-// FULL: dim == 4 * DPT, every channel test is true at compile time (the tests otherwise compile to branches in the token loop).
-template <int DPT, int MAXT, bool FULL>
-__global__ void __launch_bounds__(MAXT)
+// DPT: channels per lane (dim <= 16 DPT).  HD: one decay per head instead of one per key channel.  VEC: rows are copied 16 bytes at a time.
+template <int DPT, bool HD, bool VEC>
+__global__ void __launch_bounds__(128)
 delta_rule_kernel(DeltaArgs a) {
     extern __shared__ __align__(16) float sh[];
-    constexpr int RUN = delta_run<DPT>();
+    constexpr int DP = DLANES * DPT;
+    const int cols = blockDim.x / DLANES * DCPT, per = (HD ? 2 : 3) * DP + cols + 4;      // floats of a staged token: q | k | (g) | v | beta, kq, (g)
     const int req = blockIdx.x, h = blockIdx.y;
-    const int j = blockIdx.z * DCOLS + (threadIdx.x >> 2), part = threadIdx.x & 3;      // column, and which run of key channels
+    const int s = threadIdx.x % DLANES, jl = threadIdx.x / DLANES * DCPT, j0 = blockIdx.z * cols, j = j0 + jl;      // this thread's first column
     const int kh = h / (a.heads / a.kvh);
     const int row0 = a.req_start[req], n = a.req_start[req + 1] - row0;
+    if (n <= 0) return;
     const int dim = a.dim, vdim = a.vdim;
     const int qk = a.kvh * dim, ch = 2 * qk + a.heads * vdim, hd = a.heads * dim;
     float* S = a.state + (size_t)a.req_slot[req] * a.slot_stride + a.s_off + (size_t)h * dim * vdim;
-    const bool live = j < vdim;
     const bool fresh = a.req_pos0[req] == 0;
-    const int d0 = part * DPT;                    // this lane's channels: d0 .. d0 + DPT - 1
-    float s[DPT];
+    auto channel = [&](int i) { return (i >> 2) * (4 * DLANES) + 4 * s + (i & 3); };
+    f32x2 st[DCPT][DPT / 2];
 #pragma unroll
-    for (int i = 0; i < DPT; ++i) s[i] = (live && !fresh && d0 + i < dim) ? S[(size_t)(d0 + i) * vdim + j] : 0.f;
-    const int per = delta_token_floats(DPT, vdim);
-    const int o_k = 4 * RUN, o_g = 8 * RUN, o_v = 12 * RUN;
+    for (int c = 0; c < DCPT; ++c)
+#pragma unroll
+        for (int i = 0; i < DPT; i += 2) {
+            const bool in = !fresh && j + c < vdim;
+            const int d = channel(i);
+            st[c][i / 2] = pack2(in && d < dim ? S[(size_t)d * vdim + j + c] : 0.f, in && d + 1 < dim ? S[(size_t)(d + 1) * vdim + j + c] : 0.f);
+        }
+    if (DP != dim || j0 + cols > vdim)                 // the padding stays zero from here on
+        for (int i = threadIdx.x; i < 2 * DCHUNK * per; i += blockDim.x) sh[i] = 0.f;
+    __syncthreads();
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    auto stage = [&](int c0, float* buf) {
-        const int nc = min(DCHUNK, n - c0);
+    const int nv = min(cols, vdim - j0);
+    constexpr int O_K = DP, O_G = 2 * DP, O_V = (HD ? 2 : 3) * DP;
+    const float* q_src = a.qkv + (size_t)row0 * ch + (size_t)kh * dim;
+    const float* v_src = a.qkv + (size_t)row0 * ch + 2 * qk + (size_t)h * vdim + j0;
+    const float* g_src = a.decay + (HD ? (size_t)row0 * a.heads + h : (size_t)row0 * hd + (size_t)h * dim);
+    const float* b_src = a.beta + (size_t)row0 * a.heads + h;
+    const float* kq_src = a.kq + (size_t)row0 * a.kvh + kh;
+    auto stage = [&](unsigned c0, float* buf) {
+        const int nc = min(DCHUNK, n - (int)c0);
         for (int tt = wid; tt < nc; tt += nw) {          // a warp per token
-            const size_t t = row0 + c0 + tt;
-            float* dst = buf + (size_t)tt * per;
-            const float* q = a.qkv + t * ch + (size_t)kh * dim;
-            const float* g = a.decay + t * hd + (size_t)h * dim;
-            const float* v = a.qkv + t * ch + 2 * qk + (size_t)h * vdim;
-            for (int e = lane; e < dim; e += 32) {
-                const int at = (e / DPT) * RUN + e % DPT;
-                cp_async4(dst + at, q + e);
-                cp_async4(dst + o_k + at, q + qk + e);
-                cp_async4(dst + o_g + at, g + e);
+            float* dst = buf + tt * per;
+            const float* q = q_src + (size_t)(c0 + tt) * (unsigned)ch;
+            const float* v = v_src + (size_t)(c0 + tt) * (unsigned)ch;
+            const float* g = HD ? nullptr : g_src + (size_t)(c0 + tt) * (unsigned)hd;
+            if (VEC) {
+                for (int e = 4 * lane; e < dim; e += 128) {
+                    cp_async16(dst + e, q + e);
+                    cp_async16(dst + O_K + e, q + qk + e);
+                    if (!HD) cp_async16(dst + O_G + e, g + e);
+                }
+                for (int e = 4 * lane; e < nv; e += 128) cp_async16(dst + O_V + e, v + e);
+            } else {
+                for (int e = lane; e < dim; e += 32) {
+                    cp_async4(dst + e, q + e);
+                    cp_async4(dst + O_K + e, q + qk + e);
+                    if (!HD) cp_async4(dst + O_G + e, g + e);
+                }
+                for (int e = lane; e < nv; e += 32) cp_async4(dst + O_V + e, v + e);
             }
-            for (int e = lane; e < vdim; e += 32) cp_async4(dst + o_v + e, v + e);
-            if (lane == 0) cp_async4(dst + o_v + vdim, a.beta + t * a.heads + h);
+        }
+        const int st_ = threadIdx.x / 3, which = threadIdx.x % 3;      // (at least 64 threads: 48 numbers)
+        if (st_ < nc) {
+            float* dst = buf + st_ * per + O_V + cols + which;
+            if (which == 0) cp_async4(dst, b_src + (size_t)(c0 + st_) * (unsigned)a.heads);
+            else if (which == 1) cp_async4(dst, kq_src + (size_t)(c0 + st_) * (unsigned)a.kvh);
+            else if (HD) cp_async4(dst, g_src + (size_t)(c0 + st_) * (unsigned)a.heads);
         }
         cp_async_commit();
+    };
+    // a token's numbers in registers, read one token ahead of their use
+    struct Token { ulonglong2 q[DPT / 4], k[DPT / 4], g[HD ? 1 : DPT / 4]; float2 v; float4 sc; };
+    auto load = [&](const float* base) {
+        Token x;
+#pragma unroll
+        for (int i = 0; i < DPT / 4; ++i) {
+            x.q[i] = reinterpret_cast<const ulonglong2*>(base)[i * DLANES + s];
+            x.k[i] = reinterpret_cast<const ulonglong2*>(base + O_K)[i * DLANES + s];
+            if (!HD) x.g[i] = reinterpret_cast<const ulonglong2*>(base + O_G)[i * DLANES + s];
+        }
+        x.v = *reinterpret_cast<const float2*>(base + O_V + jl);
+        x.sc = *reinterpret_cast<const float4*>(base + O_V + cols);
+        return x;
+    };
+    float* out = a.o + (size_t)row0 * a.heads * vdim + (size_t)h * vdim + j + (s >> 3);      // the column whose sum ends in this lane
+    const bool writes = (s & 7) == 0 && j + (s >> 3) < vdim;
+    const size_t out_step = (size_t)a.heads * vdim;
+    auto token = [&](const Token& x) {
+        const f32x2 gs = pack2(x.sc.z, x.sc.z);
+        f32x2 dk[DCPT][2], dq[DCPT][2];
+#pragma unroll
+        for (int i = 0; i < DPT / 4; ++i)
+#pragma unroll
+            for (int c = 0; c < DCPT; ++c) {
+                if (!HD) {                            // a decay per head factors out of the sums
+                    st[c][2 * i] = mul2(st[c][2 * i], x.g[i].x);
+                    st[c][2 * i + 1] = mul2(st[c][2 * i + 1], x.g[i].y);
+                }
+                dk[c][0] = i ? fma2(st[c][2 * i], x.k[i].x, dk[c][0]) : mul2(st[c][0], x.k[0].x);
+                dk[c][1] = i ? fma2(st[c][2 * i + 1], x.k[i].y, dk[c][1]) : mul2(st[c][1], x.k[0].y);
+                dq[c][0] = i ? fma2(st[c][2 * i], x.q[i].x, dq[c][0]) : mul2(st[c][0], x.q[0].x);
+                dq[c][1] = i ? fma2(st[c][2 * i + 1], x.q[i].y, dq[c][1]) : mul2(st[c][1], x.q[0].y);
+            }
+        float u[DCPT], o[DCPT];
+        auto sum4 = [](f32x2 p, f32x2 q) {
+            float x0, x1, y0, y1;
+            unpack2(p, x0, x1);
+            unpack2(q, y0, y1);
+            return (x0 + x1) + (y0 + y1);
+        };
+#pragma unroll
+        for (int c = 0; c < DCPT; ++c) u[c] = sum4(dk[c][0], dk[c][1]);
+#pragma unroll
+        for (int off = DLANES / 2; off > 0; off >>= 1)
+#pragma unroll
+            for (int c = 0; c < DCPT; ++c) u[c] += __shfl_xor_sync(0xffffffffu, u[c], off);
+        if (HD)
+#pragma unroll
+            for (int c = 0; c < DCPT; ++c)
+#pragma unroll
+                for (int i = 0; i < DPT / 2; ++i) st[c][i] = mul2(st[c][i], gs);
+        const float v[DCPT] = {x.v.x, x.v.y};
+#pragma unroll
+        for (int c = 0; c < DCPT; ++c) {
+            u[c] = x.sc.x * (HD ? fmaf(-x.sc.z, u[c], v[c]) : v[c] - u[c]);
+            const f32x2 u2 = pack2(u[c], u[c]);
+#pragma unroll
+            for (int i = 0; i < DPT / 4; ++i) {
+                st[c][2 * i] = fma2(x.k[i].x, u2, st[c][2 * i]);
+                st[c][2 * i + 1] = fma2(x.k[i].y, u2, st[c][2 * i + 1]);
+            }
+        }
+        // the read-out's sums by halving: a lane hands one of its columns to its partner and keeps the other
+#pragma unroll
+        for (int c = 0; c < DCPT; ++c) o[c] = sum4(dq[c][0], dq[c][1]);
+        const bool up = s & 8;
+        float r = (up ? o[1] : o[0]) + __shfl_xor_sync(0xffffffffu, up ? o[0] : o[1], 8);
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
+        if (HD) r *= x.sc.z;
+        if (writes) *out = fmaf(up ? u[1] : u[0], x.sc.y, r);
+        out += out_step;
     };
     float* buf0 = sh;
     float* buf1 = sh + (size_t)DCHUNK * per;
@@ -833,56 +1019,49 @@ delta_rule_kernel(DeltaArgs a) {
         __syncthreads();                                  // chunk `it` has landed; everyone is done with the other buffer
         if (c0 + DCHUNK < n) stage(c0 + DCHUNK, (it & 1) ? buf0 : buf1);
         const int nc = min(DCHUNK, n - c0);
-        for (int tt = 0; tt < nc; ++tt) {
-            const float* base = cur + (size_t)tt * per;
-            const float4* q4 = reinterpret_cast<const float4*>(base + part * RUN);
-            const float4* k4 = reinterpret_cast<const float4*>(base + o_k + part * RUN);
-            const float4* g4 = reinterpret_cast<const float4*>(base + o_g + part * RUN);
-            float dot0 = 0.f, dot1 = 0.f;
-#pragma unroll
-            for (int i = 0; i < DPT; i += 4) {
-                if (FULL || d0 + i < dim) {
-                    const float4 gg = g4[i >> 2], kk = k4[i >> 2];
-                    const float ga[4] = {gg.x, gg.y, gg.z, gg.w}, ka[4] = {kk.x, kk.y, kk.z, kk.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (FULL || d0 + i + e < dim) {
-                            s[i + e] *= ga[e];
-                            if (e & 1) dot1 = fmaf(s[i + e], ka[e], dot1);
-                            else dot0 = fmaf(s[i + e], ka[e], dot0);
-                        }
-                }
-            }
-            float dot = dot0 + dot1;
-            dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-            dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-            const float u = live ? base[o_v + vdim] * (base[o_v + j] - dot) : 0.f;
-            float oa = 0.f, ob = 0.f;
-#pragma unroll
-            for (int i = 0; i < DPT; i += 4) {
-                if (FULL || d0 + i < dim) {
-                    const float4 kk = k4[i >> 2], qq = q4[i >> 2];
-                    const float ka[4] = {kk.x, kk.y, kk.z, kk.w}, qa[4] = {qq.x, qq.y, qq.z, qq.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (FULL || d0 + i + e < dim) {
-                            s[i + e] = fmaf(ka[e], u, s[i + e]);
-                            if (e & 1) ob = fmaf(s[i + e], qa[e], ob);
-                            else oa = fmaf(s[i + e], qa[e], oa);
-                        }
-                }
-            }
-            float o = oa + ob;
-            o += __shfl_xor_sync(0xffffffffu, o, 1);
-            o += __shfl_xor_sync(0xffffffffu, o, 2);
-            if (live && part == 0) a.o[(size_t)(row0 + c0 + tt) * ((size_t)a.heads * vdim) + (size_t)h * vdim + j] = o;
+        Token x = load(cur);
+        int tt = 0;
+#pragma unroll 1
+        for (; tt + 2 <= nc; tt += 2) {
+            const Token y = load(cur + (size_t)(tt + 1) * per);
+            token(x);
+            if (tt + 2 < nc) x = load(cur + (size_t)(tt + 2) * per);
+            token(y);
         }
+        if (tt < nc) token(x);
     }
-    if (live) {
 #pragma unroll
-        for (int i = 0; i < DPT; ++i)
-            if (d0 + i < dim) S[(size_t)(d0 + i) * vdim + j] = s[i];
-    }
+    for (int c = 0; c < DCPT; ++c)
+#pragma unroll
+        for (int i = 0; i < DPT; i += 2) {
+            const int d = channel(i);
+            float x, y;
+            unpack2(st[c][i / 2], x, y);
+            if (j + c < vdim && d < dim) S[(size_t)d * vdim + j + c] = x;
+            if (j + c < vdim && d + 1 < dim) S[(size_t)(d + 1) * vdim + j + c] = y;
+        }
+}
+
+template <int DPT, bool HD, bool VEC>
+static int launch_delta_rule_t(const DeltaArgs& a, int n_req, cudaStream_t stream) {
+    // 128 threads, or 64 while the wider blocks would leave SMs without a CTA
+    int threads = 128;
+    auto grid_of = [&](int th) { return dim3(n_req, a.heads, (a.vdim + th / DLANES * DCPT - 1) / (th / DLANES * DCPT)); };
+    const dim3 wide = grid_of(128);
+    if ((long long)wide.x * wide.y * wide.z < 148) threads = 64;
+    const size_t smem = (size_t)2 * DCHUNK * ((HD ? 2 : 3) * DLANES * DPT + threads / DLANES * DCPT + 4) * 4;
+    if (smem > 48 * 1024)
+        FT_CHECK_CUDA(cudaFuncSetAttribute(delta_rule_kernel<DPT, HD, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    delta_rule_kernel<DPT, HD, VEC><<<grid_of(threads), threads, smem, stream>>>(a);
+    FT_CHECK_CUDA(cudaGetLastError());
+    return 0;
+}
+template <int DPT>
+static int launch_delta_rule(const DeltaArgs& a, int n_req, cudaStream_t stream) {
+    // (every row of qkv and of the decays then starts on 16 bytes)
+    const bool vec = a.dim % 4 == 0 && a.vdim % 4 == 0 && (((uintptr_t)a.qkv | (uintptr_t)a.decay) & 15) == 0;
+    if (a.head_decay) return vec ? launch_delta_rule_t<DPT, true, true>(a, n_req, stream) : launch_delta_rule_t<DPT, true, false>(a, n_req, stream);
+    return vec ? launch_delta_rule_t<DPT, false, true>(a, n_req, stream) : launch_delta_rule_t<DPT, false, false>(a, n_req, stream);
 }
 
 // o[t, h, :] <- o / sqrt(mean(o^2) + eps) * w * act(gate[t, h, :]), one warp per (token, head); act = sigmoid or silu;
@@ -906,41 +1085,18 @@ int launch_delta(const DeltaArgs& a, const float* gate, const float* out_norm, f
     const int ch = 2 * a.kvh * a.dim + a.heads * a.vdim;
     FT_REQUIRE(a.taps >= 1 && a.taps <= 17, "channel delta: %d convolution taps are beyond 17", a.taps);
     FT_REQUIRE(a.dim <= 256 && a.vdim <= 256, "channel delta: head sizes %d / %d are beyond 256", a.dim, a.vdim);
-    FT_REQUIRE((size_t)ch * 4 <= 200 * 1024, "channel delta: %d channels do not fit in shared memory", ch);
-    static PerDeviceFlag attr;
-    if (!attr.done()) {
-        FT_CHECK_CUDA(cudaFuncSetAttribute(delta_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        attr.mark();
-    }
-    delta_prep_kernel<<<T, 256, (size_t)ch * 4, stream>>>(a);
+    FT_REQUIRE(a.kq, "channel delta: no place for the products of keys and queries");
+    const int groups = a.kvh + (a.heads * a.vdim + 127) / 128 + (a.head_decay ? 1 : a.heads);
+    if (T > 64) delta_prep_kernel<8><<<dim3((T + 7) / 8, groups), 128, 0, stream>>>(a, T);
+    else delta_prep_kernel<1><<<dim3(T, groups), 128, 0, stream>>>(a, T);
     FT_CHECK_CUDA(cudaGetLastError());
     if (a.taps > 1) {
         delta_tail_kernel<<<dim3((ch + 127) / 128, n_req), 128, 0, stream>>>(a, n_req);
         FT_CHECK_CUDA(cudaGetLastError());
     }
-    const int threads = (4 * std::min(a.vdim, DCOLS) + 31) / 32 * 32;      // four lanes per state column, whole warps
-    const int dpt = a.dim <= 32 ? 8 : a.dim <= 64 ? 16 : a.dim <= 128 ? 32 : 64;
-    const size_t smem = (size_t)2 * DCHUNK * delta_token_floats(dpt, a.vdim) * 4;
-    const dim3 grid(n_req, a.heads, (a.vdim + DCOLS - 1) / DCOLS);
-#define FT_DELTA_ONE(DPT_, FULL_)                                                                           \
-    do {                                                                                                    \
-        if (smem > 48 * 1024)                                                                               \
-            FT_CHECK_CUDA(cudaFuncSetAttribute(delta_rule_kernel<DPT_, 4 * DCOLS, FULL_>,                   \
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));    \
-        delta_rule_kernel<DPT_, 4 * DCOLS, FULL_><<<grid, threads, smem, stream>>>(a);                      \
-    } while (0)
-#define FT_DELTA(DPT_)                                  \
-    do {                                                \
-        if (a.dim == 4 * DPT_) FT_DELTA_ONE(DPT_, true); \
-        else FT_DELTA_ONE(DPT_, false);                 \
-    } while (0)
-    if (a.dim <= 32) FT_DELTA(8);
-    else if (a.dim <= 64) FT_DELTA(16);
-    else if (a.dim <= 128) FT_DELTA(32);
-    else FT_DELTA(64);
-#undef FT_DELTA
-#undef FT_DELTA_ONE
-    FT_CHECK_CUDA(cudaGetLastError());
+    if (a.dim <= 64) { if (int r = launch_delta_rule<4>(a, n_req, stream)) return r; }
+    else if (a.dim <= 128) { if (int r = launch_delta_rule<8>(a, n_req, stream)) return r; }
+    else { if (int r = launch_delta_rule<16>(a, n_req, stream)) return r; }
     const int n_pairs = T * a.heads;
     delta_out_kernel<<<(n_pairs + 3) / 4, 128, 0, stream>>>(a.o, gate, out_norm, a.vdim, eps, n_pairs, a.heads,
                                                             ldg > 0 ? ldg : a.heads * a.vdim, gate_act);

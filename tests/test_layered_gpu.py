@@ -425,3 +425,19 @@ def test_latent_attention_on_tensor_cores(sharp):
             assert rel(got, ref) < tol, ("exact" if exact else "tensor cores")
         finally:
             eng.close()
+
+
+# lanes of 4, 8 and 16 channels with and without padding, column blocks of 32 with a remainder, single columns, wide and narrow
+# copies; more than 64 tokens (eight per preparation block, a remainder) and single tokens
+@pytest.mark.parametrize("shape", [dict(heads=1, kv_heads=1, dim=64, vdim=32), dict(heads=2, kv_heads=1, dim=68, vdim=36), dict(heads=3, kv_heads=3, dim=128, vdim=129),
+                                   dict(heads=2, kv_heads=2, dim=130, vdim=5), dict(heads=2, kv_heads=1, dim=256, vdim=1), dict(heads=20, kv_heads=10, dim=8, vdim=256)])
+def test_delta_rule_sizes(shape):
+    spec, w = make([delta(conv=4, **shape)], seed=6)
+    eng = engine(spec, w)
+    try:
+        toks = tokens_of(spec, 93, 2)
+        ref = oracle_logits(spec, w, toks)
+        assert rel(feed_cut(eng, "cut", toks, [75, 1, 3, 1]), ref) < TOL
+        assert rel(feed_cut(eng, "one", toks, [93]), ref) < TOL
+    finally:
+        eng.close()
