@@ -925,6 +925,7 @@ static int run_branch(Engine* e, const Batch& b, const LayeredLayer& ll, int k, 
             launched();
         }
         if (q0 < T) {
+            if (tiles && q0 == 0) { o.out_hi = fin_hi = L.pl_hi; o.out_lo = fin_lo = L.pl_lo; }
             o.o += (size_t)q0 * o.ldo; o.out += (size_t)q0 * fin_cols;
             if (o.gate) o.gate += (size_t)q0 * o.ldg;
             if (o.x) o.x += (size_t)q0 * o.ldx;

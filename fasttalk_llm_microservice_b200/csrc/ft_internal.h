@@ -450,6 +450,7 @@ struct ReadoutArgs {
     const float* gain = nullptr;                  // [heads * vdim] or null (ones)
     float eps = 0.f;
     float* out = nullptr;                         // [T][heads * vdim]
+    void *out_hi = nullptr, *out_lo = nullptr;    // non-null: the results as bf16 hi + lo planes instead
 };
 int launch_readout(const ReadoutArgs& a, int T, cudaStream_t stream);
 

@@ -1182,35 +1182,56 @@ route_kernel(const float* __restrict__ proj, int ldp, int o_router, int E, int t
 // Counting sort of the T * top (token, choice) pairs by expert, one CTA: seg[e] .. seg[e+1] are the sorted places of
 // expert e, slot_token[place] the token whose row the expert reads, slot_pos[pair] the place of a pair.  Within an expert the
 // order is (token, choice) order, so the layout is the same from run to run.
+// Every warp has a run of neighbouring pairs: it counts them per expert, the counts of all warps are summed expert by expert, and it
+// walks its run once more, 32 pairs at a time, a pair's place being its expert's next one plus the earlier lanes with the same expert.
+// (A warp per expert that walked all pairs took 32 us for 4626 pairs; 6 us now.)
 __global__ void __launch_bounds__(1024)
 route_sort_kernel(const int* __restrict__ ids, int n_pairs, int top, int E, int* __restrict__ seg, int* __restrict__ slot_token,
                   int* __restrict__ slot_pos) {
     extern __shared__ int shi[];
-    int* cnt = shi;                    // [E + 1]
-    for (int e = threadIdx.x; e <= E; e += blockDim.x) cnt[e] = 0;
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    int* cnt = shi;                    // [warps][E]: a warp's pairs per expert, then where its next one goes
+    int* total = shi + nw * E;         // [E + 1]
+    for (int i = threadIdx.x; i < nw * E; i += blockDim.x) cnt[i] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) atomicAdd(&cnt[ids[i] + 1], 1);
+    const int run = ((n_pairs + nw - 1) / nw + 31) / 32 * 32, lo = min(wid * run, n_pairs), hi = min(lo + run, n_pairs);
+    for (int i = lo + lane; i < hi; i += 32) atomicAdd(&cnt[wid * E + ids[i]], 1);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int e = 0; e < E; ++e) cnt[e + 1] += cnt[e];
-        for (int e = 0; e <= E; ++e) seg[e] = cnt[e];
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+        int sum = 0;
+        for (int w = 0; w < nw; ++w) sum += cnt[w * E + e];
+        total[e + 1] = sum;
     }
     __syncthreads();
-    // stable placement: a warp per expert walks the pairs in order (ballot + prefix count)
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int e = wid; e < E; e += nw) {
-        int base = cnt[e];
-        for (int i0 = 0; i0 < n_pairs; i0 += 32) {
-            const int i = i0 + lane;
-            const bool mine = i < n_pairs && ids[i] == e;
-            const unsigned b = __ballot_sync(0xffffffffu, mine);
-            if (mine) {
-                const int place = base + __popc(b & ((1u << lane) - 1u));
-                slot_token[place] = i / top;
-                slot_pos[i] = place;
+    if (threadIdx.x == 0) {
+        total[0] = 0;
+        for (int e = 0; e < E; ++e) total[e + 1] += total[e];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e <= E; e += blockDim.x) {
+        seg[e] = total[e];
+        if (e < E) {
+            int next = total[e];
+            for (int w = 0; w < nw; ++w) {
+                const int c = cnt[w * E + e];
+                cnt[w * E + e] = next;
+                next += c;
             }
-            base += __popc(b);
         }
+    }
+    __syncthreads();
+    for (int i0 = lo; i0 < hi; i0 += 32) {
+        const int i = i0 + lane;
+        const int e = i < hi ? ids[i] : -1;
+        const unsigned same = __match_any_sync(0xffffffffu, e);
+        if (e >= 0) {
+            const int place = cnt[wid * E + e] + __popc(same & ((1u << lane) - 1u));
+            slot_token[place] = i / top;
+            slot_pos[i] = place;
+        }
+        __syncwarp();
+        if (e >= 0 && (same >> lane) == 1u) cnt[wid * E + e] += __popc(same);      // the last lane of the expert
+        __syncwarp();
     }
 }
 
@@ -1220,11 +1241,13 @@ int launch_route(const float* proj, int ldp, int o_router, int E, int top, int g
     FT_REQUIRE(groups >= 1 && E % groups == 0 && keep >= 1 && keep <= groups && top >= 1 && top <= (E / groups) * keep,
                "router: %d experts, %d groups, keep %d, top %d do not fit together", E, groups, keep, top);
     const size_t smem = (size_t)4 * (E + groups) * 4;
-    FT_REQUIRE(smem <= 48 * 1024 && (size_t)(E + 1) * 4 <= 48 * 1024, "router: %d experts are too many", E);
+    FT_REQUIRE(smem <= 48 * 1024 && (size_t)(2 * E + 1) * 4 <= 48 * 1024, "router: %d experts are too many", E);
     route_kernel<<<(T + 3) / 4, 128, smem, stream>>>(proj, ldp, o_router, E, top, groups, keep, ids, wts, T,
                                                      route_kind == FT_ROUTE_SIGMOID, normalise, scale > 0.f ? scale : 1.f, bias);
     FT_CHECK_CUDA(cudaGetLastError());
-    route_sort_kernel<<<1, 1024, (size_t)(E + 1) * 4, stream>>>(ids, T * top, top, E, seg, slot_token, slot_pos);
+    int warps = 32;                                    // fewer where the counts of so many would not fit
+    while (warps > 1 && (size_t)(warps * E + E + 1) * 4 > 48 * 1024) warps /= 2;
+    route_sort_kernel<<<1, warps * 32, (size_t)(warps * E + E + 1) * 4, stream>>>(ids, T * top, top, E, seg, slot_token, slot_pos);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
