@@ -46,8 +46,6 @@ __device__ __forceinline__ float cta_sum(float v, float* red) {      // red: >= 
 // x[t][c0 .. c0 + n) <- silu(x) in place, rows of stride ld; V columns (16 bytes or one) per thread
 template <int V>
 __global__ void __launch_bounds__(256) silu_cols_kernel(float* __restrict__ x, int ld, int c0, int n) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int c = (blockIdx.y * 256 + threadIdx.x) * V;
     if (c >= n) return;
     float* r = x + (size_t)blockIdx.x * ld + c0 + c;
@@ -63,14 +61,12 @@ int launch_silu_cols(float* x, int ld, int c0, int n, int T, cudaStream_t stream
     const bool v4 = ld % 4 == 0 && c0 % 4 == 0 && n % 4 == 0 && ((uintptr_t)x & 15) == 0;
     const int per = 256 * (v4 ? 4 : 1);
     const dim3 grid(T, (n + per - 1) / per);
-    if (v4) pdl_launch(silu_cols_kernel<4>, grid, 256, 0, stream, x, ld, c0, n);
-    else pdl_launch(silu_cols_kernel<1>, grid, 256, 0, stream, x, ld, c0, n);
+    if (v4) silu_cols_kernel<4><<<grid, 256, 0, stream>>>(x, ld, c0, n);
+    else silu_cols_kernel<1><<<grid, 256, 0, stream>>>(x, ld, c0, n);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 __global__ void turn_qk_kernel(TurnArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int t = blockIdx.x, half = a.rot_dims >> 1, per = half + a.dim - a.rot_dims;      // pairs, then single coordinates of a head
     const float pos = (float)a.positions[t];
     for (int i = threadIdx.x; i < (a.heads + a.kv_heads) * per; i += blockDim.x) {
@@ -92,20 +88,18 @@ __global__ void turn_qk_kernel(TurnArgs a) {
 int launch_turn_qk(const TurnArgs& a, int T, cudaStream_t stream) {
     FT_REQUIRE(a.rot_dims >= 0 && a.rot_dims <= a.dim && (a.rot_dims & 1) == 0 && (a.rot_dims == 0 || a.rot_freq),
                "rotation: bad sizes (dim %d, rotated %d)", a.dim, a.rot_dims);
-    pdl_launch(turn_qk_kernel, T, 256, 0, stream, a);
+    turn_qk_kernel<<<T, 256, 0, stream>>>(a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 // ab[t][h] = (decay[h], 1)
 __global__ void const_decay_kernel(const float* __restrict__ decay, float* __restrict__ ab, int heads, int n) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) { ab[2 * (size_t)i] = decay[i % heads]; ab[2 * (size_t)i + 1] = 1.f; }
 }
 int launch_const_decay(const float* decay, float* ab, int heads, int T, cudaStream_t stream) {
     const int n = T * heads;
-    pdl_launch(const_decay_kernel, (n + 255) / 256, 256, 0, stream, decay, ab, heads, n);
+    const_decay_kernel<<<(n + 255) / 256, 256, 0, stream>>>(decay, ab, heads, n);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -136,8 +130,6 @@ __device__ __forceinline__ float rotated(const float* __restrict__ src, const fl
 // CTA (token x, part y): the heads whose number is y modulo the parts — a step of few tokens is cut by heads so that more than a CTA
 // per token runs (one root mean square over all heads, qk_norm 2, keeps to one part).
 __global__ void __launch_bounds__(128) window_write_kernel(WindowArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     extern __shared__ float inv[];             // qk_norm: 1 / rms of every query head, then of every key head; then the pairs' trig
     const int t = blockIdx.x, part = blockIdx.y, parts = gridDim.y;
     const float* pr = a.proj + (size_t)t * a.ldp;
@@ -222,8 +214,6 @@ __device__ __forceinline__ void cp_async16_zfill(float* dst_smem, const float* s
 constexpr int kWinWarps = 4;
 template <int VPL, bool VEC>
 __global__ void __launch_bounds__(kWinWarps * 32) window_attn_kernel(WindowArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     extern __shared__ float sh[];
     float* sq = sh;                                    // [dim]
     float* sm = sq + ((a.dim + 3) & ~3);               // [warps] running maxima
@@ -320,27 +310,7 @@ __global__ void __launch_bounds__(kWinWarps * 32) window_attn_kernel(WindowArgs 
         for (int w = 0; w < kWinWarps; ++w) num += sacc[(size_t)w * a.vdim + c] * expf(sm[w] - mm);
         float r = num / den;
         if (a.gate) r *= sigmoid_f(a.gate[(size_t)t * a.ldg + h * a.vdim + c]);
-        const size_t at = ((size_t)t * a.H + h) * a.vdim + c;
-        if (a.out_hi) {
-            const __nv_bfloat16 b = __float2bfloat16_rn(r);
-            a.out_hi[at] = b;
-            a.out_lo[at] = __float2bfloat16_rn(r - __bfloat162float(b));
-        } else {
-            a.out[at] = r;
-        }
-    }
-}
-
-// Four neighbouring columns of the result, as fp32 or as the bf16 planes that the output projection reads.
-__device__ __forceinline__ void window_put4(const WindowArgs& a, size_t at, float4 o) {
-    if (a.out_hi) {
-        uint2 h, l;
-        h.x = pack_bf16(o.x, o.y); h.y = pack_bf16(o.z, o.w);
-        l.x = pack_bf16(o.x - bf16_lo(h.x), o.y - bf16_hi(h.x)); l.y = pack_bf16(o.z - bf16_lo(h.y), o.w - bf16_hi(h.y));
-        *reinterpret_cast<uint2*>(a.out_hi + at) = h;
-        *reinterpret_cast<uint2*>(a.out_lo + at) = l;
-    } else {
-        *reinterpret_cast<float4*>(a.out + at) = o;
+        a.out[((size_t)t * a.H + h) * a.vdim + c] = r;
     }
 }
 
@@ -353,8 +323,6 @@ __device__ __forceinline__ void window_put4(const WindowArgs& a, size_t at, floa
 constexpr int WT_ROWS = 64, WT_KEYS = 32, WT_THREADS = 256;
 template <int VK>
 __global__ void __launch_bounds__(WT_THREADS) window_tile_kernel(WindowArgs a, WindowTiles tm, int QT, int subs) {
-    pdl_wait();
-    pdl_launch_dependents();
     extern __shared__ __align__(16) float wsh[];
     const bool alias = a.v_in_key >= 0;       // the values are columns v_in_key.. of the key rows: no value tile of their own
     const int ldq = a.dim + 4, ldv = alias ? ldq : a.vdim, ldp = WT_KEYS + 1;
@@ -534,7 +502,7 @@ __global__ void __launch_bounds__(WT_THREADS) window_tile_kernel(WindowArgs a, W
         const int row = 8 * oy + r;
         if (row >= rows_used) continue;
         const float inv = cr[row];
-        const size_t o_at = ((size_t)(row_base + row / grp) * a.H + g * grp + row % grp) * a.vdim;
+        float* orow = a.out + ((size_t)(row_base + row / grp) * a.H + g * grp + row % grp) * a.vdim;
         const float* gate = a.gate ? a.gate + (size_t)(row_base + row / grp) * a.ldg + (g * grp + row % grp) * a.vdim : nullptr;
 #pragma unroll
         for (int k = 0; k < VK; ++k) {
@@ -544,7 +512,7 @@ __global__ void __launch_bounds__(WT_THREADS) window_tile_kernel(WindowArgs a, W
                 unpack2(acc[r][k][0], o0, o1);
                 unpack2(acc[r][k][1], o2, o3);
                 if (gate) { o0 *= sigmoid_f(gate[col]); o1 *= sigmoid_f(gate[col + 1]); o2 *= sigmoid_f(gate[col + 2]); o3 *= sigmoid_f(gate[col + 3]); }
-                window_put4(a, o_at + col, make_float4(o0 * inv, o1 * inv, o2 * inv, o3 * inv));
+                *reinterpret_cast<float4*>(orow + col) = make_float4(o0 * inv, o1 * inv, o2 * inv, o3 * inv);
             }
         }
     }
@@ -566,7 +534,7 @@ int launch_window_attention(const WindowArgs& a, int T, int n_single, const Wind
     // parts per token: as many as give about two CTAs per SM
     int parts = 1;
     while (a.qk_norm != 2 && parts < a.H && T * parts < 256 && parts < 16) parts *= 2;
-    pdl_launch(window_write_kernel, dim3(T, parts), 128, (size_t)((a.qk_norm ? a.H + a.G : 0) + a.rot_dims) * 4, stream, a);
+    window_write_kernel<<<dim3(T, parts), 128, (size_t)((a.qk_norm ? a.H + a.G : 0) + a.rot_dims) * 4, stream>>>(a);
     FT_CHECK_CUDA(cudaGetLastError());
     const int grp = a.H / a.G;
     FT_REQUIRE(a.v_in_key < 0 || (a.v_in_key + a.vdim <= a.dim && a.v_role == 0), "window attention: values inside the keys exceed them");
@@ -580,10 +548,10 @@ int launch_window_attention(const WindowArgs& a, int T, int n_single, const Wind
         dim3 grid(tm.n_tiles * subs, a.G);
         if (a.vdim <= 128) {
             FT_CHECK_CUDA(cudaFuncSetAttribute(window_tile_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
-            pdl_launch(window_tile_kernel<1>, grid, WT_THREADS, tsm, stream, a, tm, QT, subs);
+            window_tile_kernel<1><<<grid, WT_THREADS, tsm, stream>>>(a, tm, QT, subs);
         } else {
             FT_CHECK_CUDA(cudaFuncSetAttribute(window_tile_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
-            pdl_launch(window_tile_kernel<2>, grid, WT_THREADS, tsm, stream, a, tm, QT, subs);
+            window_tile_kernel<2><<<grid, WT_THREADS, tsm, stream>>>(a, tm, QT, subs);
         }
         FT_CHECK_CUDA(cudaGetLastError());
     }
@@ -595,8 +563,8 @@ int launch_window_attention(const WindowArgs& a, int T, int n_single, const Wind
     const int vpl = (a.vdim + 31) / 32;
 #define FT_WIN(V)                                                                                   \
     do {                                                                                            \
-        if (vec) pdl_launch(window_attn_kernel<V, true>, grid, kWinWarps * 32, smem, stream, a);            \
-        else pdl_launch(window_attn_kernel<V, false>, grid, kWinWarps * 32, smem, stream, a);               \
+        if (vec) window_attn_kernel<V, true><<<grid, kWinWarps * 32, smem, stream>>>(a);            \
+        else window_attn_kernel<V, false><<<grid, kWinWarps * 32, smem, stream>>>(a);               \
     } while (0)
     if (vpl <= 1) FT_WIN(1);
     else if (vpl <= 2) FT_WIN(2);
@@ -635,8 +603,6 @@ __device__ __forceinline__ void cp_async_f32x4(float* dst_smem, const float* src
 // other half, afterwards every lane holds one column and the tree goes on as usual.
 template <int LPC, int DPT, int CPT, bool VEC>
 __global__ void __launch_bounds__(RTHREADS) decay_rule_kernel(RecurArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     constexpr int VB = RTHREADS / LPC * CPT, RUN = DPT + 4, DP = LPC * RUN;
     constexpr int BUF = 2 * RCH * DP + RCH * VB + RCH * 2;      // floats of one staged chunk: keys | queries | values | (a, b)
     constexpr int NST = rule_stages(DP);
@@ -831,8 +797,8 @@ static int launch_decay_rule_t(const RecurArgs& a, int n_req, cudaStream_t strea
         FT_CHECK_CUDA(cudaFuncSetAttribute(decay_rule_kernel<LPC, DPT, CPT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     }
     dim3 grid((a.vd + VB - 1) / VB, a.heads, n_req);
-    if (vec) pdl_launch(decay_rule_kernel<LPC, DPT, CPT, true>, grid, RTHREADS, smem, stream, a);
-    else pdl_launch(decay_rule_kernel<LPC, DPT, CPT, false>, grid, RTHREADS, smem, stream, a);
+    if (vec) decay_rule_kernel<LPC, DPT, CPT, true><<<grid, RTHREADS, smem, stream>>>(a);
+    else decay_rule_kernel<LPC, DPT, CPT, false><<<grid, RTHREADS, smem, stream>>>(a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -896,8 +862,6 @@ extern "C" int ft_decay_rule(const float* q, const float* k, const float* v, con
 // Per token: values with a column of ones appended (the normaliser rides along as one more state column), and the log
 // gates i = cap tanh((z_i + b_i) / cap), f = logsigmoid(cap tanh((z_f + b_f) / cap)).
 __global__ void __launch_bounds__(128) memory_prep_kernel(MemoryArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int t = blockIdx.x, h = blockIdx.y;
     const float* pr = a.proj + (size_t)t * a.ldp;
     const int ve = a.vdim + 1;
@@ -916,8 +880,6 @@ __global__ void __launch_bounds__(128) memory_prep_kernel(MemoryArgs a) {
 // m_t = max(F_t + m_in, G_t).  Then a = exp(f + m_(t-1) - m_t), b = exp(i - m_t), floor[t] = exp(-m_t), the lower bound of the
 // read-out's denominator.  m lives in the state slot, 0 at a sequence's start.
 __global__ void __launch_bounds__(128) memory_scan_kernel(MemoryArgs a, int n_units) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (unit >= n_units) return;
     const int r = unit / a.heads, h = unit % a.heads;
@@ -950,10 +912,10 @@ __global__ void __launch_bounds__(128) memory_scan_kernel(MemoryArgs a, int n_un
 }
 int launch_memory_prep(const MemoryArgs& a, int T, int n_req, cudaStream_t stream) {
     FT_REQUIRE(a.heads >= 1 && a.cap > 0.f, "matrix memory: bad head count or gate cap");
-    pdl_launch(memory_prep_kernel, dim3(T, a.heads), 128, 0, stream, a);
+    memory_prep_kernel<<<dim3(T, a.heads), 128, 0, stream>>>(a);
     FT_CHECK_CUDA(cudaGetLastError());
     const int units = n_req * a.heads;
-    pdl_launch(memory_scan_kernel, (units + 3) / 4, 128, 0, stream, a, units);
+    memory_scan_kernel<<<(units + 3) / 4, 128, 0, stream>>>(a, units);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -965,8 +927,6 @@ int launch_memory_prep(const MemoryArgs& a, int T, int n_req, cudaStream_t strea
 // whose inputs are all rows of this step and of one request are read once for the block.
 template <int TB>
 __global__ void __launch_bounds__(256) space_conv_kernel(SpaceArgs a, int T) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int t0 = blockIdx.x * TB, nt = min(TB, T - t0), K = a.taps;
     const int c = blockIdx.y * 256 + threadIdx.x;
     if (blockIdx.y + 1 == gridDim.y)
@@ -1018,8 +978,6 @@ __global__ void __launch_bounds__(256) space_conv_kernel(SpaceArgs a, int T) {
 // The slot's tail after the step: the raw inputs of the last K-1 positions, from this step's rows or the old tail.
 constexpr int kMaxTaps = 16;
 __global__ void __launch_bounds__(256) space_tail_kernel(SpaceArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int r = blockIdx.y;
     const int start = a.req_start[r], n = a.req_start[r + 1] - start, pos0 = a.req_pos0[r], K = a.taps;
     if (n <= 0 || K <= 1) return;
@@ -1039,10 +997,10 @@ __global__ void __launch_bounds__(256) space_tail_kernel(SpaceArgs a) {
 int launch_space_prep(const SpaceArgs& a, int T, int n_req, cudaStream_t stream) {
     FT_REQUIRE(a.taps >= 1 && a.taps <= kMaxTaps, "state space: 1 to %d convolution taps (got %d)", kMaxTaps, a.taps);
     const int groups = (a.channels + 255) / 256;
-    if (T > 64) pdl_launch(space_conv_kernel<8>, dim3((T + 7) / 8, groups), 256, 0, stream, a, T);
-    else pdl_launch(space_conv_kernel<1>, dim3(T, groups), 256, 0, stream, a, T);
+    if (T > 64) space_conv_kernel<8><<<dim3((T + 7) / 8, groups), 256, 0, stream>>>(a, T);
+    else space_conv_kernel<1><<<dim3(T, groups), 256, 0, stream>>>(a, T);
     FT_CHECK_CUDA(cudaGetLastError());
-    pdl_launch(space_tail_kernel, dim3((a.channels + 255) / 256, n_req), 256, 0, stream, a);
+    space_tail_kernel<<<dim3((a.channels + 255) / 256, n_req), 256, 0, stream>>>(a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1065,8 +1023,6 @@ __device__ __forceinline__ float readout_value(const ReadoutArgs& a, int t, int 
 }
 constexpr int kReadoutKeep = 8;      // values a thread keeps in registers between the two passes
 __global__ void __launch_bounds__(256) readout_kernel(ReadoutArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red[33];
     const int t = blockIdx.x / a.norm_groups, g = blockIdx.x % a.norm_groups;
     const int n = a.heads * a.vdim / a.norm_groups, c0 = g * n;
@@ -1100,8 +1056,6 @@ __global__ void __launch_bounds__(256) readout_kernel(ReadoutArgs a) {
 // group's columns in registers between the two passes (one column at a time: 91 us for 2313 tokens of 4096 gated columns).
 template <int NV>
 __global__ void __launch_bounds__(256) readout_rows_kernel(ReadoutArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red[33];
     const int t = blockIdx.x / a.norm_groups, g = blockIdx.x % a.norm_groups;
     const int n = a.heads * a.vdim / a.norm_groups, c0 = g * n;
@@ -1163,15 +1117,15 @@ int launch_readout(const ReadoutArgs& a, int T, cudaStream_t stream) {
     if (!a.floor && a.vd == a.vdim && a.vdim % 4 == 0 && n % 4 == 0 && n <= 8192 && a.ldo % 4 == 0 && (!a.gate || a.ldg % 4 == 0) && (!a.skip || a.ldx % 4 == 0) &&
         (all & 15) == 0) {
         const int th = n <= 128 ? 32 : n <= 256 ? 64 : n <= 512 ? 128 : 256;
-        if (n <= 4 * th) pdl_launch(readout_rows_kernel<1>, T * a.norm_groups, th, 0, stream, a);
-        else if (n <= 8 * th) pdl_launch(readout_rows_kernel<2>, T * a.norm_groups, th, 0, stream, a);
-        else if (n <= 16 * th) pdl_launch(readout_rows_kernel<4>, T * a.norm_groups, th, 0, stream, a);
-        else pdl_launch(readout_rows_kernel<8>, T * a.norm_groups, th, 0, stream, a);
+        if (n <= 4 * th) readout_rows_kernel<1><<<T * a.norm_groups, th, 0, stream>>>(a);
+        else if (n <= 8 * th) readout_rows_kernel<2><<<T * a.norm_groups, th, 0, stream>>>(a);
+        else if (n <= 16 * th) readout_rows_kernel<4><<<T * a.norm_groups, th, 0, stream>>>(a);
+        else readout_rows_kernel<8><<<T * a.norm_groups, th, 0, stream>>>(a);
         FT_CHECK_CUDA(cudaGetLastError());
         return 0;
     }
     const int threads = n <= 64 ? 32 : n <= 256 ? 64 : n <= 1024 ? 128 : 256;
-    pdl_launch(readout_kernel, T * a.norm_groups, threads, 0, stream, a);
+    readout_kernel<<<T * a.norm_groups, threads, 0, stream>>>(a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

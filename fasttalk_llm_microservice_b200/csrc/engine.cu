@@ -592,7 +592,7 @@ static int dense(Engine* e, const float* A, const void* hi, const void* lo, cons
             hi = L.pl_hi;
             lo = L.pl_lo;
         }
-        FT_TRY(launch_gemm_plain(W, hi, lo, C, N, T, K, true, e->stream));
+        FT_TRY(launch_gemm_plain(W, hi, lo, C, N, T, K, false, e->stream));
         e->st.kernel_launches++;
         if (softcap > 0.f) {
             FT_TRY(launch_softcap(C, (size_t)T * N, softcap, e->stream));
@@ -796,10 +796,6 @@ static int run_branch(Engine* e, const Batch& b, const LayeredLayer& ll, int k, 
             if (rows > 0) FT_TRY(launch_paged16_mma(p, rows, st));
             launched(1 + (tc ? 1 : 0) + (rows > 0 ? 2 : 0));
         } else {
-            if (tiles && c.kind == FT_BRANCH_WINDOW_ATTENTION) {
-                fin_hi = L.pl_hi; fin_lo = L.pl_lo;
-                a.out_hi = (__nv_bfloat16*)fin_hi; a.out_lo = (__nv_bfloat16*)fin_lo;
-            }
             FT_TRY(launch_window_attention(a, T, b.n_decode, tm, st));
             launched(b.n_tiles > 0 && b.n_decode > 0 ? 3 : 2);
         }

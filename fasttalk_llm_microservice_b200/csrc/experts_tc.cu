@@ -33,7 +33,6 @@ template <int KIND>
 __global__ void __launch_bounds__(XT_THREADS, 2)
 experts_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
                   ExpertsKernelArgs a) {
-    pdl_wait();
     extern __shared__ uint8_t xt_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(xt_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint64_t full[XT_STAGES], empty[XT_STAGES], acc_full, drain;
@@ -84,7 +83,6 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_launch_dependents();      // not before its tensor memory: the next kernel takes its own ahead of its wait
     const uint32_t tmem = tmem_slot;
     if (warp == 0) {
         if (elect_one()) {
@@ -221,9 +219,9 @@ int launch_experts_tc(const ExpertsTcArgs& t, cudaStream_t stream) {
     const int tiles = t.pairs / XT_N + (t.E < t.pairs ? t.E : t.pairs);      // an upper bound: every expert may end with a partial tile
     FT_REQUIRE(tiles <= 65535, "experts (tcgen05): %d pairs are too many", t.pairs);
     const dim3 grid(t.n_rows / XT_M, tiles);
-    if (t.out) pdl_launch(experts_tc_kernel<XT_ROWS>, grid, XT_THREADS, XT_SMEM, stream, mw, mh, ml, a);
-    else if (t.act == FT_ACT_RELU2) pdl_launch(experts_tc_kernel<XT_RELU2>, grid, XT_THREADS, XT_SMEM, stream, mw, mh, ml, a);
-    else pdl_launch(experts_tc_kernel<XT_GLU>, grid, XT_THREADS, XT_SMEM, stream, mw, mh, ml, a);
+    if (t.out) experts_tc_kernel<XT_ROWS><<<grid, XT_THREADS, XT_SMEM, stream>>>(mw, mh, ml, a);
+    else if (t.act == FT_ACT_RELU2) experts_tc_kernel<XT_RELU2><<<grid, XT_THREADS, XT_SMEM, stream>>>(mw, mh, ml, a);
+    else experts_tc_kernel<XT_GLU><<<grid, XT_THREADS, XT_SMEM, stream>>>(mw, mh, ml, a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

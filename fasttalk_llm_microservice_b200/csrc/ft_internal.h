@@ -31,26 +31,6 @@ struct PerDeviceFlag {
     }
 };
 
-// Launch of a kernel that begins with pdl_wait(): its blocks may be set up while the kernel before it in the stream is still running
-// (programmatic dependent launch).  Every kernel of the layered models waits before it touches memory and then lets its successor start,
-// so "the kernel before has ended" holds along the whole stream as without the attribute.  A kernel with tensor memory lets it start
-// only once all of its own is allocated: a projection allocates ahead of its wait, and would otherwise hold columns that the kernel it
-// waits for still needs.
-template <class... P, class... A>
-inline void pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);      // (an error stays for cudaGetLastError)
-}
-
 // ---- gemm.cu
 int make_tmap_bf16_k64(CUtensorMap* map, const void* base, int rows, int K, int box_rows);
 int make_tmap_f16_3d(CUtensorMap* map, const void* base, int d0, int d1, int d2, int b0, int b1, int b2);
@@ -318,7 +298,6 @@ struct WindowArgs {
     int H = 0, G = 0, dim = 0, vdim = 0, window = 0;
     float scale = 1.f, softcap = 0.f;
     float* out = nullptr;                         // [T][H * vdim]
-    __nv_bfloat16 *out_hi = nullptr, *out_lo = nullptr;      // non-null: the result as bf16 hi + lo planes instead
     // options, off by default
     int qk_norm = 0;                              // q and k divided by their root mean square per head (before rotation)
     float eps = 0.f;

@@ -30,7 +30,6 @@ __device__ __forceinline__ void ht_copy16(uint32_t dst_smem, const void* src) {
 
 template <int NT>
 __global__ void __launch_bounds__(HT_THREADS) linear_heads_kernel(LinearArgs a, int* err) {
-    pdl_wait();
     constexpr int W_BYTES = HT_ROWS * 128, X_BYTES = NT * 128, STAGE = W_BYTES + 2 * X_BYTES;
     constexpr int COLS = NT < 32 ? 32 : NT;
     constexpr int PIECES = (NT * 8 + HT_THREADS - 1) / HT_THREADS;      // (token row, 8 columns) pieces per thread and block
@@ -56,7 +55,6 @@ __global__ void __launch_bounds__(HT_THREADS) linear_heads_kernel(LinearArgs a, 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_launch_dependents();      // not before its tensor memory: the next kernel takes its own ahead of its wait
     const uint32_t tmem = tmem_slot, base = smem_u32(smem);
     const int nkb = (a.K + HT_KB - 1) / HT_KB;
 
@@ -181,7 +179,7 @@ int launch_nt(const LinearArgs& a, int* err, cudaStream_t stream) {
         attr.mark();
     }
     const dim3 grid((a.N + HT_ROWS - 1) / HT_ROWS, (a.M + NT - 1) / NT, a.P);
-    pdl_launch(linear_heads_kernel<NT>, grid, HT_THREADS, SMEM, stream, a, err);
+    linear_heads_kernel<NT><<<grid, HT_THREADS, SMEM, stream>>>(a, err);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -56,8 +56,6 @@ constexpr int LBM = 64, LBN = 64, LBK = 16, LTHREADS = 256;
 
 template <bool VEC>
 __global__ void __launch_bounds__(LTHREADS) linear_tile_kernel(LinearArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float sA[LBK][LBM + 4];
     __shared__ float sW[LBK][LBN + 4];
     __shared__ int s_info[3];
@@ -186,8 +184,6 @@ constexpr int LWARPS = 8, LROWS_MANY = 16, LROWS_FEW = 4, LSTAGE = 8192;
 
 template <bool PAIR, bool VEC, int LROWS>
 __global__ void __launch_bounds__(LWARPS * 32) linear_rows_kernel(LinearArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     constexpr int LKC = LSTAGE / LROWS;
     constexpr int CPW = PAIR ? 2 : 4;                 // output columns per warp
     constexpr int WR = PAIR ? 2 * CPW : CPW;          // weight rows per warp
@@ -311,8 +307,8 @@ int launch_linear(const LinearArgs& a, int rows_bound, cudaStream_t stream) {
         const bool handful = a.seg ? rows_bound <= 3 * a.P : a.M <= LROWS_FEW;
 #define FT_ROWS(PAIR_, VEC_)                                                                                             \
     do {                                                                                                                 \
-        if (handful) pdl_launch(linear_rows_kernel<PAIR_, VEC_, LROWS_FEW>, grid, LWARPS * 32, 0, stream, a);                    \
-        else pdl_launch(linear_rows_kernel<PAIR_, VEC_, LROWS_MANY>, grid, LWARPS * 32, 0, stream, a);                           \
+        if (handful) linear_rows_kernel<PAIR_, VEC_, LROWS_FEW><<<grid, LWARPS * 32, 0, stream>>>(a);                    \
+        else linear_rows_kernel<PAIR_, VEC_, LROWS_MANY><<<grid, LWARPS * 32, 0, stream>>>(a);                           \
     } while (0)
         if (pair) {
             if (v8) FT_ROWS(true, true);
@@ -330,8 +326,8 @@ int launch_linear(const LinearArgs& a, int rows_bound, cudaStream_t stream) {
     dim3 grid((a.N + LBN - 1) / LBN, 1, 1);
     if (a.seg) grid.y = (rows_bound + LBM - 1) / LBM + a.P;
     else { grid.y = (a.M + LBM - 1) / LBM; grid.z = a.P; }
-    if (vec) pdl_launch(linear_tile_kernel<true>, grid, LTHREADS, 0, stream, a);
-    else pdl_launch(linear_tile_kernel<false>, grid, LTHREADS, 0, stream, a);
+    if (vec) linear_tile_kernel<true><<<grid, LTHREADS, 0, stream>>>(a);
+    else linear_tile_kernel<false><<<grid, LTHREADS, 0, stream>>>(a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -347,15 +343,11 @@ __device__ __forceinline__ void store_planes(__nv_bfloat16* hi, __nv_bfloat16* l
 
 __global__ void to_planes_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
                                  size_t n) {
-    pdl_wait();
-    pdl_launch_dependents();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         store_planes(hi, lo, i, x[i]);
 }
 
 __global__ void softcap_kernel(float* __restrict__ x, size_t n, float cap) {
-    pdl_wait();
-    pdl_launch_dependents();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         x[i] = cap * tanhf(x[i] / cap);
 }
@@ -363,8 +355,6 @@ __global__ void softcap_kernel(float* __restrict__ x, size_t n, float cap) {
 // planes of the rows an index list names: out row i = planes(src[idx[i]])
 __global__ void gather_planes_kernel2(const float* __restrict__ src, const int* __restrict__ idx, __nv_bfloat16* __restrict__ hi,
                                       __nv_bfloat16* __restrict__ lo, int W) {
-    pdl_wait();
-    pdl_launch_dependents();
     const size_t i = blockIdx.x;
     const float* r = src + (size_t)idx[i] * W;
     for (int c = threadIdx.x; c < W; c += blockDim.x) store_planes(hi, lo, i * W + c, r[c]);
@@ -373,8 +363,6 @@ __global__ void gather_planes_kernel2(const float* __restrict__ src, const int* 
 // gu [rows][2 ff] with columns (2j, 2j+1) = (gate_j, up_j)  ->  planes of their gated product (GluSpec), [rows][ff]
 __global__ void glu_planes_kernel(const float* __restrict__ gu, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, size_t n,
                                   int ff, GluSpec glu) {
-    pdl_wait();
-    pdl_launch_dependents();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const float2 v = reinterpret_cast<const float2*>(gu)[i];
         store_planes(hi, lo, i, glu_value(glu, v.x, v.y, glu.bias ? (int)(i % ff) : 0));
@@ -384,8 +372,6 @@ __global__ void glu_planes_kernel(const float* __restrict__ gu, __nv_bfloat16* _
 // u [rows][ff]  ->  planes of relu(u)^2
 __global__ void relu2_planes_kernel(const float* __restrict__ u, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
                                     size_t n) {
-    pdl_wait();
-    pdl_launch_dependents();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const float v = fmaxf(u[i], 0.f);
         store_planes(hi, lo, i, v * v);
@@ -393,28 +379,28 @@ __global__ void relu2_planes_kernel(const float* __restrict__ u, __nv_bfloat16* 
 }
 
 int launch_gather_planes_rows(const float* src, const int* idx, void* hi, void* lo, int n, int W, cudaStream_t stream) {
-    pdl_launch(gather_planes_kernel2, n, 256, 0, stream, src, idx, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, W);
+    gather_planes_kernel2<<<n, 256, 0, stream>>>(src, idx, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, W);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 int launch_act_planes(const float* gu, void* hi, void* lo, int rows, int ff, int act, const GluSpec& glu, cudaStream_t stream) {
     const size_t n = (size_t)rows * ff;
     const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-    if (act == FT_ACT_RELU2) pdl_launch(relu2_planes_kernel, blocks, 256, 0, stream, gu, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n);
-    else pdl_launch(glu_planes_kernel, blocks, 256, 0, stream, gu, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n, ff, glu);
+    if (act == FT_ACT_RELU2) relu2_planes_kernel<<<blocks, 256, 0, stream>>>(gu, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n);
+    else glu_planes_kernel<<<blocks, 256, 0, stream>>>(gu, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n, ff, glu);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 
 int launch_to_planes(const float* x, void* hi, void* lo, size_t n, cudaStream_t stream) {
     const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-    pdl_launch(to_planes_kernel, blocks, 256, 0, stream, x, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n);
+    to_planes_kernel<<<blocks, 256, 0, stream>>>(x, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 int launch_softcap(float* x, size_t n, float cap, cudaStream_t stream) {
     const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-    pdl_launch(softcap_kernel, blocks, 256, 0, stream, x, n, cap);
+    softcap_kernel<<<blocks, 256, 0, stream>>>(x, n, cap);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -425,8 +411,6 @@ __global__ void __launch_bounds__(256)
 embed_norm_kernel(const int* __restrict__ tokens, const __nv_bfloat16* __restrict__ embed, float* __restrict__ x,
                   float* __restrict__ hn, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, int W, float eps,
                   float gain, const float* __restrict__ gain_w) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red[33];
     const int t = blockIdx.x;
     const __nv_bfloat16* e = embed + (size_t)tokens[t] * W;
@@ -453,8 +437,6 @@ combine_norm_kernel(float* __restrict__ x, float* __restrict__ hn, const float* 
                     int o_rg2, const float* __restrict__ rg_bias, const float* __restrict__ mix,
                     const float* __restrict__ eout, const float* __restrict__ wt, const int* __restrict__ slot_pos,
                     int top, int W, float eps, float gain, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red[33];
     extern __shared__ float row[];
     const int t = blockIdx.x;
@@ -484,8 +466,6 @@ combine_norm_kernel(float* __restrict__ x, float* __restrict__ hn, const float* 
 
 // rows of the normed stream that the head reads: out[i] = hn[idx[i]]
 __global__ void gather_rows_kernel(const float* __restrict__ src, const int* __restrict__ idx, float* __restrict__ dst, int W) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int i = blockIdx.x;
     const float* s = src + (size_t)idx[i] * W;
     for (int c = threadIdx.x; c < W; c += blockDim.x) dst[(size_t)i * W + c] = s[c];
@@ -493,7 +473,7 @@ __global__ void gather_rows_kernel(const float* __restrict__ src, const int* __r
 
 int launch_embed_norm(const int* tokens, const void* embed, float* x, float* hn, void* hi, void* lo, int T, int W, float eps,
                       float gain, const float* gain_w, cudaStream_t stream) {
-    pdl_launch(embed_norm_kernel, T, 256, 0, stream, tokens, (const __nv_bfloat16*)embed, x, hn, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo,
+    embed_norm_kernel<<<T, 256, 0, stream>>>(tokens, (const __nv_bfloat16*)embed, x, hn, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo,
                                              W, eps, gain_w ? 1.f : gain, gain_w);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
@@ -501,13 +481,13 @@ int launch_embed_norm(const int* tokens, const void* embed, float* x, float* hn,
 int launch_combine_norm(float* x, float* hn, const float* proj, int ldp, int o_rg1, int o_rg2, const float* rg_bias,
                         const float* mix, const float* eout, const float* wt, const int* slot_pos, int top, int T, int W,
                         float eps, float gain, void* hi, void* lo, cudaStream_t stream) {
-    pdl_launch(combine_norm_kernel, T, 256, (size_t)W * 4, stream, x, hn, proj, ldp, o_rg1, o_rg2, rg_bias, mix, eout, wt, slot_pos,
+    combine_norm_kernel<<<T, 256, (size_t)W * 4, stream>>>(x, hn, proj, ldp, o_rg1, o_rg2, rg_bias, mix, eout, wt, slot_pos,
                                                           top, W, eps, gain, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 int launch_gather_rows(const float* src, const int* idx, float* dst, int n, int W, cudaStream_t stream) {
-    pdl_launch(gather_rows_kernel, n, 256, 0, stream, src, idx, dst, W);
+    gather_rows_kernel<<<n, 256, 0, stream>>>(src, idx, dst, W);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -517,8 +497,6 @@ int launch_gather_rows(const float* src, const int* idx, float* dst, int n, int 
 // pos % 64 of the layer's caches ([page][64][rank + rot] fp32; bf16 as latent_chunk16 lays a page out); the rotated part
 // of every query head goes to qlat.  Pairs (i, i + rot / 2); the angle's sine and cosine are formed once per token.
 __global__ void __launch_bounds__(128) latent_prep_kernel(LatentArgs a, int row16) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red[33];
     extern __shared__ float trig[];                        // [rot / 2] cosines, [rot / 2] sines
     const int t = blockIdx.x, rank = a.rank, rot = a.rot, half = rot >> 1;
@@ -589,8 +567,6 @@ __device__ __forceinline__ float latent_finish(float m, float l, const LatentArg
 
 template <int NR, int KB>
 __global__ void __launch_bounds__(128) latent_attn_kernel(LatentArgs a, int n_pairs, int n_split) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int pair = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int split = blockIdx.y;
     if (pair >= n_pairs) return;
@@ -678,7 +654,7 @@ __global__ void __launch_bounds__(128) latent_attn_kernel(LatentArgs a, int n_pa
 int launch_latent_prep(const LatentArgs& a, int T, cudaStream_t stream) {
     FT_REQUIRE(a.proj && a.norm_w && (a.cache || a.cache16) && (a.rot == 0 || (a.rot_freq && (a.qlat || a.qlat16) && a.rot % 2 == 0)),
                "latent prep: missing operands");
-    pdl_launch(latent_prep_kernel, T, 128, (size_t)a.rot * 4, stream, a, latent_row16(a.rank, a.rot));
+    latent_prep_kernel<<<T, 128, (size_t)a.rot * 4, stream>>>(a, latent_row16(a.rank, a.rot));
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -711,7 +687,7 @@ int launch_latent_attn(const LatentArgs& a, int T, cudaStream_t stream) {
         FT_REQUIRE(a.cache && a.qlat, "latent attention: no fp32 cache or queries");
         const int kd = a.rank + a.rot;
         const dim3 grid((n_pairs + 3) / 4, n_split);
-#define FT_LAT(NR_, KB_) pdl_launch(latent_attn_kernel<NR_, KB_>, grid, 128, 0, stream, a, n_pairs, n_split)
+#define FT_LAT(NR_, KB_) latent_attn_kernel<NR_, KB_><<<grid, 128, 0, stream>>>(a, n_pairs, n_split)
         if (kd <= 32) FT_LAT(1, 8);
         else if (kd <= 64) FT_LAT(2, 8);
         else if (kd <= 128) FT_LAT(4, 8);
@@ -737,8 +713,6 @@ int launch_latent_attn(const LatentArgs& a, int T, cudaStream_t stream) {
 template <int TB>
 __global__ void __launch_bounds__(128)
 delta_prep_kernel(DeltaArgs a, int T) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red[3][TB][4];
     const int t0 = blockIdx.x * TB, nt = min(TB, T - t0), g = blockIdx.y;
     const int qk = a.kvh * a.dim, ch = 2 * qk + a.heads * a.vdim, hd = a.heads * a.dim;
@@ -867,8 +841,6 @@ delta_prep_kernel(DeltaArgs a, int T) {
 
 // New tail of raw convolution inputs per (request, channel): the last taps-1 entries of (old tail ++ this step's inputs).
 __global__ void delta_tail_kernel(DeltaArgs a, int n_req) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int req = blockIdx.y;
     const int ch = 2 * a.kvh * a.dim + a.heads * a.vdim;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -900,8 +872,6 @@ constexpr int DCHUNK = 16, DLANES = 16, DCPT = 2;
 template <int DPT, bool HD, bool VEC>
 __global__ void __launch_bounds__(128)
 delta_rule_kernel(DeltaArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     extern __shared__ __align__(16) float sh[];
     constexpr int DP = DLANES * DPT;
     const int cols = blockDim.x / DLANES * DCPT, per = (HD ? 2 : 3) * DP + cols + 4;      // floats of a staged token: q | k | (g) | v | beta, kq, (g)
@@ -1082,7 +1052,7 @@ static int launch_delta_rule_t(const DeltaArgs& a, int n_req, cudaStream_t strea
     const size_t smem = (size_t)2 * DCHUNK * ((HD ? 2 : 3) * DLANES * DPT + threads / DLANES * DCPT + 4) * 4;
     if (smem > 48 * 1024)
         FT_CHECK_CUDA(cudaFuncSetAttribute(delta_rule_kernel<DPT, HD, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    pdl_launch(delta_rule_kernel<DPT, HD, VEC>, grid_of(threads), threads, smem, stream, a);
+    delta_rule_kernel<DPT, HD, VEC><<<grid_of(threads), threads, smem, stream>>>(a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1099,8 +1069,6 @@ static int launch_delta_rule(const DeltaArgs& a, int n_req, cudaStream_t stream)
 __global__ void __launch_bounds__(128)
 delta_out_kernel(float* __restrict__ o, const float* __restrict__ gate, const float* __restrict__ w, int vdim, float eps,
                  int n_pairs, int heads, int ldg, int gate_act) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int pair = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (pair >= n_pairs) return;
     float* p = o + (size_t)pair * vdim;
@@ -1119,18 +1087,18 @@ int launch_delta(const DeltaArgs& a, const float* gate, const float* out_norm, f
     FT_REQUIRE(a.dim <= 256 && a.vdim <= 256, "channel delta: head sizes %d / %d are beyond 256", a.dim, a.vdim);
     FT_REQUIRE(a.kq, "channel delta: no place for the products of keys and queries");
     const int groups = a.kvh + (a.heads * a.vdim + 127) / 128 + (a.head_decay ? 1 : a.heads);
-    if (T > 64) pdl_launch(delta_prep_kernel<8>, dim3((T + 7) / 8, groups), 128, 0, stream, a, T);
-    else pdl_launch(delta_prep_kernel<1>, dim3(T, groups), 128, 0, stream, a, T);
+    if (T > 64) delta_prep_kernel<8><<<dim3((T + 7) / 8, groups), 128, 0, stream>>>(a, T);
+    else delta_prep_kernel<1><<<dim3(T, groups), 128, 0, stream>>>(a, T);
     FT_CHECK_CUDA(cudaGetLastError());
     if (a.taps > 1) {
-        pdl_launch(delta_tail_kernel, dim3((ch + 127) / 128, n_req), 128, 0, stream, a, n_req);
+        delta_tail_kernel<<<dim3((ch + 127) / 128, n_req), 128, 0, stream>>>(a, n_req);
         FT_CHECK_CUDA(cudaGetLastError());
     }
     if (a.dim <= 64) { if (int r = launch_delta_rule<4>(a, n_req, stream)) return r; }
     else if (a.dim <= 128) { if (int r = launch_delta_rule<8>(a, n_req, stream)) return r; }
     else { if (int r = launch_delta_rule<16>(a, n_req, stream)) return r; }
     const int n_pairs = T * a.heads;
-    pdl_launch(delta_out_kernel, (n_pairs + 3) / 4, 128, 0, stream, a.o, gate, out_norm, a.vdim, eps, n_pairs, a.heads,
+    delta_out_kernel<<<(n_pairs + 3) / 4, 128, 0, stream>>>(a.o, gate, out_norm, a.vdim, eps, n_pairs, a.heads,
                                                             ldg > 0 ? ldg : a.heads * a.vdim, gate_act);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
@@ -1143,8 +1111,6 @@ int launch_delta(const DeltaArgs& a, const float* gate, const float* out_norm, f
 __global__ void __launch_bounds__(128)
 route_kernel(const float* __restrict__ proj, int ldp, int o_router, int E, int top, int groups, int keep, int* __restrict__ ids,
              float* __restrict__ wts, int T, int sigmoid_scores, int normalise, float scale, const float* __restrict__ bias) {
-    pdl_wait();
-    pdl_launch_dependents();
     extern __shared__ float sh[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + wid;
@@ -1222,8 +1188,6 @@ route_kernel(const float* __restrict__ proj, int ldp, int o_router, int E, int t
 __global__ void __launch_bounds__(1024)
 route_sort_kernel(const int* __restrict__ ids, int n_pairs, int top, int E, int* __restrict__ seg, int* __restrict__ slot_token,
                   int* __restrict__ slot_pos) {
-    pdl_wait();
-    pdl_launch_dependents();
     extern __shared__ int shi[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     int* cnt = shi;                    // [warps][E]: a warp's pairs per expert, then where its next one goes
@@ -1278,12 +1242,12 @@ int launch_route(const float* proj, int ldp, int o_router, int E, int top, int g
                "router: %d experts, %d groups, keep %d, top %d do not fit together", E, groups, keep, top);
     const size_t smem = (size_t)4 * (E + groups) * 4;
     FT_REQUIRE(smem <= 48 * 1024 && (size_t)(2 * E + 1) * 4 <= 48 * 1024, "router: %d experts are too many", E);
-    pdl_launch(route_kernel, (T + 3) / 4, 128, smem, stream, proj, ldp, o_router, E, top, groups, keep, ids, wts, T,
+    route_kernel<<<(T + 3) / 4, 128, smem, stream>>>(proj, ldp, o_router, E, top, groups, keep, ids, wts, T,
                                                      route_kind == FT_ROUTE_SIGMOID, normalise, scale > 0.f ? scale : 1.f, bias);
     FT_CHECK_CUDA(cudaGetLastError());
     int warps = 32;                                    // fewer where the counts of so many would not fit
     while (warps > 1 && (size_t)(warps * E + E + 1) * 4 > 48 * 1024) warps /= 2;
-    pdl_launch(route_sort_kernel, 1, warps * 32, (size_t)(warps * E + E + 1) * 4, stream, ids, T * top, top, E, seg, slot_token, slot_pos);
+    route_sort_kernel<<<1, warps * 32, (size_t)(warps * E + E + 1) * 4, stream>>>(ids, T * top, top, E, seg, slot_token, slot_pos);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

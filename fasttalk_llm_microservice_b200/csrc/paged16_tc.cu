@@ -71,7 +71,6 @@ bool paged_tc_cfg(const Paged16Args& a, PagedTcCfg& c) {
 template <int PER_SM>
 __global__ void __launch_bounds__(LT_THREADS, PER_SM)
 paged16_tc_kernel(Paged16Args a, WindowTiles tm, PagedTcCfg cfg, int subs, int* err) {
-    pdl_wait();
     using TM = LtTmem<PER_SM>;
     constexpr int NBUF = TM::NBUF;                                     // score buffers
     extern __shared__ uint8_t smem_raw[];
@@ -122,7 +121,6 @@ paged16_tc_kernel(Paged16Args a, WindowTiles tm, PagedTcCfg cfg, int subs, int* 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_launch_dependents();      // not before its tensor memory: the next kernel takes its own ahead of its wait
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 0) {
@@ -445,8 +443,8 @@ int launch_paged16_tc(const Paged16Args& a, const WindowTiles& tm, int* err, cud
     }
     const int subs = (c.span * c.grp + LT_ROWS - 1) / LT_ROWS;
     const dim3 grid(tm.n_tiles * subs * a.G, c.groups);
-    if (c.per_sm == 2) pdl_launch(paged16_tc_kernel<2>, grid, LT_THREADS, c.smem, stream, a, tm, c, subs, err);
-    else pdl_launch(paged16_tc_kernel<1>, grid, LT_THREADS, c.smem, stream, a, tm, c, subs, err);
+    if (c.per_sm == 2) paged16_tc_kernel<2><<<grid, LT_THREADS, c.smem, stream>>>(a, tm, c, subs, err);
+    else paged16_tc_kernel<1><<<grid, LT_THREADS, c.smem, stream>>>(a, tm, c, subs, err);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -37,8 +37,6 @@ __device__ __forceinline__ void planes_put(__nv_bfloat16* hi, __nv_bfloat16* lo,
 __global__ void __launch_bounds__(256)
 embed_scale_kernel(const int* __restrict__ tokens, const __nv_bfloat16* __restrict__ embed, float scale, float* __restrict__ x,
                    float* __restrict__ hist, int W) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int t = blockIdx.x;
     const __nv_bfloat16* e = embed + (size_t)tokens[t] * W;
     for (int c = threadIdx.x; c < W; c += blockDim.x) {
@@ -48,7 +46,7 @@ embed_scale_kernel(const int* __restrict__ tokens, const __nv_bfloat16* __restri
     }
 }
 int launch_embed_scale(const int* tokens, const void* embed, float scale, float* x, float* hist, int T, int W, cudaStream_t stream) {
-    pdl_launch(embed_scale_kernel, T, 256, 0, stream, tokens, (const __nv_bfloat16*)embed, scale, x, hist, W);
+    embed_scale_kernel<<<T, 256, 0, stream>>>(tokens, (const __nv_bfloat16*)embed, scale, x, hist, W);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -63,8 +61,6 @@ constexpr int kCanonMaxTaps = 17;
 // request are read once for the block (2313 tokens of 2048 columns, one CTA per token: 31 us; now 14 us).
 template <int TB>
 __global__ void __launch_bounds__(256) canon_kernel(CanonArgs a, int T) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int t0 = blockIdx.x * TB, nt = min(TB, T - t0), W = a.W, taps = a.taps, keep = taps - 1;
     const int c = blockIdx.y * 256 + threadIdx.x;
     if (c >= W) return;
@@ -120,8 +116,8 @@ int launch_canon(const CanonArgs& a, int T, cudaStream_t stream) {
     FT_REQUIRE(!a.w || (a.taps >= 1 && a.taps <= kCanonMaxTaps && a.state), "input convolution: %d taps are beyond %d", a.taps,
                kCanonMaxTaps);
     const int cols = (a.W + 255) / 256;
-    if (T > 64) pdl_launch(canon_kernel<8>, dim3((T + 7) / 8, cols), 256, 0, stream, a, T);
-    else pdl_launch(canon_kernel<1>, dim3(T, cols), 256, 0, stream, a, T);
+    if (T > 64) canon_kernel<8><<<dim3((T + 7) / 8, cols), 256, 0, stream>>>(a, T);
+    else canon_kernel<1><<<dim3(T, cols), 256, 0, stream>>>(a, T);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -142,8 +138,6 @@ __device__ __forceinline__ float post_y(const PostNormArgs& a, size_t i, int c) 
     return y;
 }
 __global__ void __launch_bounds__(256) postnorm_kernel(PostNormArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red[33];
     extern __shared__ float sm[];
     const int t = blockIdx.x, W = a.W;
@@ -212,8 +206,6 @@ __global__ void __launch_bounds__(256) postnorm_kernel(PostNormArgs a) {
 // sum and the result (one column at a time through shared memory: 34 us for 2313 rows of 2048, 52 at a layer's end; now 15 and 22 us).
 template <int NV>
 __global__ void __launch_bounds__(256) postnorm_rows_kernel(PostNormArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red[33];
     const int t = blockIdx.x, n4 = a.W >> 2;
     int r = 0, pos0 = 0, n = 1;
@@ -280,12 +272,12 @@ int launch_postnorm(const PostNormArgs& a, int T, cudaStream_t stream) {
     const uintptr_t all = (uintptr_t)a.x | (uintptr_t)a.x_out | (uintptr_t)a.y0 | (uintptr_t)a.y1 | (uintptr_t)a.b0 | (uintptr_t)a.b1 | (uintptr_t)a.post_w |
                           (uintptr_t)a.hist | (a.save_off >= 0 ? (uintptr_t)a.state | (uintptr_t)(a.slot_stride * 4) | (uintptr_t)(a.save_off * 4) : 0);
     if (!a.cw && a.W % 4 == 0 && a.W <= 8192 && (all & 15) == 0) {
-        if (a.W <= 1024) pdl_launch(postnorm_rows_kernel<1>, T, 256, 0, stream, a);
-        else if (a.W <= 2048) pdl_launch(postnorm_rows_kernel<2>, T, 256, 0, stream, a);
-        else if (a.W <= 4096) pdl_launch(postnorm_rows_kernel<4>, T, 256, 0, stream, a);
-        else pdl_launch(postnorm_rows_kernel<8>, T, 256, 0, stream, a);
+        if (a.W <= 1024) postnorm_rows_kernel<1><<<T, 256, 0, stream>>>(a);
+        else if (a.W <= 2048) postnorm_rows_kernel<2><<<T, 256, 0, stream>>>(a);
+        else if (a.W <= 4096) postnorm_rows_kernel<4><<<T, 256, 0, stream>>>(a);
+        else postnorm_rows_kernel<8><<<T, 256, 0, stream>>>(a);
     } else {
-        pdl_launch(postnorm_kernel, T, 256, (size_t)a.W * 8, stream, a);
+        postnorm_kernel<<<T, 256, (size_t)a.W * 8, stream>>>(a);
     }
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
@@ -295,8 +287,6 @@ int launch_postnorm(const PostNormArgs& a, int T, cudaStream_t stream) {
 __global__ void __launch_bounds__(256)
 rms_rows_kernel(const float* __restrict__ x, const int* __restrict__ rows, const float* __restrict__ w, float gain,
                 float* __restrict__ out, int W, float eps) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red[33];
     const float* src = x + (size_t)(rows ? rows[blockIdx.x] : blockIdx.x) * W;
     float ss = 0.f;
@@ -307,7 +297,7 @@ rms_rows_kernel(const float* __restrict__ x, const int* __restrict__ rows, const
 }
 int launch_rms_rows(const float* x, const int* rows, const float* w, float gain, float* out, int n, int W, float eps,
                     cudaStream_t stream) {
-    pdl_launch(rms_rows_kernel, n, 256, 0, stream, x, rows, w, gain, out, W, eps);
+    rms_rows_kernel<<<n, 256, 0, stream>>>(x, rows, w, gain, out, W, eps);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -315,8 +305,6 @@ int launch_rms_rows(const float* x, const int* rows, const float* w, float gain,
 __global__ void __launch_bounds__(128)
 rms_cols_kernel(const float* __restrict__ src, int lds, int src_off, const float* __restrict__ w, float* __restrict__ dst, int ldd,
                 int dst_off, int n, float eps) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red[33];
     const float* s = src + (size_t)blockIdx.x * lds + src_off;
     float* d = dst + (size_t)blockIdx.x * ldd + dst_off;
@@ -328,7 +316,7 @@ rms_cols_kernel(const float* __restrict__ src, int lds, int src_off, const float
 }
 int launch_rms_cols(const float* src, int lds, int src_off, const float* w, float* dst, int ldd, int dst_off, int n, float eps,
                     int T, cudaStream_t stream) {
-    pdl_launch(rms_cols_kernel, T, 128, 0, stream, src, lds, src_off, w, dst, ldd, dst_off, n, eps);
+    rms_cols_kernel<<<T, 128, 0, stream>>>(src, lds, src_off, w, dst, ldd, dst_off, n, eps);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -339,8 +327,6 @@ int launch_rms_cols(const float* src, int lds, int src_off, const float* w, floa
 __global__ void __launch_bounds__(128)
 latent_stage_kernel(const float* __restrict__ q, int heads, int dim, int rot, const float* __restrict__ proj, int ldp, int o_k,
                     int rank, const float* __restrict__ w, float eps, float* __restrict__ stage, int lds) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red[33];
     const int t = blockIdx.x, kd = rot + rank;
     float* st = stage + (size_t)t * lds;
@@ -363,7 +349,7 @@ latent_stage_kernel(const float* __restrict__ q, int heads, int dim, int rot, co
 }
 int launch_latent_stage(const float* q, int heads, int dim, int rot, const float* proj, int ldp, int o_k, int rank, const float* w,
                         float eps, float* stage, int lds, int T, cudaStream_t stream) {
-    pdl_launch(latent_stage_kernel, T, 128, 0, stream, q, heads, dim, rot, proj, ldp, o_k, rank, w, eps, stage, lds);
+    latent_stage_kernel<<<T, 128, 0, stream>>>(q, heads, dim, rot, proj, ldp, o_k, rank, w, eps, stage, lds);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -49,8 +49,6 @@ __device__ __forceinline__ float turned(const float* __restrict__ x, int c, int 
 // ------------------------------------------------------------------ one token per request
 template <int CV>
 __global__ void __launch_bounds__(RT_THREADS) retention_step_kernel(RetentionArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     extern __shared__ __align__(16) float rs_smem[];
     const int D = a.dim, V = a.vdim, h = blockIdx.x, r = blockIdx.y, t = a.req_start[r], tid = threadIdx.x;
     float* sq = rs_smem;                                 // [D]
@@ -138,8 +136,6 @@ __global__ void __launch_bounds__(RT_THREADS) retention_step_kernel(RetentionArg
 // ------------------------------------------------------------------ portions: bf16 rows
 // q16, k16 [row][heads][Dp], v16 [row][heads][Vp] of the step's rows from `row0` on (row index counted from there)
 __global__ void __launch_bounds__(256) retention_pack_kernel(RetentionArgs a, int row0, int Dp, int Vp) {
-    pdl_wait();
-    pdl_launch_dependents();
     extern __shared__ float trig[];
     const int t = row0 + blockIdx.x, H = a.heads, D = a.dim, V = a.vdim, half = a.rot_dims >> 1;
     const float* pr = a.proj + (size_t)t * a.ldp;
@@ -256,7 +252,6 @@ __device__ __forceinline__ void tile_out(float* tile, int ld, uint32_t tmem, int
 // ------------------------------------------------------------------ what a run adds to the state
 // D[d][v] (TMEM, M = 128 key channels, N = up to 128 value columns) = Kd^T V over the run's tokens; both operands MN-major.
 __global__ void __launch_bounds__(RT_THREADS) retention_gain_kernel(RetentionArgs a, WindowTiles tm, int Dp, int Vp, int* err) {
-    pdl_wait();
     extern __shared__ uint8_t rg_raw[];
     __shared__ float pw[RT_RUN];
     __shared__ uint64_t done;
@@ -278,7 +273,6 @@ __global__ void __launch_bounds__(RT_THREADS) retention_gain_kernel(RetentionArg
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_launch_dependents();      // not before its tensor memory: the next kernel takes its own ahead of its wait
     const uint32_t tmem = tmem_slot;
     stage_rows(v_s, (const __nv_bfloat16*)a.v16 + ((size_t)run.row * a.heads + h) * Vp + v0, (size_t)a.heads * Vp, nv / 64, run.n);
     const __nv_bfloat16* ks = (const __nv_bfloat16*)a.k16 + ((size_t)run.row * a.heads + h) * Dp;
@@ -357,8 +351,6 @@ __global__ void __launch_bounds__(RT_THREADS) retention_gain_kernel(RetentionArg
 // ws of a run: what it adds -> what it starts from.  CV numbers per thread.
 template <int CV>
 __global__ void __launch_bounds__(256) retention_carry_kernel(RetentionArgs a, WindowTiles tm, int first_req) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int j = blockIdx.z, h = blockIdx.y, e = (blockIdx.x * blockDim.x + threadIdx.x) * CV, DV = a.dim * a.vdim;
     if (e >= DV) return;
     const int len = tm.req_q_start[j + 1] - tm.req_q_start[j], n_runs = (len + RT_RUN - 1) / RT_RUN;
@@ -397,7 +389,6 @@ __global__ void __launch_bounds__(256) retention_carry_kernel(RetentionArgs a, W
 // its lo plane that of v once the run's part is.
 constexpr int RT_COL_S = 0, RT_COL_PH = 0, RT_COL_PL = 64, RT_COL_O1 = 0, RT_COL_O2 = 128;
 __global__ void __launch_bounds__(RT_THREADS, 2) retention_runs_kernel(RetentionArgs a, WindowTiles tm, int Dp, int Vp, int raw, int first_req, int* err) {
-    pdl_wait();
     extern __shared__ uint8_t rr_raw[];
     __shared__ float pw[RT_RUN + 1];
     __shared__ uint64_t done[3];
@@ -427,7 +418,6 @@ __global__ void __launch_bounds__(RT_THREADS, 2) retention_runs_kernel(Retention
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_launch_dependents();      // not before its tensor memory: the next kernel takes its own ahead of its wait
     const uint32_t tmem = tmem_slot;
     if (tid == 0) {
         const uint32_t idesc_qk = umma_idesc_bf16(RT_RUN, RT_RUN);
@@ -676,8 +666,8 @@ int launch_retention_step(const RetentionArgs& a, int n_req, cudaStream_t stream
     const size_t smem = (size_t)(((2 * a.dim + a.rot_dims + 33 + 3) & ~3) + 2 * ((a.vdim + 3) & ~3) + RT_THREADS * cv) * 4;
     FT_REQUIRE(smem <= 48 * 1024, "retention step: head sizes %d / %d are too large", a.dim, a.vdim);
     const dim3 grid(a.heads, n_req);
-    if (v4) pdl_launch(retention_step_kernel<4>, grid, RT_THREADS, smem, stream, a);
-    else pdl_launch(retention_step_kernel<1>, grid, RT_THREADS, smem, stream, a);
+    if (v4) retention_step_kernel<4><<<grid, RT_THREADS, smem, stream>>>(a);
+    else retention_step_kernel<1><<<grid, RT_THREADS, smem, stream>>>(a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -691,17 +681,17 @@ int launch_retention_tc(const RetentionArgs& a, const WindowTiles& tm, int first
         FT_CHECK_CUDA(cudaFuncSetAttribute(retention_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
         attr.mark();
     }
-    pdl_launch(retention_pack_kernel, rows, 256, (size_t)a.rot_dims * 4, stream, a, row0, Dp, Vp);
+    retention_pack_kernel<<<rows, 256, (size_t)a.rot_dims * 4, stream>>>(a, row0, Dp, Vp);
     FT_CHECK_CUDA(cudaGetLastError());
     const dim3 grid(tm.n_tiles, a.heads, groups);
-    pdl_launch(retention_gain_kernel, grid, RT_THREADS, RT_GAIN_SMEM, stream, a, tm, Dp, Vp, err);
+    retention_gain_kernel<<<grid, RT_THREADS, RT_GAIN_SMEM, stream>>>(a, tm, Dp, Vp, err);
     FT_CHECK_CUDA(cudaGetLastError());
     const int dv = a.dim * a.vdim;
     const bool v4 = a.vdim % 4 == 0 && a.slot_stride % 4 == 0 && a.s_off % 4 == 0 && ((uintptr_t)a.state & 15) == 0;
-    if (v4) pdl_launch(retention_carry_kernel<4>, dim3((dv / 4 + 255) / 256, a.heads, portions), 256, 0, stream, a, tm, first_req);
-    else pdl_launch(retention_carry_kernel<1>, dim3((dv + 255) / 256, a.heads, portions), 256, 0, stream, a, tm, first_req);
+    if (v4) retention_carry_kernel<4><<<dim3((dv / 4 + 255) / 256, a.heads, portions), 256, 0, stream>>>(a, tm, first_req);
+    else retention_carry_kernel<1><<<dim3((dv + 255) / 256, a.heads, portions), 256, 0, stream>>>(a, tm, first_req);
     FT_CHECK_CUDA(cudaGetLastError());
-    pdl_launch(retention_runs_kernel, grid, RT_THREADS, runs_smem(a.dim, a.vdim), stream, a, tm, Dp, Vp, !retention_one_pass(a.vdim), first_req, err);
+    retention_runs_kernel<<<grid, RT_THREADS, runs_smem(a.dim, a.vdim), stream>>>(a, tm, Dp, Vp, !retention_one_pass(a.vdim), first_req, err);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -19,8 +19,6 @@ __device__ __forceinline__ void put_row(float* f32, void* hi, void* lo, size_t a
 
 template <int V>
 __global__ void __launch_bounds__(256) sandwich_joint_kernel(SandwichArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red[33];
     extern __shared__ __align__(16) float row[];          // [W]: the sublayer's result, then the new row of the stream
     const int t = blockIdx.x, W = a.W;
@@ -118,8 +116,8 @@ int launch_sandwich_joint(const SandwichArgs& a, int T, cudaStream_t stream) {
             attr.mark();
         }
     }
-    if (v4) pdl_launch(sandwich_joint_kernel<4>, T, 256, smem, stream, a);
-    else pdl_launch(sandwich_joint_kernel<1>, T, 256, smem, stream, a);
+    if (v4) sandwich_joint_kernel<4><<<T, 256, smem, stream>>>(a);
+    else sandwich_joint_kernel<1><<<T, 256, smem, stream>>>(a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
