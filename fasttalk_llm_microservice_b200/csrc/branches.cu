@@ -787,6 +787,87 @@ __global__ void __launch_bounds__(RTHREADS) decay_rule_kernel(RecurArgs a) {
         }
 }
 
+// A step of single tokens: one pass over the state, which bounds it.  CTA (request, head, TX units of V columns): the threads of a row
+// group read neighbouring units, eight rows on their way per thread, and the row groups' shares of the read-out meet in shared
+// memory.  (More tokens than one are taken one after the other, each with a pass of its own.)  16 tokens, 16 heads of 128 x 128: the kernel
+// above, which stages chunks of 16 tokens for lanes that hold the state, took 17 us, this one 9; 64 heads of 128 x 64 25 and 12 us.
+template <int V>
+__global__ void __launch_bounds__(256) decay_step_kernel(RecurArgs a, int TX) {
+    extern __shared__ __align__(16) float sh[];
+    float* part = sh;                                 // [256][V]
+    float *sk = sh + 256 * V, *sq = sk + a.dim;
+    const int r = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+    const int t0 = a.req_start[r], t1 = a.req_start[r + 1];
+    const int tx = tid % TX, rg = tid / TX, RG = 256 / TX, c = (blockIdx.z * TX + tx) * V;
+    const bool live = c < a.vd;
+    const int gh = h / (a.heads / a.qk_heads);
+    float* S = a.state + (size_t)a.req_slot[r] * a.slot_stride + a.s_off + (size_t)h * a.dim * a.vd + c;
+    bool old = a.req_pos0[r] > 0;
+    for (int t = t0; t < t1; ++t, old = true) {
+        for (int d = tid; d < a.dim; d += 256) {
+            sk[d] = a.k[(size_t)t * a.ldk + (size_t)gh * a.dim + d];
+            sq[d] = a.q[(size_t)t * a.ldq + (size_t)gh * a.dim + d];
+        }
+        const float da = a.ab[((size_t)t * a.heads + h) * 2], db = a.ab[((size_t)t * a.heads + h) * 2 + 1];
+        float v[V], o[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            v[i] = live ? db * a.v[(size_t)t * a.ldv + (size_t)h * a.vd + c + i] : 0.f;
+            o[i] = 0.f;
+        }
+        __syncthreads();
+        if (live)
+            for (int d0 = rg; d0 < a.dim; d0 += 8 * RG) {
+                float x[8][V];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int d = d0 + i * RG;
+                    if (V == 4) {
+                        const float4 f = old && d < a.dim ? *reinterpret_cast<const float4*>(S + (size_t)d * a.vd) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        x[i][0] = f.x; x[i][1 % V] = f.y; x[i][2 % V] = f.z; x[i][3 % V] = f.w;
+                    } else {
+                        x[i][0] = old && d < a.dim ? S[(size_t)d * a.vd] : 0.f;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int d = d0 + i * RG;
+                    if (d >= a.dim) break;
+                    const float kk = sk[d], qq = sq[d];
+#pragma unroll
+                    for (int e = 0; e < V; ++e) {
+                        x[i][e] = fmaf(da, x[i][e], v[e] * kk);
+                        o[e] = fmaf(x[i][e], qq, o[e]);
+                    }
+                    if (V == 4) *reinterpret_cast<float4*>(S + (size_t)d * a.vd) = make_float4(x[i][0], x[i][1 % V], x[i][2 % V], x[i][3 % V]);
+                    else S[(size_t)d * a.vd] = x[i][0];
+                }
+            }
+#pragma unroll
+        for (int e = 0; e < V; ++e) part[tid * V + e] = o[e];
+        __syncthreads();
+        for (int i = tid; i < TX * V; i += 256) {
+            const int col = blockIdx.z * TX * V + i;
+            float sum = 0.f;
+            for (int g = 0; g < RG; ++g) sum += part[g * TX * V + i];
+            if (col < a.vd) a.o[(size_t)t * a.ldo + (size_t)h * a.vd + col] = sum;
+        }
+        __syncthreads();
+    }
+}
+static int launch_decay_step(const RecurArgs& a, int n_req, cudaStream_t stream) {
+    const bool wide = a.vd % 4 == 0 && a.slot_stride % 4 == 0 && a.s_off % 4 == 0 && ((uintptr_t)a.state & 15) == 0;
+    const int units = wide ? a.vd / 4 : a.vd;
+    int TX = 8;
+    while (TX < 32 && TX < units) TX *= 2;
+    const dim3 grid(n_req, a.heads, (units + TX - 1) / TX);
+    const size_t smem = (size_t)(256 * (wide ? 4 : 1) + 2 * a.dim) * 4;
+    if (wide) decay_step_kernel<4><<<grid, 256, smem, stream>>>(a, TX);
+    else decay_step_kernel<1><<<grid, 256, smem, stream>>>(a, TX);
+    FT_CHECK_CUDA(cudaGetLastError());
+    return 0;
+}
+
 template <int LPC, int DPT, int CPT>
 static int launch_decay_rule_t(const RecurArgs& a, int n_req, cudaStream_t stream) {
     constexpr int VB = RTHREADS / LPC * CPT, DP = LPC * (DPT + 4);
@@ -807,13 +888,12 @@ static int launch_decay_rule_t(const RecurArgs& a, int n_req, cudaStream_t strea
 // fewest lanes whose runs cover dim and four columns per thread — the widest column blocks, the best-coalesced state
 // traffic and the fewest shared-memory reads per multiply-add; then, while fewer than 96 CTAs would run (one long prompt
 // with few heads): two columns per thread, more lanes with shorter runs, at last one column (measured order).  The split
-// changes the order of a sum, nothing else.  a.lanes fixes LPC.  T: tokens in the step (unused by the present rule, kept
-// for callers that tune).
+// changes the order of a sum, nothing else.  a.lanes fixes LPC.  Steps of single tokens (no more rows than requests) take the step kernel.
 int launch_decay_rule(const RecurArgs& a, int n_req, int T, cudaStream_t stream) {
-    (void)T;
     FT_REQUIRE(a.heads >= 1 && a.qk_heads >= 1 && a.heads % a.qk_heads == 0 && a.dim >= 1 && a.dim <= 1024 && a.vd >= 1,
                "decay rule: bad sizes (heads %d, key heads %d, dim %d, values %d)", a.heads, a.qk_heads, a.dim, a.vd);
     if (n_req <= 0) return 0;
+    if (a.lanes == 0 && T > 0 && T <= n_req) return launch_decay_step(a, n_req, stream);
     int lpc = 4, dpt = 4;
     while (dpt < 16 && lpc * dpt < a.dim) dpt *= 2;
     while (lpc < 32 && lpc * dpt < a.dim) lpc *= 2;

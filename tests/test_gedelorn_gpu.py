@@ -530,3 +530,43 @@ def test_decay_rule_kernel_alone(lanes, heads, qk_heads, dim, vd):
     assert rc == 0, native.last_error()
     assert rel(o.cpu().double().numpy(), ref_o.numpy()) < 1e-5
     assert rel(dst.cpu().double().numpy(), ref_state.numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("heads,qk_heads,dim,vd,pad", [(2, 2, 128, 128, 0), (3, 1, 96, 80, 0), (4, 2, 64, 257, 0), (2, 1, 7, 20, 1), (1, 1, 513, 1, 0)])
+def test_decay_rule_single_tokens(heads, qk_heads, dim, vd, pad):
+    """One token per request (units of four columns and of one, slots that break the 16-byte rows, fresh and continued states), and a
+    request of several tokens in a launch whose caller named fewer rows."""
+    from fasttalk_llm_microservice_b200 import build, native
+    build.build()
+    lib = native.load()
+    g = torch.Generator().manual_seed(dim + vd)
+    dev = "cuda"
+    for lens, rows in (([1] * 5, 5), ([1, 3, 1], 3)):
+        T, R = sum(lens), len(lens)
+        pos0 = [0 if r % 2 else 11 for r in range(R)]
+        q, k = torch.randn(T, qk_heads * dim, generator=g) * dim ** -0.5, torch.randn(T, qk_heads * dim, generator=g)
+        v = torch.randn(T, heads * vd, generator=g)
+        ab = torch.rand(T, heads, 2, generator=g).contiguous()
+        stride = heads * dim * vd + pad
+        state = torch.randn(R * stride, generator=g)
+        start = [0] + [sum(lens[:i + 1]) for i in range(R)]
+        ref_o, ref_state = torch.zeros(T, heads, vd, dtype=torch.float64), state.double().clone()
+        rep = lambda x: x.double().reshape(T, qk_heads, dim).repeat_interleave(heads // qk_heads, 1)
+        q64, k64, v64 = rep(q), rep(k), v.double().reshape(T, heads, vd)
+        for r in range(R):
+            S = ref_state[r * stride:r * stride + heads * dim * vd].reshape(heads, dim, vd) * (pos0[r] > 0)
+            for t in range(start[r], start[r + 1]):
+                S = ab[t, :, 0].double()[:, None, None] * S + (ab[t, :, 1].double()[:, None] * k64[t])[:, :, None] * v64[t][:, None, :]
+                ref_o[t] = torch.einsum("hdv,hd->hv", S, q64[t])
+            ref_state[r * stride:r * stride + heads * dim * vd] = S.reshape(-1)
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+        rs, rp, sl = i32(start), i32(pos0), i32(list(range(R)))
+        dq, dk, dv, dab, dst = q.to(dev), k.to(dev), v.to(dev), ab.to(dev), state.to(dev)
+        o = torch.zeros(T, heads * vd, device=dev)
+        rc = lib.ft_decay_rule(dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dab.data_ptr(), o.data_ptr(), dst.data_ptr(), rs.data_ptr(),
+                               rp.data_ptr(), sl.data_ptr(), R, heads, qk_heads, dim, vd, stride, 0, rows, None)
+        torch.cuda.synchronize()
+        assert rc == 0, native.last_error()
+        # 24-bit sums of dim terms
+        assert rel(o.cpu().double().numpy(), ref_o.reshape(T, -1).numpy()) < 2e-6
+        assert rel(dst.cpu().double().numpy(), ref_state.numpy()) < 1e-6
