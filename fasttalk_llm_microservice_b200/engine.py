@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import hashlib
+from array import array
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -242,7 +243,13 @@ class Engine:
         logits are wanted).  All entries run as one batch; returns float32 [wanted, vocab] in entry order."""
         keys = np.array([session_key(s) for s, _, _ in entries], dtype=np.uint64)
         counts = np.array([len(t) for _, t, _ in entries], dtype=np.int32)
-        toks = np.ascontiguousarray(np.concatenate([np.asarray(t, dtype=np.int32) for _, t, _ in entries]))
+        flat = array("i")
+        for _, t, _ in entries:
+            try:
+                flat.fromlist(t)                       # (several times faster than numpy on a list of Python integers)
+            except TypeError:                          # not a list, or not one of integers
+                flat.frombytes(np.ascontiguousarray(t, dtype=np.int32).tobytes())
+        toks = np.frombuffer(flat, dtype=np.int32) if len(flat) else np.empty(0, dtype=np.int32)
         want, off = [], 0
         for _, t, wn in entries:
             want += [off + int(i) for i in wn]
