@@ -709,7 +709,7 @@ int launch_latent_attn(const LatentArgs& a, int T, cudaStream_t stream) {
 // normed rows, the decay exp(-exp(A_log_h) * softplus(a + dt_bias)) per head and key channel (or per head), beta = sigmoid.
 // qkv out: [T][channels] with channels = 2 * kvh * dim + heads * vdim in the order q | k | v.
 // CTA (tokens x .. + TB - 1, group y): group y < kvh is a q and a k head, then come 128 value channels each, then decays and betas.  A thread keeps its channels over the TB tokens, so that the rows the taps share come out of L1 (one CTA per
-// token, all channels after one another: 121 us for 2313 tokens of 6144 channels).
+// token, all channels after one another: 121 us for 2313 tokens of 6144 channels; now 73 us).
 template <int TB>
 __global__ void __launch_bounds__(128)
 delta_prep_kernel(DeltaArgs a, int T) {
@@ -864,8 +864,9 @@ __global__ void delta_tail_kernel(DeltaArgs a, int n_req) {
 // so that both sums over key channels are taken in one pass and only one of them, S^T k, lies on the chain from token to token:
 // a few multiply-adds, four shuffles, u, the update.  q, k, g, v of DCHUNK tokens at a time are copied into shared memory one
 // chunk ahead; channels beyond dim are zeros.
-// Bound by that chain (one or two warps per scheduler).  Four lanes per column with one column per thread, unpacked, both sums one
-// after the other: 515 us for three requests of 771 tokens, 16 heads of 128 x 128.
+// Bound by that chain and by the instructions around it (two to three warps per scheduler).  Four lanes per column with one column per
+// thread, unpacked, both sums one after the other took 515 us for three requests of 771 tokens, 16 heads of 128 x 128; this form
+// 277 us (four columns per thread, half as many warps: 506 us).
 constexpr int DCHUNK = 16, DLANES = 16, DCPT = 2;
 
 // DPT: channels per lane (dim <= 16 DPT).  HD: one decay per head instead of one per key channel.  VEC: rows are copied 16 bytes at a time.
@@ -1184,7 +1185,7 @@ route_kernel(const float* __restrict__ proj, int ldp, int o_router, int E, int t
 // order is (token, choice) order, so the layout is the same from run to run.
 // Every warp has a run of neighbouring pairs: it counts them per expert, the counts of all warps are summed expert by expert, and it
 // walks its run once more, 32 pairs at a time, a pair's place being its expert's next one plus the earlier lanes with the same expert.
-// (A warp per expert that walked all pairs took 32 us for 4626 pairs; 6 us now.)
+// (A warp per expert that walked all pairs took 32 us for 4626 pairs; 8 us now.)
 __global__ void __launch_bounds__(1024)
 route_sort_kernel(const int* __restrict__ ids, int n_pairs, int top, int E, int* __restrict__ seg, int* __restrict__ slot_token,
                   int* __restrict__ slot_pos) {

@@ -58,7 +58,7 @@ int launch_embed_scale(const int* tokens, const void* embed, float scale, float*
 // two launches in stream order, so a step never reads a ring entry that it has already replaced.
 constexpr int kCanonMaxTaps = 17;
 // A CTA takes TB tokens of 256 columns, a thread one column.  Up to four taps whose inputs are all rows of this step and of one
-// request are read once for the block (2313 tokens of 2048 columns, one CTA per token: 31 us; now 14 us).
+// request are read once for the block (2313 tokens of 2048 columns, one CTA per token: 31 us; now 15 us).
 template <int TB>
 __global__ void __launch_bounds__(256) canon_kernel(CanonArgs a, int T) {
     const int t0 = blockIdx.x * TB, nt = min(TB, T - t0), W = a.W, taps = a.taps, keep = taps - 1;
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(256) postnorm_kernel(PostNormArgs a) {
     }
 }
 // The same without the next input, rows of whole 16-byte groups: NV groups of four columns per thread stay in registers between the
-// sum and the result (one column at a time through shared memory: 34 us for 2313 rows of 2048, 52 at a layer's end; now 15 and 22 us).
+// sum and the result (one column at a time through shared memory: 41 us for 2313 rows of 2048, the mean of a layer's two joints; now 17 us).
 template <int NV>
 __global__ void __launch_bounds__(256) postnorm_rows_kernel(PostNormArgs a) {
     __shared__ float red[33];
