@@ -15,7 +15,7 @@ def main(rep, title):
     rows = list(csv.reader(out.splitlines()))
     hdr, units = rows[0], rows[1]
     cols = [c for c in WANT if c in hdr]
-    print(f"## {title}\n\nsource: `{rep}` (`ncu --set full --clock-control none --import-source on`)\n")
+    print(f"## {title}\n\nsource: `{rep}`\n")
     print("| kernel | grid | " + " | ".join(cols) + " |")
     print("|---|---|" + "---|" * len(cols))
     for r in rows[2:]:
