@@ -1528,6 +1528,10 @@ static int engine_step(Engine* e, std::unique_lock<std::mutex>& lk) {
     int produced = 0;
     auto emit = [&](Request* r) {
         const int tok = h[m.o_sampled + r->logits_row];
+        if (tok < 0 || tok >= c.vocab) {             // the next step would read the embedding table with it
+            finish_request(e, r, 4, -1);
+            return;
+        }
         r->last_token = tok;
         r->n_generated++;
         produced++;

@@ -279,6 +279,7 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
     int argmax = sm.idx[0];
     for (int p = 1; p < C; ++p)
         if (sm.val[p] > maxv) { maxv = sm.val[p]; argmax = sm.idx[p]; }      // shares are in index order: the first maximum wins
+    if (argmax == 0x7fffffff) argmax = 0;            // no logit above minus infinity (all of them minus infinity or NaN): an index of the row all the same
     if (greedy) {
         if (rank == 0 && threadIdx.x == 0) out_tokens[b] = argmax;
         return;

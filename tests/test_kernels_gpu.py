@@ -632,6 +632,20 @@ def test_sample_rows_without_numbers(K):
         tok = K.sample(logits, n, torch.full((6,), top_k, device=DEV, dtype=torch.int32), torch.full((6,), top_p, device=DEV),
                        torch.arange(6, device=DEV, dtype=torch.int64)).tolist()
         assert tok[0] >= V - 5 and tok[1] == 777 and 0 <= tok[2] < V and tok[2] != 3 and tok[5] % 2 == 1
+        assert all(0 <= t < V for t in tok)
+
+
+@pytest.mark.parametrize("V", [1, 7, 4096, 4100, 32768, 128256])
+def test_sample_rows_without_a_largest_logit(K, V):
+    """Rows of minus infinities, of NaN, and of both, greedy and drawn, one CTA per row up to eight: the token is one of the row's."""
+    logits = torch.full((3, V), -float("inf"), device=DEV)
+    logits[1] = float("nan")
+    logits[2, ::2] = float("nan")
+    for temp, top_k, top_p in [(0.0, 0, 1.0), (0.8, 0, 1.0), (0.8, 20, 0.9), (0.8, 0, 0.0)]:
+        tok = K.sample(logits, torch.full((3,), temp, device=DEV), torch.full((3,), top_k, device=DEV, dtype=torch.int32),
+                       torch.full((3,), top_p, device=DEV), torch.arange(3, device=DEV, dtype=torch.int64)).tolist()
+        assert all(0 <= t < V for t in tok), (temp, top_k, top_p, tok)
+    assert all(0 <= t < V for t in K.sample(logits).tolist())
 
 
 def test_gemm_split_k_alternating_arrival_words(K):
