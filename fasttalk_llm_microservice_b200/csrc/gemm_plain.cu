@@ -251,8 +251,15 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         }
     }
     tc_fence_before();
+    __syncthreads();                                      // the columns have been read; this CTA's share lies in its shared memory
+    if (warp == 1) {
+        // Before the cluster's barrier: a CTA that waits for the others holds no columns.  With them it could keep one of another
+        // stream's kernel from its columns, and that one a CTA of this cluster on another SM.
+        tc_fence_after();
+        tmem_dealloc(tmem, COLS);
+    }
     if (S > 1) {
-        cluster_sync_all();                               // every share of the row tile lies in its CTA's shared memory
+        cluster_sync_all();                               // every share of the row tile is there
         if (warp >= 2) {
             const int f = threadIdx.x - 64;
             const uint32_t at = smem_u32(smem) + (uint32_t)f * 4;
@@ -267,12 +274,6 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             }
         }
         cluster_sync_all();                               // nobody leaves while its tile is being read
-    } else {
-        __syncthreads();
-    }
-    if (warp == 1) {
-        tc_fence_after();
-        tmem_dealloc(tmem, COLS);
     }
 }
 
@@ -402,7 +403,9 @@ int launch_gemm_plain(const void* w, const void* hi, const void* lo, float* out,
     if (stages > PL_MAX_STAGES) stages = PL_MAX_STAGES;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    fill(cfg, attr, dim3(2 * (units < clusters ? units : clusters)), PL_THREADS, (size_t)stages * stage + 1024, pdl, stream);
+    // the whole ring's memory, also where the stages take less: a pair's CTA holds all columns while it waits for its partner, so no
+    // other kernel with columns of its own may have room beside it
+    fill(cfg, attr, dim3(2 * (units < clusters ? units : clusters)), PL_THREADS, PL_RING + 1024, pdl, stream);
     FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_plain_pair_kernel, mw, mh, ml, out, n_out, T, K / PL_BK, stages, bn));
     return 0;
 }

@@ -583,6 +583,29 @@ def test_gemm_plain_fp32(K, T, n_out, Kd):
     assert bool((guard[T] == 7.0).all())
 
 
+def test_gemm_plain_on_two_streams(K):
+    """Launches of few tokens (K shared by clusters of four CTAs, three chunks each) beside launches of CTA pairs with 32-token
+    tiles, on two streams at once: both kinds hold tensor-memory columns, and neither may wait for the other's."""
+    from fasttalk_llm_microservice_b200 import native as N
+    g = torch.Generator(device=DEV).manual_seed(5)
+    calls = []
+    for T, n_out, Kd in [(16, 2048, 768), (16, 4096, 384), (160, 1024, 512), (129, 2048, 384)]:
+        w = (torch.randn(n_out, Kd, device=DEV, generator=g) * 0.05).bfloat16()
+        x, x_lo = K.split_hi_lo(torch.randn(T, Kd, device=DEV, generator=g))
+        calls.append((w, x, x_lo, n_out, T, Kd, torch.empty(T, n_out, device=DEV)))
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for i in range(200):
+        for s, st in enumerate(streams):
+            w, x, x_lo, n_out, T, Kd, out = calls[2 * s + i % 2]
+            N.check(N.load().ft_gemm_bf16(N.ptr(w), N.ptr(x), N.ptr(x_lo), N.ptr(out), 0, n_out, T, Kd, 1, 0, st.cuda_stream), "ft_gemm_bf16")
+    torch.cuda.synchronize()
+    for w, x, x_lo, n_out, T, Kd, out in calls:
+        xs = x.double() + x_lo.double()
+        # (bound as above)
+        assert bool(((out.double() - xs @ w.double().T).abs() <= (xs.abs() @ w.double().abs().T) * (4.0 * Kd ** 0.5 * 2.0 ** -24) + 1e-30).all())
+
+
 def _draw_point(seed):
     """The 24-bit point of [0, 1) that a row's seed stands for (splitmix64)."""
     m = (1 << 64) - 1
