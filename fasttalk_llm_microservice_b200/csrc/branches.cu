@@ -1036,7 +1036,8 @@ __global__ void __launch_bounds__(256) space_conv_kernel(SpaceArgs a, int T) {
         for (int i = 0; i < TB; ++i) {
             float acc = bias;
 #pragma unroll
-            for (int j = 3; j >= 0; --j) acc = fmaf(w[j], v[i + j], acc);      // the current token's tap first, as below
+            for (int j = 3; j >= 0; --j)                 // the current token's tap first, as below; rows out of reach are left out:
+                if (j >= 4 - K) acc = fmaf(w[j], v[i + j], acc);      // a zero tap would make a NaN of an infinite one
             put(t0 + i, acc);
         }
         return;

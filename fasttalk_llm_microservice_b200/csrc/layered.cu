@@ -776,7 +776,8 @@ delta_prep_kernel(DeltaArgs a, int T) {
             for (int i = 0; i < TB; ++i) {
                 float s = 0.f;
 #pragma unroll
-                for (int x = 0; x < 4; ++x) s = fmaf(w[x], v[i + x], s);
+                for (int x = 0; x < 4; ++x)
+                    if (x >= 4 - taps) s = fmaf(w[x], v[i + x], s);      // (a row out of reach may hold an infinity: no zero tap)
                 y[i] = s / (1.f + expf(-s));
             }
         } else {

@@ -85,7 +85,8 @@ __global__ void __launch_bounds__(256) canon_kernel(CanonArgs a, int T) {
         for (int i = 0; i < TB; ++i) {
             float acc = 0.f;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) acc = fmaf(w[k], v[i + k], acc);
+            for (int k = 0; k < 4; ++k)
+                if (k >= 4 - taps) acc = fmaf(w[k], v[i + k], acc);      // (a row out of reach may hold an infinity: no zero tap)
             put(t0 + i, v[i + 3] + acc);
         }
         return;

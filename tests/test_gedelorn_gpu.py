@@ -570,3 +570,28 @@ def test_decay_rule_single_tokens(heads, qk_heads, dim, vd, pad):
         # 24-bit sums of dim terms
         assert rel(o.cpu().double().numpy(), ref_o.reshape(T, -1).numpy()) < 2e-6
         assert rel(dst.cpu().double().numpy(), ref_state.numpy()) < 1e-6
+
+
+def test_short_taps_do_not_reach_an_infinite_row_further_back():
+    """A convolution of two taps in a step of more than 64 tokens: state coordinates to read out with that overflow at one token
+    spoil that token and the next, no more."""
+    m = space(heads=4, vdim=8, state=12, groups=1, norm_groups=1, conv=2)
+    spec, w = make([layer(m)], seed=8)
+    w["embed"][:, 0] = 0.0
+    w["embed"][5] = 0.0
+    w["embed"][5, 0] = 1.0
+    inner, n = 32, 12
+    w["l0.mix.in"][:, 0] = 0.0
+    w["l0.mix.in"][2 * inner + n:2 * inner + 2 * n, 0] = 3e38
+    toks = [t if t != 5 else 6 for t in tokens_of(spec, 90, 2)]
+    toks[42] = 5
+    with torch.no_grad():
+        ref = O.forward(spec.config(), w, toks, dtype=torch.float32).numpy()
+    clean = [i for i in range(90) if i not in (42, 43)]
+    assert np.isfinite(ref[clean]).all() and not np.isfinite(ref[42]).all()
+    eng = engine(spec, w)
+    try:
+        got = eng.feed([("s", toks, list(range(90)))])
+        assert rel(got[clean], ref[clean]) < TOL
+    finally:
+        eng.close()

@@ -441,3 +441,30 @@ def test_delta_rule_sizes(shape):
         assert rel(feed_cut(eng, "one", toks, [93]), ref) < TOL
     finally:
         eng.close()
+
+
+def pulse(spec, w, at, name, value):
+    """Token `at` alone has a number in coordinate 0 of its embedding, and of the projections only `name` reads it, `value` times."""
+    w["embed"][:, 0] = 0.0
+    w["embed"][at] = 0.0
+    w["embed"][at, 0] = 1.0
+    for n, t in w.items():
+        if n.startswith("l0.") and t.dim() == 2 and t.shape[1] == spec.width:
+            t[:, 0] = value if n in name else 0.0
+
+
+def test_short_taps_do_not_reach_an_infinite_query_further_back():
+    """Convolutions of two taps in steps of more than 64 tokens: the query that overflows spoils its own token and the next, no more."""
+    spec, w = make([delta(heads=2, kv_heads=2, dim=32, vdim=16, conv=2)], seed=8)
+    pulse(spec, w, 5, ["l0.mix.q"], 3e38)
+    toks = [t if t != 5 else 6 for t in tokens_of(spec, 90, 2)]
+    toks[42] = 5
+    ref = oracle_logits(spec, w, toks)
+    clean = [i for i in range(90) if i not in (42, 43)]
+    assert np.isfinite(ref[clean]).all() and not np.isfinite(ref[42]).all()
+    eng = engine(spec, w, exact_f32=True)
+    try:
+        got = feed_cut(eng, "s", toks, [90])
+        assert rel(got[clean], ref[clean]) < TOL
+    finally:
+        eng.close()

@@ -516,3 +516,35 @@ def test_served_through_the_handler(tmp_path, monkeypatch):
         h.close()
         runner.shutdown()
         runner.engine.close()
+
+
+def test_short_taps_do_not_reach_an_infinite_row_further_back():
+    """Input convolutions of two taps in a step of more than 256 tokens (where they run apart from the post norms): a stream
+    coordinate that overflows between mixer and feed-forward spoils its own token and the next, no more."""
+    spec, w = make([layer(attention(heads=2, kv_heads=2, dim=8, vdim=8, size=1, keep_first=0, v_mix=False), dense())], seed=8, taps=2, embed_scale=1.0)
+    # coordinate 0: large at token 5, read by nothing; coordinate 1: what token 5 alone puts into value 0, which alone reaches coordinate 0
+    w["embed"][:, :2] = 0.0
+    w["embed"][5, 0], w["embed"][5, 1] = 3.3e38, 2.0
+    for n in ("q", "k", "v"):
+        w[f"l0.mix.{n}"][:, :2] = 0.0
+    w["l0.mix.v"][0] = 0.0
+    w["l0.mix.v"][0, 1], w["l0.mix.v.b"][0] = 1.0, 0.0
+    w["l0.mix.o"][0] = 0.0
+    w["l0.mix.o"][0, 0], w["l0.mix.o.b"][0] = 8.0, 0.0
+    w["l0.canon1"][:2] = 0.0
+    w["l0.norm1"][0] = 3e38
+    for n in ("gate", "up"):
+        w[f"l0.mlp.{n}"][:, 0] = 0.0
+    w["l0.mlp.down"][0] = 0.0
+    toks = [t if t != 5 else 6 for t in tokens_of(spec, 300, 2)]
+    toks[42] = 5
+    with torch.no_grad():
+        ref = O.forward(spec.config(), w, toks, dtype=torch.float32).numpy()
+    clean = [i for i in range(300) if i not in (42, 43)]
+    assert np.isfinite(ref[clean]).all() and not np.isfinite(ref[42]).all()
+    eng = engine(spec, w)
+    try:
+        got = eng.feed([("s", toks, list(range(300)))])
+        assert rel(got[clean], ref[clean]) < TOL
+    finally:
+        eng.close()
