@@ -836,7 +836,8 @@ delta_prep_kernel(DeltaArgs a, int T) {
                 const int d = threadIdx.x + 128 * x;
                 if (d < a.dim) { dst[d] = q[x][i] * sq; dst[qk + d] = k[x][i] * sk; }
             }
-            if (threadIdx.x == 0) a.kq[(size_t)(t0 + i) * a.kvh + g] = s[2] * sq * sk;
+            // a row whose squares overflow is scaled to zeros, and so is its product, which may have overflowed as well
+            if (threadIdx.x == 0) a.kq[(size_t)(t0 + i) * a.kvh + g] = sq > 0.f && sk > 0.f ? s[2] * sq * sk : 0.f;
         }
 }
 

@@ -468,3 +468,22 @@ def test_short_taps_do_not_reach_an_infinite_query_further_back():
         assert rel(got[clean], ref[clean]) < TOL
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("q,k", [(1e20, 1e20), (1e12, 1e30), (1e30, 1.0)])
+def test_rows_whose_squares_overflow_count_as_zeros(q, k):
+    """The norm of such a row has no value in 32 bits and its factor is zero; its product with the other row is zero, too."""
+    spec, w = make([delta(heads=2, kv_heads=2, dim=32, vdim=16, conv=1)], seed=8)
+    w["l0.mix.q.conv"][:] = w["l0.mix.k.conv"][:] = 1.0
+    pulse(spec, w, 5, [], 0.0)
+    w["l0.mix.q"][:, 0], w["l0.mix.k"][:, 0] = q, k
+    toks = [t if t != 5 else 6 for t in tokens_of(spec, 80, 2)]
+    toks[33] = 5
+    ref = oracle_logits(spec, w, toks)
+    assert np.isfinite(ref).all()
+    eng = engine(spec, w, exact_f32=True)
+    try:
+        for n, cuts in (("whole", [80]), ("single", [1])):
+            assert rel(feed_cut(eng, n, toks, cuts), ref) < TOL, n
+    finally:
+        eng.close()
