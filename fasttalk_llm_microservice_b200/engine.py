@@ -46,6 +46,20 @@ class EngineLimits:
     debug_logit_rows: int = 0
 
 
+def _flat_tokens(rows: Sequence[Sequence[int]]) -> np.ndarray:
+    """All rows' tokens in one int32 array.  Lists of integers take the short way (several times faster than numpy on Python
+    integers); everything else is numpy's, what it takes and what it refuses."""
+    flat = array("i")
+    try:
+        for t in rows:
+            flat.fromlist(t)
+    except (TypeError, OverflowError):                 # not a list, or not one of small integers
+        flat = None
+    if flat:
+        return np.frombuffer(flat, dtype=np.int32)
+    return np.ascontiguousarray(np.concatenate([np.asarray(t, dtype=np.int32) for t in rows]))
+
+
 class Engine:
     def __init__(self, spec: ModelSpec, weights: Dict[str, torch.Tensor], limits: Optional[EngineLimits] = None,
                  eos_ids: Sequence[int] = LLAMA3_EOS, device: Optional[torch.device] = None,
@@ -243,13 +257,7 @@ class Engine:
         logits are wanted).  All entries run as one batch; returns float32 [wanted, vocab] in entry order."""
         keys = np.array([session_key(s) for s, _, _ in entries], dtype=np.uint64)
         counts = np.array([len(t) for _, t, _ in entries], dtype=np.int32)
-        flat = array("i")
-        for _, t, _ in entries:
-            try:
-                flat.fromlist(t)                       # (several times faster than numpy on a list of Python integers)
-            except TypeError:                          # not a list, or not one of integers
-                flat.frombytes(np.ascontiguousarray(t, dtype=np.int32).tobytes())
-        toks = np.frombuffer(flat, dtype=np.int32) if len(flat) else np.empty(0, dtype=np.int32)
+        toks = _flat_tokens([t for _, t, _ in entries])
         want, off = [], 0
         for _, t, wn in entries:
             want += [off + int(i) for i in wn]

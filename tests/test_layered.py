@@ -5,6 +5,7 @@ import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 import torch
 
@@ -100,3 +101,23 @@ def test_trace_runner_is_an_executable_with_help():
     assert os.access(path, os.X_OK)
     r = subprocess.run([sys.executable, path, "--help"], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and "--max-tokens" in r.stdout
+
+
+@pytest.mark.parametrize("rows", [
+    [[1, 2, 3]], [[5], [6], [7, 8]], [[], [4]], [[]], [[True, 2]], [[np.int64(9), 4], [3]], [(1, 2), [3]], [np.array([1, 2], dtype=np.int64), [3]],
+    [torch.tensor([4, 5])], [[1.0, 2.0], [3]], [[1, 2, 2.0]], [[-1, 2**31 - 1]], [[np.int64(2**40)]],
+    [], [[2**31]], [[1, 2], [[3, 4]]], [["a"]], [[None]], [3],
+], ids=str)
+def test_fed_tokens_are_taken_and_refused_as_numpy_does(rows):
+    from fasttalk_llm_microservice_b200.engine import _flat_tokens
+
+    def plain():
+        return np.ascontiguousarray(np.concatenate([np.asarray(t, dtype=np.int32) for t in rows]))
+    try:
+        ref = plain()
+    except Exception as e:
+        with pytest.raises(type(e)):
+            _flat_tokens(rows)
+        return
+    got = _flat_tokens(rows)
+    assert got.dtype == np.int32 and got.shape == ref.shape and got.flags.c_contiguous and (got == ref).all()
