@@ -548,3 +548,33 @@ def test_short_taps_do_not_reach_an_infinite_row_further_back():
         assert rel(got[clean], ref[clean]) < TOL
     finally:
         eng.close()
+
+
+# one decay per head: lanes of 4, 8 and 16 channels with and without padding, 16-byte and 4-byte copies, column blocks with a
+# remainder, single columns; with 20 heads of 128 columns 160 blocks of 128 threads, otherwise 64 threads
+@pytest.mark.parametrize("shape", [dict(heads=1, kv_heads=1, dim=64, vdim=32), dict(heads=2, kv_heads=1, dim=68, vdim=36), dict(heads=20, kv_heads=10, dim=128, vdim=128),
+                                   dict(heads=3, kv_heads=3, dim=128, vdim=129), dict(heads=2, kv_heads=2, dim=130, vdim=5), dict(heads=2, kv_heads=1, dim=256, vdim=1),
+                                   dict(heads=10, kv_heads=5, dim=256, vdim=256), dict(heads=20, kv_heads=10, dim=8, vdim=256)])
+def test_delta_rule_sizes_with_a_decay_per_head(shape):
+    spec, w = make([layer(delta(conv=4, **shape))], seed=6)
+    eng = engine(spec, w)
+    try:
+        toks = tokens_of(spec, 93, 2)
+        ref = oracle_logits(spec, w, toks)
+        assert rel(feed_cut(eng, "cut", toks, [75, 1, 3, 1]), ref) < TOL
+        eng.close_session("cut")
+        assert rel(feed_cut(eng, "one", toks, [93]), ref) < TOL
+        # requests of unequal length in one step of more than 64 rows: blocks of eight tokens that straddle two of them, one shorter
+        # than the taps, one that goes on from its state; then a token of each
+        parts = {"one": toks[:19], "a": toks[:33], "b": toks[:2], "c": toks[:45]}
+        whole = {n: (toks + t if n == "one" else t) for n, t in parts.items()}
+        got = eng.feed([(n, t, list(range(len(t)))) for n, t in parts.items()])
+        after = eng.feed([(n, [7], [0]) for n in parts])
+        at = 0
+        for i, (n, t) in enumerate(parts.items()):
+            full = oracle_logits(spec, w, whole[n] + [7])
+            assert rel(got[at:at + len(t)], full[-1 - len(t):-1]) < TOL, n
+            assert rel(after[i:i + 1], full[-1:]) < TOL, n
+            at += len(t)
+    finally:
+        eng.close()
