@@ -217,6 +217,18 @@ __device__ __forceinline__ uint32_t cluster_id_x() {
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same shared-memory variable in another CTA of the cluster.
+__device__ __forceinline__ uint32_t peer_addr(const void* p, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ unsigned peer_ld(const unsigned* p, int rank) {
+    unsigned v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_addr(p, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ float peer_ld(const float* p, int rank) { return __uint_as_float(peer_ld(reinterpret_cast<const unsigned*>(p), rank)); }
 // Tile load issued by EITHER CTA of the pair into its own shared memory; the bytes are counted on
 // the LEADER's mbarrier (same offset in the even CTA).
 __device__ __forceinline__ void tma_tile_2d_pair(void* dst_smem, const CUtensorMap* map, int c0, int c1,

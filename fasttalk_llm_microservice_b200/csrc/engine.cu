@@ -592,7 +592,7 @@ static int dense(Engine* e, const float* A, const void* hi, const void* lo, cons
             hi = L.pl_hi;
             lo = L.pl_lo;
         }
-        FT_TRY(launch_gemm_plain(W, hi, lo, C, N, T, K, false, e->stream));
+        FT_TRY(launch_gemm_plain(W, hi, lo, C, N, T, K, e->stream));
         e->st.kernel_launches++;
         if (softcap > 0.f) {
             FT_TRY(launch_softcap(C, (size_t)T * N, softcap, e->stream));

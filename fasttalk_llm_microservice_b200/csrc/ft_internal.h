@@ -32,6 +32,7 @@ struct PerDeviceFlag {
 };
 
 // ---- gemm.cu
+int device_sms();                                     // of the CURRENT device
 int make_tmap_bf16_k64(CUtensorMap* map, const void* base, int rows, int K, int box_rows);
 int make_tmap_f16_3d(CUtensorMap* map, const void* base, int d0, int d1, int d2, int b0, int b1, int b2);
 int gemm_pick_bn(int T, bool hilo);
@@ -46,8 +47,7 @@ int launch_gemm(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap*
                 const CUtensorMap* mx_half = nullptr, const CUtensorMap* mx_lo_half = nullptr);
 
 // ---- gemm_plain.cu: out[t][n] = sum_k (hi + lo)[t][k] W[n][k], fp32 results without a fused layer step
-bool gemm_plain_ok(int n_out, int T, int K);
-int launch_gemm_plain(const void* w, const void* hi, const void* lo, float* out, int n_out, int T, int K, bool pdl, cudaStream_t stream);
+int launch_gemm_plain(const void* w, const void* hi, const void* lo, float* out, int n_out, int T, int K, cudaStream_t stream);
 
 // ---- elementwise.cu
 int launch_add_rmsnorm(float* resid, const float* partials, int n_splits, size_t split_stride,

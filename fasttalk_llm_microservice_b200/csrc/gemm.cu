@@ -1033,7 +1033,7 @@ int make_tmap_f16_3d(CUtensorMap* map, const void* base, int d0, int d1, int d2,
     return 0;
 }
 
-static int device_sms() {          // of the CURRENT device
+int device_sms() {
     static int sms[kMaxDevices] = {};
     const int slot = current_device_slot();
     if (!sms[slot]) {
@@ -1385,7 +1385,7 @@ extern "C" int ft_gemm_fused(const void* w, const void* x, const void* x_lo, int
     if (n_splits <= 0)
         n_splits = epi->mode == FT_EPI_PARTIAL || staged ? gemm_pick_splits(n_out, T, K, sms, hilo) : 1;
     if (hilo && epi->mode == FT_EPI_PARTIAL && n_splits == 1)      // one unsplit fp32 result: the kernels made for it
-        return launch_gemm_plain(w, x, x_lo, reinterpret_cast<float*>(epi->out), n_out, T, K, false, static_cast<cudaStream_t>(stream));
+        return launch_gemm_plain(w, x, x_lo, reinterpret_cast<float*>(epi->out), n_out, T, K, static_cast<cudaStream_t>(stream));
     CUtensorMap mw, mx, mxl;
     if (int r = make_tmap_bf16_k64(&mw, w, n_out, K, GEMM_BM)) return r;
     if (int r = make_tmap_bf16_k64(&mx, x, T, K, bn)) return r;

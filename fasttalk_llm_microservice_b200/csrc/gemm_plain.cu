@@ -58,13 +58,11 @@ gemm_plain_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     cluster_sync_all();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    pdl_launch_dependents();
     if (warp == 0) {
         if (elect_one()) {
             // weights are read again by every token tile; a launch of one token tile streams them
             const bool multi = T > bn;
             const uint64_t pol_w = multi ? policy_evict_last() : policy_evict_first(), pol_x = multi ? policy_evict_first() : policy_evict_last();
-            pdl_wait();
             int it = 0;
             for (int u = cl; u < units; u += n_cl) {
                 const int row0 = (2 * (u % row_pairs) + rank) * PL_BM, tok0 = u / row_pairs * bn + rank * (bn / 2);
@@ -107,7 +105,6 @@ gemm_plain_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             }
         }
     } else if (warp >= 2) {
-        pdl_wait();
         const int quarter = warp & 3, half = (warp - 2) >> 2;
         uint32_t use = 0;
         for (int u = cl; u < units; u += n_cl, ++use) {
@@ -148,14 +145,6 @@ gemm_plain_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 // ------------------------------------------------------------------ few tokens
 constexpr int PF_THREADS = 192;                           // TMA warp, MMA warp, four epilogue warps
 
-__device__ __forceinline__ float peer_f32(uint32_t addr, int rank) {
-    uint32_t r;
-    float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(r) : "memory");
-    return v;
-}
-
 // grid (row tiles, S), clusters of (1, S): CTA (x, s) takes the s-th share of K of weight rows 128 x .. 128 x + 127.
 template <int BN>
 __global__ void __launch_bounds__(PF_THREADS)
@@ -189,24 +178,15 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    pdl_launch_dependents();
     if (warp == 0) {
         if (elect_one()) {
             const uint64_t pol_w = policy_evict_first(), pol_x = policy_evict_last();
-            const int pre = min(n_iter, stages);
-            for (int i = 0; i < pre; ++i) {               // the weights do not depend on the kernel before
-                mbar_expect_tx(&full[i], STAGE);
-                tma_tile_2d(smem + (size_t)i * STAGE, &map_w, (kc0 + i) * PL_BK, row0, &full[i], pol_w);
-            }
-            pdl_wait();
             for (int i = 0; i < n_iter; ++i) {
                 const int s = i % stages;
                 uint8_t* st = smem + (size_t)s * STAGE;
-                if (i >= pre) {
-                    mbar_wait(&empty[s], ((i / stages) - 1) & 1);
-                    mbar_expect_tx(&full[s], STAGE);
-                    tma_tile_2d(st, &map_w, (kc0 + i) * PL_BK, row0, &full[s], pol_w);
-                }
+                if (i >= stages) mbar_wait(&empty[s], ((i / stages) - 1) & 1);
+                mbar_expect_tx(&full[s], STAGE);
+                tma_tile_2d(st, &map_w, (kc0 + i) * PL_BK, row0, &full[s], pol_w);
                 tma_tile_2d(st + PL_A, &map_hi, (kc0 + i) * PL_BK, 0, &full[s], pol_x);
                 tma_tile_2d(st + PL_A + PLANE, &map_lo, (kc0 + i) * PL_BK, 0, &full[s], pol_x);
             }
@@ -228,7 +208,6 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             umma_commit(&acc_full);
         }
     } else {
-        pdl_wait();                                       // out may still be read by the kernel before
         mbar_wait(&acc_full, 0);
         tc_fence_after();
         const int quarter = warp & 3, f = quarter * 32 + lane;
@@ -262,11 +241,11 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         cluster_sync_all();                               // every share of the row tile is there
         if (warp >= 2) {
             const int f = threadIdx.x - 64;
-            const uint32_t at = smem_u32(smem) + (uint32_t)f * 4;
+            const float* mine = reinterpret_cast<const float*>(smem) + f;      // (the same place in every CTA)
             for (int t = rank; t < T; t += S) {
                 float v[8];
 #pragma unroll
-                for (int p = 0; p < 8; ++p) v[p] = p < S ? peer_f32(at + (uint32_t)t * (PL_BM * 4), p) : 0.f;
+                for (int p = 0; p < 8; ++p) v[p] = p < S ? peer_ld(mine + t * PL_BM, p) : 0.f;
                 float sum = v[0];
 #pragma unroll
                 for (int p = 1; p < 8; ++p) sum += v[p];
@@ -277,43 +256,20 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     }
 }
 
-int sm_count() {
-    static int sms[kMaxDevices] = {};
-    int& n = sms[current_device_slot()];
-    if (!n) {
-        int dev = 0, v = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
-        n = v;
-    }
-    return n;
-}
-
 constexpr int PL_RING = 222 * 1024;                       // shared memory for the stages (+ 1 KB to align them)
 
-void fill(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, dim3 grid, int threads, size_t smem, bool pdl, cudaStream_t stream) {
-    cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-}
-
 template <int BN>
-int launch_few(const CUtensorMap& mw, const CUtensorMap& mh, const CUtensorMap& ml, float* out, int n_out, int T, int K, bool pdl, cudaStream_t stream) {
+int launch_few(const CUtensorMap& mw, const CUtensorMap& mh, const CUtensorMap& ml, float* out, int n_out, int T, int K, cudaStream_t stream) {
     constexpr int STAGE = PL_A + 2 * BN * PL_BK * 2;
     const int kc = K / PL_BK, tiles = n_out / PL_BM;
     // CTAs per row tile: as many as leave each three chunks and the grid one CTA per SM, two from four CTAs per tile on (weights of
     // 10752 x 2048 and 64 tokens: 12.8 us with S = 1, 16.1 with 2; 8576 x 2048 and 16 tokens: 8.5 us with S = 2, 7.9 with 4)
     int S = 8;
-    while (S > 1 && (kc / S < 3 || tiles * S > (S >= 4 ? 2 : 1) * sm_count())) S /= 2;
+    while (S > 1 && (kc / S < 3 || tiles * S > (S >= 4 ? 2 : 1) * device_sms())) S /= 2;
     // A deep ring where a CTA has an SM for itself, half of one otherwise.  Clusters of four or eight always leave room for a second CTA:
     // they must lie within one GPC, and with one CTA per SM sixteen clusters of eight do not all find one (2048 x 4096, 16 tokens:
     // 12.9 us with 160 KB per CTA, more than with half the CTAs).
-    const int budget = tiles * S <= sm_count() && S <= 2 ? 200 * 1024 : 104 * 1024;
+    const int budget = tiles * S <= device_sms() && S <= 2 ? 200 * 1024 : 104 * 1024;
     int stages = budget / STAGE;
     if (stages > PL_MAX_STAGES) stages = PL_MAX_STAGES;
     if (stages > (kc + S - 1) / S) stages = (kc + S - 1) / S;
@@ -327,12 +283,16 @@ int launch_few(const CUtensorMap& mw, const CUtensorMap& mh, const CUtensorMap& 
         FT_CHECK_CUDA(cudaFuncSetAttribute(gemm_plain_few_kernel<BN>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         attr_set.mark();
     }
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[2];
-    fill(cfg, attr, dim3(tiles, S), PF_THREADS, smem, pdl, stream);
-    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
-    attr[cfg.numAttrs].val.clusterDim.x = 1; attr[cfg.numAttrs].val.clusterDim.y = S; attr[cfg.numAttrs].val.clusterDim.z = 1;
-    ++cfg.numAttrs;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles, S);
+    cfg.blockDim = dim3(PF_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = S; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
     FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_plain_few_kernel<BN>, mw, mh, ml, out, n_out, T, kc, stages));
     return 0;
 }
@@ -344,7 +304,7 @@ int plain_clusters() {
     if (!n) {
         FT_CHECK_CUDA(cudaFuncSetAttribute(gemm_plain_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PL_RING + 1024));
         cudaLaunchConfig_t q = {};
-        q.gridDim = dim3(sm_count() & ~1);
+        q.gridDim = dim3(device_sms() & ~1);
         q.blockDim = dim3(PL_THREADS);
         q.dynamicSmemBytes = PL_RING + 1024;
         cudaLaunchAttribute qa[1];
@@ -353,7 +313,7 @@ int plain_clusters() {
         q.attrs = qa;
         q.numAttrs = 1;
         int v = 0;
-        if (cudaOccupancyMaxActiveClusters(&v, gemm_plain_pair_kernel, &q) != cudaSuccess || v <= 0) v = sm_count() / 2;
+        if (cudaOccupancyMaxActiveClusters(&v, gemm_plain_pair_kernel, &q) != cudaSuccess || v <= 0) v = device_sms() / 2;
         n = v;
     }
     return n;
@@ -376,10 +336,9 @@ int plain_token_tile(int row_pairs, int T, int clusters) {
 
 }  // namespace
 
-bool gemm_plain_ok(int n_out, int T, int K) { return n_out >= PL_BM && n_out % PL_BM == 0 && K >= PL_BK && K % PL_BK == 0 && T >= 1; }
-
-int launch_gemm_plain(const void* w, const void* hi, const void* lo, float* out, int n_out, int T, int K, bool pdl, cudaStream_t stream) {
-    FT_REQUIRE(w && hi && lo && out && gemm_plain_ok(n_out, T, K), "gemm (plain): bad sizes or operands (n_out %d, T %d, K %d)", n_out, T, K);
+int launch_gemm_plain(const void* w, const void* hi, const void* lo, float* out, int n_out, int T, int K, cudaStream_t stream) {
+    FT_REQUIRE(w && hi && lo && out && n_out >= PL_BM && n_out % PL_BM == 0 && K >= PL_BK && K % PL_BK == 0 && T >= 1,
+               "gemm (plain): bad sizes or operands (n_out %d, T %d, K %d)", n_out, T, K);
     CUtensorMap mw, mh, ml;
     if (int r = make_tmap_bf16_k64(&mw, w, n_out, K, PL_BM)) return r;
     if (T <= 128) {
@@ -387,10 +346,10 @@ int launch_gemm_plain(const void* w, const void* hi, const void* lo, float* out,
         if (int r = make_tmap_bf16_k64(&mh, hi, T, K, bn)) return r;
         if (int r = make_tmap_bf16_k64(&ml, lo, T, K, bn)) return r;
         switch (bn) {
-            case 16: return launch_few<16>(mw, mh, ml, out, n_out, T, K, pdl, stream);
-            case 32: return launch_few<32>(mw, mh, ml, out, n_out, T, K, pdl, stream);
-            case 64: return launch_few<64>(mw, mh, ml, out, n_out, T, K, pdl, stream);
-            default: return launch_few<128>(mw, mh, ml, out, n_out, T, K, pdl, stream);
+            case 16: return launch_few<16>(mw, mh, ml, out, n_out, T, K, stream);
+            case 32: return launch_few<32>(mw, mh, ml, out, n_out, T, K, stream);
+            case 64: return launch_few<64>(mw, mh, ml, out, n_out, T, K, stream);
+            default: return launch_few<128>(mw, mh, ml, out, n_out, T, K, stream);
         }
     }
     const int clusters = plain_clusters();
@@ -401,12 +360,10 @@ int launch_gemm_plain(const void* w, const void* hi, const void* lo, float* out,
     const int units = row_pairs * ((T + bn - 1) / bn), stage = PL_A + bn * PL_BK * 2;
     int stages = PL_RING / stage;
     if (stages > PL_MAX_STAGES) stages = PL_MAX_STAGES;
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[1];
     // the whole ring's memory, also where the stages take less: a pair's CTA holds all columns while it waits for its partner, so no
     // other kernel with columns of its own may have room beside it
-    fill(cfg, attr, dim3(2 * (units < clusters ? units : clusters)), PL_THREADS, PL_RING + 1024, pdl, stream);
-    FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_plain_pair_kernel, mw, mh, ml, out, n_out, T, K / PL_BK, stages, bn));
+    gemm_plain_pair_kernel<<<2 * (units < clusters ? units : clusters), PL_THREADS, PL_RING + 1024, stream>>>(mw, mh, ml, out, n_out, T, K / PL_BK, stages, bn);
+    FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 

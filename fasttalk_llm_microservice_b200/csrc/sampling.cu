@@ -43,17 +43,6 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long x) {
     return x ^ (x >> 31);
 }
 
-// The same shared-memory variable in another CTA of the cluster.
-__device__ __forceinline__ uint32_t peer_addr(const void* p, int rank) {
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ unsigned peer_ld(const unsigned* p, int rank) {
-    unsigned v;
-    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_addr(p, rank)) : "memory");
-    return v;
-}
 __device__ __forceinline__ void peer_st(int* p, int rank, int v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer_addr(p, rank)), "r"(v) : "memory");
 }
