@@ -1,7 +1,9 @@
 // Kernels of the layered model family: decoders described layer by layer (ft_layer_desc), whose sizes are all run-time
 // values.  The residual stream, the normed layer input, every projection output, attention scores and weights, router
 // scores and the recurrent state are fp32; weights are bf16 and are multiplied as the fp32 numbers they are, with fp32
-// accumulation in a fixed order per output element — a row's result does not depend on which other rows share its launch.
+// accumulation.  The order of each kernel's sums is fixed per output element; which kernel runs depends on the sizes of the step
+// (few rows, tiles, the tensor cores; there K is cut among CTAs for up to 128 rows, and a scalar-decay step of single tokens has a
+// kernel of its own), so the rows that share a step can change a result by rounding, by nothing else.
 //
 //   linear              C[r, n] = sum_k A[row(r), k] * W[p][n, k]: plain, batched over heads (column offsets per problem)
 //                       or grouped over experts (row segments per problem, rows gathered through an index list), with
@@ -13,7 +15,7 @@
 //                       latent space (q W_uk), scores, softmax and the weighted sum run over the cached latents, values
 //                       are expanded afterwards (W_uv): only the latent is ever stored
 //   channel delta       short causal convolutions + SiLU + unit norms + per-channel decays, then the gated delta rule
-//                       token by token with one thread per state column, state and convolution tails in per-session slots
+//                       token by token with the state in registers, state and convolution tails in per-session slots
 //   router              softmax over all experts, group-limited top-k, counting sort of (token, choice) pairs by expert
 #include "common.cuh"
 #include "ft_internal.h"
@@ -708,8 +710,9 @@ int launch_latent_attn(const LatentArgs& a, int T, cudaStream_t stream) {
 // tail of raw inputs; zeros before position 0), unit norms of q and k per head (q also times dim^-1/2), the product k q of a head's
 // normed rows, the decay exp(-exp(A_log_h) * softplus(a + dt_bias)) per head and key channel (or per head), beta = sigmoid.
 // qkv out: [T][channels] with channels = 2 * kvh * dim + heads * vdim in the order q | k | v.
-// CTA (tokens x .. + TB - 1, group y): group y < kvh is a q and a k head, then come 128 value channels each, then decays and betas.  A thread keeps its channels over the TB tokens, so that the rows the taps share come out of L1 (one CTA per
-// token, all channels after one another: 121 us for 2313 tokens of 6144 channels; now 73 us).
+// CTA (tokens x .. + TB - 1, group y): group y < kvh is a q and a k head, then come 128 value channels each, then decays and
+// betas.  A thread keeps its channels over the TB tokens, so that the rows the taps share come out of L1 (one CTA per token, all
+// channels after one another: 121 us for 2313 tokens of 6144 channels; now 73 us).
 template <int TB>
 __global__ void __launch_bounds__(128)
 delta_prep_kernel(DeltaArgs a, int T) {
@@ -1051,7 +1054,7 @@ static int launch_delta_rule_t(const DeltaArgs& a, int n_req, cudaStream_t strea
     int threads = 128;
     auto grid_of = [&](int th) { return dim3(n_req, a.heads, (a.vdim + th / DLANES * DCPT - 1) / (th / DLANES * DCPT)); };
     const dim3 wide = grid_of(128);
-    if ((long long)wide.x * wide.y * wide.z < 148) threads = 64;
+    if ((long long)wide.x * wide.y * wide.z < device_sms()) threads = 64;
     const size_t smem = (size_t)2 * DCHUNK * ((HD ? 2 : 3) * DLANES * DPT + threads / DLANES * DCPT + 4) * 4;
     if (smem > 48 * 1024)
         FT_CHECK_CUDA(cudaFuncSetAttribute(delta_rule_kernel<DPT, HD, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
