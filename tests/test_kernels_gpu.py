@@ -567,7 +567,7 @@ def test_sample_full_vocab_row(K):
 @pytest.mark.parametrize("T", [1, 16, 17, 33, 128, 129, 161, 600, 2313])
 @pytest.mark.parametrize("n_out,Kd", [(128, 64), (384, 192), (2048, 2048), (4352, 1024), (640, 8192)])
 def test_gemm_plain_fp32(K, T, n_out, Kd):
-    """Unsplit fp32 results of both planes: K shared by a cluster (up to 128 tokens) and CTA pairs with token tiles of every width,
+    """Unsplit fp32 results of both planes: K shared by a cluster (up to 128 tokens) and CTA pairs with token tiles of 32 to 192,
     odd row tile counts, ragged last tiles.  Both planes are exact inputs of the reference; what is left is the rounding of fp32
     sums of Kd products in another order, at most Kd * 2^-24 of the sum of magnitudes and in practice its square root."""
     g = torch.Generator(device=DEV).manual_seed(T * 7 + n_out)
@@ -581,6 +581,13 @@ def test_gemm_plain_fp32(K, T, n_out, Kd):
     bound = (xs.abs() @ w.double().abs().T) * (4.0 * Kd ** 0.5 * 2.0 ** -24)
     assert bool(((guard[:T].double() - ref).abs() <= bound + 1e-30).all())
     assert bool((guard[T] == 7.0).all())
+
+
+@pytest.mark.parametrize("T,n_out,Kd", [(391, 7680, 64), (586, 5632, 320), (963, 12800, 192), (1002, 12672, 64)])
+def test_gemm_plain_widest_token_tiles(K, T, n_out, Kd):
+    """Token tiles of 224 (two sizes) and 256 (two sizes, one with an odd number of row tiles), which take the fewest rounds here
+    whether 70 CTA pairs fit the device or 74: both accumulators up to all 512 columns, the shortest rings, a ragged last tile."""
+    test_gemm_plain_fp32(K, T, n_out, Kd)
 
 
 def test_gemm_plain_on_two_streams(K):
