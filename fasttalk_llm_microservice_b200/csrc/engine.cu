@@ -1467,7 +1467,9 @@ static int engine_step(Engine* e, std::unique_lock<std::mutex>& lk) {
     // sampling parameters per logit row
     float* hf = reinterpret_cast<float*>(h);
     unsigned long long* hseed = reinterpret_cast<unsigned long long*>(h + m.o_seed);
+    bool drawn = false;                              // any row that is not greedy
     auto put_sampling = [&](Request* r) {
+        drawn |= !(r->temperature <= 1e-6f);
         const int lr = r->logits_row;
         hf[m.o_temp + lr] = r->temperature;
         h[m.o_topk + lr] = r->top_k;
@@ -1482,7 +1484,7 @@ static int engine_step(Engine* e, std::unique_lock<std::mutex>& lk) {
     FT_TRY(upload_meta(e));
     FT_TRY(forward(e, b));
     if (b.n_logit_rows > 0) {
-        const float* dtemp = reinterpret_cast<const float*>(m.d + m.o_temp);
+        const float* dtemp = drawn ? reinterpret_cast<const float*>(m.d + m.o_temp) : nullptr;
         const float* dtopp = reinterpret_cast<const float*>(m.d + m.o_topp);
         const unsigned long long* dseed = reinterpret_cast<const unsigned long long*>(m.d + m.o_seed);
         FT_TRY(launch_sample(e->logits, b.n_logit_rows, c.vocab, dtemp, m.d + m.o_topk, dtopp, dseed,

@@ -32,6 +32,9 @@ struct SampleSmem {
     float val[SAMPLE_MAX_CTAS], above, target;
     int idx[SAMPLE_MAX_CTAS];
     int bin, single;
+    unsigned long long seed;                                          // the row's own settings, read while its logits are
+    int top_k;
+    float top_p;
     float warp_f[SAMPLE_WARPS];
     int warp_i[SAMPLE_WARPS];
 };
@@ -49,6 +52,23 @@ __device__ __forceinline__ void peer_st(int* p, int rank, int v) {
 __device__ __forceinline__ void peer_st(float* p, int rank, float v) { peer_st(reinterpret_cast<int*>(p), rank, __float_as_int(v)); }
 __device__ __forceinline__ void peer_st(double* p, int rank, double v) {
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(peer_addr(p, rank)), "d"(v) : "memory");
+}
+
+// The same for one CTA of C; alone it needs neither.
+template <int C, typename T>
+__device__ __forceinline__ void peer_put(T* p, int rank, T v) {
+    if (C == 1) *p = v;
+    else peer_st(p, rank, v);
+}
+template <int C>
+__device__ __forceinline__ unsigned peer_get(const unsigned* p, int rank) {
+    return C == 1 ? *p : peer_ld(p, rank);
+}
+// A barrier of all CTAs of a row; one CTA needs no more than its own.
+template <int C>
+__device__ __forceinline__ void row_sync() {
+    if (C == 1) __syncthreads();
+    else cluster_sync_all();
 }
 
 // e = exp((x - max) / T) as its bit pattern; 0 where the difference has no value (NaN logits, infinity minus infinity)
@@ -85,10 +105,11 @@ __device__ __forceinline__ int walk_down(float v, int n, float& acc, float targe
 // weight is the sum of the elements, and the target `part` of the sum of all elements with key >= min_key; otherwise the weight is
 // their number and the target `part` itself.  The bins are walked from the top in 32-bit sums, 64 at a time and then one by one,
 // whatever C is.  Every thread of the cluster calls; the result is the same for all.
-template <bool MASS>
-__device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, float part, int rank, int C, SampleSmem& sm) {
+template <bool MASS, int C>
+__device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, float part, int rank, SampleSmem& sm) {
     const int shifts[3] = {20, 9, 0}, bits[3] = {11, 11, 9};
-    const int groups = SAMPLE_GROUPS / C, w = threadIdx.x >> 5, l = threadIdx.x & 31;      // this CTA's groups of 64 bins
+    constexpr int groups = SAMPLE_GROUPS / C;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;      // this CTA's groups of 64 bins
     uint32_t prefix = 0, mask = 0;
     float above = 0.f, target = part;
     for (int lvl = 0; lvl < 3; ++lvl) {
@@ -107,7 +128,7 @@ __device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, floa
                 if (MASS && (off & 1023u)) atomicAdd(&sm.lo[b], off & 1023u);
             }
         }
-        cluster_sync_all();                          // every histogram of the cluster is complete
+        row_sync<C>();                          // every histogram of the cluster is complete
         // warp w sums groups w and w + 16 of this CTA over the cluster, two bins of each per lane
         float wt[2][2];
         unsigned ct[2][2];
@@ -119,17 +140,17 @@ __device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, floa
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const int b = (rank * groups + g) * 64 + 32 * j + l;
-                unsigned pc[SAMPLE_MAX_CTAS], ph[SAMPLE_MAX_CTAS], pl[SAMPLE_MAX_CTAS];      // all reads in flight before the first sum
+                unsigned pc[C], ph[C], pl[C];        // all reads in flight before the first sum
 #pragma unroll
-                for (int p = 0; p < SAMPLE_MAX_CTAS; ++p) {
-                    pc[p] = p < C ? peer_ld(&sm.cnt[b], p) : 0u;
-                    ph[p] = MASS && p < C ? peer_ld(&sm.hi[b], p) : 0u;
-                    pl[p] = MASS && p < C ? peer_ld(&sm.lo[b], p) : 0u;
+                for (int p = 0; p < C; ++p) {
+                    pc[p] = peer_get<C>(&sm.cnt[b], p);
+                    ph[p] = MASS ? peer_get<C>(&sm.hi[b], p) : 0u;
+                    pl[p] = MASS ? peer_get<C>(&sm.lo[b], p) : 0u;
                 }
                 unsigned c = 0;
                 unsigned long long off = 0;
 #pragma unroll
-                for (int p = 0; p < SAMPLE_MAX_CTAS; ++p) {
+                for (int p = 0; p < C; ++p) {
                     c += pc[p];
                     off += ((unsigned long long)ph[p] << 10) + pl[p];
                 }
@@ -148,11 +169,11 @@ __device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, floa
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
             if (l < C) {
-                peer_st(&sm.group[rank * groups + g], l, sum);
-                if (MASS && lvl == 0) peer_st(&sm.total[rank * groups + g], l, all);
+                peer_put<C>(&sm.group[rank * groups + g], l, sum);
+                if (MASS && lvl == 0) peer_put<C>(&sm.total[rank * groups + g], l, all);
             }
         }
-        cluster_sync_all();                          // the groups' sums are everywhere; the histograms have been read
+        row_sync<C>();                          // the groups' sums are everywhere; the histograms have been read
         if (w < groups) {
             if (MASS && lvl == 0) {
                 double z = sm.total[l];
@@ -180,14 +201,14 @@ __device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, floa
                     }
                     const unsigned c = bin < 32 ? __shfl_sync(0xffffffffu, ct[x][0], bin) : __shfl_sync(0xffffffffu, ct[x][1], bin - 32);
                     if (l < C) {
-                        peer_st(&sm.bin, l, max(in, 0) * 64 + bin);
-                        peer_st(&sm.single, l, c == 1u);
-                        peer_st(&sm.above, l, over);
-                        peer_st(&sm.target, l, target);
+                        peer_put<C>(&sm.bin, l, max(in, 0) * 64 + bin);
+                        peer_put<C>(&sm.single, l, (int)(c == 1u));
+                        peer_put<C>(&sm.above, l, over);
+                        peer_put<C>(&sm.target, l, target);
                     }
                 }
         }
-        cluster_sync_all();
+        row_sync<C>();
         prefix |= (uint32_t)sm.bin << shift;
         mask |= (uint32_t)(nb - 1) << shift;
         above = sm.above;
@@ -197,15 +218,17 @@ __device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, floa
     return prefix < min_key ? min_key : prefix;
 }
 
+// C CTAs per row (a cluster; consecutive blocks)
+template <int C>
 __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
 sample_kernel(const float* __restrict__ logits, int V, int span, int cache, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
-              const unsigned long long* __restrict__ seeds, int* __restrict__ out_tokens, int C) {
+              const unsigned long long* __restrict__ seeds, int* __restrict__ out_tokens) {
     __shared__ SampleSmem sm;
     extern __shared__ __align__(16) uint32_t keys[];
-    const int b = blockIdx.x / C, rank = blockIdx.x % C;      // clusters are runs of C consecutive blocks
+    const int b = blockIdx.x / C, rank = blockIdx.x % C;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    if (C > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     pdl_wait();
     pdl_launch_dependents();
     const int lo = min(rank * span, V), hi = min(lo + span, V);
@@ -215,6 +238,11 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
     const float temp = temperature ? temperature[b] : 0.f;
     const bool greedy = temp <= 1e-6f;
     s.cached = greedy ? 0 : min(s.n, cache);
+    if (!greedy && threadIdx.x == SAMPLE_THREADS - 1) {
+        sm.seed = seeds ? seeds[b] : 0x1234ull + b;
+        sm.top_k = top_k ? top_k[b] : 0;
+        sm.top_p = top_p ? top_p[b] : 1.f;
+    }
 
     // ---- max (+ argmax, lowest index on ties); the logits of a sampled row stay in shared memory
     float best = -INFINITY;
@@ -240,10 +268,18 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
             }
         }
     } else {
-        for (int i = threadIdx.x; i < s.n; i += SAMPLE_THREADS) {
-            const float v = x[i];
-            take(v, i);
-            if (i < s.cached) keys[i] = __float_as_uint(v);
+        for (int i = threadIdx.x; i < s.n; i += 8 * SAMPLE_THREADS) {      // eight in flight
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (i + u * SAMPLE_THREADS < s.n) v[u] = __ldcg(x + i + u * SAMPLE_THREADS);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int c = i + u * SAMPLE_THREADS;
+                if (c >= s.n) break;
+                take(v[u], c);
+                if (c < s.cached) keys[c] = __float_as_uint(v[u]);
+            }
         }
     }
 #pragma unroll
@@ -254,83 +290,105 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
     }
     if (l == 0) { sm.warp_f[w] = best; sm.warp_i[w] = best_i; }
     __syncthreads();
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // every CTA of the cluster has started
+    if (C > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // every CTA of the cluster has started
     if (threadIdx.x == 0) {
         for (int i = 1; i < SAMPLE_WARPS; ++i)
             if (sm.warp_f[i] > best || (sm.warp_f[i] == best && sm.warp_i[i] < best_i)) { best = sm.warp_f[i]; best_i = sm.warp_i[i]; }
         for (int p = 0; p < C; ++p) {
-            peer_st(&sm.val[rank], p, best);
-            peer_st(&sm.idx[rank], p, best_i);
+            peer_put<C>(&sm.val[rank], p, best);
+            peer_put<C>(&sm.idx[rank], p, best_i);
         }
     }
-    cluster_sync_all();
+    row_sync<C>();
     float maxv = sm.val[0];
-    int argmax = sm.idx[0];
-    for (int p = 1; p < C; ++p)
-        if (sm.val[p] > maxv) { maxv = sm.val[p]; argmax = sm.idx[p]; }      // shares are in index order: the first maximum wins
-    if (argmax == 0x7fffffff) argmax = 0;            // no logit above minus infinity (all of them minus infinity or NaN): an index of the row all the same
+    for (int p = 1; p < C; ++p) maxv = fmaxf(maxv, sm.val[p]);
+    auto most_likely = [&]() {                       // shares are in index order: the first maximum wins
+        int at = sm.idx[0];
+        float v = sm.val[0];
+        for (int p = 1; p < C; ++p)
+            if (sm.val[p] > v) { v = sm.val[p]; at = sm.idx[p]; }
+        return at == 0x7fffffff ? 0 : at;            // no logit above minus infinity (all of them minus infinity or NaN): an index of the row all the same
+    };
     if (greedy) {
-        if (rank == 0 && threadIdx.x == 0) out_tokens[b] = argmax;
+        if (rank == 0 && threadIdx.x == 0) out_tokens[b] = most_likely();
         return;
     }
     s.maxv = maxv;
     s.inv_t = 1.f / temp;
-    for (int i = threadIdx.x; i < s.cached; i += SAMPLE_THREADS) keys[i] = weight_key(__uint_as_float(keys[i]), maxv, s.inv_t);
-    __syncthreads();
-    const int k = top_k ? top_k[b] : 0;
-    const float p = top_p ? top_p[b] : 1.f;
-
+    const int k = sm.top_k;
+    const float p = sm.top_p;
+    // The draw sees the row as SAMPLE_PARTS runs of `part` elements, 1 / C of them in this CTA's share.  A run is summed by one warp
+    // and the runs' sums are added in order whatever C is, so that a token does not depend on how the row was shared out.
+    constexpr int runs = SAMPLE_PARTS / C;
+    const int part = span / runs;
+    auto sum_runs = [&](auto&& weight) {
+        for (int q = w; q < runs; q += SAMPLE_WARPS) {
+            const int qhi = min((q + 1) * part, s.n);
+            float mine = 0.f;
+            int i = q * part + l;
+            for (; i + 7 * 32 < qhi; i += 8 * 32) {       // eight reads in flight, added one by one
+                float e[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) e[u] = weight(i + u * 32);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) mine += e[u];
+            }
+            for (; i < qhi; i += 32) mine += weight(i);
+            mine = warp_sum(mine);
+            if (l == 0)
+                for (int peer = 0; peer < C; ++peer) peer_put<C>(&sm.mass[rank * runs + q], peer, mine);
+        }
+    };
     uint32_t thr = 0;           // keep keys >= thr
-    if (k > 0 && k < V) thr = radix_threshold<false>(s, 0u, (float)k, rank, C, sm);
-    if (p < 1.f) {
-        if (p > 0.f) thr = radix_threshold<true>(s, thr, p, rank, C, sm);
-        else thr = 0xffffffffu;                      // an empty nucleus: the most likely token
-    }
-
-    // ---- draw: the row as SAMPLE_PARTS runs of `part` elements, 1 / C of them in this CTA's share.  A run is summed by one warp and
-    // the runs' sums are added in order whatever C is, so that a token does not depend on how the row was shared out.
     auto kept = [&](int i) {
         const uint32_t key = s.at(i);
         return key >= thr ? __uint_as_float(key) : 0.f;
     };
-    const int part = span / (SAMPLE_PARTS / C);
-    for (int q = w; q < SAMPLE_PARTS / C; q += SAMPLE_WARPS) {
-        const int qhi = min((q + 1) * part, s.n);
-        float mine = 0.f;
-        int i = q * part + l;
-        for (; i + 7 * 32 < qhi; i += 8 * 32) {       // eight reads in flight, added one by one
-            float e[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) e[u] = kept(i + u * 32);
-#pragma unroll
-            for (int u = 0; u < 8; ++u) mine += e[u];
+    if (C <= 2 && !(k > 0 && k < V) && !(p < 1.f)) {
+        // a row without filters whose runs occupy all warps is summed while its weights are formed
+        sum_runs([&](int i) {
+            const uint32_t key = weight_key(i < s.cached ? __uint_as_float(keys[i]) : x[i], maxv, s.inv_t);
+            if (i < s.cached) keys[i] = key;
+            return __uint_as_float(key);
+        });
+    } else {
+        for (int i = threadIdx.x; i < s.cached; i += SAMPLE_THREADS) keys[i] = weight_key(__uint_as_float(keys[i]), maxv, s.inv_t);
+        __syncthreads();
+        if (k > 0 && k < V) thr = radix_threshold<false, C>(s, 0u, (float)k, rank, sm);
+        if (p < 1.f) {
+            if (p > 0.f) thr = radix_threshold<true, C>(s, thr, p, rank, sm);
+            else thr = 0xffffffffu;                  // an empty nucleus: the most likely token
         }
-        for (; i < qhi; i += 32) mine += kept(i);
-        mine = warp_sum(mine);
-        if (l == 0)
-            for (int peer = 0; peer < C; ++peer) peer_st(&sm.mass[rank * (SAMPLE_PARTS / C) + q], peer, mine);
+        sum_runs(kept);
     }
-    cluster_sync_all();                              // nothing is read from or written to another CTA after this
-    float tot = 0.f;
-    for (int q = 0; q < SAMPLE_PARTS; ++q) tot += sm.mass[q];
+    row_sync<C>();                              // nothing is read from or written to another CTA after this
+    // a run's sum per lane; the sum of all runs in order, of which a lane keeps the part before its own
+    const float run_sum = sm.mass[l];
+    float tot = 0.f, ahead = 0.f;
+    for (int q0 = 0; q0 < SAMPLE_PARTS; q0 += 8) {
+        float x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = __shfl_sync(0xffffffffu, run_sum, q0 + u);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (l == q0 + u) ahead = tot;
+            tot += x[u];
+        }
+    }
     if (!(tot > 0.f)) {
-        if (rank == 0 && threadIdx.x == 0) out_tokens[b] = argmax;
+        if (rank == 0 && threadIdx.x == 0) out_tokens[b] = most_likely();
         return;
     }
-    const unsigned long long r = splitmix64(seeds ? seeds[b] : 0x1234ull + b);
-    const float u = (float)(r >> 40) * (1.0f / 16777216.0f) * tot;      // [0, tot)
-    float before = 0.f;
-    int in = SAMPLE_PARTS - 1;
-    for (int q = 0; q < SAMPLE_PARTS; ++q) {
-        if (before + sm.mass[q] > u) { in = q; break; }
-        before += sm.mass[q];
-    }
+    const float u = (float)(splitmix64(sm.seed) >> 40) * (1.0f / 16777216.0f) * tot;      // [0, tot)
+    const unsigned past = __ballot_sync(0xffffffffu, ahead + run_sum > u);
+    int in = past ? __ffs(past) - 1 : SAMPLE_PARTS - 1;
+    const float before = past ? __shfl_sync(0xffffffffu, ahead, in) : tot;
     while (in > 0 && sm.mass[in] == 0.f) --in;        // rounding pushed u past the total: the last run that holds mass
-    if (in / (SAMPLE_PARTS / C) != rank) return;
+    if (in / runs != rank) return;
     // Inside the run: blocks of 32 elements, an inclusive scan in each.  All warps scan blocks and leave every block's sum and the
     // largest kept prefix in it; the running sum over the blocks then stops at the first one with a prefix beyond the point.
     const float need = u - before;
-    const int wlo = in % (SAMPLE_PARTS / C) * part, whi = min(wlo + part, s.n);
+    const int wlo = in % runs * part, whi = min(wlo + part, s.n);
     float* bsum = reinterpret_cast<float*>(sm.cnt);
     float* bmax = reinterpret_cast<float*>(sm.hi);
     auto scan = [&](int b0, float& e) {
@@ -390,19 +448,12 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
     }
 }
 
-int launch_sample(const float* logits, int B, int V, const float* temperature, const int* top_k,
-                  const float* top_p, const unsigned long long* seeds, int* out_tokens, bool pdl,
-                  cudaStream_t stream) {
-    FT_REQUIRE(B >= 1 && V >= 1, "sample: B=%d V=%d", B, V);
-    // CTAs per row: a share of 4096 logits keeps 512 threads busy for longer than a cluster barrier takes
-    int C = 1;
-    while (C < SAMPLE_MAX_CTAS && V > 4096 * C) C *= 2;
-    while (C > 1 && (long long)B * C > 0x7fffffffll) C /= 2;
-    const int span = (V + SAMPLE_PARTS - 1) / SAMPLE_PARTS * (SAMPLE_PARTS / C);      // a multiple of 4: shares start on 16 bytes where the rows do
-    const int cache = span < SAMPLE_CACHE ? span : SAMPLE_CACHE;
+template <int C>
+static int launch_rows(const float* logits, int B, int V, int span, int cache, const float* temperature, const int* top_k, const float* top_p,
+                       const unsigned long long* seeds, int* out_tokens, bool pdl, cudaStream_t stream) {
     static PerDeviceFlag attr_set;
     if (!attr_set.done()) {
-        FT_CHECK_CUDA(cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_CACHE * 4));
+        FT_CHECK_CUDA(cudaFuncSetAttribute(sample_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_CACHE * 4));
         attr_set.mark();
     }
     cudaLaunchConfig_t cfg = {};
@@ -411,15 +462,51 @@ int launch_sample(const float* logits, int B, int V, const float* temperature, c
     cfg.dynamicSmemBytes = temperature ? (size_t)cache * 4 : 0;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = C; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    int n = 0;
+    if (C > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = C; attr[n].val.clusterDim.y = 1; attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 2 : 1;
-    FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, sample_kernel, logits, V, span, cache, temperature, top_k, top_p, seeds,
-                                     out_tokens, C));
+    cfg.numAttrs = n;
+    FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, sample_kernel<C>, logits, V, span, cache, temperature, top_k, top_p, seeds, out_tokens));
     return 0;
+}
+
+int launch_sample(const float* logits, int B, int V, const float* temperature, const int* top_k,
+                  const float* top_p, const unsigned long long* seeds, int* out_tokens, bool pdl,
+                  cudaStream_t stream) {
+    FT_REQUIRE(B >= 1 && V >= 1, "sample: B=%d V=%d", B, V);
+    // CTAs per row: a share of 4096 logits keeps 512 threads busy for longer than a cluster barrier takes.  Rows of up to 65536
+    // logits, and greedy ones, take no more CTAs than are resident at once, two per SM, and beyond half of the SMs in rows not those
+    // that only shorten a share below 16384.  Nucleus / plain / greedy rows, with eight CTAs each whatever the batch and (last)
+    // with one CTA that reads the row again in every pass, as it once was:
+    //   256 rows of 32768   49 / 16 / 5.3 us   139 / 60 / 23    99 / 25 / 6.7
+    //   128 rows of 50257   49 / 18 / 6.6       88 / 41 / 14    72 / 20 / 4.9
+    // A longer row that is sampled wants its weights in shared memory whatever the batch (128 rows of 128256: 124 us in eight CTAs,
+    // 145 in two; 96 rows: 96 and 139); its greedy neighbours pay for that (14 us, alone 7.9).
+    const int sms = device_sms();
+    const bool bounded = V <= 65536 || !temperature;
+    const int per = bounded && 2LL * B > sms ? 16384 : 4096;
+    int C = 1;
+    while (C < SAMPLE_MAX_CTAS && V > per * C && (!bounded || 2LL * C * B <= 2LL * sms)) C *= 2;
+    while (C > 1 && (long long)B * C > 0x7fffffffll) C /= 2;
+    const int span = (V + SAMPLE_PARTS - 1) / SAMPLE_PARTS * (SAMPLE_PARTS / C);      // a multiple of 4: shares start on 16 bytes where the rows do
+    // half of the weights where that lets a second CTA onto the SM and there is one (256 rows of 50257: 87 us, 126 with all)
+    const int room = bounded && C <= 2 && (long long)B * C > sms ? SAMPLE_CACHE / 2 : SAMPLE_CACHE;
+    const int cache = span < room ? span : room;
+    switch (C) {
+        case 1: return launch_rows<1>(logits, B, V, span, cache, temperature, top_k, top_p, seeds, out_tokens, pdl, stream);
+        case 2: return launch_rows<2>(logits, B, V, span, cache, temperature, top_k, top_p, seeds, out_tokens, pdl, stream);
+        case 4: return launch_rows<4>(logits, B, V, span, cache, temperature, top_k, top_p, seeds, out_tokens, pdl, stream);
+        default: return launch_rows<8>(logits, B, V, span, cache, temperature, top_k, top_p, seeds, out_tokens, pdl, stream);
+    }
 }
 
 }  // namespace ft

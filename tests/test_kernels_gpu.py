@@ -647,6 +647,26 @@ def test_sample_against_the_sorted_row(K, B, V):
             assert float(cum[t] - prob[t]) - slack <= u <= float(cum[t]) + slack, (temp, k, p, b)
 
 
+@pytest.mark.parametrize("V", [1000, 4097, 32768, 50257, 128256])
+def test_sample_token_does_not_depend_on_the_batch(K, V):
+    """A row's share of CTAs (eight to one) and of cached weights follows the batch and the row's length; its token does not."""
+    g = torch.Generator(device=DEV).manual_seed(V)
+    rows = torch.randn(4, V, device=DEV, generator=g) * 2.5
+    rows[3, V // 2] = rows[3, V // 3] = float(rows.max()) + 1.0          # a tie: the lower index wins
+    for temp, k, p in [(0.0, 0, 1.0), (1.0, 0, 1.0), (0.7, 0, 0.9), (0.7, 40, 0.9), (1.3, 5, 1.0)]:
+        first = None
+        for B in (4, 40, 76, 152, 300):
+            n = -(-B // 4)
+            logits = rows.repeat(n, 1)[:B].contiguous()
+            seeds = torch.arange(4, device=DEV, dtype=torch.int64).repeat(n)[:B] * 7919 + 5
+            tok = K.sample(logits, torch.full((B,), temp, device=DEV), torch.full((B,), k, device=DEV, dtype=torch.int32),
+                           torch.full((B,), p, device=DEV), seeds)
+            first = tok if first is None else first
+            assert torch.equal(tok, first.repeat(n)[:B]), (temp, k, p, B)
+            if temp == 0.0:
+                assert torch.equal(K.sample(logits), tok) and int(tok[3]) == V // 3
+
+
 def test_sample_rows_without_numbers(K):
     """Infinities and NaN: minus infinity is never drawn, an infinite logit wins, a NaN is never drawn, the index stays inside."""
     V = 32768
