@@ -1,14 +1,14 @@
 // Plain projections on tcgen05: out[t][n] = sum_k (hi + lo)[t][k] W[n][k] in fp32, no fused layer step — every projection of the
 // layered models, and ft_gemm_bf16 / ft_gemm_fused with unsplit fp32 results.  Operands as in gemm.cu (W rows are the UMMA A operand,
-// the activation's two bf16 planes the B operand, both products into one fp32 accumulator in TMEM); two kernels:
+// the activation's two bf16 planes the B operand, fp32 accumulators in TMEM); two kernels:
 //
 //   many tokens   CTA pairs (cta_group::2) that walk units of 256 weight rows x `bn` tokens, two accumulators, as gemm_pair_kernel
 //                 does, with a token tile whose width is a run-time value.  A projection of 2313 tokens and 2048 rows is 152 units of
 //                 128 tokens for 74 pairs: three rounds, the last one nearly empty; 160 tokens wide it is 120 units in two.  The
 //                 width that the launcher takes is the one with the least time over all rounds (plain_token_tile).
 //                 Measured (2313 tokens, hi + lo, one CTA per tile before): 2048 -> 2048 45 -> 40 us, 2048 -> 10752 182 -> 143 us.
-//   few tokens    one token tile; K is shared by the up to eight CTAs of a cluster, which add their partial tiles through distributed
-//                 shared memory in rank order: no slabs, no arrival words, no second launch.  Bound by latency (launch, first load,
+//   few tokens    up to 128, where few_tokens() says so: one token tile; K is shared by the up to eight CTAs of a cluster, which
+//                 add their partial tiles through distributed shared memory in rank order: no slabs, no arrival words, no second launch.  Bound by latency (launch, first load,
 //                 one pass over a few chunks), and per chunk by the tensor core's reads of the weight tile, which both planes share
 //                 (16 tokens, 2048 x 2048: one CTA per 128 rows 13.1 us, K shared by eight 6.6, one product for both planes 5.9).
 #include "common.cuh"
@@ -145,6 +145,27 @@ gemm_plain_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 // ------------------------------------------------------------------ few tokens
 constexpr int PF_THREADS = 192;                           // TMA warp, MMA warp, four epilogue warps
 
+// One weight row's partial sums of every S-th token, added in rank order, sixteen reads of the cluster's shared memory on their way
+// per thread.  (One token at a time with S reads: 512 x 512 and 128 tokens, S = 2, 14.7 us; S = 2 and this 12.)
+template <int S>
+__device__ __forceinline__ void add_shares(const float* mine, float* dst, int n_out, int T, int rank) {
+    constexpr int U = 16 / S;
+    for (int t0 = rank; t0 < T; t0 += S * U) {
+        float v[U][S];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int p = 0; p < S; ++p) v[u][p] = t0 + u * S < T ? peer_ld(mine + (t0 + u * S) * PL_BM, p) : 0.f;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            float sum = v[u][0];
+#pragma unroll
+            for (int p = 1; p < S; ++p) sum += v[u][p];
+            if (t0 + u * S < T) dst[(size_t)(t0 + u * S) * n_out] = sum;
+        }
+    }
+}
+
 // grid (row tiles, S), clusters of (1, S): CTA (x, s) takes the s-th share of K of weight rows 128 x .. 128 x + 127.
 template <int BN>
 __global__ void __launch_bounds__(PF_THREADS)
@@ -240,17 +261,11 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     if (S > 1) {
         cluster_sync_all();                               // every share of the row tile is there
         if (warp >= 2) {
-            const int f = threadIdx.x - 64;
-            const float* mine = reinterpret_cast<const float*>(smem) + f;      // (the same place in every CTA)
-            for (int t = rank; t < T; t += S) {
-                float v[8];
-#pragma unroll
-                for (int p = 0; p < 8; ++p) v[p] = p < S ? peer_ld(mine + t * PL_BM, p) : 0.f;
-                float sum = v[0];
-#pragma unroll
-                for (int p = 1; p < 8; ++p) sum += v[p];
-                out[(size_t)t * n_out + row0 + f] = sum;
-            }
+            const float* mine = reinterpret_cast<const float*>(smem) + threadIdx.x - 64;      // (the same place in every CTA)
+            float* dst = out + row0 + threadIdx.x - 64;
+            if (S == 2) add_shares<2>(mine, dst, n_out, T, rank);
+            else if (S == 4) add_shares<4>(mine, dst, n_out, T, rank);
+            else add_shares<8>(mine, dst, n_out, T, rank);
         }
         cluster_sync_all();                               // nobody leaves while its tile is being read
     }
@@ -258,14 +273,32 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 
 constexpr int PL_RING = 222 * 1024;                       // shared memory for the stages (+ 1 KB to align them)
 
+// CTAs that share a row tile's K: as many as leave each three chunks and the grid one CTA per SM, from four CTAs per tile on nearly two
+// (10752 x 2048 and 64 tokens: 14.7 us with S = 1, 17.2 with 2; 296 CTAs in clusters of four do not all find a place within their GPCs at
+// once: 9472 x 3072, 64 tokens, 24.4 us, 15.3 in 148).  Where K is short the sharing costs what it saves: none up to 512 columns (4096 x 512,
+// 48 tokens: 6.5 us with S = 1, 9.0 with 2), and up to 1984 only as far as 64 CTAs, 128 for one narrow token tile (8192 x 1024, 64 tokens:
+// 9.8 us with S = 1, 12.0 with 2; 4096 x 1024, 16 tokens: 7.2 with 2, 6.8 with 4).
+int few_shares(int tiles, int kc, int T) {
+    if (kc <= 8) return 1;
+    int S = 8;
+    while (S > 1 && (kc / S < 3 || tiles * S > (kc < 32 ? (T <= 16 && tiles < 64 ? 128 : 64) : S >= 4 ? 7 * device_sms() / 4 : device_sms()))) S /= 2;
+    return S;
+}
+// Up to 128 tokens on the few-token kernel, or (more than 48) on CTA pairs.  The few-token kernel wins where K can be shared: 64 tokens
+// and 4096 x 2048 10.3 against 12.5 us, 128 tokens and 2048 x 8192 21.1 against 37.  From 65 tokens on its token tile is as wide as the
+// pairs' and adding the shares takes longer than they save, unless K is long or the row tiles are few (128 tokens: 8192 x 1024 15.3 against
+// 9.7 us, 12288 x 4096 30.7 against 25.1, but 3072 x 3072 14.7 against 18.7).  Unshared, with a short K or on more than half of the SMs,
+// pairs are ahead from 49 tokens on (64 tokens: 4096 x 512 7.1 against 6.4, 16384 x 2048 15.8 against 14.7).
+bool few_tokens(int tiles, int kc, int T, int S) {
+    if (T <= 48) return true;
+    if (T <= 64) return S > 1 || (kc > 8 && 2 * tiles <= device_sms());
+    return T <= 128 && S >= 4 && (kc >= 48 || (kc >= 32 && tiles <= (T <= 80 ? 32 : 16)));
+}
+
 template <int BN>
-int launch_few(const CUtensorMap& mw, const CUtensorMap& mh, const CUtensorMap& ml, float* out, int n_out, int T, int K, cudaStream_t stream) {
+int launch_few(const CUtensorMap& mw, const CUtensorMap& mh, const CUtensorMap& ml, float* out, int n_out, int T, int K, int S, cudaStream_t stream) {
     constexpr int STAGE = PL_A + 2 * BN * PL_BK * 2;
     const int kc = K / PL_BK, tiles = n_out / PL_BM;
-    // CTAs per row tile: as many as leave each three chunks and the grid one CTA per SM, two from four CTAs per tile on (weights of
-    // 10752 x 2048 and 64 tokens: 12.8 us with S = 1, 16.1 with 2; 8576 x 2048 and 16 tokens: 8.5 us with S = 2, 7.9 with 4)
-    int S = 8;
-    while (S > 1 && (kc / S < 3 || tiles * S > (S >= 4 ? 2 : 1) * device_sms())) S /= 2;
     // A deep ring where a CTA has an SM for itself, half of one otherwise.  Clusters of four or eight always leave room for a second CTA:
     // they must lie within one GPC, and with one CTA per SM sixteen clusters of eight do not all find one (2048 x 4096, 16 tokens:
     // 12.9 us with 160 KB per CTA, more than with half the CTAs).
@@ -341,15 +374,16 @@ int launch_gemm_plain(const void* w, const void* hi, const void* lo, float* out,
                "gemm (plain): bad sizes or operands (n_out %d, T %d, K %d)", n_out, T, K);
     CUtensorMap mw, mh, ml;
     if (int r = make_tmap_bf16_k64(&mw, w, n_out, K, PL_BM)) return r;
-    if (T <= 128) {
+    const int S = few_shares(n_out / PL_BM, K / PL_BK, T);
+    if (few_tokens(n_out / PL_BM, K / PL_BK, T, S)) {
         const int bn = gemm_pick_bn(T, true);
         if (int r = make_tmap_bf16_k64(&mh, hi, T, K, bn)) return r;
         if (int r = make_tmap_bf16_k64(&ml, lo, T, K, bn)) return r;
         switch (bn) {
-            case 16: return launch_few<16>(mw, mh, ml, out, n_out, T, K, stream);
-            case 32: return launch_few<32>(mw, mh, ml, out, n_out, T, K, stream);
-            case 64: return launch_few<64>(mw, mh, ml, out, n_out, T, K, stream);
-            default: return launch_few<128>(mw, mh, ml, out, n_out, T, K, stream);
+            case 16: return launch_few<16>(mw, mh, ml, out, n_out, T, K, S, stream);
+            case 32: return launch_few<32>(mw, mh, ml, out, n_out, T, K, S, stream);
+            case 64: return launch_few<64>(mw, mh, ml, out, n_out, T, K, S, stream);
+            default: return launch_few<128>(mw, mh, ml, out, n_out, T, K, S, stream);
         }
     }
     const int clusters = plain_clusters();

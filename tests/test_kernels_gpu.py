@@ -583,6 +583,13 @@ def test_gemm_plain_fp32(K, T, n_out, Kd):
     assert bool((guard[T] == 7.0).all())
 
 
+@pytest.mark.parametrize("T,n_out,Kd", [(48, 512, 512), (49, 512, 512), (64, 4096, 256), (16, 4096, 1024), (17, 4096, 1024), (64, 9600, 640), (49, 9600, 640),
+                                        (65, 2048, 2048), (80, 4096, 2048), (81, 4096, 2048), (100, 1024, 3072), (127, 9472, 3072), (65, 128, 64)])
+def test_gemm_plain_few_tokens_or_pairs(K, T, n_out, Kd):
+    """Both sides of every line between the few-token kernel (K whole, or shared by two, four and eight CTAs) and CTA pairs."""
+    test_gemm_plain_fp32(K, T, n_out, Kd)
+
+
 @pytest.mark.parametrize("T,n_out,Kd", [(391, 7680, 64), (586, 5632, 320), (963, 12800, 192), (1002, 12672, 64)])
 def test_gemm_plain_widest_token_tiles(K, T, n_out, Kd):
     """Token tiles of 224 (two sizes) and 256 (two sizes, one with an odd number of row tiles), which take the fewest rounds here
@@ -591,12 +598,12 @@ def test_gemm_plain_widest_token_tiles(K, T, n_out, Kd):
 
 
 def test_gemm_plain_on_two_streams(K):
-    """Launches of few tokens (K shared by clusters of four CTAs, three chunks each) beside launches of CTA pairs with 32-token
+    """Launches of few tokens (K shared by clusters of four and eight CTAs, three chunks each) beside launches of CTA pairs with 32-token
     tiles, on two streams at once: both kinds hold tensor-memory columns, and neither may wait for the other's."""
     from fasttalk_llm_microservice_b200 import native as N
     g = torch.Generator(device=DEV).manual_seed(5)
     calls = []
-    for T, n_out, Kd in [(16, 2048, 768), (16, 4096, 384), (160, 1024, 512), (129, 2048, 384)]:
+    for T, n_out, Kd in [(16, 2048, 768), (16, 1024, 1536), (160, 1024, 512), (129, 2048, 384)]:
         w = (torch.randn(n_out, Kd, device=DEV, generator=g) * 0.05).bfloat16()
         x, x_lo = K.split_hi_lo(torch.randn(T, Kd, device=DEV, generator=g))
         calls.append((w, x, x_lo, n_out, T, Kd, torch.empty(T, n_out, device=DEV)))
