@@ -856,12 +856,27 @@ __global__ void __launch_bounds__(256) decay_step_kernel(RecurArgs a, int TX) {
         __syncthreads();
     }
 }
-static int launch_decay_step(const RecurArgs& a, int n_req, cudaStream_t stream) {
-    const bool wide = a.vd % 4 == 0 && a.slot_stride % 4 == 0 && a.s_off % 4 == 0 && ((uintptr_t)a.state & 15) == 0;
-    const int units = wide ? a.vd / 4 : a.vd;
-    int TX = 8;
-    while (TX < 32 && TX < units) TX *= 2;
-    const dim3 grid(n_req, a.heads, (units + TX - 1) / TX);
+// Units per CTA: 32 of a row's where there are so many.  A thread then has dim / 8 rows: with few channels and a full grid more units, so
+// that it has eight (64 requests of 16 heads of 32 x 1024: 64.9 us with 32 units, 50.3 with 64), and while fewer CTAs than half of the
+// SMs would run fewer units, until it has no more than the eight rows that are on their way together (one request of two heads of 256 x 256:
+// 5.8 us with 32 units, 3.6 with eight).
+struct StepPlan { bool wide; int TX; long long ctas; };
+static StepPlan decay_step_plan(const RecurArgs& a, int n_req) {
+    StepPlan p;
+    p.wide = a.vd % 4 == 0 && a.slot_stride % 4 == 0 && a.s_off % 4 == 0 && ((uintptr_t)a.state & 15) == 0;
+    const int units = p.wide ? a.vd / 4 : a.vd, sms = device_sms();
+    auto ctas = [&](int tx) { return (long long)n_req * a.heads * ((units + tx - 1) / tx); };
+    p.TX = 4;
+    while (p.TX < 32 && p.TX < units) p.TX *= 2;
+    while (p.TX < 256 && p.TX < units && a.dim * p.TX < 8 * 256 && ctas(2 * p.TX) >= sms) p.TX *= 2;
+    while (p.TX > 4 && a.dim * p.TX > 8 * 256 && ctas(p.TX) < sms / 2) p.TX /= 2;
+    p.ctas = ctas(p.TX);
+    return p;
+}
+static int launch_decay_step(const RecurArgs& a, int n_req, const StepPlan& p, cudaStream_t stream) {
+    const bool wide = p.wide;
+    const int TX = p.TX;
+    const dim3 grid(n_req, a.heads, ((wide ? a.vd / 4 : a.vd) + TX - 1) / TX);
     const size_t smem = (size_t)(256 * (wide ? 4 : 1) + 2 * a.dim) * 4;
     if (wide) decay_step_kernel<4><<<grid, 256, smem, stream>>>(a, TX);
     else decay_step_kernel<1><<<grid, 256, smem, stream>>>(a, TX);
@@ -889,12 +904,19 @@ static int launch_decay_rule_t(const RecurArgs& a, int n_req, cudaStream_t strea
 // fewest lanes whose runs cover dim and four columns per thread — the widest column blocks, the best-coalesced state
 // traffic and the fewest shared-memory reads per multiply-add; then, while fewer than 96 CTAs would run (one long prompt
 // with few heads): two columns per thread, more lanes with shorter runs, at last one column (measured order).  The split
-// changes the order of a sum, nothing else.  a.lanes fixes LPC.  Steps of single tokens (no more rows than requests) take the step kernel.
+// changes the order of a sum, nothing else.  a.lanes fixes LPC.  Steps of single tokens (no more rows than requests) take the
+// step kernel, except where many small states make a full grid.
 int launch_decay_rule(const RecurArgs& a, int n_req, int T, cudaStream_t stream) {
     FT_REQUIRE(a.heads >= 1 && a.qk_heads >= 1 && a.heads % a.qk_heads == 0 && a.dim >= 1 && a.dim <= 1024 && a.vd >= 1,
                "decay rule: bad sizes (heads %d, key heads %d, dim %d, values %d)", a.heads, a.qk_heads, a.dim, a.vd);
     if (n_req <= 0) return 0;
-    if (a.lanes == 0 && T > 0 && T <= n_req) return launch_decay_step(a, n_req, stream);
+    if (a.lanes == 0 && T > 0 && T <= n_req) {
+        // Not where a thread would have a row or two and the CTAs queue up: states so small go faster through the kernel by lanes
+        // (64 requests of 16 heads of 16 x 64: 7.0 us, by lanes 4.8; of 64 heads of 32 x 64: 21.5 and 19.8, but of 16 heads 8.5 and 10.4).
+        const StepPlan p = decay_step_plan(a, n_req);
+        const int rows = a.dim * p.TX / 256;
+        if (rows >= 4 || p.ctas <= (rows < 2 ? 2 : 16) * device_sms()) return launch_decay_step(a, n_req, p, stream);
+    }
     int lpc = 4, dpt = 4;
     while (dpt < 16 && lpc * dpt < a.dim) dpt *= 2;
     while (lpc < 32 && lpc * dpt < a.dim) lpc *= 2;

@@ -572,6 +572,33 @@ def test_decay_rule_single_tokens(heads, qk_heads, dim, vd, pad):
         assert rel(dst.cpu().double().numpy(), ref_state.numpy()) < 1e-6
 
 
+@pytest.mark.parametrize("R,heads,dim,vd", [(1, 2, 256, 256), (1, 1, 512, 64), (2, 3, 512, 12), (5, 16, 32, 1024), (3, 8, 16, 1024), (40, 8, 16, 64), (80, 32, 40, 64), (3, 2, 128, 33)])
+def test_decay_rule_single_tokens_by_grid(R, heads, dim, vd):
+    """Units per CTA from 4 to 128 by channels, columns and grid, and many small states, which take the kernel by lanes."""
+    from fasttalk_llm_microservice_b200 import build, native
+    build.build()
+    lib = native.load()
+    g = torch.Generator(device="cuda").manual_seed(dim + vd)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    q, k, v = rnd(R, heads * dim) * dim ** -0.5, rnd(R, heads * dim), rnd(R, heads * vd)
+    ab = torch.rand(R, heads, 2, device="cuda", generator=g)
+    state = rnd(R, heads, dim, vd)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    pos0 = i32([0 if r % 2 else 11 for r in range(R)])
+    S = ab.double()[:, :, :1, None] * state.double() * (pos0 > 0)[:, None, None, None]
+    S = S + (ab.double()[:, :, 1:] * k.double().reshape(R, heads, dim))[..., None] * v.double().reshape(R, heads, 1, vd)
+    ref = torch.einsum("rhdv,rhd->rhv", S, q.double().reshape(R, heads, dim))
+    o = torch.zeros(R, heads * vd, device="cuda")
+    start, slot = i32(list(range(R + 1))), i32(list(range(R)))
+    rc = lib.ft_decay_rule(q.data_ptr(), k.data_ptr(), v.data_ptr(), ab.data_ptr(), o.data_ptr(), state.data_ptr(), start.data_ptr(), pos0.data_ptr(),
+                           slot.data_ptr(), R, heads, heads, dim, vd, heads * dim * vd, 0, R, None)
+    torch.cuda.synchronize()
+    assert rc == 0, native.last_error()
+    # 24-bit sums of dim terms
+    assert rel(o.cpu().double().numpy(), ref.reshape(R, -1).cpu().numpy()) < 2e-6
+    assert rel(state.cpu().double().numpy(), S.cpu().numpy()) < 1e-6
+
+
 def test_short_taps_do_not_reach_an_infinite_row_further_back():
     """A convolution of two taps in a step of more than 64 tokens: state coordinates to read out with that overflow at one token
     spoil that token and the next, no more."""
