@@ -1251,8 +1251,10 @@ int launch_route(const float* proj, int ldp, int o_router, int E, int top, int g
     route_kernel<<<(T + 3) / 4, 128, smem, stream>>>(proj, ldp, o_router, E, top, groups, keep, ids, wts, T,
                                                      route_kind == FT_ROUTE_SIGMOID, normalise, scale > 0.f ? scale : 1.f, bias);
     FT_CHECK_CUDA(cudaGetLastError());
-    int warps = 32;                                    // fewer where the counts of so many would not fit
-    while (warps > 1 && (size_t)(warps * E + E + 1) * 4 > 48 * 1024) warps /= 2;
+    // Every expert's thread walks the warps' counts, so few pairs take few warps (one token's two choices of 16 experts: all 32
+    // took a microsecond more); fewer, too, where the counts of so many would not fit.
+    int warps = 32;
+    while (warps > 1 && (warps * 16 >= std::max(T * top, E) || (size_t)(warps * E + E + 1) * 4 > 48 * 1024)) warps /= 2;
     route_sort_kernel<<<1, warps * 32, (size_t)(warps * E + E + 1) * 4, stream>>>(ids, T * top, top, E, seg, slot_token, slot_pos);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
