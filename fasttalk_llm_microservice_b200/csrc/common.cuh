@@ -214,8 +214,11 @@ __device__ __forceinline__ uint32_t cluster_id_x() {
     asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
     return r;
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 // The same shared-memory variable in another CTA of the cluster.
 __device__ __forceinline__ uint32_t peer_addr(const void* p, int rank) {

@@ -252,14 +252,15 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     }
     tc_fence_before();
     __syncthreads();                                      // the columns have been read; this CTA's share lies in its shared memory
+    if (S > 1) cluster_arrive();
     if (warp == 1) {
-        // Before the cluster's barrier: a CTA that waits for the others holds no columns.  With them it could keep one of another
-        // stream's kernel from its columns, and that one a CTA of this cluster on another SM.
+        // Before the wait: a CTA that waits for the others holds no columns.  With them it could keep one of another stream's kernel
+        // from its columns, and that one a CTA of this cluster on another SM.
         tc_fence_after();
         tmem_dealloc(tmem, COLS);
     }
     if (S > 1) {
-        cluster_sync_all();                               // every share of the row tile is there
+        cluster_wait();                                   // every share of the row tile is there
         if (warp >= 2) {
             const float* mine = reinterpret_cast<const float*>(smem) + threadIdx.x - 64;      // (the same place in every CTA)
             float* dst = out + row0 + threadIdx.x - 64;
