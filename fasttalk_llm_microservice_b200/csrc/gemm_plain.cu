@@ -202,12 +202,19 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     if (warp == 0) {
         if (elect_one()) {
             const uint64_t pol_w = policy_evict_first(), pol_x = policy_evict_last();
+            const int pre = min(n_iter, stages);
+            for (int i = 0; i < pre; ++i) {               // the weights first: they come from memory, the activations out of L2
+                mbar_expect_tx(&full[i], STAGE);
+                tma_tile_2d(smem + (size_t)i * STAGE, &map_w, (kc0 + i) * PL_BK, row0, &full[i], pol_w);
+            }
             for (int i = 0; i < n_iter; ++i) {
                 const int s = i % stages;
                 uint8_t* st = smem + (size_t)s * STAGE;
-                if (i >= stages) mbar_wait(&empty[s], ((i / stages) - 1) & 1);
-                mbar_expect_tx(&full[s], STAGE);
-                tma_tile_2d(st, &map_w, (kc0 + i) * PL_BK, row0, &full[s], pol_w);
+                if (i >= pre) {
+                    mbar_wait(&empty[s], ((i / stages) - 1) & 1);
+                    mbar_expect_tx(&full[s], STAGE);
+                    tma_tile_2d(st, &map_w, (kc0 + i) * PL_BK, row0, &full[s], pol_w);
+                }
                 tma_tile_2d(st + PL_A, &map_hi, (kc0 + i) * PL_BK, 0, &full[s], pol_x);
                 tma_tile_2d(st + PL_A + PLANE, &map_lo, (kc0 + i) * PL_BK, 0, &full[s], pol_x);
             }
@@ -276,13 +283,15 @@ constexpr int PL_RING = 222 * 1024;                       // shared memory for t
 
 // CTAs that share a row tile's K: as many as leave each three chunks and the grid one CTA per SM, from four CTAs per tile on nearly two
 // (10752 x 2048 and 64 tokens: 14.7 us with S = 1, 17.2 with 2; 296 CTAs in clusters of four do not all find a place within their GPCs at
-// once: 9472 x 3072, 64 tokens, 24.4 us, 15.3 in 148).  Where K is short the sharing costs what it saves: none up to 512 columns (4096 x 512,
-// 48 tokens: 6.5 us with S = 1, 9.0 with 2), and up to 1984 only as far as 64 CTAs, 128 for one narrow token tile (8192 x 1024, 64 tokens:
-// 9.8 us with S = 1, 12.0 with 2; 4096 x 1024, 16 tokens: 7.2 with 2, 6.8 with 4).
+// once: 9472 x 3072, 64 tokens, 24.4 us, 15.3 in 148).  Where K is short the sharing costs what it saves: up to 512 columns none (64 tokens
+// of 4096 x 512: 6.4 us, 10.2 with S = 2 and one token at a time), and up to 1984 fewer CTAs for more than 32 tokens, whose shares take
+// longer to add (24 tokens of 8192 x 1024: 8.0 us with S = 4, 8.3 with 1; 64 tokens: 10.3 and 9.7; 3072 x 1024: 8.3 and 8.9).
 int few_shares(int tiles, int kc, int T) {
     if (kc <= 8) return 1;
+    const int sms = device_sms();
+    auto most = [&](int S) { return kc < 32 && T > 32 ? (S == 8 ? 192 : S == 4 ? 136 : 80) : S >= 4 ? (T > 32 ? 14 : 15) * sms / 8 : sms; };
     int S = 8;
-    while (S > 1 && (kc / S < 3 || tiles * S > (kc < 32 ? (T <= 16 && tiles < 64 ? 128 : 64) : S >= 4 ? 7 * device_sms() / 4 : device_sms()))) S /= 2;
+    while (S > 1 && (kc / S < 3 || tiles * S > most(S))) S /= 2;
     return S;
 }
 // Up to 128 tokens on the few-token kernel, or (more than 48) on CTA pairs.  The few-token kernel wins where K can be shared: 64 tokens
