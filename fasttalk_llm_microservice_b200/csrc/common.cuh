@@ -231,7 +231,11 @@ __device__ __forceinline__ unsigned peer_ld(const unsigned* p, int rank) {
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_addr(p, rank)) : "memory");
     return v;
 }
-__device__ __forceinline__ float peer_ld(const float* p, int rank) { return __uint_as_float(peer_ld(reinterpret_cast<const unsigned*>(p), rank)); }
+__device__ __forceinline__ float peer_ld_at(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
 // Tile load issued by EITHER CTA of the pair into its own shared memory; the bytes are counted on
 // the LEADER's mbarrier (same offset in the even CTA).
 __device__ __forceinline__ void tma_tile_2d_pair(void* dst_smem, const CUtensorMap* map, int c0, int c1,

@@ -145,27 +145,6 @@ gemm_plain_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 // ------------------------------------------------------------------ few tokens
 constexpr int PF_THREADS = 192;                           // TMA warp, MMA warp, four epilogue warps
 
-// One weight row's partial sums of every S-th token, added in rank order, sixteen reads of the cluster's shared memory on their way
-// per thread.  (One token at a time with S reads: 512 x 512 and 128 tokens, S = 2, 14.7 us; S = 2 and this 12.)
-template <int S>
-__device__ __forceinline__ void add_shares(const float* mine, float* dst, int n_out, int T, int rank) {
-    constexpr int U = 16 / S;
-    for (int t0 = rank; t0 < T; t0 += S * U) {
-        float v[U][S];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int p = 0; p < S; ++p) v[u][p] = t0 + u * S < T ? peer_ld(mine + (t0 + u * S) * PL_BM, p) : 0.f;
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            float sum = v[u][0];
-#pragma unroll
-            for (int p = 1; p < S; ++p) sum += v[u][p];
-            if (t0 + u * S < T) dst[(size_t)(t0 + u * S) * n_out] = sum;
-        }
-    }
-}
-
 // grid (row tiles, S), clusters of (1, S): CTA (x, s) takes the s-th share of K of weight rows 128 x .. 128 x + 127.
 template <int BN>
 __global__ void __launch_bounds__(PF_THREADS)
@@ -269,11 +248,40 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     if (S > 1) {
         cluster_wait();                                   // every share of the row tile is there
         if (warp >= 2) {
+            // This CTA adds every S-th token's shares, one weight row per thread, in rank order.  Eight reads of the cluster's memory are on
+            // their way per thread, whatever S is (one token at a time: 128 tokens of 512 x 512 with S = 2 14.7 us, so 12).
             const float* mine = reinterpret_cast<const float*>(smem) + threadIdx.x - 64;      // (the same place in every CTA)
             float* dst = out + row0 + threadIdx.x - 64;
-            if (S == 2) add_shares<2>(mine, dst, n_out, T, rank);
-            else if (S == 4) add_shares<4>(mine, dst, n_out, T, rank);
-            else add_shares<8>(mine, dst, n_out, T, rank);
+            const int ls = __ffs(S) - 1;
+            uint32_t from[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) from[q] = peer_addr(mine, q & (S - 1));
+            if (S == 8) {
+                for (int t = rank; t < T; t += 8) {
+                    float v[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) v[q] = peer_ld_at(from[q] + (uint32_t)t * (PL_BM * 4));
+                    float sum = v[0];
+#pragma unroll
+                    for (int q = 1; q < 8; ++q) sum += v[q];
+                    dst[(size_t)t * n_out] = sum;
+                }
+            } else {
+                for (int t0 = rank; t0 < T; t0 += 8) {            // tokens t0, t0 + S, ..
+                    float v[8], sum = 0.f;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const int t = t0 + (q >> ls << ls);
+                        v[q] = t < T ? peer_ld_at(from[q] + (uint32_t)t * (PL_BM * 4)) : 0.f;
+                    }
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const int t = t0 + (q >> ls << ls);
+                        sum = (q & (S - 1)) ? sum + v[q] : v[q];
+                        if ((q & (S - 1)) == S - 1 && t < T) dst[(size_t)t * n_out] = sum;
+                    }
+                }
+            }
         }
         cluster_sync_all();                               // nobody leaves while its tile is being read
     }
