@@ -12,7 +12,7 @@
 //
 // What bounds it: a chain of short passes over data in shared memory and of cluster barriers (3 per radix pass).  One CTA per row
 // with every pass reading the row again took 153 us for one row of 128256 and 203 us for 64 (greedy and sampled rows mixed);
-// the cluster takes 30 and 78 us.
+// the cluster takes 26 and 73 us.
 #include "common.cuh"
 #include "ft_internal.h"
 
