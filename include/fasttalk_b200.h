@@ -644,7 +644,8 @@ int ft_attn_prefill(const void* q, const void* kv_layer, const int* page_table, 
                     const int* tile_q0, int n_tiles, void* out, void* out_lo, int nq, int nkv, int d,
                     int q_rows, void* stream);
 
-/* K7: per-row temperature / top-k / top-p sampling (argmax when temperature <= 0). */
+/* K7: per-row temperature / top-k / top-p sampling (argmax when temperature <= 0; a null temperature says so for all rows).
+ * A row without any logit above minus infinity gives index 0. */
 int ft_sample(const float* logits, int B, int V, const float* temperature, const int* top_k,
               const float* top_p, const unsigned long long* seeds, int* out_tokens, void* stream);
 
