@@ -905,7 +905,7 @@ static int launch_decay_rule_t(const RecurArgs& a, int n_req, cudaStream_t strea
 // traffic and the fewest shared-memory reads per multiply-add; then, while fewer than 96 CTAs would run (one long prompt
 // with few heads): two columns per thread, more lanes with shorter runs, at last one column (measured order).  The split
 // changes the order of a sum, nothing else.  a.lanes fixes LPC.  Steps of single tokens (no more rows than requests) take the
-// step kernel, except where many small states make a full grid.
+// step kernel, except where many small states make a full grid; portions of many tokens go to the tensor cores (decay_tc.cu).
 int launch_decay_rule(const RecurArgs& a, int n_req, int T, cudaStream_t stream) {
     FT_REQUIRE(a.heads >= 1 && a.qk_heads >= 1 && a.heads % a.qk_heads == 0 && a.dim >= 1 && a.dim <= 1024 && a.vd >= 1,
                "decay rule: bad sizes (heads %d, key heads %d, dim %d, values %d)", a.heads, a.qk_heads, a.dim, a.vd);
@@ -917,6 +917,7 @@ int launch_decay_rule(const RecurArgs& a, int n_req, int T, cudaStream_t stream)
         const int rows = a.dim * p.TX / 256;
         if (rows >= 4 || p.ctas <= (rows < 2 ? 2 : 16) * device_sms()) return launch_decay_step(a, n_req, p, stream);
     }
+    if (a.lanes == 0 && decay_tc_ahead(a, n_req, T)) return launch_decay_tc(a, n_req, stream);
     int lpc = 4, dpt = 4;
     while (dpt < 16 && lpc * dpt < a.dim) dpt *= 2;
     while (lpc < 32 && lpc * dpt < a.dim) lpc *= 2;

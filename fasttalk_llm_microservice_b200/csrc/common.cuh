@@ -130,6 +130,24 @@ __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity
     return false;
 }
 
+// The same for many warps at once: a try sleeps up to 2 us in hardware, so that waiting warps leave the issue slots to the others.
+__device__ __forceinline__ bool mbar_sleep_limited(uint64_t* bar, uint32_t parity, volatile int* dead) {
+    for (int i = 0; i < kWaitLimit / 4; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity), "r"(2000)
+            : "memory");
+        if (ok) return true;
+        if (*dead) return false;
+    }
+    *dead = 1;
+    return false;
+}
+
 // ------------------------------------------------------------------ L2 cache policies
 __device__ __forceinline__ uint64_t policy_evict_first() {
     uint64_t p;

@@ -921,8 +921,19 @@ static int run_branch(Engine* e, const Batch& b, const LayeredLayer& ll, int k, 
         o.ldo = r.ldo;
         if (r0 < b.n_req) {
             r.req_start += r0; r.req_pos0 += r0; r.req_slot += r0;
-            FT_TRY(launch_decay_rule(r, b.n_req - r0, T - q0, st));
-            launched();
+            r.err = e->h_kernel_err;
+            // decoding sessions beside portions: each in a launch of its own, with the kernel that suits it
+            const int single = b.n_decode - r0, rest = b.n_req - b.n_decode;
+            RecurArgs p = r;
+            if (single > 0) { p.req_start += single; p.req_pos0 += single; p.req_slot += single; }
+            if (single > 0 && rest > 0 && decay_tc_ahead(p, rest, T - b.n_decode)) {
+                FT_TRY(launch_decay_rule(r, single, single, st));
+                FT_TRY(launch_decay_rule(p, rest, T - b.n_decode, st));
+                launched(2);
+            } else {
+                FT_TRY(launch_decay_rule(r, b.n_req - r0, T - q0, st));
+                launched();
+            }
         }
         if (q0 < T) {
             if (tiles && q0 == 0) { o.out_hi = fin_hi = L.pl_hi; o.out_lo = fin_lo = L.pl_lo; }

@@ -532,6 +532,64 @@ def test_decay_rule_kernel_alone(lanes, heads, qk_heads, dim, vd):
     assert rel(dst.cpu().double().numpy(), ref_state.numpy()) < 1e-5
 
 
+@pytest.mark.parametrize("heads,qk_heads,dim,vd,pad", [(2, 2, 128, 128, 0), (3, 1, 96, 80, 0), (2, 2, 64, 65, 0), (2, 1, 65, 9, 1), (1, 1, 20, 129, 3), (2, 1, 128, 257, 0)])
+@pytest.mark.parametrize("odd", ["", "infinite", "growing"])
+def test_decay_rule_portions(heads, qk_heads, dim, vd, pad, odd):
+    """Runs of 128 tokens on the tensor cores: ends of runs one token short, whole, one too long and around the length below which they go
+    token by token, fresh and continued states, decays of zero and one, rows of very different size, slots and columns off 16 bytes; runs
+    with infinities and NaN (which must not reach an earlier token or another head) or decays beyond one."""
+    from fasttalk_llm_microservice_b200 import build, native
+    build.build()
+    lib = native.load()
+    g = torch.Generator(device="cuda").manual_seed(dim * 7 + vd)
+    dev = "cuda"
+    lens = [127, 128, 129, 128 + 15, 128 + 16, 300, 1]
+    T, R = sum(lens), len(lens)
+    start = [sum(lens[:i]) for i in range(R + 1)]
+    rnd = lambda *s: torch.randn(*s, device=dev, generator=g)
+    size = torch.exp2(torch.randint(-12, 13, (T, 1, 1), device=dev, generator=g).float())
+    q, k = (rnd(T, qk_heads, dim) * dim ** -0.5 * size), rnd(T, qk_heads, dim) * size.flip(0)
+    v, ab = rnd(T, heads, vd), torch.rand(T, heads, 2, device=dev, generator=g)
+    ab[::97, :, 0], ab[5::31, :, 0], ab[11::53, :, 0] = 0.0, 1.0, 1.0 + 2.0 ** -20
+    if odd == "infinite":
+        v[40, 0, 3], k[start[2] + 100, 0, 1], q[start[5] + 10, 0, 0] = float("inf"), float("nan"), float("-inf")
+    if odd == "growing":
+        ab[start[4] + 50, :, 0] = 1.5
+    stride = heads * dim * vd + pad
+    state = rnd(R * stride)
+    pos0 = [0 if r % 2 else 11 for r in range(R)]
+    ref_o, ref_state = torch.zeros(T, heads, vd, dtype=torch.float64, device=dev), state.double().clone()
+    abs_o, abs_state = torch.zeros_like(ref_o), ref_state.clone()      # the same sums of absolute values
+    q64, k64 = (x.double().repeat_interleave(heads // qk_heads, 1) for x in (q, k))
+    for r in range(R):
+        S = ref_state[r * stride:r * stride + heads * dim * vd].reshape(heads, dim, vd) * (pos0[r] > 0)
+        A = S.abs()
+        for t in range(start[r], start[r + 1]):
+            put = k64[t][:, :, None] * (ab[t, :, 1:].double() * v[t].double())[:, None, :]
+            S, A = ab[t, :, 0].double()[:, None, None] * S + put, ab[t, :, 0].double()[:, None, None] * A + put.abs()
+            ref_o[t], abs_o[t] = (S * q64[t][:, :, None]).sum(1), (A * q64[t][:, :, None].abs()).sum(1)
+        ref_state[r * stride:r * stride + heads * dim * vd] = S.reshape(-1)
+        abs_state[r * stride:r * stride + heads * dim * vd] = A.reshape(-1)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    rs, rp, sl = i32(start), i32(pos0), i32(list(range(R)))
+    o = torch.full((T, heads, vd), 7.0, device=dev)
+    rc = lib.ft_decay_rule(q.data_ptr(), k.data_ptr(), v.data_ptr(), ab.data_ptr(), o.data_ptr(), state.data_ptr(), rs.data_ptr(), rp.data_ptr(),
+                           sl.data_ptr(), R, heads, qk_heads, dim, vd, stride, 0, T, None)
+    torch.cuda.synchronize()
+    assert rc == 0, native.last_error()
+    states = lambda x: x[:R * stride].reshape(R, stride)[:, :heads * dim * vd]
+    for got, ref, size, rows in ((o, ref_o, abs_o, T * heads), (states(state), states(ref_state), states(abs_state), R * heads)):
+        got, ref, size = got.double().reshape(rows, -1), ref.reshape(rows, -1), size.reshape(rows, -1)
+        assert torch.equal(torch.isfinite(got), torch.isfinite(ref))
+        fin = torch.isfinite(ref).all(1) & torch.isfinite(size).all(1)
+        assert fin.any() and (odd == "infinite") == (not fin.all())
+        # a row (a token's head, a state) against the sum of its terms' sizes: eight times the rounding of one fp32 number
+        err = (got[fin] - ref[fin]).norm(dim=1) / size[fin].norm(dim=1).clamp_min(1e-30)
+        assert err.max() < 8 * 2.0 ** -24, err.max()
+    if pad:
+        assert torch.equal(state.reshape(R, stride)[:, -pad:].double(), ref_state.reshape(R, stride)[:, -pad:])
+
+
 @pytest.mark.parametrize("heads,qk_heads,dim,vd,pad", [(2, 2, 128, 128, 0), (3, 1, 96, 80, 0), (4, 2, 64, 257, 0), (2, 1, 7, 20, 1), (1, 1, 513, 1, 0)])
 def test_decay_rule_single_tokens(heads, qk_heads, dim, vd, pad):
     """One token per request (units of four columns and of one, slots that break the 16-byte rows, fresh and continued states), and a
