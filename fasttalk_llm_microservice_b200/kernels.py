@@ -191,10 +191,19 @@ def attn_prefill(q: torch.Tensor, kv_layer: torch.Tensor, page_table: torch.Tens
     for r in range(len(req_slot)):
         for q0 in range(0, req_q_start[r + 1] - req_q_start[r], 64):
             tile_req.append(r); tile_q0.append(q0)
-    i32 = lambda v: torch.tensor(v, device=dev, dtype=torch.int32)
-    t_qs, t_slot, t_pos0, t_treq, t_tq0 = i32(req_q_start), i32(req_slot), i32(req_pos0), i32(tile_req), i32(tile_q0)
-    out = torch.zeros(T, nq * d, device=dev, dtype=torch.bfloat16)
-    out_lo = torch.zeros_like(out)
+    # The lists go up in one copy that the host does not wait for (five waiting ones cost 60 us of GPU time between calls).  While a
+    # stream is captured the copy is an ordinary one, which capture refuses: a replay would read memory that is no longer this call's.
+    i32 = lambda v: torch.tensor(v, device="cpu", dtype=torch.int32).reshape(-1)
+    parts = [i32(v) for v in (req_q_start, req_slot, req_pos0, tile_req, tile_q0)]
+    lists = torch.cat(parts)
+    waits = dev.index != torch.cuda.current_device() or torch.cuda.is_current_stream_capturing()
+    lists = lists.to(dev) if waits else lists.pin_memory().to(dev, non_blocking=True)
+    t_qs, t_slot, t_pos0, t_treq, t_tq0 = lists.split([p.numel() for p in parts])
+    # rows that no request owns are zeros
+    starts = parts[0].tolist()[:len(req_slot) + 1]
+    owned = bool(starts) and starts[0] == 0 and starts[-1] == T and all(x <= y for x, y in zip(starts, starts[1:]))
+    out = (torch.empty if owned else torch.zeros)(T, nq * d, device=dev, dtype=torch.bfloat16)
+    out_lo = torch.empty_like(out) if owned else torch.zeros_like(out)
     N.check(N.load().ft_attn_prefill(N.ptr(q), N.ptr(kv_layer), N.ptr(page_table), page_table.shape[1],
                                      N.ptr(t_qs), N.ptr(t_slot), N.ptr(t_pos0), N.ptr(t_treq), N.ptr(t_tq0),
                                      len(tile_req), N.ptr(out), N.ptr(out_lo), nq, nkv, d, T if tensor_cores else 0,

@@ -9,6 +9,7 @@ leave every kernel as bf16 hi + lo planes; hi + lo must match the fp32 reference
 """
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -490,6 +491,28 @@ def test_attn_prefill(K, nq, nkv, d, reqs):
         ref = O.attention(q[q_start[r]:q_start[r + 1]].float(), ks[r].float(), vs[r].float(), p0)
         got = out[q_start[r]:q_start[r + 1]]
         assert rel_err(got, ref) < 2e-3, (r, rel_err(got, ref))
+
+
+@pytest.mark.parametrize("before,after", [(0, 0), (3, 0), (0, 5), (2, 66)])
+@pytest.mark.parametrize("as_given", [list, np.array, torch.tensor])
+def test_attn_prefill_rows_without_a_request(K, before, after, as_given):
+    """Rows before the first request and behind the last one are zeros, whatever the memory held; lists, arrays and tensors of places."""
+    nq, nkv, d, reqs = 8, 2, 64, [(0, 70), (9, 0), (33, 64)]
+    g = torch.Generator(device=DEV).manual_seed(before * 7 + after)
+    kv, pt, ks, vs = build_paged_kv(K, [max(1, p + n) for p, n in reqs], nkv, d, g)
+    q_start = [before]
+    for _, n in reqs:
+        q_start.append(q_start[-1] + n)
+    T = q_start[-1] + after
+    q = torch.randn(T, nq, d, device=DEV, generator=g).half()
+    dirty = [torch.full((T, nq * d), float("nan"), device=DEV, dtype=torch.bfloat16) for _ in range(4)]
+    del dirty
+    out = hilo(*K.attn_prefill(q, kv, pt, as_given(q_start), as_given(list(range(len(reqs)))), as_given([p for p, _ in reqs])))
+    assert torch.equal(out[:before], torch.zeros_like(out[:before])) and torch.equal(out[q_start[-1]:], torch.zeros_like(out[q_start[-1]:]))
+    for r, (p0, n) in enumerate(reqs):
+        if n:
+            ref = O.attention(q[q_start[r]:q_start[r + 1]].float(), ks[r].float(), vs[r].float(), p0)
+            assert rel_err(out[q_start[r]:q_start[r + 1]], ref) < 2e-3
 
 
 @pytest.mark.parametrize("nq,nkv,d", [(8, 2, 64), (6, 2, 64), (32, 8, 64), (32, 8, 128), (24, 8, 128), (3, 1, 128)])
