@@ -542,7 +542,10 @@ int launch_window_attention(const WindowArgs& a, int T, int n_single, const Wind
     const bool tiled = tm.n_tiles > 0 && (a.dim & 3) == 0 && (a.vdim & 3) == 0 && grp <= WT_ROWS && a.vdim <= 256 && tsm <= 220 * 1024 &&
                        (a.v_in_key < 0 || (a.v_in_key & 3) == 0);
     int rows_each = T;                                 // rows of the one-CTA-per-(token, head) kernel
-    if (tiled) {
+    if (tm.n_tiles > 0 && window_tc_ok(a)) {
+        rows_each = n_single;
+        if (int r = launch_window_tc(a, tm, stream)) return r;
+    } else if (tiled) {
         rows_each = n_single;
         const int QT = WT_ROWS / grp, subs = (64 + QT - 1) / QT;
         dim3 grid(tm.n_tiles * subs, a.G);

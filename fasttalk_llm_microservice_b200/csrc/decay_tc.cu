@@ -33,7 +33,6 @@ constexpr int DR_LDQ = 132, DR_LDO = 68;                 // floats between rows 
 constexpr int DR_COL_Q = 0, DR_COL_U = 0, DR_COL_S = 192, DR_COL_P = 192, DR_COL_ST = 320, DR_COL_O = 384;
 constexpr unsigned DR_BIG_IN = (127u + 36) << 23, DR_BIG_STATE = (127u + 80) << 23, DR_DECAY = 0x3f820000u;      // 2^36, 2^80, 1 + 2^-6
 
-__device__ __forceinline__ unsigned warp_umax(unsigned v) { return __reduce_max_sync(0xffffffffu, v); }
 __device__ __forceinline__ void cp16_zfill(float* dst, const float* src, int bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
 }
@@ -69,23 +68,6 @@ __device__ __forceinline__ void hold(f32x2* x) {
 #pragma unroll
     for (int i = 0; i < N; ++i) asm volatile("" : "+l"(x[i]));
 }
-// 32 lanes x 8 columns
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
-                 "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
-// 16 numbers of a row as three slices, 64 columns apart
-__device__ __forceinline__ void slices_to_tmem(f32x2* x, float inv, uint32_t at) {
-    uint32_t w[8];
-    slice_first<8>(x, inv, w);
-    tmem_st8(at, w);
-    slice_next<8>(x, w);
-    tmem_st8(at + 64, w);
-    slice_last<8>(x, w);
-    tmem_st8(at + 128, w);
-}
-
 template <bool VEC, int DB>
 __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, int* err) {
     extern __shared__ uint8_t dr_raw[];
@@ -360,7 +342,7 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
                 f32x2 qx[8];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) *reinterpret_cast<ulonglong2*>(qx + 2 * i) = *reinterpret_cast<const ulonglong2*>(qr + 16 * x + 4 * i);
-                slices_to_tmem(qx, slice_inv(q_top), lanes + DR_COL_Q + part * 16 + 8 * x);
+                slices_to_tmem<64>(qx, slice_inv(q_top), lanes + DR_COL_Q + part * 16 + 8 * x);
             }
             __syncthreads();                             // the queries have been read: the keys take their place
             hold<8 * DB>(kx[0]);
@@ -481,7 +463,7 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
             for (int x = 0; x < 2; ++x) {
                 const uint32_t at = lanes + DR_COL_P + part * 16 + 8 * x;
                 if (part <= (warp & 3)) {
-                    slices_to_tmem(sc + 8 * x, slice_inv(p_top), at);
+                    slices_to_tmem<64>(sc + 8 * x, slice_inv(p_top), at);
                 } else {
                     const uint32_t zero[8] = {};
 #pragma unroll

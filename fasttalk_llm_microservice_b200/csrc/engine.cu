@@ -796,6 +796,7 @@ static int run_branch(Engine* e, const Batch& b, const LayeredLayer& ll, int k, 
             if (rows > 0) FT_TRY(launch_paged16_mma(p, rows, st));
             launched(1 + (tc ? 1 : 0) + (rows > 0 ? 2 : 0));
         } else {
+            a.err = e->h_kernel_err;
             FT_TRY(launch_window_attention(a, T, b.n_decode, tm, st));
             launched(b.n_tiles > 0 && b.n_decode > 0 ? 3 : 2);
         }

@@ -322,6 +322,7 @@ struct WindowArgs {
     int ldg = 0;
     float temp_coef = 0.f;                        // q *= 1 + temp_coef * ln(1 + floor((p + 1) / temp_every)); temp_every 0: no
     int temp_every = 0;
+    int* err = nullptr;                           // set where a wait inside a kernel ran out
 };
 // The step's prompt portions as the batch builder lists them: 64-token query tiles (request, first token), and per request
 // its first row in the step, its page-table row and the position of its first token.
@@ -331,6 +332,8 @@ struct WindowTiles {
 };
 // n_single: how many of the step's first rows are single tokens of running sequences (they precede the portions)
 int launch_window_attention(const WindowArgs& a, int T, int n_single, const WindowTiles& tm, cudaStream_t stream);
+bool window_tc_ok(const WindowArgs& a);           // window_tc.cu: portions on the tensor cores
+int launch_window_tc(const WindowArgs& a, const WindowTiles& tm, cudaStream_t stream);
 
 // ---- paged16.cu / paged16_tc.cu: softmax attention over a paged bf16 cache (the serving form of latent attention and of window
 // attention without a window).  A page holds, per key head, `blocks` blocks of [64 tokens][64 columns] whose 128-byte rows have

@@ -16,6 +16,7 @@ namespace ft {
 constexpr int kSliceBits = 10;
 constexpr float kSliceMagic = 12582912.f;               // 1.5 * 2^23: x + magic - magic is x rounded to a whole number
 
+__device__ __forceinline__ unsigned warp_umax(unsigned v) { return __reduce_max_sync(0xffffffffu, v); }
 // Bit patterns of |x| order as the numbers do, infinities and NaN above all of them.
 __device__ __forceinline__ unsigned abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 constexpr int kSliceMinExp = -100;                      // rows below 2^-100 share its unit
@@ -102,6 +103,23 @@ __device__ __forceinline__ void slice8(f32x2* x, float inv, uint8_t* at, int pla
     *reinterpret_cast<uint4*>(at + plane) = make_uint4(w[0], w[1], w[2], w[3]);
     slice_last<4>(x, w);
     *reinterpret_cast<uint4*>(at + 2 * plane) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+// 32 lanes x 8 columns
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+                 "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+// 16 numbers of a row as three slices, PITCH columns apart
+template <int PITCH>
+__device__ __forceinline__ void slices_to_tmem(f32x2* x, float inv, uint32_t at) {
+    uint32_t w[8];
+    slice_first<8>(x, inv, w);
+    tmem_st8(at, w);
+    slice_next<8>(x, w);
+    tmem_st8(at + PITCH, w);
+    slice_last<8>(x, w);
+    tmem_st8(at + 2 * PITCH, w);
 }
 // The products beside first x first, smallest first: (slice of A, slice of B)
 constexpr int kSlicePairs = 5;

@@ -132,6 +132,51 @@ def test_whole_prompt_matches_oracle(layers):
         eng.close()
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(5, 5, 64, 64), (6, 2, 128, 96), (8, 1, 20, 128), (4, 2, 100, 64), (7, 1, 64, 4)])
+@pytest.mark.parametrize("size,keep_first", [(64, 0), (65, 70), (200, 3)])
+def test_attention_of_portions_by_group_and_head_size(heads, kv_heads, dim, vdim, size, keep_first):
+    """128 rows of a run: groups of 1, 2, 3, 7 and 8 query heads (64 to 16 tokens, rows left over), heads in one and two blocks of 64 with padding,
+    windows of a whole tile of keys and one more, kept tokens over several tiles; portions that start inside tiles."""
+    spec, w = make([layer(attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, size=size, keep_first=keep_first, scale=1.3 * dim ** -0.5,
+                                    rows=24, bias_max=150))], seed=heads + dim)
+    eng = engine(spec, w)
+    try:
+        toks = tokens_of(spec, 310, 4)
+        ref = oracle_logits(spec, w, toks)
+        assert rel(eng.feed([("whole", toks, list(range(len(toks))))]), ref) < TOL
+        assert rel(feed_cut(eng, "cut", toks, [63, 1, 100, 2, 144]), ref) < TOL
+    finally:
+        eng.close()
+
+
+def test_attention_of_portions_with_numbers_beyond_the_slices():
+    """Values of 1e13 and more (plain fp32 rows) against the oracle; a token without a finite number is felt by the same positions as when the
+    tokens come one by one, and changes nothing before it or beyond the window's reach."""
+    layers = [layer(attention(heads=6, kv_heads=2, dim=32, vdim=32, size=24, keep_first=0, v_mix=False))]
+
+    def huge(w):
+        w["embed"][7] *= 1e13
+    spec, w = make(layers, seed=8, tweak=huge)
+    toks = [t if t not in (7, 8) else 9 for t in tokens_of(spec, 200, 2)]
+    toks[90] = 7
+    eng = engine(spec, w)
+    try:
+        assert rel(eng.feed([("s", toks, list(range(200)))]), oracle_logits(spec, w, toks)) < TOL
+    finally:
+        eng.close()
+    w["embed"][8] = float("inf")
+    toks[90] = 8
+    eng = engine(spec, w)
+    try:
+        whole = eng.feed([("s", toks, list(range(200)))])
+        single = feed_cut(eng, "t", toks, [1])
+        fin = np.isfinite(single).all(1)
+        assert fin[:90].all() and not fin[90] and fin[140:].all() and (np.isfinite(whole).all(1) == fin).all()
+        assert rel(whole[fin], single[fin]) < TOL
+    finally:
+        eng.close()
+
+
 @pytest.mark.parametrize("taps", [1, 2, 6])
 def test_other_sizes_and_taps(taps):
     layers = [layer(attention(heads=10, kv_heads=5, dim=12, vdim=14, size=33, keep_first=2, scale=0.5, rows=12, bias_max=17.5), dense(ff=50)),
