@@ -11,8 +11,10 @@
 // The draw walks the kept set in index order.
 //
 // What bounds it: a chain of short passes over data in shared memory and of cluster barriers (3 per radix pass).  One CTA per row
-// with every pass reading the row again took 153 us for one row of 128256 and 203 us for 64 (greedy and sampled rows mixed);
-// the cluster takes 26 and 73 us.
+// with every pass reading the row again took 153 us for one row of 128256 and 203 us for 64 (greedy and sampled rows mixed); the
+// cluster took 28 and 69 us on the device with a pass of its own for every step, and takes 19 and 50 with the first histogram filled
+// where the weights are formed, two additions an element, a bin's reads from the other CTAs spread over all warps, and walks whose
+// sums are one addition a step.
 #include "common.cuh"
 #include "ft_internal.h"
 
@@ -32,7 +34,9 @@ struct SampleSmem {
     float val[SAMPLE_MAX_CTAS], above, target;
     int idx[SAMPLE_MAX_CTAS];
     int bin, single;
-    unsigned long long seed;                                          // the row's own settings, read while its logits are
+    unsigned bins_c[SAMPLE_THREADS];                                  // this CTA's bins over the cluster, by parts of it: elements, offsets
+    unsigned long long bins_o[SAMPLE_THREADS];
+    float rnd;                                                        // the row's own number in [0, 1) and settings, read while its logits are
     int top_k;
     float top_p;
     float warp_f[SAMPLE_WARPS];
@@ -84,19 +88,83 @@ struct SampleShare {
     int n, cached;
     float maxv, inv_t;
     __device__ __forceinline__ uint32_t at(int i) const { return i < cached ? key[i] : weight_key(x[i], maxv, inv_t); }
+    // the elements for which `in` holds, four cached ones at a time: mostly none of the four
+    template <class P, class F>
+    __device__ __forceinline__ void each(P&& in, F&& f) const {
+        const int n4 = cached >> 2;
+#pragma unroll 2
+        for (int i = threadIdx.x; i < n4; i += SAMPLE_THREADS) {
+            const uint4 v = reinterpret_cast<const uint4*>(key)[i];
+            if (in(v.x) | in(v.y) | in(v.z) | in(v.w)) {
+                if (in(v.x)) f(v.x);
+                if (in(v.y)) f(v.y);
+                if (in(v.z)) f(v.z);
+                if (in(v.w)) f(v.w);
+            }
+        }
+        for (int i = 4 * n4 + threadIdx.x; i < n; i += SAMPLE_THREADS) {
+            const uint32_t k = at(i);
+            if (in(k)) f(k);
+        }
+    }
 };
+
+// One element in the histograms: its bin's count and, for masses, its offset in the bin.  Shares of up to 16384 elements take two
+// additions: `cnt` holds the count above the sum of the offsets' bits 17 .. 19 (at most 7 * 16384), `lo` that of the other 17.  Longer
+// ones take three, the offset's upper and lower ten bits apart.
+constexpr int SAMPLE_PACKED = 16384;
+constexpr int SAMPLE_SHIFT0 = 20, SAMPLE_BITS0 = 11;      // the first pass's bins
+template <bool MASS>
+__device__ __forceinline__ void count_key(SampleSmem& sm, uint32_t key, int shift, int nb, bool packed) {
+    const uint32_t b = (key >> shift) & (nb - 1), off = key & ((1u << shift) - 1);
+    if (MASS && packed) {
+        atomicAdd(&sm.cnt[b], (1u << 17) | (off >> 17));
+        if (off & 0x1ffffu) atomicAdd(&sm.lo[b], off & 0x1ffffu);
+        return;
+    }
+    atomicAdd(&sm.cnt[b], 1u);
+    if (MASS && (off >> 10)) atomicAdd(&sm.hi[b], off >> 10);
+    if (MASS && (off & 1023u)) atomicAdd(&sm.lo[b], off & 1023u);
+}
+// What a CTA's histograms hold for bin b
+template <bool MASS, int C>
+__device__ __forceinline__ void read_bin(const SampleSmem& sm, int b, int rank, bool packed, unsigned& c, unsigned& hi, unsigned& lo) {
+    c = peer_get<C>(&sm.cnt[b], rank);
+    hi = MASS && !packed ? peer_get<C>(&sm.hi[b], rank) : 0u;
+    lo = MASS ? peer_get<C>(&sm.lo[b], rank) : 0u;
+}
+template <bool MASS>
+__device__ __forceinline__ void add_bin(unsigned pc, unsigned ph, unsigned pl, bool packed, unsigned& c, unsigned long long& off) {
+    if (MASS && packed) {
+        c += pc >> 17;
+        off += ((unsigned long long)(pc & 0x1ffffu) << 17) + pl;
+    } else {
+        c += pc;
+        off += ((unsigned long long)ph << 10) + pl;
+    }
+}
 
 // Adds the n lanes' values to acc one by one from the last lane down and stops at the first that would reach the target; -1: none does.
 __device__ __forceinline__ int walk_down(float v, int n, float& acc, float target) {
     for (int top = n - 8; top >= 0; top -= 8) {
-        float x[8];
+        float x[9];                                  // the sums in order first: one addition a step, the comparisons beside them
+        x[0] = acc;
+        unsigned hit = 0;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) x[u] = __shfl_sync(0xffffffffu, v, top + 7 - u);
+        for (int u = 0; u < 8; ++u) x[u + 1] = __shfl_sync(0xffffffffu, v, top + 7 - u);
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            if (acc + x[u] >= target) return top + 7 - u;
-            acc += x[u];
+            x[u + 1] += x[u];
+            if (x[u + 1] >= target) hit |= 1u << u;
         }
+        if (hit) {
+            const int first = __ffs(hit) - 1;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (u == first) acc = x[u];
+            return top + 7 - first;
+        }
+        acc = x[8];
     }
     return -1;
 }
@@ -105,31 +173,43 @@ __device__ __forceinline__ int walk_down(float v, int n, float& acc, float targe
 // weight is the sum of the elements, and the target `part` of the sum of all elements with key >= min_key; otherwise the weight is
 // their number and the target `part` itself.  The bins are walked from the top in 32-bit sums, 64 at a time and then one by one,
 // whatever C is.  Every thread of the cluster calls; the result is the same for all.
+// counted: the first pass's histograms of this CTA are there (min_key 0).
 template <bool MASS, int C>
-__device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, float part, int rank, SampleSmem& sm) {
-    const int shifts[3] = {20, 9, 0}, bits[3] = {11, 11, 9};
+__device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, float part, int rank, SampleSmem& sm, bool counted, bool packed) {
+    const int shifts[3] = {SAMPLE_SHIFT0, 9, 0}, bits[3] = {SAMPLE_BITS0, 11, 9};
     constexpr int groups = SAMPLE_GROUPS / C;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;      // this CTA's groups of 64 bins
     uint32_t prefix = 0, mask = 0;
     float above = 0.f, target = part;
     for (int lvl = 0; lvl < 3; ++lvl) {
         const int shift = shifts[lvl], nb = 1 << bits[lvl];
-        for (int i = threadIdx.x; i < SAMPLE_BINS; i += SAMPLE_THREADS) {
-            sm.cnt[i] = 0;
-            if (MASS) sm.hi[i] = sm.lo[i] = 0;
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < s.n; i += SAMPLE_THREADS) {
-            const uint32_t key = s.at(i);
-            if (key >= min_key && (key & mask) == prefix) {
-                const uint32_t b = (key >> shift) & (nb - 1), off = key & ((1u << shift) - 1);
-                atomicAdd(&sm.cnt[b], 1u);
-                if (MASS && (off >> 10)) atomicAdd(&sm.hi[b], off >> 10);
-                if (MASS && (off & 1023u)) atomicAdd(&sm.lo[b], off & 1023u);
+        if (!counted || lvl > 0) {
+            for (int i = threadIdx.x; i < SAMPLE_BINS; i += SAMPLE_THREADS) {
+                sm.cnt[i] = 0;
+                if (MASS) sm.hi[i] = sm.lo[i] = 0;
             }
+            __syncthreads();
+            s.each([&](uint32_t key) { return key >= min_key && (key & mask) == prefix; },
+                   [&](uint32_t key) { count_key<MASS>(sm, key, shift, nb, packed); });
         }
         row_sync<C>();                          // every histogram of the cluster is complete
-        // warp w sums groups w and w + 16 of this CTA over the cluster, two bins of each per lane
+        // The CTA's bins over the cluster: from four CTAs on a thread adds up one bin of four of them (whole numbers: in any order), so that
+        // all warps have their reads on the way together; then warp w sums groups w and w + 16, two bins of each per lane.
+        constexpr bool SPREAD = C >= 4;
+        constexpr int mine = SAMPLE_BINS / C;
+        if (SPREAD) {
+            const int b = rank * mine + threadIdx.x % mine, p0 = threadIdx.x / mine * 4;
+            unsigned pc[4], ph[4], pl[4];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) read_bin<MASS, C>(sm, b, p0 + p, packed, pc[p], ph[p], pl[p]);
+            unsigned c = 0;
+            unsigned long long off = 0;
+#pragma unroll
+            for (int p = 0; p < 4; ++p) add_bin<MASS>(pc[p], ph[p], pl[p], packed, c, off);
+            sm.bins_c[threadIdx.x] = c;
+            sm.bins_o[threadIdx.x] = off;
+            __syncthreads();
+        }
         float wt[2][2];
         unsigned ct[2][2];
 #pragma unroll
@@ -139,20 +219,21 @@ __device__ uint32_t radix_threshold(const SampleShare& s, uint32_t min_key, floa
             double all = 0.0;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                const int b = (rank * groups + g) * 64 + 32 * j + l;
-                unsigned pc[C], ph[C], pl[C];        // all reads in flight before the first sum
-#pragma unroll
-                for (int p = 0; p < C; ++p) {
-                    pc[p] = peer_get<C>(&sm.cnt[b], p);
-                    ph[p] = MASS ? peer_get<C>(&sm.hi[b], p) : 0u;
-                    pl[p] = MASS ? peer_get<C>(&sm.lo[b], p) : 0u;
-                }
+                const int at = g * 64 + 32 * j + l, b = rank * mine + at;
                 unsigned c = 0;
                 unsigned long long off = 0;
+                if (SPREAD) {
 #pragma unroll
-                for (int p = 0; p < C; ++p) {
-                    c += pc[p];
-                    off += ((unsigned long long)ph[p] << 10) + pl[p];
+                    for (int p = 0; p < C / 4; ++p) {
+                        c += sm.bins_c[p * mine + at];
+                        off += sm.bins_o[p * mine + at];
+                    }
+                } else {
+                    unsigned pc[C], ph[C], pl[C];        // all reads in flight before the first sum
+#pragma unroll
+                    for (int p = 0; p < C; ++p) read_bin<MASS, C>(sm, b, p, packed, pc[p], ph[p], pl[p]);
+#pragma unroll
+                    for (int p = 0; p < C; ++p) add_bin<MASS>(pc[p], ph[p], pl[p], packed, c, off);
                 }
                 double m = (double)c;
                 if (MASS && c) {
@@ -239,10 +320,13 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
     const bool greedy = temp <= 1e-6f;
     s.cached = greedy ? 0 : min(s.n, cache);
     if (!greedy && threadIdx.x == SAMPLE_THREADS - 1) {
-        sm.seed = seeds ? seeds[b] : 0x1234ull + b;
+        sm.rnd = (float)(splitmix64(seeds ? seeds[b] : 0x1234ull + b) >> 40) * (1.0f / 16777216.0f);
         sm.top_k = top_k ? top_k[b] : 0;
         sm.top_p = top_p ? top_p[b] : 1.f;
     }
+
+    if (!greedy)
+        for (int i = threadIdx.x; i < SAMPLE_BINS; i += SAMPLE_THREADS) sm.cnt[i] = sm.hi[i] = sm.lo[i] = 0;
 
     // ---- max (+ argmax, lowest index on ties); the logits of a sampled row stay in shared memory
     float best = -INFINITY;
@@ -291,12 +375,18 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
     if (l == 0) { sm.warp_f[w] = best; sm.warp_i[w] = best_i; }
     __syncthreads();
     if (C > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // every CTA of the cluster has started
-    if (threadIdx.x == 0) {
-        for (int i = 1; i < SAMPLE_WARPS; ++i)
-            if (sm.warp_f[i] > best || (sm.warp_f[i] == best && sm.warp_i[i] < best_i)) { best = sm.warp_f[i]; best_i = sm.warp_i[i]; }
-        for (int p = 0; p < C; ++p) {
-            peer_put<C>(&sm.val[rank], p, best);
-            peer_put<C>(&sm.idx[rank], p, best_i);
+    if (w == 0) {                                    // lane p tells CTA p
+        best = sm.warp_f[l & (SAMPLE_WARPS - 1)];
+        best_i = sm.warp_i[l & (SAMPLE_WARPS - 1)];
+#pragma unroll
+        for (int o = SAMPLE_WARPS / 2; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
+            if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
+        }
+        if (l < C) {
+            peer_put<C>(&sm.val[rank], l, best);
+            peer_put<C>(&sm.idx[rank], l, best_i);
         }
     }
     row_sync<C>();
@@ -326,12 +416,12 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
             const int qhi = min((q + 1) * part, s.n);
             float mine = 0.f;
             int i = q * part + l;
-            for (; i + 7 * 32 < qhi; i += 8 * 32) {       // eight reads in flight, added one by one
-                float e[8];
+            for (; i + 15 * 32 < qhi; i += 16 * 32) {     // sixteen reads in flight, added one by one
+                float e[16];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) e[u] = weight(i + u * 32);
+                for (int u = 0; u < 16; ++u) e[u] = weight(i + u * 32);
 #pragma unroll
-                for (int u = 0; u < 8; ++u) mine += e[u];
+                for (int u = 0; u < 16; ++u) mine += e[u];
             }
             for (; i < qhi; i += 32) mine += weight(i);
             mine = warp_sum(mine);
@@ -344,6 +434,10 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
         const uint32_t key = s.at(i);
         return key >= thr ? __uint_as_float(key) : 0.f;
     };
+    auto kept_here = [&](int i) {                    // of a share that is cached whole
+        const uint32_t key = keys[i];
+        return key >= thr ? __uint_as_float(key) : 0.f;
+    };
     if (C <= 2 && !(k > 0 && k < V) && !(p < 1.f)) {
         // a row without filters whose runs occupy all warps is summed while its weights are formed
         sum_runs([&](int i) {
@@ -352,14 +446,34 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
             return __uint_as_float(key);
         });
     } else {
-        for (int i = threadIdx.x; i < s.cached; i += SAMPLE_THREADS) keys[i] = weight_key(__uint_as_float(keys[i]), maxv, s.inv_t);
+        // the weights, and with them the histograms of the first pass of the first filter
+        const bool by_count = k > 0 && k < V, by_mass = p < 1.f && p > 0.f, packed = span <= SAMPLE_PACKED;
+        auto form = [&](auto&& add) {
+            const int n4 = s.cached >> 2;
+            auto key_of = [&](uint32_t bits) {
+                const uint32_t key = weight_key(__uint_as_float(bits), maxv, s.inv_t);
+                add(key);
+                return key;
+            };
+#pragma unroll 2
+            for (int i = threadIdx.x; i < n4; i += SAMPLE_THREADS) {
+                const uint4 v = reinterpret_cast<const uint4*>(keys)[i];
+                reinterpret_cast<uint4*>(keys)[i] = make_uint4(key_of(v.x), key_of(v.y), key_of(v.z), key_of(v.w));
+            }
+            for (int i = 4 * n4 + threadIdx.x; i < s.cached; i += SAMPLE_THREADS) keys[i] = key_of(keys[i]);
+            for (int i = s.cached + threadIdx.x; i < s.n; i += SAMPLE_THREADS) add(weight_key(x[i], maxv, s.inv_t));
+        };
+        if (by_count) form([&](uint32_t key) { count_key<false>(sm, key, SAMPLE_SHIFT0, 1 << SAMPLE_BITS0, packed); });
+        else if (by_mass) form([&](uint32_t key) { count_key<true>(sm, key, SAMPLE_SHIFT0, 1 << SAMPLE_BITS0, packed); });
+        else form([](uint32_t) {});
         __syncthreads();
-        if (k > 0 && k < V) thr = radix_threshold<false, C>(s, 0u, (float)k, rank, sm);
+        if (by_count) thr = radix_threshold<false, C>(s, 0u, (float)k, rank, sm, true, packed);
         if (p < 1.f) {
-            if (p > 0.f) thr = radix_threshold<true, C>(s, thr, p, rank, sm);
+            if (p > 0.f) thr = radix_threshold<true, C>(s, thr, p, rank, sm, !by_count, packed);
             else thr = 0xffffffffu;                  // an empty nucleus: the most likely token
         }
-        sum_runs(kept);
+        if (s.cached == s.n) sum_runs(kept_here);
+        else sum_runs(kept);
     }
     row_sync<C>();                              // nothing is read from or written to another CTA after this
     // a run's sum per lane; the sum of all runs in order, of which a lane keeps the part before its own
@@ -379,7 +493,7 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
         if (rank == 0 && threadIdx.x == 0) out_tokens[b] = most_likely();
         return;
     }
-    const float u = (float)(splitmix64(sm.seed) >> 40) * (1.0f / 16777216.0f) * tot;      // [0, tot)
+    const float u = sm.rnd * tot;               // [0, tot)
     const unsigned past = __ballot_sync(0xffffffffu, ahead + run_sum > u);
     int in = past ? __ffs(past) - 1 : SAMPLE_PARTS - 1;
     const float before = past ? __shfl_sync(0xffffffffu, ahead, in) : tot;
@@ -391,9 +505,7 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
     const int wlo = in % runs * part, whi = min(wlo + part, s.n);
     float* bsum = reinterpret_cast<float*>(sm.cnt);
     float* bmax = reinterpret_cast<float*>(sm.hi);
-    auto scan = [&](int b0, float& e) {
-        const int i = b0 + l;
-        e = i < whi ? kept(i) : 0.f;
+    auto scan = [&](float e) {
         float inc = e;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -402,40 +514,56 @@ sample_kernel(const float* __restrict__ logits, int V, int span, int cache, cons
         }
         return inc;
     };
+    auto element = [&](int i) { return i < whi ? kept(i) : 0.f; };
     int last_kept = -1;
     float run = 0.f;
     for (int c0 = wlo; c0 < whi; c0 += 32 * SAMPLE_BINS) {      // (one round, except for rows of more than two million)
         const int blocks = (min(c0 + 32 * SAMPLE_BINS, whi) - c0 + 31) / 32;
         __syncthreads();
-        for (int q = w; q < blocks; q += SAMPLE_WARPS) {
-            float e;
-            const float inc = scan(c0 + 32 * q, e);
-            const float most = warp_max(e > 0.f ? inc : -1.f);
-            if (l == 31) { bsum[q] = inc; bmax[q] = most; }
+        for (int q0 = w; q0 < (blocks + 7 & ~7); q0 += 4 * SAMPLE_WARPS) {      // four blocks at a time; those behind the last hold nothing
+            float e[4], inc[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) e[x] = element(c0 + 32 * (q0 + x * SAMPLE_WARPS) + l);
+#pragma unroll
+            for (int x = 0; x < 4; ++x) inc[x] = scan(e[x]);
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int q = q0 + x * SAMPLE_WARPS;
+                const unsigned most = __reduce_max_sync(0xffffffffu, e[x] > 0.f ? __float_as_uint(inc[x]) : 0u);      // (sums of kept ones are above zero)
+                if (l == 31 && q < SAMPLE_BINS) { bsum[q] = inc[x]; bmax[q] = most ? __uint_as_float(most) : -1.f; }
+            }
         }
         __syncthreads();
         int q = blocks;
         for (int q8 = 0; q8 < blocks && q == blocks; q8 += 8) {      // every thread walks the same way, eight blocks read at a time
-            float bs[8], bm[8];
+            float before[9], bm[8];
+            unsigned hit = 0, any = 0;
+            before[0] = run;
 #pragma unroll
-            for (int x = 0; x < 8; ++x) { bs[x] = bsum[q8 + x]; bm[x] = bmax[q8 + x]; }
+            for (int x = 0; x < 8; ++x) { before[x + 1] = bsum[q8 + x]; bm[x] = bmax[q8 + x]; }
 #pragma unroll
-            for (int x = 0; x < 8; ++x)
-                if (q8 + x < blocks && q == blocks) {
-                    if (bm[x] >= 0.f && run + bm[x] > need) q = q8 + x;
-                    else {
-                        if (bm[x] >= 0.f) last_kept = q8 + x;
-                        run += bs[x];
-                    }
-                }
+            for (int x = 0; x < 8; ++x) {
+                before[x + 1] += before[x];
+                if (bm[x] >= 0.f && before[x] + bm[x] > need) hit |= 1u << x;
+                if (bm[x] >= 0.f) any |= 1u << x;
+            }
+            if (hit) {
+                const int first = __ffs(hit) - 1;
+                q = q8 + first;
+#pragma unroll
+                for (int x = 0; x < 8; ++x)
+                    if (x == first) run = before[x];
+            } else {
+                if (any) last_kept = q8 + 31 - __clz(any);
+                run = before[8];
+            }
         }
         if (q < blocks || last_kept >= 0) {
             if (w != 0) {
                 if (q < blocks) return;
             } else {
-                float e;
                 const int at = c0 + 32 * (q < blocks ? q : last_kept);
-                const float inc = scan(at, e);
+                const float e = element(at + l), inc = scan(e);
                 const unsigned hit = __ballot_sync(0xffffffffu, e > 0.f && run + inc > need), any = __ballot_sync(0xffffffffu, e > 0.f);
                 if (q < blocks) {
                     if (l == 0) out_tokens[b] = lo + at + __ffs(hit) - 1;

@@ -677,6 +677,23 @@ def test_sample_against_the_sorted_row(K, B, V):
             assert float(cum[t] - prob[t]) - slack <= u <= float(cum[t]) + slack, (temp, k, p, b)
 
 
+@pytest.mark.parametrize("V", [4 * 16384, 8 * 16384, 8 * 16384 + 32, 8 * 16384 + 37])
+def test_sample_rows_whose_weights_share_a_bin(K, V):
+    """Shares of 16384 elements, the most whose counts and offsets are added up together, and longer ones: every weight falls into the first
+    histogram's bin below one, next to its upper end, so that no sum could be larger.  Same oracle as above."""
+    g = torch.Generator(device=DEV).manual_seed(V)
+    logits = 0.02 * torch.rand(2, V, device=DEV, generator=g)
+    for k, p in [(0, 0.5), (0, 0.97), (V // 3, 0.6)]:
+        seeds = torch.randint(1 << 62, (2,), device=DEV, generator=g, dtype=torch.int64)
+        tok = K.sample(logits, torch.ones(2, device=DEV), torch.full((2,), k, device=DEV, dtype=torch.int32), torch.full((2,), p, device=DEV), seeds)
+        for b in range(2):
+            prob = O.sampling_support(logits[b].cpu(), 1.0, k, p)
+            cum, t, u = torch.cumsum(prob, 0), int(tok[b]), _draw_point(seeds[b])
+            # logits of 24 bits tie at the edge of the kept set: twenty of a row's more or less
+            slack = 1e-5 + 20 * float(prob[prob > 0].min())
+            assert float(cum[t] - prob[t]) - slack <= u <= float(cum[t]) + slack, (k, p, b)
+
+
 @pytest.mark.parametrize("V", [1000, 4097, 32768, 50257, 128256])
 def test_sample_token_does_not_depend_on_the_batch(K, V):
     """A row's share of CTAs (eight to one) and of cached weights follows the batch and the row's length; its token does not."""
