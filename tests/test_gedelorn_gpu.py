@@ -484,6 +484,20 @@ def test_served_through_the_handler(tmp_path, monkeypatch):
         runner.engine.close()
 
 
+@pytest.mark.parametrize("width,ff,experts,top,sessions", [(520, 512, 8, 3, 2), (520, 1032, 7, 7, 1), (1032, 2056, 3, 2, 7), (3208, 1024, 5, 1, 4)])
+def test_experts_of_a_few_pairs(width, ff, experts, top, sessions):
+    """Pairs that go past weights in shared memory: experts without a pair, with one, and with two groups of four rows; sixteen and eight weight rows a CTA."""
+    spec, w = make([layer(memory(), moe(ff=ff, experts=experts, top=top, shared=0))], width=width, vocab=90, seed=ff)
+    eng = engine(spec, w, max_batch=8, max_sessions=8)
+    try:
+        toks = [tokens_of(spec, 3, 50 + i) for i in range(sessions)]
+        got = np.stack([eng.feed([(i, [t[j]], [0]) for i, t in enumerate(toks)]) for j in range(3)], 1)
+        for i, t in enumerate(toks):
+            assert rel(got[i], oracle_logits(spec, w, t)) < TOL
+    finally:
+        eng.close()
+
+
 # ------------------------------------------------------------------------------------------------ the rule alone
 @pytest.mark.parametrize("lanes", [0, 4, 8, 16, 32])
 @pytest.mark.parametrize("heads,qk_heads,dim,vd", [(3, 3, 20, 9), (4, 2, 64, 33), (2, 1, 128, 16), (1, 1, 7, 70)])

@@ -177,6 +177,21 @@ def test_attention_of_portions_with_numbers_beyond_the_slices():
         eng.close()
 
 
+@pytest.mark.parametrize("width,ff,sessions", [(520, 2056, 1), (1032, 528, 3), (1024, 1024, 4), (2048, 520, 5), (3208, 512, 7), (520, 6400, 2), (520, 512, 8), (520, 512, 9)])
+def test_projections_of_a_few_rows(width, ff, sessions):
+    """One to eight rows (and one more) against long weight rows: sixteen and eight weight rows a CTA, steps of 256 channels with and without a rest, outputs
+    that fill no CTA, gate and up side by side, a second group of rows."""
+    spec, w = make([layer(attention(heads=2, kv_heads=1, dim=16, vdim=12), dense(ff=ff))], width=width, vocab=333, seed=ff)
+    eng = engine(spec, w, max_batch=9, max_sessions=9)
+    try:
+        toks = [tokens_of(spec, 4, 30 + i) for i in range(sessions)]
+        got = np.stack([eng.feed([(i, [t[j]], [0]) for i, t in enumerate(toks)]) for j in range(4)], 1)
+        for i, t in enumerate(toks):
+            assert rel(got[i], oracle_logits(spec, w, t)) < TOL
+    finally:
+        eng.close()
+
+
 @pytest.mark.parametrize("taps", [1, 2, 6])
 def test_other_sizes_and_taps(taps):
     layers = [layer(attention(heads=10, kv_heads=5, dim=12, vdim=14, size=33, keep_first=2, scale=0.5, rows=12, bias_max=17.5), dense(ff=50)),
