@@ -493,6 +493,26 @@ def test_attn_prefill(K, nq, nkv, d, reqs):
         assert rel_err(got, ref) < 2e-3, (r, rel_err(got, ref))
 
 
+@pytest.mark.parametrize("nq,nkv,d", [(4, 1, 64), (3, 1, 64), (4, 1, 128), (6, 2, 128), (32, 8, 64)])
+@pytest.mark.parametrize("reqs", [[(23 * 64 - 20, 19)], [(23 * 64 - 20, 21)], [(24 * 64 - 1, 64)], [(1990, 65), (5, 3)], [(5 * 64, 64), (11 * 64, 1)],
+                                  [(1500, 90), (64, 64), (0, 70), (2300, 1)]])
+def test_attn_prefill_keys_shared_out(K, nq, nkv, d, reqs):
+    """Clusters of two, four and eight CTAs per tile: tiles of keys just below and at three per CTA, a tile of queries across two tiles of keys, requests too short
+    to be shared beside long ones, groups that leave rows over; against the mma.sync kernel and the oracle."""
+    g = torch.Generator(device=DEV).manual_seed(nq * 17 + d + len(reqs))
+    kv, pt, ks, vs = build_paged_kv(K, [p + n for p, n in reqs], nkv, d, g)
+    q_start = [0]
+    for _, n in reqs:
+        q_start.append(q_start[-1] + n)
+    q = (torch.randn(q_start[-1], nq, d, device=DEV, generator=g) * 1.5).half()
+    args = (q, kv, pt, q_start, list(range(len(reqs))), [p for p, _ in reqs])
+    tc, ms = hilo(*K.attn_prefill(*args)), hilo(*K.attn_prefill(*args, tensor_cores=False))
+    assert torch.isfinite(tc).all() and rel_err(tc, ms) < 1.5e-3
+    for r, (p0, n) in enumerate(reqs):
+        ref = O.attention(q[q_start[r]:q_start[r + 1]].float(), ks[r].float(), vs[r].float(), p0)
+        assert rel_err(tc[q_start[r]:q_start[r + 1]], ref) < 2e-3, r
+
+
 @pytest.mark.parametrize("before,after", [(0, 0), (3, 0), (0, 5), (2, 66)])
 @pytest.mark.parametrize("as_given", [list, np.array, torch.tensor])
 def test_attn_prefill_rows_without_a_request(K, before, after, as_given):
