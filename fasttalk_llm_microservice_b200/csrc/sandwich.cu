@@ -95,6 +95,95 @@ __global__ void __launch_bounds__(256) sandwich_joint_kernel(SandwichArgs a) {
     }
 }
 
+// The same with a row's numbers in registers, N passes of them: every load is on the way before the first sum, two barriers in all.
+template <int N>
+__global__ void __launch_bounds__(256) sandwich_joint_regs_kernel(SandwichArgs a) {
+    __shared__ float red[2][8];
+    const int t = blockIdx.x, W = a.W, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool sub = a.y0 || a.y1 || a.top > 0;
+    float* xr = a.x + (size_t)t * W;
+    const __nv_bfloat16* emb = a.tokens ? (const __nv_bfloat16*)a.embed + (size_t)a.tokens[t] * W : nullptr;
+    float x[N][4], y[N][4], w1[N][4], w2[N][4];
+    auto total = [&](float v, float* r) {
+        v = warp_sum(v);
+        if (lane == 0) r[warp] = v;
+        __syncthreads();
+        return ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
+    };
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        const int c = (n * 256 + threadIdx.x) * 4;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[n][i] = y[n][i] = w1[n][i] = w2[n][i] = 0.f;
+        if (c >= W) continue;
+        if (emb) {
+            ld_cols_bf16<4>(x[n], emb + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[n][i] *= a.embed_scale;
+        } else {
+            ld_cols<4>(x[n], xr + c);
+        }
+        if (sub) ld_cols<4>(w1[n], a.post_w + c);
+        if (a.next_w) ld_cols<4>(w2[n], a.next_w + c);
+        float v[4];
+        for (int k = 0; k < a.top; ++k) {
+            ld_cols<4>(v, a.eout + (size_t)a.slot_pos[(size_t)t * a.top + k] * W + c);
+            const float wk = a.wt[(size_t)t * a.top + k];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[n][i] = fmaf(wk, v[i], y[n][i]);
+        }
+        if (a.y0) {
+            ld_cols<4>(v, a.y0 + (size_t)t * W + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[n][i] = fmaf(a.s0, v[i], y[n][i]);
+        }
+        if (a.b0) {
+            ld_cols<4>(v, a.b0 + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[n][i] += v[i];
+        }
+        if (a.y1) {
+            ld_cols<4>(v, a.y1 + (size_t)t * W + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[n][i] = fmaf(a.s1, v[i], y[n][i]);
+        }
+    }
+    if (sub) {
+        float ss = 0.f;
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ss = fmaf(y[n][i], y[n][i], ss);
+        const float r1 = 1.f / sqrtf(total(ss, red[0]) / (float)W + a.eps);
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[n][i] += y[n][i] * r1 * w1[n][i];
+    }
+    float s2 = 0.f;
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        const int c = (n * 256 + threadIdx.x) * 4;
+        if (c >= W) continue;
+        if (sub || emb) st_cols<4>(xr + c, x[n]);
+        if (a.cat_x) put_row<4>(a.cat, a.cat_hi, a.cat_lo, (size_t)t * 2 * W + c, x[n]);
+        if (a.cat_x0) put_row<4>(a.cat, a.cat_hi, a.cat_lo, (size_t)t * 2 * W + W + c, x[n]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s2 = fmaf(x[n][i], x[n][i], s2);
+    }
+    if (!a.next_w) return;
+    const float r2 = 1.f / sqrtf(total(s2, red[1]) / (float)W + a.eps);
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        const int c = (n * 256 + threadIdx.x) * 4;
+        if (c >= W) continue;
+        float v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = x[n][i] * r2 * w2[n][i];
+        put_row<4>(a.hn, a.hi, a.lo, (size_t)t * W + c, v);
+    }
+}
+
 }  // namespace
 
 int launch_sandwich_joint(const SandwichArgs& a, int T, cudaStream_t stream) {
@@ -116,7 +205,13 @@ int launch_sandwich_joint(const SandwichArgs& a, int T, cudaStream_t stream) {
             attr.mark();
         }
     }
-    if (v4) sandwich_joint_kernel<4><<<T, 256, smem, stream>>>(a);
+    // Few rows: up to 4096 columns in registers (16 rows of 2048: 4.1 us, through shared memory 5.4).  Many rows want the other kernel's occupancy
+    // (2313 rows: 18.4 and 16.2 us).
+    const bool regs = v4 && T <= 2 * device_sms();
+    if (regs && a.W <= 1024) sandwich_joint_regs_kernel<1><<<T, 256, 0, stream>>>(a);
+    else if (regs && a.W <= 2048) sandwich_joint_regs_kernel<2><<<T, 256, 0, stream>>>(a);
+    else if (regs && a.W <= 4096) sandwich_joint_regs_kernel<4><<<T, 256, 0, stream>>>(a);
+    else if (v4) sandwich_joint_kernel<4><<<T, 256, smem, stream>>>(a);
     else sandwich_joint_kernel<1><<<T, 256, smem, stream>>>(a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;

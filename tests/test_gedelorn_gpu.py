@@ -484,7 +484,7 @@ def test_served_through_the_handler(tmp_path, monkeypatch):
         runner.engine.close()
 
 
-@pytest.mark.parametrize("width,ff,experts,top,sessions", [(520, 512, 8, 3, 2), (520, 1032, 7, 7, 1), (1032, 2056, 3, 2, 7), (3208, 1024, 5, 1, 4)])
+@pytest.mark.parametrize("width,ff,experts,top,sessions", [(520, 512, 8, 3, 2), (520, 1032, 7, 7, 1), (1032, 2056, 3, 2, 7), (3208, 1024, 5, 1, 4), (4104, 512, 2, 1, 1)])
 def test_experts_of_a_few_pairs(width, ff, experts, top, sessions):
     """Pairs that go past weights in shared memory: experts without a pair, with one, and with two groups of four rows; sixteen and eight weight rows a CTA."""
     spec, w = make([layer(memory(), moe(ff=ff, experts=experts, top=top, shared=0))], width=width, vocab=90, seed=ff)
