@@ -24,9 +24,6 @@
 // warp 1 = TMEM owner + MMA issuer (one elected thread), warps 2..5 = softmax / epilogue of half 0, warps 6..9 of
 // half 1 (warp w may touch TMEM lanes 32 * (w % 4) .. +31), one thread per query row.
 //
-// Few tiles over many keys (a follow-up turn of a few sessions) leave SMs idle, or a second round nearly empty: then a cluster of two to eight
-// CTAs shares a tile's keys out, and each puts D / S columns of the result together from the others' shared memory.
-//
 // What bounds it (in-kernel clock64 timeline + ncu, profiles/r02_attn_prefill_tc.md): per 64-key tile the softmax
 // warps spend ~1200 clk in the exponentials — 64 x 256 of them at the SFU's 16 / clk / SM — and ~1300 clk in the
 // latency-bound rest (TMEM load ~450, row maximum, hand-over); both halves go through these phases in lock step, so
@@ -46,7 +43,6 @@ constexpr int TC_TOK = 64;                   // query tokens per CTA
 constexpr int TC_SUB_BYTES = kKvTile * 128;  // one [64 tokens][64 dims] fp16 sub-slab = 8 KB; also 64 rows of a Q block
 constexpr int TC_QBLK_BYTES = TC_ROWS * 128; // one 128-row x 64-dim block of Q = 16 KB
 constexpr float TC_RESCALE_THRESHOLD = 8.f;  // log2 units
-constexpr int TC_MAX_SPLIT = 8;              // CTAs that share a tile's keys: a portable cluster
 
 template <int D>
 struct TcCfg {
@@ -73,53 +69,6 @@ __device__ __forceinline__ void mbar_wait_sleep(uint64_t* bar, uint32_t parity) 
     while (!mbar_try_wait(bar, parity)) __nanosleep(20);
 }
 
-// A warp's 32 rows (of eight warps' 256) from the sums of S CTAs: this CTA's D / S columns of every row, 16 bytes per lane, the other CTAs' reads of
-// 16 / S groups of rows on their way together (one at a time they took 6 us).
-template <int D, int G, int S>
-__device__ __forceinline__ void merge_rows(float* rows_s, float2* ml_s, int w, int lane, int share, int n_tok, size_t row0, int nq,
-                                           __nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ out_lo) {
-    constexpr int UNITS = D / S / 4, PER = 32 / UNITS, AHEAD = UNITS < 16 / S ? UNITS : 16 / S;      // lanes per row, rows at a time
-    const int mine = w * 32 + lane;
-    float f[S], top = -INFINITY, sum = 0.f;
-    float2 ml[S];
-#pragma unroll
-    for (int p = 0; p < S; ++p) ml[p] = make_float2(peer_ld_at(peer_addr(&ml_s[mine].x, p)), peer_ld_at(peer_addr(&ml_s[mine].y, p)));
-#pragma unroll
-    for (int p = 0; p < S; ++p) top = fmaxf(top, ml[p].x);
-#pragma unroll
-    for (int p = 0; p < S; ++p) {
-        f[p] = ml[p].x == -INFINITY ? 0.f : exp2f(ml[p].x - top);
-        sum = fmaf(f[p], ml[p].y, sum);
-    }
-    const float inv = 1.f / sum;
-    const int u = lane % UNITS, col = share * (D / S) + u * 4;
-    for (int r0 = 0; r0 < 32; r0 += PER * AHEAD) {
-        float4 x[AHEAD][S];
-#pragma unroll
-        for (int i = 0; i < AHEAD; ++i)
-#pragma unroll
-            for (int p = 0; p < S; ++p) x[i][p] = peer_ld4(rows_s + (w * 32 + r0 + i * PER + lane / UNITS) * (D + 4) + col, p);
-#pragma unroll
-        for (int i = 0; i < AHEAD; ++i) {
-            const int r = r0 + i * PER + lane / UNITS, half_row = (w * 32 + r) % TC_ROWS, tok = (w * 32 + r) / TC_ROWS * 32 + half_row / G;
-            float o[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int p = 0; p < S; ++p) {
-                const float fp = __shfl_sync(0xffffffffu, f[p], r);
-                o[0] = fmaf(fp, x[i][p].x, o[0]); o[1] = fmaf(fp, x[i][p].y, o[1]); o[2] = fmaf(fp, x[i][p].z, o[2]); o[3] = fmaf(fp, x[i][p].w, o[3]);
-            }
-            const float k = __shfl_sync(0xffffffffu, inv, r);
-            if (half_row >= 32 * G || tok >= n_tok) continue;
-            const size_t at = (row0 + (size_t)tok * nq + half_row % G) * D + col;
-            const uint32_t h0 = pack_bf16(o[0] * k, o[1] * k), h1 = pack_bf16(o[2] * k, o[3] * k);
-            *reinterpret_cast<uint2*>(out + at) = make_uint2(h0, h1);
-            if (out_lo)
-                *reinterpret_cast<uint2*>(out_lo + at) = make_uint2(pack_bf16(o[0] * k - bf16_lo(h0), o[1] * k - bf16_hi(h0)),
-                                                                    pack_bf16(o[2] * k - bf16_lo(h1), o[3] * k - bf16_hi(h1)));
-        }
-    }
-}
-
 template <int D, int G>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t* __restrict__ kv_layer,
@@ -127,7 +76,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
                        const int* __restrict__ req_slot, const int* __restrict__ req_pos0,
                        const int* __restrict__ tile_req, const int* __restrict__ tile_q0,
                        __nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ out_lo, int nq, int nkv,
-                       float scale_log2, int stagger_on, int split) {
+                       float scale_log2, int stagger_on) {
     using C = TcCfg<D>;
     constexpr int KH = C::KH;
     constexpr int R = 32 * G;                                 // real rows of a half (row = token * G + head)
@@ -188,7 +137,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
 
     // the engine lists a request's q tiles in order, so the LAST tiles see the most keys: take the list back to
     // front, otherwise the longest CTAs start last and the grid ends in a long tail
-    const int share = (int)blockIdx.x % split, tile_idx = ((int)gridDim.x - 1 - (int)blockIdx.x) / split;
+    const int tile_idx = (int)gridDim.x - 1 - (int)blockIdx.x;
     const int req = tile_req[tile_idx];
     const int q0 = tile_q0[tile_idx];
     const int q_row0 = req_q_start[req];
@@ -197,17 +146,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
     const int kvh = blockIdx.y;
     const int rows_here = q_len - q0 < TC_TOK ? q_len - q0 : TC_TOK;
     const int last_pos = pos0 + q0 + rows_here - 1;
-    // the cluster's CTAs share the keys out (three tiles each at least) and put their sums together at the end
-    const int all_tiles = last_pos / kKvTile + 1;
-    const bool shared = split > 1 && all_tiles >= 3 * split;
-    const int j0 = shared ? all_tiles * share / split : 0;
-    const int n_tiles = shared ? all_tiles * (share + 1) / split - j0 : share == 0 ? all_tiles : 0;
-    float m_ref = -INFINITY, l_run = 0.f;                        // a softmax thread's row: maximum in scaled (log2) units, sum
+    const int n_tiles = last_pos / kKvTile + 1;
     const int* pt = page_table + (size_t)req_slot[req] * max_pages;
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
-        if (lane == 0 && n_tiles > 0) {
+        if (lane == 0) {
             mbar_expect_tx(q_full, 2 * KH * R * 128);
             for (int h = 0; h < 2; ++h)
                 for (int kh = 0; kh < KH; ++kh)
@@ -218,7 +162,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
         uint32_t phase = 0;
         for (int t0 = 0; t0 < n_tiles; t0 += 32) {
             const int mine = t0 + lane;
-            const int my_page = mine < n_tiles ? pt[j0 + mine] : 0;
+            const int my_page = mine < n_tiles ? pt[mine] : 0;
             const int n = n_tiles - t0 < 32 ? n_tiles - t0 : 32;
             for (int i = 0; i < n; ++i) {
                 const int page = __shfl_sync(0xffffffffu, my_page, i);
@@ -233,7 +177,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (n_tiles > 0 && elect_one()) {
+        if (elect_one()) {
             constexpr uint32_t idesc_qk = umma_idesc_f16(TC_ROWS, kKvTile, false);
             constexpr uint32_t idesc_pv = umma_idesc_f16(TC_ROWS, D, true);
             const uint32_t q_addr = smem_u32(q_s);
@@ -301,6 +245,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
         const bool valid = row < R && q0 + tok < q_len;
         const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
         const uint32_t s_taddr0 = lane_base + C::COL_S + 2 * h * 64, o_taddr = lane_base + C::COL_O + h * D;
+        float m_ref = -INFINITY, l_run = 0.f;                    // m_ref in scaled (log2) units
         for (int j = 0; j < n_tiles; ++j) {
             mbar_wait(&s_full[2 * h + (j & 1)], (j >> 1) & 1);
             tc_fence_after();
@@ -310,12 +255,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
             for (int c = 0; c < 4; ++c) tmem_ld16_nowait(s_taddr + 16 * c, sr + 16 * c);
             tmem_ld_wait();
             float t4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // four chains instead of one of 64
-            const int key0 = (j0 + j) * kKvTile;
-            if (key0 + kKvTile - 1 > pos) {                      // diagonal tile: causal mask
+            if (j * kKvTile + kKvTile - 1 > pos) {               // diagonal tile: causal mask
 #pragma unroll
                 for (int c = 0; c < 64; ++c) {
                     float v = __uint_as_float(sr[c]);
-                    v = key0 + c <= pos ? v : -INFINITY;
+                    v = j * kKvTile + c <= pos ? v : -INFINITY;
                     sr[c] = __float_as_uint(v);
                     t4[c & 3] = fmaxf(t4[c & 3], v);
                 }
@@ -335,8 +279,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
             } else if (__any_sync(0xffffffffu, grow)) {          // tcgen05.ld / st are warp-wide: rescale all 32 rows
                 mbar_wait(&pv_done[2 * h + ((j - 1) & 1)], ((j - 1) >> 1) & 1);     // O_h complete up to tile j - 1
                 tc_fence_after();
-                // rows that did not grow: m_new >= m_ref, alpha <= 1; rows that see none of a share's keys: nothing to rescale
-                const float alpha = m_new == -INFINITY ? 1.f : exp2f(m_ref - m_new);
+                const float alpha = exp2f(m_ref - m_new);        // rows that did not grow: m_new >= m_ref, alpha <= 1
                 l_run *= alpha;
                 m_ref = m_new;
 #pragma unroll
@@ -373,13 +316,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
             if (lane == 0) mbar_arrive(&p_full[2 * h + (j & 1)]);
         }
         // ---- epilogue: O / l -> bf16 hi + lo planes
-        if (n_tiles > 0) mbar_wait(&pv_done[2 * h + ((n_tiles - 1) & 1)], ((n_tiles - 1) >> 1) & 1);
+        mbar_wait(&pv_done[2 * h + ((n_tiles - 1) & 1)], ((n_tiles - 1) >> 1) & 1);
         tc_fence_after();
         const float inv = 1.f / l_run;
         const size_t off = ((size_t)(q_row0 + q0 + tok) * nq + head) * D;
 #pragma unroll
         for (int c = 0; c < D / 16; ++c) {
-            if (shared || n_tiles == 0) break;
             uint32_t orr[16];
             tmem_ld16_nowait(o_taddr + 16 * c, orr);
             tmem_ld_wait();
@@ -402,36 +344,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
             }
         }
     }
-    if (shared) {
-        // Every CTA leaves its rows' sums, maxima and sums of weights in its shared memory (all products and copies are through), and puts its part of the
-        // columns together from all of them.
-        float* rows_s = reinterpret_cast<float*>(smem);
-        float2* ml_s = reinterpret_cast<float2*>(rows_s + 2 * TC_ROWS * (D + 4));
-        const int h = (warp - 2) >> 2, at = h * TC_ROWS + (warp & 3) * 32 + lane;
-        __syncthreads();
-        if (warp >= 2) {
-            const uint32_t o_taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + C::COL_O + h * D;
-#pragma unroll
-            for (int c = 0; c < D / 16; ++c) {
-                float o[16];
-                tmem_ld16(o_taddr + 16 * c, o);
-#pragma unroll
-                for (int k = 0; k < 16; k += 4) *reinterpret_cast<float4*>(rows_s + at * (D + 4) + 16 * c + k) = make_float4(o[k], o[k + 1], o[k + 2], o[k + 3]);
-            }
-            ml_s[at] = make_float2(m_ref, l_run);
-        }
-        __syncwarp();
-        cluster_sync_all();
-        if (warp >= 2) {
-            const size_t row0 = (size_t)(q_row0 + q0) * nq + kvh * G;
-            const int n_tok = min(TC_TOK, q_len - q0);
-            if (split == 2) merge_rows<D, G, 2>(rows_s, ml_s, warp - 2, lane, share, n_tok, row0, nq, out, out_lo);
-            else if (split == 4) merge_rows<D, G, 4>(rows_s, ml_s, warp - 2, lane, share, n_tok, row0, nq, out, out_lo);
-            else merge_rows<D, G, 8>(rows_s, ml_s, warp - 2, lane, share, n_tok, row0, nq, out, out_lo);
-        }
-        __syncwarp();
-        cluster_sync_all();                                      // no CTA ends while another reads its rows
-    }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
@@ -452,30 +364,6 @@ static std::mutex g_qmap_mu;
 static QMapEntry g_qmaps[16];
 static int g_qmap_n = 0, g_qmap_next = 0;
 
-// Clusters of S CTAs (one per SM, all in one part of the chip) that run at once.
-template <int D, int G>
-static int resident_clusters(int S) {
-    static int known[kMaxDevices][4] = {};
-    const int at = S == 1 ? 0 : S == 2 ? 1 : S == 4 ? 2 : 3;
-    int& n = known[current_device_slot()][at];
-    if (n == 0) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(S * 128);
-        cfg.blockDim = dim3(TC_THREADS);
-        cfg.dynamicSmemBytes = TcCfg<D>::SMEM;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = S; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        int c = 0;
-        if (S == 1) c = device_sms();
-        else if (cudaOccupancyMaxActiveClusters(&c, attn_prefill_tc_kernel<D, G>, &cfg) != cudaSuccess || c < 1) { cudaGetLastError(); c = 1; }
-        n = c;
-    }
-    return n;
-}
-
 template <int D, int G>
 static int launch_tc(const CUtensorMap& map, const void* kv_layer, const int* page_table, int max_pages,
                      const int* req_q_start, const int* req_slot, const int* req_pos0, const int* tile_req,
@@ -486,42 +374,21 @@ static int launch_tc(const CUtensorMap& map, const void* kv_layer, const int* pa
         FT_CHECK_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel<D, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
         attr_set.mark();
     }
-    // CTAs per q tile and KV head: the number whose rounds of resident clusters take least, with the longest row of the page table as the keys
-    // (requests with fewer than three tiles per CTA stay with one) and four key tiles' time for a round's start and end, nine where sums are put
-    // together.  One CTA / two / four / eight, us, d = 128 unless said otherwise: 6 x 211 tokens over 5003 (168 tiles) 170 / 149 / 184 / 280, 2 x 200
-    // over 3000 with 7 tiles of 8 heads 57 / 37 / 48 / 80, 60 over 5003 at d = 64 (8 tiles) 77 / 45 / 28 / 21, 3 x 60 over 1000 21 / 17 / 14 / 23.
-    int split = 1;
-    {
-        const double len = max_pages < 96 ? max_pages : 96;
-        double best = 0;
-        for (int S = 1; S <= TC_MAX_SPLIT; S *= 2) {
-            const int per = resident_clusters<D, G>(S);
-            const double t = (double)((n_tiles * nkv + per - 1) / per) * (len / S + (S == 1 ? 4.0 : 9.0));
-            if (S == 1 || (len >= 3 * S && t < best)) { best = t; split = S; }
-        }
-    }
     const float scale_log2 = 1.4426950408889634f / sqrtf((float)D);
     static const int stagger_on = getenv("FT_TC_STAGGER") ? atoi(getenv("FT_TC_STAGGER")) : 1;       // A/B switch; measured: 4–6 % at d = 64
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(n_tiles * split, nkv);
+    cfg.gridDim = dim3(n_tiles, nkv);
     cfg.blockDim = dim3(TC_THREADS);
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    int n_attr = 0;
-    if (pdl) {
-        attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n_attr++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    if (split > 1) {
-        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-        attr[n_attr].val.clusterDim.x = split; attr[n_attr].val.clusterDim.y = 1; attr[n_attr++].val.clusterDim.z = 1;
-    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = n_attr;
+    cfg.numAttrs = pdl ? 1 : 0;
     FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_prefill_tc_kernel<D, G>, map, (const uint8_t*)kv_layer, page_table, max_pages,
                                      req_q_start, req_slot, req_pos0, tile_req, tile_q0, (__nv_bfloat16*)out,
-                                     (__nv_bfloat16*)out_lo, nq, nkv, scale_log2, stagger_on, split));
+                                     (__nv_bfloat16*)out_lo, nq, nkv, scale_log2, stagger_on));
     return 0;
 }
 

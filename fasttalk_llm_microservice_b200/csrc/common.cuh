@@ -254,11 +254,6 @@ __device__ __forceinline__ float peer_ld_at(uint32_t addr) {
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
     return v;
 }
-__device__ __forceinline__ float4 peer_ld4(const float* p, int rank) {      // p on 16 bytes
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(peer_addr(p, rank)) : "memory");
-    return v;
-}
 // Tile load issued by EITHER CTA of the pair into its own shared memory; the bytes are counted on
 // the LEADER's mbarrier (same offset in the even CTA).
 __device__ __forceinline__ void tma_tile_2d_pair(void* dst_smem, const CUtensorMap* map, int c0, int c1,

@@ -496,9 +496,9 @@ def test_attn_prefill(K, nq, nkv, d, reqs):
 @pytest.mark.parametrize("nq,nkv,d", [(4, 1, 64), (3, 1, 64), (4, 1, 128), (6, 2, 128), (32, 8, 64)])
 @pytest.mark.parametrize("reqs", [[(23 * 64 - 20, 19)], [(23 * 64 - 20, 21)], [(24 * 64 - 1, 64)], [(1990, 65), (5, 3)], [(5 * 64, 64), (11 * 64, 1)],
                                   [(1500, 90), (64, 64), (0, 70), (2300, 1)]])
-def test_attn_prefill_keys_shared_out(K, nq, nkv, d, reqs):
-    """Clusters of two, four and eight CTAs per tile: tiles of keys just below and at three per CTA, a tile of queries across two tiles of keys, requests too short
-    to be shared beside long ones, groups that leave rows over; against the mma.sync kernel and the oracle."""
+def test_attn_prefill_few_tiles_over_many_keys(K, nq, nkv, d, reqs):
+    """Follow-up turns over long histories: a tile of queries across two tiles of keys, short requests beside long ones, groups that leave rows over; against the
+    mma.sync kernel and the oracle."""
     g = torch.Generator(device=DEV).manual_seed(nq * 17 + d + len(reqs))
     kv, pt, ks, vs = build_paged_kv(K, [p + n for p, n in reqs], nkv, d, g)
     q_start = [0]
@@ -511,6 +511,31 @@ def test_attn_prefill_keys_shared_out(K, nq, nkv, d, reqs):
     for r, (p0, n) in enumerate(reqs):
         ref = O.attention(q[q_start[r]:q_start[r + 1]].float(), ks[r].float(), vs[r].float(), p0)
         assert rel_err(tc[q_start[r]:q_start[r + 1]], ref) < 2e-3, r
+
+
+@pytest.mark.parametrize("nq,nkv,d", [(32, 8, 64), (32, 8, 128), (6, 2, 128)])
+@pytest.mark.parametrize("p0,n", [(1472, 21), (5 * 64, 64), (0, 300)])
+def test_attn_prefill_rows_depend_on_nothing_else(K, nq, nkv, d, p0, n):
+    """A request's rows are the same to the last bit alone, behind other requests (nothing behind it: its last tile's unused rows take part in when a warp rescales its
+    sums), and with a page table as wide as a deployed engine's (128 pages)."""
+    g = torch.Generator(device=DEV).manual_seed(p0 + n + d)
+    reqs = [(p0, n), (0, 90), (700, 33), (2000, 1), (0, 640)]
+    kv, pt, _, _ = build_paged_kv(K, [a + b for a, b in reqs], nkv, d, g)
+    q = [(torch.randn(b, nq, d, device=DEV, generator=g) * 1.5).half() for _, b in reqs]
+
+    def rows(which, table):
+        start = [0]
+        for r in which:
+            start.append(start[-1] + reqs[r][1])
+        out = K.attn_prefill(torch.cat([q[r] for r in which]), kv, table, start, which, [reqs[r][0] for r in which])
+        at = start[which.index(0)]
+        return torch.stack([x[at:at + n] for x in out])
+    narrow = pt[:, :(p0 + n + 63) // 64].contiguous()
+    wide = torch.cat([pt, torch.zeros(pt.shape[0], 128 - pt.shape[1], device=DEV, dtype=pt.dtype)], 1)
+    alone = rows([0], narrow)
+    for which in ([0], [1, 0], [2, 1, 0], [4, 3, 2, 1, 0]):
+        for table in (pt, wide):
+            assert torch.equal(rows(which, table), alone), (which, table.shape)
 
 
 @pytest.mark.parametrize("before,after", [(0, 0), (3, 0), (0, 5), (2, 66)])
