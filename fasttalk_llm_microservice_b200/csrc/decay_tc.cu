@@ -3,16 +3,20 @@
 // The token-by-token kernel (branches.cu) is a serial chain: one warp per scheduler, 0.28 us a token whatever runs beside it.  Here a CTA
 // (request, head, 64 value columns) takes 128 tokens at a time.  With W_ij = a_(j+1) .. a_i and S the state before the run:
 //     o_i = sum_{j<=i} W_ij (q_i . k_j) b_j v_j  +  (a_0 .. a_i) S^T q_i          S <- (a_0 .. a_(n-1)) S + sum_j W_(n-1)j k_j (b_j v_j)^T
-// Four products per run, 128 x 128 x D, 128 x 64 x D and twice 128 x 64 x 128, each as six fp16 products: 8400 clocks of the tensor pipe.  A
-// run takes 26000: forming the slices (some 10000 instruction slots per scheduler) and the barriers between the steps bound the kernel, then
+// Four products per run, 128 x 128 x D, 128 x 64 x D and twice 128 x 64 x 128, each as eight bf16 products: 11200 clocks of the tensor pipe.  A
+// run takes 27000: forming the slices (some 10000 instruction slots per scheduler) and the barriers between the steps bound the kernel, then
 // the 200 KB per run that an SM reads and writes.  The state stays on the chip (16 numbers per thread, fp32) from the first run to the last;
-// decays are products of at most 128 numbers to 40 bits (never quotients or logarithms: a decay of zero is nothing special), rounded once.
-// Three requests of 683 tokens: 16 heads of 128 x 128 188 -> 97 us, 64 heads of 128 x 64 280 -> 213 us, 8 heads of 128 x 257 189 -> 125 us.
-// Error against 64 bits over 2048 tokens: results 1.1e-7 -> 6e-8, states 8e-8 -> 5e-8.
+// decays are products of at most 128 numbers to 40 bits (never quotients or logarithms: a decay of zero is nothing special), and what a score or a state is
+// multiplied by keeps those bits, so that each of them is rounded once.
+// Three requests of 683 tokens: 16 heads of 128 x 128 188 -> 106 us.
+// Error against 64 bits over 2048 tokens: results 1.1e-7 -> 6.0e-8, states 8.4e-8 -> 5.1e-8; by single elements beside numbers 2^30 as large it is that of fp32.
 //
 // Shared memory: slices of the keys | of the run's values (first weighted for the state, then for the results) | of the state.
 // TMEM columns: the state 320..383 until the scores' slices need the place; queries' slices 0..191, after their last product what the run adds to the state 0..127; scores' second
 // accumulator 192..319, their slices as an operand 192..383; scores' first accumulator 384..511, then the results (first | second accumulator).
+//
+// What a token's row does not depend on (later tokens, other columns) leaves no trace in it: masked products are zeros in every slice, and no number is formed in
+// units of another.  Only whether its run goes token by token follows from the whole run.
 //
 // A run that holds infinities, NaN, numbers beyond 2^36 or decays beyond 1 by more than rounding, and runs of few tokens, go token by token: a product
 // with a masked zero must not make a NaN of another token's infinity.  Every wait has a limit; a CTA whose wait runs out marks `err`, leaves NaN and ends.
@@ -20,10 +24,13 @@
 #include "ft_internal.h"
 #include "slices.cuh"
 
+#include <algorithm>
+#include <cmath>
+
 namespace ft {
 namespace {
 
-constexpr int DR_RUN = 128, DR_WARPS = 16, DR_THREADS = DR_WARPS * 32, DR_COLS = 64, DR_PARTS = DR_WARPS / 4;
+constexpr int DR_RUN = 128, DR_WARPS = 16, DR_THREADS = DR_WARPS * 32, DR_COLS = 64;
 constexpr int DR_FEW = 16;                               // tokens below which a run goes token by token (0.8 us each)
 constexpr int DR_ISSUER = 12;                            // the warp that issues the products: its part of the scores lies above the diagonal
 constexpr int DR_BLK = DR_RUN * 128;                     // bytes of one [128 rows][64 columns] block
@@ -46,20 +53,20 @@ __device__ __forceinline__ Two mul(Two a, Two b) {
 __device__ __forceinline__ Two shfl_up16(Two v, int o) { return {__shfl_up_sync(0xffffffffu, v.h, o, 16), __shfl_up_sync(0xffffffffu, v.l, o, 16)}; }
 __device__ __forceinline__ Two shfl_down16(Two v, int o) { return {__shfl_down_sync(0xffffffffu, v.h, o, 16), __shfl_down_sync(0xffffffffu, v.l, o, 16)}; }
 
-// D[tmem] (+)= A[tmem] B[smem] over N steps of 16 along the contraction; KMAJOR: B's blocks of 64 lie DR_BLK apart.  Everything but the
-// addresses is known to the compiler: operands that are put together at run time cost the issuing thread 150 clocks a product, four
-// times what the tensor cores take for it.
+// D = A[tmem] B[smem] over N steps of 16 along the contraction, the seven small products `rest` columns from first x first.  Slices of A are 64 columns apart, slices
+// of B `plane` bytes; KMAJOR: B's blocks of 64 lie DR_BLK apart.  Everything but the addresses is known to the compiler: operands that are put together at
+// run time cost the issuing thread 150 clocks a product, four times what the tensor cores take for it.
 template <bool KMAJOR, int N>
-__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool first) {
+__device__ __forceinline__ void mma_slices(uint32_t d, int rest, uint32_t a, uint64_t b, int plane, uint32_t idesc) {
 #pragma unroll
-    for (int k = 0; k < N; ++k)
-        umma_f16_ts(d, a + k * 8, b + (KMAJOR ? (k >> 2) * (DR_BLK >> 4) + (k & 3) * 2 : k * (2048 >> 4)), idesc, !first || k > 0);
-}
-// the five products beside first x first: D (+)= A B, slices of A 64 columns apart, slices of B `plane` bytes
-template <bool KMAJOR, int N>
-__device__ __forceinline__ void mma_rest(uint32_t d, uint32_t a, uint64_t b, int plane, uint32_t idesc) {
+    for (int p = 0; p <= kSlicePairs; ++p) {
+        const bool last = p == kSlicePairs;
+        const int sa = last ? 0 : slice_a(p), sb = last ? 0 : slice_b(p);
 #pragma unroll
-    for (int p = 0; p < kSlicePairs; ++p) mma_ts<KMAJOR, N>(d, a + 64 * slice_a(p), b + slice_b(p) * (plane >> 4), idesc, p == 0);
+        for (int k = 0; k < N; ++k)
+            umma_f16_ts(last ? d : d + rest, a + 64 * sa + k * 8,
+                        b + sb * (plane >> 4) + (KMAJOR ? (k >> 2) * (DR_BLK >> 4) + (k & 3) * 2 : k * (2048 >> 4)), idesc, k > 0 || (p > 0 && !last));
+    }
 }
 
 // Nothing is computed from x before this point: work moved up across barriers would need more registers than there are.
@@ -73,14 +80,13 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
     extern __shared__ uint8_t dr_raw[];
     __shared__ Two pref[DR_RUN], suff[DR_RUN], full[8];      // products of decays inside a block of 16 tokens: up to and with i, behind j, all
     __shared__ Two mid[8][8], tail[8], head[9];          // of whole blocks: between two, behind one, before one (head[8]: of the run)
-    __shared__ __align__(16) float ywk[DR_RUN];          // a block's decays behind j, times the unit of key j
-    __shared__ __align__(16) float near[DR_RUN][20];     // decays inside a row's own block of 16
-    __shared__ float sa[DR_RUN], sb[DR_RUN], kunit[DR_RUN];
-    __shared__ unsigned qtop[DR_PARTS][DR_RUN], ptop[DR_PARTS][DR_RUN], wtop[3][DR_WARPS];
+    __shared__ __align__(16) float behind[2][DR_RUN];    // a block's decays behind j, times b_j: h and l of a Two
+    __shared__ __align__(16) float near[2][DR_RUN][20];  // decays inside a row's own block of 16, times b_j
+    __shared__ float sa[DR_RUN], sb[DR_RUN];
     __shared__ float red[4][DR_COLS];
     __shared__ uint64_t done[4];
     __shared__ uint32_t tmem_slot;
-    __shared__ int odd;                                  // 1: the run goes token by token
+    __shared__ int odd, state_big;                       // 1: the run, or the one behind this state, goes token by token
     __shared__ volatile int dead;
     const int r = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * DR_COLS, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int t0 = a.req_start[r], t1 = a.req_start[r + 1];
@@ -94,6 +100,7 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
         for (int i = 0; i < 4; ++i) mbar_init(&done[i], 1);
         fence_mbar_init();
         dead = 0;
+        state_big = 0;
     }
     if (warp == 0) {
         tmem_alloc(&tmem_slot, 512);
@@ -120,26 +127,18 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot, lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    unsigned s_top = 0;                                  // the largest of the state, known to all threads
-    auto all_top = [&](const unsigned* w) { return warp_umax(w[lane & (DR_WARPS - 1)]); };
-    auto state_top = [&]() {
+    // the state's slices to shared memory, [channel][64 columns]
+    auto state_out = [&]() {
         float t = 0.f;
 #pragma unroll
         for (int i = 0; i < 16; i += 2) t = top3(t, st[i], st[i + 1]);
-        const unsigned m = warp_umax(abs_bits(t));
-        if (lane == 0) wtop[2][warp] = m;
-        __syncthreads();
-        s_top = all_top(wtop[2]);
-    };
-    // the state's slices to shared memory, [channel][64 columns]
-    auto state_out = [&]() {
-        const float inv = slice_inv(s_top);
+        if (abs_bits(t) >= DR_BIG_STATE) state_big = 1;
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
             f32x2 v[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[e] = pack2(st[x * 8 + 2 * e], st[x * 8 + 2 * e + 1]);
-            slice8(v, inv, s_s + row * 128 + (((part * 2 + x) ^ (row & 7)) << 4), DR_BLK);
+            slice8(v, s_s + row * 128 + (((part * 2 + x) ^ (row & 7)) << 4), DR_BLK);
         }
     };
     // four numbers of a row: columns c .. of n, zeros beyond
@@ -193,14 +192,14 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
         v[0] = mul2(v[0], f2);
         v[1] = mul2(v[1], f2);
     };
-    auto values_out = [&](f32x2 (*x)[2], float inv) {
+    auto values_out = [&](f32x2 (*x)[2]) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int j = vr + 32 * i;
-            slice4(x[i], inv, v_s + j * 128 + (((vc >> 1) ^ (j & 7)) << 4) + (vc & 1) * 8, DR_BLK);
+            slice4(x[i], v_s + j * 128 + (((vc >> 1) ^ (j & 7)) << 4) + (vc & 1) * 8, DR_BLK);
         }
     };
-    constexpr uint32_t id128 = umma_idesc_f16(128, DR_RUN), id64 = umma_idesc_f16(128, DR_COLS, true);
+    constexpr uint32_t id128 = slice_idesc(128, DR_RUN), id64 = slice_idesc(128, DR_COLS, true);
     const uint64_t kd = umma_desc_k128(smem_u32(k_s)), vd = umma_desc_mn128(smem_u32(v_s), DR_BLK), sd = umma_desc_mn128(smem_u32(s_s), DR_BLK);
     unsigned ph = 0;
     bool ok = true;
@@ -214,13 +213,11 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
     stage_q(t0);
     load_k(kx, t0);
     load_v(v0, t0);
-    if (carried) {
-        state_top();
-        state_out();
-    }
+    if (carried) state_out();
+    __syncthreads();
     for (int base = t0; base < t1; base += DR_RUN) {
         const int n = min(DR_RUN, t1 - base);
-        if (tid == 0) odd = n < DR_FEW || s_top >= DR_BIG_STATE;
+        if (tid == 0) odd = n < DR_FEW || state_big;
         if (tid < DR_RUN) {
             const float d = ab_x.x;
             sa[tid] = d;
@@ -243,31 +240,19 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        // ---- the largest numbers of rows and tiles
-        unsigned bad = 0, k_top;
+        // ---- numbers that do not go as slices
+        bool bad = false;
         const float* qr = q_stage + row * DR_LDQ + part * 32;
         {
+            if (tid == 0) state_big = 0;
             float t = 0.f;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const float4 f = *reinterpret_cast<const float4*>(qr + 4 * i);
                 t = top3(top3(t, f.x, f.y), f.z, f.w);
             }
-            unsigned m = abs_bits(t);
-            qtop[part][row] = m;
-            bad |= m >= DR_BIG_IN;
-            m = abs_bits(top_of<8 * DB>(kx[0]));
-            m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
-            k_top = m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
-            bad |= m >= DR_BIG_IN;
-            if (kq == 0) kunit[kr] = slice_unit(min(m, DR_BIG_IN));
-            bad |= abs_bits(top_of<8>(v0[0])) >= DR_BIG_IN;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) scale_v(v0[i], sb[vr + 32 * i]);
-            m = warp_umax(abs_bits(top_of<8>(v0[0])));
-            bad |= m >= DR_BIG_IN;
-            if (lane == 0) wtop[0][warp] = m;
-            if (tid < DR_RUN) bad |= abs_bits(sa[tid]) > DR_DECAY;
+            bad = abs_bits(top_of<8>(v0[0], top_of<8 * DB>(kx[0], t))) >= DR_BIG_IN;
+            if (tid < DR_RUN) bad |= abs_bits(sa[tid]) > DR_DECAY || abs_bits(sb[tid]) >= DR_BIG_IN;
             if (tid >= DR_THREADS - 64) {
                 const int b = tid & 7, c = (tid >> 3) & 7;
                 Two f[8], p = {1.f, 0.f};
@@ -315,42 +300,40 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
                 __syncthreads();
             }
             carried = true;
-            state_top();
             state_out();
+            __syncthreads();
             ab_x = load_ab(base + DR_RUN);
             load_k(kx, base + DR_RUN);
             load_v(v0, base + DR_RUN);
             continue;
         }
-        // ---- queries and keys as slices; the state waits in tensor memory meanwhile; what a token's value weighs in the state after the run, with its key's unit
-        unsigned q_top = 0;
+        // ---- queries and keys as slices; the state waits in tensor memory meanwhile; what a token's value weighs in the state after the run
         {
             tmem_st16(lanes + DR_COL_ST + c0, reinterpret_cast<const uint32_t*>(st));
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int j = vr + 32 * i;
-                const Two p = mul(suff[j], tail[j >> 4]);
+                const Two p = mul(mul(suff[j], tail[j >> 4]), {sb[j], 0.f});
                 scale_v(v0[i], p.h + p.l);
-                scale_v(v0[i], kunit[j]);
             }
-            const unsigned m = warp_umax(abs_bits(top_of<8>(v0[0])));
-            if (lane == 0) wtop[1][warp] = m;
-            if (tid < DR_RUN) ywk[tid] = (suff[tid].h + suff[tid].l) * kunit[tid];
-            q_top = max(max(qtop[0][row], qtop[1][row]), max(qtop[2][row], qtop[3][row]));
+            if (tid < DR_RUN) {
+                const Two p = mul(suff[tid], {sb[tid], 0.f});
+                behind[0][tid] = p.h;
+                behind[1][tid] = p.l;
+            }
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
                 f32x2 qx[8];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) *reinterpret_cast<ulonglong2*>(qx + 2 * i) = *reinterpret_cast<const ulonglong2*>(qr + 16 * x + 4 * i);
-                slices_to_tmem<64>(qx, slice_inv(q_top), lanes + DR_COL_Q + part * 16 + 8 * x);
+                slices_to_tmem<64>(qx, lanes + DR_COL_Q + part * 16 + 8 * x);
             }
             __syncthreads();                             // the queries have been read: the keys take their place
             hold<8 * DB>(kx[0]);
-            const float k_inv = slice_inv(k_top);
 #pragma unroll
             for (int i = 0; i < 4 * DB; ++i) {
                 const int u = kq + 4 * i;                // units of four channels, two to 16 bytes of a slice
-                slice4(kx[i], k_inv, k_s + (u >> 4) * DR_BLK + kr * 128 + (((u >> 1 & 7) ^ (kr & 7)) << 4) + (u & 1) * 8, DR_K);
+                slice4(kx[i], k_s + (u >> 4) * DR_BLK + kr * 128 + (((u >> 1 & 7) ^ (kr & 7)) << 4) + (u & 1) * 8, DR_K);
             }
             tmem_st_wait();
         }
@@ -361,25 +344,25 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
         // ---- scores
         if (warp == DR_ISSUER) {
             if (elect_one()) {
-                mma_rest<true, 4 * DB>(tmem + DR_COL_S, tmem + DR_COL_Q, kd, DR_K, id128);
-                mma_ts<true, 4 * DB>(tmem + DR_COL_O, tmem + DR_COL_Q, kd, id128, true);
+                mma_slices<true, 4 * DB>(tmem + DR_COL_O, DR_COL_S - DR_COL_O, tmem + DR_COL_Q, kd, DR_K, id128);
                 umma_commit(&done[0]);
             }
             __syncwarp();
         }
-        const unsigned v_top = all_top(wtop[0]), g_top = all_top(wtop[1]);
         f32x2 sc[16];
         {
             hold<8>(v0[0]);
-            values_out(v0, slice_inv(g_top));
-            // decays from token j to the row's, times the unit of key j: inside the row's own block
+            values_out(v0);
+            // what token j's values weigh in the row's result but for the score, inside the row's own block
             if (part == (warp & 3)) {
                 const int b0 = row & ~15;
                 Two p = {1.f, 0.f};
 #pragma unroll
                 for (int e = 15; e >= 0; --e) {
                     const bool seen = e <= (row & 15);
-                    near[row][e] = seen ? (p.h + p.l) * kunit[b0 + e] : 0.f;
+                    const Two w = mul(p, {sb[b0 + e], 0.f});
+                    near[0][row][e] = seen ? w.h : 0.f;
+                    near[1][row][e] = seen ? w.l : 0.f;
                     const Two q = mul(p, {sa[b0 + e], 0.f});
                     p.h = seen ? q.h : p.h;
                     p.l = seen ? q.l : p.l;
@@ -390,8 +373,7 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
             __syncwarp();
         }
         if (ok) {
-            // times the decays, zero above the diagonal
-            unsigned m = 0;
+            // times the decays and b, zero above the diagonal
             const int bi = row >> 4;
             if (part <= (warp & 3)) {
 #pragma unroll
@@ -400,24 +382,24 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
                     f32x2 s[8], u[8];
                     tmem_ld16_nowait(lanes + DR_COL_S + b * 16, reinterpret_cast<uint32_t*>(s));
                     tmem_ld16_nowait(lanes + DR_COL_O + b * 16, reinterpret_cast<uint32_t*>(u));
-                    float f = b == bi ? 1.f : 0.f;
-                    if (b < bi) {
-                        const Two p = mul(pref[row], mid[b][bi]);
-                        f = p.h + p.l;
-                    }
-                    const f32x2 f2 = pack2(f, f);
-                    const float* y = b == bi ? near[row] : ywk + b * 16;
+                    Two f = {b == bi ? 1.f : 0.f, 0.f};
+                    if (b < bi) f = mul(pref[row], mid[b][bi]);
+                    const f32x2 fh = pack2(f.h, f.h), fl = pack2(f.l, f.l), minus = pack2(-1.f, -1.f);
+                    const float *yh = b == bi ? near[0][row] : behind[0] + b * 16, *yl = b == bi ? near[1][row] : behind[1] + b * 16;
                     tmem_ld_wait();
 #pragma unroll
                     for (int e = 0; e < 8; e += 2) {
-                        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(y + 2 * e);
-                        sc[x * 8 + e] = mul2(add2(s[e], u[e]), mul2(w.x, f2));
-                        sc[x * 8 + e + 1] = mul2(add2(s[e + 1], u[e + 1]), mul2(w.y, f2));
+                        const ulonglong2 h = *reinterpret_cast<const ulonglong2*>(yh + 2 * e), l = *reinterpret_cast<const ulonglong2*>(yl + 2 * e);
+                        // (u + rest) (wh + wl), rounded once
+                        auto weighted = [&](f32x2 u, f32x2 s, f32x2 h, f32x2 l) {
+                            const f32x2 wh = mul2(h, fh), wl = fma2(l, fh, fma2(h, fl, fma2(h, fh, mul2(wh, minus))));
+                            return fma2(u, wh, fma2(u, wl, mul2(rest_of(u, s), wh)));
+                        };
+                        sc[x * 8 + e] = weighted(u[e], s[e], h.x, l.x);
+                        sc[x * 8 + e + 1] = weighted(u[e + 1], s[e + 1], h.y, l.y);
                     }
                 }
-                m = abs_bits(top_of<16>(sc));
             }
-            ptop[part][row] = m;
         }
         fence_proxy_async();                             // the weighted values
         tc_fence_before();
@@ -427,10 +409,7 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
         // ---- what the state gives, in the scores' place; then what the run adds to it, in the queries' place
         if (warp == DR_ISSUER) {
             if (elect_one()) {
-                if (carried) {
-                    mma_rest<false, 4 * DB>(tmem + DR_COL_O + 64, tmem + DR_COL_Q, sd, DR_BLK, id64);
-                    mma_ts<false, 4 * DB>(tmem + DR_COL_O, tmem + DR_COL_Q, sd, id64, true);
-                }
+                if (carried) mma_slices<false, 4 * DB>(tmem + DR_COL_O, 64, tmem + DR_COL_Q, sd, DR_BLK, id64);
                 umma_commit(&done[1]);
             }
             __syncwarp();
@@ -452,18 +431,15 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
             __syncwarp();
         }
         // ---- weights of the values as slices
-        unsigned p_top = 0;
         float o[16];
-        const float q_unit = slice_unit(q_top);
         {
-            p_top = max(max(ptop[0][row], ptop[1][row]), max(ptop[2][row], ptop[3][row]));
             load_v(v0, base);
             tmem_ld16(lanes + DR_COL_ST + c0, st);
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
                 const uint32_t at = lanes + DR_COL_P + part * 16 + 8 * x;
                 if (part <= (warp & 3)) {
-                    slices_to_tmem<64>(sc + 8 * x, slice_inv(p_top), at);
+                    slices_to_tmem<64>(sc + 8 * x, at);
                 } else {
                     const uint32_t zero[8] = {};
 #pragma unroll
@@ -477,20 +453,17 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
             __syncwarp();
             if (carried && ok) {
                 const Two p = mul(pref[row], head[row >> 4]);
-                const float f = (p.h + p.l) * (q_unit * slice_unit(s_top));
                 float y[16];
                 tmem_ld16(lanes + DR_COL_O + c0, o);
                 tmem_ld16(lanes + DR_COL_O + 64 + c0, y);
 #pragma unroll
-                for (int i = 0; i < 16; ++i) o[i] = (o[i] + y[i]) * f;
+                for (int i = 0; i < 16; ++i) o[i] = __fmaf_rn(o[i], p.h, __fmaf_rn(o[i], p.l, rest_of(o[i], y[i]) * p.h));
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) scale_v(v0[i], sb[vr + 32 * i]);
             tmem_st_wait();
             ok = ok && mbar_sleep_limited(&done[2], ph, &dead);     // the weighted values and the keys have been read
             tc_fence_after();
             __syncwarp();
-            if (ok) values_out(v0, slice_inv(v_top));
+            if (ok) values_out(v0);
         }
         fence_proxy_async();
         tc_fence_before();
@@ -499,8 +472,7 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
         if (!ok) break;
         if (warp == DR_ISSUER) {
             if (elect_one()) {
-                mma_rest<false, 8>(tmem + DR_COL_O + 64, tmem + DR_COL_P, vd, DR_BLK, id64);
-                mma_ts<false, 8>(tmem + DR_COL_O, tmem + DR_COL_P, vd, id64, true);
+                mma_slices<false, 8>(tmem + DR_COL_O, 64, tmem + DR_COL_P, vd, DR_BLK, id64);
                 umma_commit(&done[3]);
             }
             __syncwarp();
@@ -508,15 +480,13 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
         stage_q(base + DR_RUN);
         // ---- the state meanwhile
         {
-            const float f = head[8].h + head[8].l, g = slice_unit(g_top);
+            const Two f = head[8];
             float u[16], x[16];
             tmem_ld16(lanes + DR_COL_U + c0, u);
             tmem_ld16(lanes + DR_COL_U + 64 + c0, x);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) st[i] = mine ? __fmaf_rn(f, st[i], (u[i] + x[i]) * g) : 0.f;
+            for (int i = 0; i < 16; ++i) st[i] = mine ? __fmaf_rn(f.h, st[i], __fmaf_rn(f.l, st[i], rest_of(u[i], x[i]))) + u[i] : 0.f;
         }
-        state_top();
-        const float f_o = slice_unit(p_top) * (q_unit * slice_unit(v_top));
         if (base + DR_RUN < t1) state_out();
         carried = true;
         ok = mbar_sleep_limited(&done[3], ph, &dead);
@@ -529,8 +499,8 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, 
 #pragma unroll
             for (int i = 0; i < 16; i += 4)
                 *reinterpret_cast<float4*>(o_stage + row * DR_LDO + c0 + i) =
-                    make_float4(__fmaf_rn(x[i] + y[i], f_o, o[i]), __fmaf_rn(x[i + 1] + y[i + 1], f_o, o[i + 1]),
-                                __fmaf_rn(x[i + 2] + y[i + 2], f_o, o[i + 2]), __fmaf_rn(x[i + 3] + y[i + 3], f_o, o[i + 3]));
+                    make_float4(x[i] + (rest_of(x[i], y[i]) + o[i]), x[i + 1] + (rest_of(x[i + 1], y[i + 1]) + o[i + 1]),
+                                x[i + 2] + (rest_of(x[i + 2], y[i + 2]) + o[i + 2]), x[i + 3] + (rest_of(x[i + 3], y[i + 3]) + o[i + 3]));
         }
         tc_fence_before();
         ok = __syncthreads_and(ok);
@@ -598,22 +568,30 @@ int launch_runs(const RecurArgs& a, dim3 grid, cudaStream_t stream) {
 
 }  // namespace
 
-// A run of 128 tokens takes about 14 us whatever the sizes (one CTA per SM), after 5 us for the launch and the first operands; the kernel that
-// goes token by token 0.275 us a token, and in proportion longer when more than about 175 of its CTAs of 64 columns run.  Mean portions of L
-// tokens, us by tokens / here: 3 requests x 16 heads of 128 x 128, L = 32: 13 / 21, 67: 23 / 22, 683: 188 / 97; 16 requests, L = 64: 56 / 76,
-// 128: 102 / 84; 3 x 64 heads of 128 x 64 (two waves of CTAs), 683: 280 / 213; 3 x 8 heads of 128 x 257, 683: 189 / 125.
+static bool vectors(const RecurArgs& a) {
+    return ((a.dim | a.vd | a.ldk | a.ldq | a.ldv) & 3) == 0 && (((uintptr_t)a.k | (uintptr_t)a.q | (uintptr_t)a.v) & 15) == 0;
+}
+// Both kernels' times in us from 1500 pairs of measurements (1 to 64 heads, 20 x 70 to 128 x 257, 1 to 40 portions of 17 to 1500 tokens; a mean of 7 % off).
+// This one: rounds of CTAs, one per SM, of 4.5 us and 16.2 a run of 128 tokens (12.6 up to 64 channels), up to an eighth more when all SMs read, a fifth more off 16
+// bytes; the last tokens of a portion take as long as a run from a dozen on.  Token by token: 4 us and per token 0.17 us with up to 30 CTAs, 0.0012 us more with each further
+// one (of 64 columns, or 128 up to 64 channels).  By tokens / here, portions of L tokens: one of 16 heads of 128 x 128, L = 64: 15 / 20, 128: 26 / 20, 150: 30 / 35, 256: 48 /
+// 36, 1500: 262 / 192; three, 683: 189 / 103; 40 of them (nine rounds), 100: 175 / 204, 128: 216 / 209, 150: 252 / 345; 16 of 64 heads of 128 x 64, 128: 173 / 175, 200: 263 /
+// 289; eight heads of 128 x 257, 128: 26 / 27, 200: 38 / 44, 1024: 179 / 166.  Shorter portions than 64 never gained.
 bool decay_tc_ahead(const RecurArgs& a, int n_req, int T) {
     if (a.dim > 128 || n_req < 1 || n_req > 65535) return false;
-    const double L = (double)T / n_req, ctas = (double)n_req * a.heads * ((a.vd + DR_COLS - 1) / DR_COLS), sms = device_sms();
-    const double whole = (double)(int)(L / DR_RUN), runs = whole + (L - whole * DR_RUN >= DR_FEW ? 1.0 : 0.0);
-    const double waves = (double)(long long)((ctas + sms - 1) / sms);
-    return L >= 64 && waves * (5.0 + 14.0 * runs) < 0.275 * L * (ctas > 1.2 * sms ? ctas / (1.2 * sms) : 1.0);
+    const double L = (double)T / n_req, sms = device_sms();
+    if (L < 64) return false;
+    const double heads = (double)n_req * a.heads, ctas = heads * ((a.vd + DR_COLS - 1) / DR_COLS), token_ctas = heads * (a.dim <= 64 ? (a.vd + 127) / 128 : (a.vd + 63) / 64);
+    const double whole = (double)(int)(L / DR_RUN), runs = whole + std::min(1.0, (L - whole * DR_RUN) / 12);
+    const double run = (a.dim <= 64 ? 12.6 : 16.2) * (vectors(a) ? 1.0 : 1.2) * (1.0 + 0.13 * std::min(1.0, ctas / sms));
+    const double here = std::ceil(ctas / sms) * (4.5 + run * runs), by_tokens = 4.0 + L * std::max(0.17, 0.13 + 0.0012 * token_ctas);
+    return here < 0.9 * by_tokens;
 }
 
 int launch_decay_tc(const RecurArgs& a, int n_req, cudaStream_t stream) {
     FT_REQUIRE(a.dim <= 128 && n_req >= 1 && n_req <= 65535, "decay rule (tcgen05): %d channels, %d requests do not fit", a.dim, n_req);
     const dim3 grid((a.vd + DR_COLS - 1) / DR_COLS, a.heads, n_req);
-    const bool vec = ((a.dim | a.vd | a.ldk | a.ldq | a.ldv) & 3) == 0 && (((uintptr_t)a.k | (uintptr_t)a.q | (uintptr_t)a.v) & 15) == 0;
+    const bool vec = vectors(a);
     if (a.dim <= 64) return vec ? launch_runs<true, 1>(a, grid, stream) : launch_runs<false, 1>(a, grid, stream);
     return vec ? launch_runs<true, 2>(a, grid, stream) : launch_runs<false, 2>(a, grid, stream);
 }

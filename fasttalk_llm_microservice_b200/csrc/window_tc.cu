@@ -1,11 +1,12 @@
-// Window attention of prompt portions on the tensor cores, in fp32 accuracy (slices.cuh): scores, softmax weights and their sums are what
-// the fp32 kernel of branches.cu makes of the same cache rows, to the last bits.
+// Window attention of prompt portions on the tensor cores, in fp32 accuracy (slices.cuh): against 64 bits scores, softmax weights and their sums come out as near as
+// those of the fp32 kernels of branches.cu, or nearer, and a row shows nothing of keys that it does not see.
 //
 // A CTA takes 128 rows: a run of up to 64 tokens times the query heads of one key head.  Keys come 64 at a time from the first one the run's
-// first token sees; every key and value row becomes three fp16 slices in shared memory once per CTA and serves all rows.  Scores: six
+// first token sees; every key and value row becomes three bf16 slices in shared memory once per CTA and serves all rows.  Scores: eight
 // products 128 x 64 x D.  Softmax on the CUDA cores, a row by four threads of the same lane of four warps.  Weights as slices in tensor
-// memory, six products 128 x V x 64, and the sums join the rows' fp32 registers (rescaled there).  The fp32 kernel (64 rows and 32 keys at
-// a time, multiply-adds and shared-memory reads bound it, 20 TFLOP/s of products) took 5.6 us per tile of half the keys and half the rows.
+// memory, eight products 128 x V x 64, and the sums join the rows' fp32 registers (rescaled there).  The fp32 kernel (64 rows and 32 keys at
+// a time, multiply-adds and shared-memory reads bound it, 20 TFLOP/s of products) took 5.6 us per tile of half the keys and half the rows.  2313 tokens of 16
+// heads of 128, window 512: 389 -> 132 us with a cap, 436 -> 145 us with a bias by distance.
 //
 // Per tile: value slices and the last tile's sums beside the scores' products, the next tile's key slices beside the sums' products;
 // softmax alone.  Two barriers for the CTA, one for the four warps of a row.
@@ -32,7 +33,7 @@ constexpr int WR_COL_Q = 0, WR_COL_S = 128, WR_COL_P = 128, WR_COL_O = 256;
 constexpr int WR_ISSUE_S = 15, WR_ISSUE_O = 10;         // the warps that issue scores' and sums' products, which holds them up for most of the products' time
 constexpr unsigned WR_BIG = (127u + 36) << 23;
 
-// tanh of up to 0.6 in size: x + x^3 Q(x^2), Q fitted to the smallest relative error over the range (2.6e-9; 0.73 ulp in fp32).  tanhf takes
+// tanh of up to 0.6 in size: x + x^3 Q(x^2), Q fitted to the smallest relative error over the range (6.0e-9; 0.68 ulp in fp32).  tanhf takes
 // forty instructions an element on either of its two ways, 6000 clocks a tile.
 constexpr float kTanhSmall = 0.6f;
 __device__ __forceinline__ float tanh_small(float x) {
@@ -98,9 +99,7 @@ __device__ __noinline__ void window_row(const WindowArgs& a, const int* pt, int 
 template <int DB, int VB>
 __global__ void __launch_bounds__(WR_THREADS, 1) window_runs_kernel(WindowArgs a, WindowTiles tm, int QT, int subs) {
     extern __shared__ uint8_t wr_raw[];
-    __shared__ __align__(16) float kunit[WR_KEYS];
     __shared__ float part_max[4][WR_ROWS], part_sum[4][WR_ROWS];
-    __shared__ unsigned qtop[4][WR_ROWS], vtop[WR_WARPS];
     __shared__ uint64_t done[2];                         // scores, sums
     __shared__ uint32_t tmem_slot;
     __shared__ int odd;
@@ -141,25 +140,18 @@ __global__ void __launch_bounds__(WR_THREADS, 1) window_runs_kernel(WindowArgs a
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot, lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    float q_scale;                                       // the row's unit times the score scale
     {
         constexpr int N = 8 * DB;                        // pairs of a thread
         f32x2 qx[N];
         const float* src = stage + row * WR_LDQ + part * 2 * N;
 #pragma unroll
         for (int i = 0; i < N / 2; ++i) *reinterpret_cast<ulonglong2*>(qx + 2 * i) = *reinterpret_cast<const ulonglong2*>(src + 4 * i);
-        const unsigned top = abs_bits(top_of<N>(qx));
-        qtop[part][row] = top;
-        if (top >= WR_BIG) odd = 1;
-        __syncthreads();
-        const unsigned q_top = max(max(qtop[0][row], qtop[1][row]), max(qtop[2][row], qtop[3][row]));
-        q_scale = slice_unit(min(q_top, WR_BIG)) * a.scale;
-        const float inv = slice_inv(min(q_top, WR_BIG));
+        if (abs_bits(top_of<N>(qx)) >= WR_BIG) odd = 1;
 #pragma unroll
         for (int x = 0; x < DB; ++x) {
             uint32_t w[8];
             const int c = part * 2 * N + 16 * x;         // first of 16 channels
-            slice_first<8>(qx + 8 * x, inv, w);
+            slice_first<8>(qx + 8 * x, w);
             tmem_st8(lanes + WR_COL_Q + c / 2, w);
             slice_next<8>(qx + 8 * x, w);
             tmem_st8(lanes + WR_COL_Q + 64 + c / 2, w);
@@ -198,35 +190,27 @@ __global__ void __launch_bounds__(WR_THREADS, 1) window_runs_kernel(WindowArgs a
     auto load_v = [&](int it) { load(vx, 2 * VB, it, a.vdim, (size_t)a.G * a.dim + (size_t)g * a.vdim); };
     auto place = [&](uint8_t* base, int u) { return base + (u >> 4) * WR_KBLK + kr * 128 + ((((u >> 1) & 7) ^ (kr & 7)) << 4) + (u & 1) * 8; };
     auto keys_out = [&]() {
-        unsigned m = abs_bits(top_of<4 * DB>(kx[0]));
+        if (abs_bits(top_of<4 * VB>(vx[0], top_of<4 * DB>(kx[0]))) >= WR_BIG) odd = 1;
 #pragma unroll
-        for (int o = 1; o < 8; o *= 2) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (m >= WR_BIG) odd = 1;
-        m = min(m, WR_BIG);
-        if (kq == 0) kunit[kr] = slice_unit(m);
-        const float inv = slice_inv(m);
-#pragma unroll
-        for (int i = 0; i < 2 * DB; ++i) slice4(kx[i], inv, place(k_s, kq + 8 * i), K_PLANE);
-        m = warp_umax(abs_bits(top_of<4 * VB>(vx[0])));
-        if (m >= WR_BIG) odd = 1;
-        if (lane == 0) vtop[warp] = m;
+        for (int i = 0; i < 2 * DB; ++i) slice4(kx[i], place(k_s, kq + 8 * i), K_PLANE);
     };
-    constexpr uint32_t id_s = umma_idesc_f16(WR_ROWS, WR_KEYS), id_o = umma_idesc_f16(WR_ROWS, 64 * VB, true);
+    constexpr uint32_t id_s = slice_idesc(WR_ROWS, WR_KEYS), id_o = slice_idesc(WR_ROWS, 64 * VB, true);
     const uint64_t kd = umma_desc_k128(smem_u32(k_s)), vd = umma_desc_mn128(smem_u32(v_s), WR_KBLK), qd = umma_desc_k128(smem_u32(ql_s));
     // all operands but the addresses are known to the compiler: see decay_tc.cu
     auto issue_scores = [&]() {
         if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < 4 * DB; ++k)             // third slice of the queries, from shared memory
-                umma_bf16(tmem + WR_COL_S + 64, qd + (k >> 2) * (WR_QBLK >> 4) + (k & 3) * 2, kd + (k >> 2) * (WR_KBLK >> 4) + (k & 3) * 2, id_s, k > 0);
-#pragma unroll
-            for (int p = 1; p <= kSlicePairs; ++p) {
+            for (int p = 0; p <= kSlicePairs; ++p) {
                 const bool last = p == kSlicePairs;
                 const int sa = last ? 0 : slice_a(p), sb = last ? 0 : slice_b(p);
+                const uint32_t d = tmem + WR_COL_S + (last ? 0 : 64);
 #pragma unroll
-                for (int k = 0; k < 4 * DB; ++k)
-                    umma_f16_ts(tmem + WR_COL_S + (last ? 0 : 64), tmem + WR_COL_Q + 64 * sa + 8 * k,
-                                kd + sb * (K_PLANE >> 4) + (k >> 2) * (WR_KBLK >> 4) + (k & 3) * 2, id_s, !last || k > 0);
+                for (int k = 0; k < 4 * DB; ++k) {
+                    const uint64_t b = kd + sb * (K_PLANE >> 4) + (k >> 2) * (WR_KBLK >> 4) + (k & 3) * 2;
+                    const bool more = k > 0 || (p > 0 && !last);
+                    if (sa == 2) umma_bf16(d, qd + (k >> 2) * (WR_QBLK >> 4) + (k & 3) * 2, b, id_s, more);      // third slice of the queries, from shared memory
+                    else umma_f16_ts(d, tmem + WR_COL_Q + 64 * sa + 8 * k, b, id_s, more);
+                }
             }
             umma_commit(&done[0]);
         }
@@ -266,10 +250,8 @@ __global__ void __launch_bounds__(WR_THREADS, 1) window_runs_kernel(WindowArgs a
     if (!plain && warp == WR_ISSUE_S) issue_scores();
     for (int it = 0; it < nt && !plain; ++it) {
         // ---- values as slices while the scores are made
-        const unsigned v_top = warp_umax(vtop[lane & (WR_WARPS - 1)]);
-        const float v_inv = slice_inv(v_top);
 #pragma unroll
-        for (int i = 0; i < 2 * VB; ++i) slice4(vx[i], v_inv, place(v_s, kq + 8 * i), V_PLANE);
+        for (int i = 0; i < 2 * VB; ++i) slice4(vx[i], place(v_s, kq + 8 * i), V_PLANE);
         load_k(it + 1);
         ok = mbar_sleep_limited(&done[0], it & 1, &dead);
         tc_fence_after();
@@ -284,13 +266,7 @@ __global__ void __launch_bounds__(WR_THREADS, 1) window_runs_kernel(WindowArgs a
             tmem_ld_wait();
             const int k0 = first_key(it) + part * 16, kend = end_key(it);
 #pragma unroll
-            for (int e = 0; e < 16; e += 4) {
-                const float4 k4 = *reinterpret_cast<const float4*>(kunit + part * 16 + e);
-                s[e] = (s[e] + u[e]) * (q_scale * k4.x);
-                s[e + 1] = (s[e + 1] + u[e + 1]) * (q_scale * k4.y);
-                s[e + 2] = (s[e + 2] + u[e + 2]) * (q_scale * k4.z);
-                s[e + 3] = (s[e + 3] + u[e + 3]) * (q_scale * k4.w);
-            }
+            for (int e = 0; e < 16; ++e) s[e] = __fmaf_rn(s[e], a.scale, rest_of(s[e], u[e]) * a.scale);
             if (a.softcap > 0.f) {
                 float big = 0.f;
 #pragma unroll
@@ -345,7 +321,7 @@ __global__ void __launch_bounds__(WR_THREADS, 1) window_runs_kernel(WindowArgs a
             f32x2 w[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) w[e] = pack2(s[2 * e], s[2 * e + 1]);
-            slices_to_tmem<32>(w, slice_inv(127u << 23), lanes + WR_COL_P + part * 8);      // weights are at most one
+            slices_to_tmem<32>(w, lanes + WR_COL_P + part * 8);
         }
         load_v(it + 1);
         tmem_st_wait();
@@ -367,8 +343,7 @@ __global__ void __launch_bounds__(WR_THREADS, 1) window_runs_kernel(WindowArgs a
         plain = odd != 0;
         if (it + 1 < nt && !plain && warp == WR_ISSUE_S) issue_scores();
         // ---- this tile's sums join the row's
-        const float v_unit = slice_unit(v_top) * slice_unit(127u << 23);
-        const f32x2 c2 = pack2(corr, corr), u2 = pack2(v_unit, v_unit);
+        const f32x2 c2 = pack2(corr, corr);
 #pragma unroll
         for (int x = 0; x < VB; ++x) {
             f32x2 o0[8], o1[8];
@@ -376,7 +351,7 @@ __global__ void __launch_bounds__(WR_THREADS, 1) window_runs_kernel(WindowArgs a
             tmem_ld16_nowait(lanes + WR_COL_O + 128 + (part * VB + x) * 16, reinterpret_cast<uint32_t*>(o1));
             tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 8; ++e) acc[x * 8 + e] = fma2(add2(o0[e], o1[e]), u2, mul2(acc[x * 8 + e], c2));
+            for (int e = 0; e < 8; ++e) acc[x * 8 + e] = add2(o0[e], fma2(acc[x * 8 + e], c2, rest_of(o0[e], o1[e])));
         }
     }
     if (!ok) {

@@ -498,6 +498,21 @@ def test_experts_of_a_few_pairs(width, ff, experts, top, sessions):
         eng.close()
 
 
+@pytest.mark.parametrize("dim,scale,cap", [(64, 1.0, 6.0), (64, 1.0, 18.0), (64, 1.0, 60.0), (128, 0.3, 10.0), (128, 1.0, 0.0)])
+def test_window_of_portions_in_fp32_accuracy(dim, scale, cap):
+    """A prompt as a whole (matrix products of slices, caps on both sides of 0.6) is no further from 64 bits than its tokens one by one (fp32 multiply-adds):
+    the quarter is for another order of sums.  A slice or a term of the small tanh less would be tens of times off."""
+    spec, w = make([layer(parallel(window(heads=4, kv_heads=2, dim=dim, size=200, rot=(16, 5000.0), softcap=cap, scale=scale)))], width=256, seed=dim)
+    toks = tokens_of(spec, 400, 4)
+    ref = oracle_logits(spec, w, toks)
+    eng = engine(spec, w)
+    try:
+        off = lambda x: np.linalg.norm(x - ref)
+        assert off(eng.feed([("whole", toks, list(range(400)))])) < 1.25 * off(feed_cut(eng, "single", toks, [1]))
+    finally:
+        eng.close()
+
+
 # ------------------------------------------------------------------------------------------------ the rule alone
 @pytest.mark.parametrize("lanes", [0, 4, 8, 16, 32])
 @pytest.mark.parametrize("heads,qk_heads,dim,vd", [(3, 3, 20, 9), (4, 2, 64, 33), (2, 1, 128, 16), (1, 1, 7, 70)])
@@ -602,6 +617,75 @@ def test_decay_rule_portions(heads, qk_heads, dim, vd, pad, odd):
         assert err.max() < 8 * 2.0 ** -24, err.max()
     if pad:
         assert torch.equal(state.reshape(R, stride)[:, -pad:].double(), ref_state.reshape(R, stride)[:, -pad:])
+
+
+@pytest.mark.parametrize("what", ["columns", "tokens", "state", "later", "behind a zero decay", "keys", "small"])
+@pytest.mark.parametrize("size", [10, 20, 30])
+def test_decay_rule_portions_by_element(what, size):
+    """Every number by itself against 64 bits, beside numbers 2^size as large: columns of the values, tokens, states, a later token, one that a decay
+    of zero has removed, channels of the keys; and everything small.  What an element does not depend on leaves no trace in it, and what it depends on
+    counts with the sizes of its own terms."""
+    from fasttalk_llm_microservice_b200 import build, native
+    build.build()
+    lib = native.load()
+    dev, heads, dim, vd = "cuda", 2, 128, 96
+    g = torch.Generator(device=dev).manual_seed(size * 11 + len(what))
+    lens = [300, 128, 77]
+    T, R = sum(lens), len(lens)
+    start = [sum(lens[:i]) for i in range(R + 1)]
+    rnd = lambda *s: torch.randn(*s, device=dev, generator=g)
+    q, k, v, ab = rnd(T, heads, dim) * dim ** -0.5, rnd(T, heads, dim), rnd(T, heads, vd), 1 - 0.2 * torch.rand(T, heads, 2, device=dev, generator=g) ** 2
+    state, big, plain = rnd(R, heads, dim, vd), 2.0 ** size, v.clone()
+    some = lambda *s: torch.rand(*s, device=dev, generator=g) < 0.2
+    if what == "columns":
+        v *= torch.where(some(heads, vd), big, 1.0)
+    elif what == "tokens":
+        v *= torch.where(some(T, 1, 1), big, 1.0)
+        q *= torch.where(some(T, 1, 1), big, 1.0)
+    elif what == "state":
+        state *= torch.where(some(R, heads, dim, 1), big, 1.0)
+    elif what == "later":
+        for r in range(R):
+            v[start[r] + 70] *= big
+    elif what == "behind a zero decay":
+        for r in range(R):
+            v[start[r] + 20] *= big
+            ab[start[r] + 23, :, 0] = 0.0
+    elif what == "keys":
+        k *= torch.where(some(heads, dim), big, 1.0)
+    else:
+        q, k, v, state = q / big, k / big, v / big, state / big ** 2
+    pos0 = [5, 0, 9]
+    ref_o, abs_o = (torch.zeros(T, heads, vd, dtype=torch.float64, device=dev) for _ in range(2))
+    ref_s, abs_s = (torch.zeros(R, heads, dim, vd, dtype=torch.float64, device=dev) for _ in range(2))
+    for r in range(R):
+        S = state[r].double() * (pos0[r] > 0)
+        A = S.abs()
+        for t in range(start[r], start[r + 1]):
+            put = k[t].double()[:, :, None] * (ab[t, :, 1:].double() * v[t].double())[:, None, :]
+            S, A = ab[t, :, 0].double()[:, None, None] * S + put, ab[t, :, 0].double()[:, None, None] * A + put.abs()
+            ref_o[t], abs_o[t] = (S * q[t].double()[:, :, None]).sum(1), (A * q[t].double()[:, :, None].abs()).sum(1)
+        ref_s[r], abs_s[r] = S, A
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    rs, rp, sl = i32(start), i32(pos0), i32(list(range(R)))
+
+    def rule(v, state):
+        o = torch.full((T, heads, vd), 7.0, device=dev)
+        rc = lib.ft_decay_rule(q.data_ptr(), k.data_ptr(), v.data_ptr(), ab.data_ptr(), o.data_ptr(), state.data_ptr(), rs.data_ptr(), rp.data_ptr(),
+                               sl.data_ptr(), R, heads, heads, dim, vd, heads * dim * vd, 0, T, None)
+        torch.cuda.synchronize()
+        assert rc == 0, native.last_error()
+        return o
+    other = rule(plain, state.clone())
+    o = rule(v, state)
+    if what == "later":
+        for r in range(R):
+            assert torch.equal(o[start[r]:start[r] + 70], other[start[r]:start[r] + 70])
+    # Token by token a number passes up to 300 roundings of half of 2^-23 of its size, in random directions; by runs of 128 fewer of them, and sums of 128 products cut
+    # off by up to 2^-24 of the largest.  64 * 2^-24 holds either way of summing; operands that lost a slice's last eight bits would be off by 2^-16.
+    for got, ref, size_ in ((o, ref_o, abs_o), (state, ref_s, abs_s)):
+        err = ((got.double() - ref).abs() / size_.clamp_min(1e-300)).max()
+        assert err < 64 * 2.0 ** -24, float(err) * 2 ** 24
 
 
 @pytest.mark.parametrize("heads,qk_heads,dim,vd,pad", [(2, 2, 128, 128, 0), (3, 1, 96, 80, 0), (4, 2, 64, 257, 0), (2, 1, 7, 20, 1), (1, 1, 513, 1, 0)])

@@ -177,6 +177,44 @@ def test_attention_of_portions_with_numbers_beyond_the_slices():
         eng.close()
 
 
+@pytest.mark.parametrize("dim,scale", [(64, 0.125), (128, 1.0), (128, 4.0), (32, 8.0)])
+def test_attention_of_portions_in_fp32_accuracy(dim, scale):
+    """A prompt as a whole (matrix products of slices) is no further from 64 bits than its tokens one by one (fp32 multiply-adds), whatever the scores' size: the quarter is
+    for another order of sums."""
+    spec, w = make([layer(attention(heads=4, kv_heads=2, dim=dim, vdim=64, size=200, scale=scale, rows=24, bias_max=150))], seed=dim, width=256)
+    toks = tokens_of(spec, 400, 4)
+    ref = oracle_logits(spec, w, toks)
+    eng = engine(spec, w)
+    try:
+        off = lambda x: np.linalg.norm(x - ref)
+        assert off(eng.feed([("whole", toks, list(range(400)))])) < 1.25 * off(feed_cut(eng, "single", toks, [1]))
+    finally:
+        eng.close()
+
+
+@pytest.mark.parametrize("size", [10, 20, 25, 30, 35])
+def test_attention_of_portions_beside_a_large_value(size):
+    """One token's value is 2^size as large as the others'.  Positions before it and beyond the window's reach do not see it: row by row they are the oracle's, and to
+    the last bit what they are beside an ordinary token, in whichever tile of keys it lies."""
+    layers = [layer(attention(heads=6, kv_heads=2, dim=32, vdim=32, size=24, keep_first=0, v_mix=False))]
+
+    def huge(w):
+        w["embed"][7] *= 2.0 ** size
+    spec, w = make(layers, seed=8, tweak=huge)
+    toks = [t if t != 7 else 9 for t in tokens_of(spec, 200, 2)]
+    plain = list(toks)
+    toks[90] = 7
+    eng = engine(spec, w)
+    try:
+        got, beside = (eng.feed([(name, t, list(range(200)))]) for name, t in (("s", toks), ("p", plain)))
+        ref = oracle_logits(spec, w, toks)
+        row = np.abs(got - ref).max(1) / np.abs(ref).max(1)
+        assert row.max() < TOL, row.argmax()
+        assert np.array_equal(got[:88], beside[:88]) and np.array_equal(got[140:], beside[140:])
+    finally:
+        eng.close()
+
+
 @pytest.mark.parametrize("width,ff,sessions", [(520, 2056, 1), (1032, 528, 3), (1024, 1024, 4), (2048, 520, 5), (3208, 512, 7), (520, 6400, 2), (520, 512, 8), (520, 512, 9)])
 def test_projections_of_a_few_rows(width, ff, sessions):
     """One to eight rows (and one more) against long weight rows: sixteen and eight weight rows a CTA, steps of 256 channels with and without a rest, outputs
