@@ -603,7 +603,7 @@ static int dense(Engine* e, const float* A, const void* hi, const void* lo, cons
     LinearArgs a;
     a.A = A; a.lda = K; a.W = (const __nv_bfloat16*)W; a.ldw = K; a.C = C; a.ldc = N; a.M = T; a.N = N; a.K = K;
     if (softcap > 0.f) { a.epi = LIN_SOFTCAP; a.cap = softcap; }
-    FT_TRY(launch_linear(a, T, e->stream));
+    FT_TRY(launch_linear(a, T, e->h_kernel_err, e->stream));
     e->st.kernel_launches++;
     return 0;
 }
@@ -611,7 +611,7 @@ static int dense(Engine* e, const float* A, const void* hi, const void* lo, cons
 // Projections of every head side by side: as dense(), one launch for all heads.
 static int heads(Engine* e, const LinearArgs& a) {
     if (e->lay->tensor && a.M >= kTensorMinRows && linear_heads_ok(a)) return launch_linear_heads(a, e->h_kernel_err, e->stream);
-    return launch_linear(a, a.M, e->stream);
+    return launch_linear(a, a.M, e->h_kernel_err, e->stream);
 }
 
 // layer forms whose feed-forward reads a normed input of its own: its projections (the router among them) are not part of w_in
@@ -666,11 +666,11 @@ static int run_experts(Engine* e, const ft_layer_desc& c, const float* logits, i
         }
         gu.w_stride = (long long)n_up * W; gu.ldw = W; gu.C = L.act; gu.ldc = c.ff; gu.seg = L.seg;
         gu.N = n_up; gu.K = W; gu.P = c.experts; gu.epi = act == FT_ACT_RELU2 ? LIN_RELU2 : LIN_SWIGLU_PAIR; gu.glu = glu;
-        FT_TRY(launch_linear(gu, T * top, st));
+        FT_TRY(launch_linear(gu, T * top, e->h_kernel_err, st));
         LinearArgs dn;
         dn.A = L.act; dn.lda = c.ff; dn.W = (const __nv_bfloat16*)c.w_down; dn.w_stride = (long long)W * c.ff;
         dn.ldw = c.ff; dn.C = L.eout; dn.ldc = W; dn.seg = L.seg; dn.N = W; dn.K = c.ff; dn.P = c.experts;
-        FT_TRY(launch_linear(dn, T * top, st));
+        FT_TRY(launch_linear(dn, T * top, e->h_kernel_err, st));
     }
     launched(4);
     return 0;
@@ -693,7 +693,7 @@ static int run_mlp(Engine* e, const void* hi, const void* lo, const void* w_up, 
     LinearArgs up;
     up.A = L.hn; up.lda = W; up.W = (const __nv_bfloat16*)w_up; up.ldw = W; up.C = L.ffb; up.ldc = ff; up.M = T; up.N = n_up;
     up.K = W; up.epi = act == FT_ACT_RELU2 ? LIN_RELU2 : LIN_SWIGLU_PAIR; up.glu = glu;
-    FT_TRY(launch_linear(up, T, st));
+    FT_TRY(launch_linear(up, T, e->h_kernel_err, st));
     e->st.kernel_launches++;
     return dense(e, L.ffb, nullptr, nullptr, w_down, out, T, W, ff);
 }
@@ -774,7 +774,7 @@ static int run_branch(Engine* e, const Batch& b, const LayeredLayer& ll, int k, 
             f.A = L.b2; f.lda = H * (D + R); f.a_col_stride = D + R;
             f.W = (const __nv_bfloat16*)c.w_uk_t; f.w_stride = (long long)C * D; f.ldw = D;
             f.C = L.lstage + R; f.ldc = ls; f.c_col_stride = kd; f.M = T; f.N = C; f.K = D; f.P = H;
-            FT_TRY(launch_linear(f, T, st));
+            FT_TRY(launch_linear(f, T, e->h_kernel_err, st));
             launched(3);
             a.proj = L.lstage; a.ldp = ls; a.o_q = 0; a.o_k = H * kd; a.o_v = -1; a.v_in_key = R;
             a.G = 1; a.dim = kd; a.vdim = C;
@@ -806,7 +806,7 @@ static int run_branch(Engine* e, const Batch& b, const LayeredLayer& ll, int k, 
             v.W = (const __nv_bfloat16*)c.w_uv; v.w_stride = (long long)c.vdim * c.kv_rank; v.ldw = c.kv_rank;
             v.C = L.b3; v.ldc = c.heads * c.vdim; v.c_col_stride = c.vdim;
             v.M = T; v.N = c.vdim; v.K = c.kv_rank; v.P = c.heads;
-            FT_TRY(launch_linear(v, T, st));
+            FT_TRY(launch_linear(v, T, e->h_kernel_err, st));
             launched();
             fin = L.b3;
         }
@@ -829,7 +829,7 @@ static int run_branch(Engine* e, const Batch& b, const LayeredLayer& ll, int k, 
             LinearArgs dtp;
             dtp.A = L.b1; dtp.lda = nl; dtp.W = (const __nv_bfloat16*)c.w_dt; dtp.ldw = kdt; dtp.C = L.b2; dtp.ldc = inner;
             dtp.M = T; dtp.N = inner; dtp.K = kdt;
-            FT_TRY(launch_linear(dtp, T, st));
+            FT_TRY(launch_linear(dtp, T, e->h_kernel_err, st));
         }
         ScanArgs sc;
         sc.x = L.bv; sc.ldx = inner; sc.dt_raw = L.b2; sc.ldd = inner; sc.B = L.b1 + R; sc.C = L.b1 + R + N; sc.ldbc = nl;
@@ -1090,7 +1090,7 @@ static int forward_layered(Engine* e, const Batch& b) {
                 LinearArgs a;
                 a.A = L.proj + c.o_a1; a.lda = ld; a.W = (const __nv_bfloat16*)c.w_a2; a.ldw = c.rank_a;
                 a.C = L.b1; a.ldc = c.heads * c.dim; a.M = T; a.N = c.heads * c.dim; a.K = c.rank_a;
-                FT_TRY(launch_linear(a, T, st));
+                FT_TRY(launch_linear(a, T, e->h_kernel_err, st));
                 da.araw = L.b1;
             } else {                        // one decay per head and token, straight from the stacked projection
                 da.araw = L.proj + c.o_a1; da.head_decay = 1; da.ld_araw = ld;
@@ -1099,7 +1099,7 @@ static int forward_layered(Engine* e, const Batch& b) {
                 LinearArgs g;
                 g.A = L.proj + c.o_g1; g.lda = ld; g.W = (const __nv_bfloat16*)c.w_g2; g.ldw = c.rank_g;
                 g.C = L.b2; g.ldc = c.heads * c.vdim; g.M = T; g.N = c.heads * c.vdim; g.K = c.rank_g;
-                FT_TRY(launch_linear(g, T, st));
+                FT_TRY(launch_linear(g, T, e->h_kernel_err, st));
                 gate = L.b2; ldg = 0;
             }
             da.proj = L.proj; da.ldp = ld; da.o_q = c.o_q; da.o_beta = c.o_beta;

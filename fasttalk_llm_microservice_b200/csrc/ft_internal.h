@@ -138,11 +138,11 @@ struct LinearArgs {
     float c16_scale = 1.f;
     GluSpec glu;                                  // LIN_SWIGLU_PAIR
 };
-// rows_bound: M when batched; an upper bound of seg[P] when grouped
-int launch_linear(const LinearArgs& a, int rows_bound, cudaStream_t stream);
+// rows_bound: M when batched; an upper bound of seg[P] when grouped.  err: set where a wait inside a kernel ran out
+int launch_linear(const LinearArgs& a, int rows_bound, int* err, cudaStream_t stream);
 // linear_stream.cu: a few rows per problem, the weights through shared memory
 bool linear_stream_ok(const LinearArgs& a);
-int launch_linear_stream(const LinearArgs& a, cudaStream_t stream);
+int launch_linear_stream(const LinearArgs& a, int* err, cudaStream_t stream);
 // ---- heads_tc.cu: a batched LinearArgs (seg, a_rows null) on tcgen05, fp32 activations as bf16 hi + lo planes; K and N whole
 // 32-column pieces.  err as for launch_paged16_tc
 bool linear_heads_ok(const LinearArgs& a);

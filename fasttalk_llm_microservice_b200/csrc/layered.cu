@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(LWARPS * 32) linear_rows_kernel(LinearArgs a) 
     }
 }
 
-int launch_linear(const LinearArgs& a, int rows_bound, cudaStream_t stream) {
+int launch_linear(const LinearArgs& a, int rows_bound, int* err, cudaStream_t stream) {
     if (rows_bound <= 0 || a.N <= 0) return 0;
     FT_REQUIRE(a.K >= 1 && a.P >= 1, "linear: bad sizes");
     FT_REQUIRE(a.epi != LIN_SWIGLU_PAIR || (a.N & 1) == 0, "linear: the paired epilogue needs an even number of rows");
@@ -302,7 +302,7 @@ int launch_linear(const LinearArgs& a, int rows_bound, cudaStream_t stream) {
     // weights and more.  Steps at width 2048, us by rows / through shared memory: Gedelorn of one session 412 / 309, four 518 / 372, eight
     // 757 / 456; Vonedra 282 / 199, 342 / 238, 464 / 288; the experts of 16 sessions (32 pairs over 16 of 1024 x 2048 and 2048 x 1024) 56 / 38.
     // Experts of 512 x 1024 and 1024 x 512 lose with the same pairs, whose groups of four rows wait for one another (a step 452 / 503).
-    if (few && linear_stream_ok(a) && (a.seg ? rows_bound <= a.P || (long long)a.N * a.K >= (1 << 21) : a.M <= 8)) return launch_linear_stream(a, stream);
+    if (few && linear_stream_ok(a) && (a.seg ? rows_bound <= a.P || (long long)a.N * a.K >= (1 << 21) : a.M <= 8)) return launch_linear_stream(a, err, stream);
     if (few) {
         const bool pair = a.epi == LIN_SWIGLU_PAIR;
         const int cols = pair ? a.N / 2 : a.N;

@@ -6,6 +6,8 @@
 //
 // The kernel by rows (layered.cu: a warp per four columns, 16 bytes of each on the way, rows staged first) took 30.8 and 25 us for the 32 pairs of 16
 // sessions over 16 experts of 1024 x 2048 and of 2048 x 1024 (58 MB of weights each, 9 us at the copy rate); this one takes 19 each.
+//
+// The wait for the weights has a limit; a CTA whose wait runs out marks `err`, leaves NaN and ends.
 #include "common.cuh"
 #include "ft_internal.h"
 
@@ -30,7 +32,7 @@ __device__ __forceinline__ float transpose_sum(float (&v)[32], int lane) {
 }
 
 template <bool PAIR, int NC>
-__global__ void __launch_bounds__(LS_WARPS * 32) linear_stream_kernel(LinearArgs a) {
+__global__ void __launch_bounds__(LS_WARPS * 32) linear_stream_kernel(LinearArgs a, int* err) {
     constexpr int HALVES = NC / 8;                           // groups of eight weight rows
     extern __shared__ __align__(128) uint8_t ls_w[];
     __shared__ float red[LS_WARPS][32];
@@ -119,18 +121,22 @@ __global__ void __launch_bounds__(LS_WARPS * 32) linear_stream_kernel(LinearArgs
         }
         __syncthreads();
     }
+    if (!ok && tid == 0) {                                   // the results are NaN; the CTA's copies may still be on their way into its memory
+        if (err) *err = 1;
+        for (int i = 0; i < kWaitLimit && !mbar_try_wait(&full, 0); ++i) {}
+    }
 }
 
 int weight_rows(int K) { return (size_t)16 * K * 2 <= LS_MAX_BYTES ? 16 : (size_t)8 * K * 2 <= LS_MAX_BYTES ? 8 : 0; }
 
 template <bool PAIR, int NC>
-int launch(const LinearArgs& a, cudaStream_t stream) {
+int launch(const LinearArgs& a, int* err, cudaStream_t stream) {
     static PerDeviceFlag attr;
     if (!attr.done()) {
         FT_CHECK_CUDA(cudaFuncSetAttribute(linear_stream_kernel<PAIR, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, LS_MAX_BYTES));
         attr.mark();
     }
-    linear_stream_kernel<PAIR, NC><<<dim3((a.N + NC - 1) / NC, a.P), LS_WARPS * 32, (size_t)NC * a.K * 2, stream>>>(a);
+    linear_stream_kernel<PAIR, NC><<<dim3((a.N + NC - 1) / NC, a.P), LS_WARPS * 32, (size_t)NC * a.K * 2, stream>>>(a, err);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -142,11 +148,11 @@ bool linear_stream_ok(const LinearArgs& a) {
     return a.K >= 512 && weight_rows(a.K) > 0 && (a.K & 7) == 0 && (a.ldw & 7) == 0 && (a.lda & 3) == 0 && (a.a_col_stride & 3) == 0 && (a.w_stride & 7) == 0 &&
            ((uintptr_t)a.A & 15) == 0 && ((uintptr_t)a.W & 15) == 0;
 }
-int launch_linear_stream(const LinearArgs& a, cudaStream_t stream) {
+int launch_linear_stream(const LinearArgs& a, int* err, cudaStream_t stream) {
     FT_REQUIRE(linear_stream_ok(a) && a.P <= 65535, "linear (few rows): K %d, row strides %d and %d do not fit", a.K, a.lda, a.ldw);
     const bool pair = a.epi == LIN_SWIGLU_PAIR;
-    if (weight_rows(a.K) == 16) return pair ? launch<true, 16>(a, stream) : launch<false, 16>(a, stream);
-    return pair ? launch<true, 8>(a, stream) : launch<false, 8>(a, stream);
+    if (weight_rows(a.K) == 16) return pair ? launch<true, 16>(a, err, stream) : launch<false, 16>(a, err, stream);
+    return pair ? launch<true, 8>(a, err, stream) : launch<false, 8>(a, err, stream);
 }
 
 }  // namespace ft
