@@ -16,7 +16,7 @@
 // sums 256..511 (first | second accumulator).
 //
 // Where a query, key or value is infinite, NaN or beyond 2^36 the CTA's rows go one by one through plain fp32 code: a hidden key's weight of
-// zero must not make a NaN of its value.  Every wait has a limit; a CTA whose wait runs out marks `err` and ends.
+// zero must not make a NaN of its value.  Every wait has a limit; a CTA whose wait runs out marks `err`, leaves NaN and ends.
 #include "common.cuh"
 #include "ft_internal.h"
 #include "slices.cuh"
@@ -356,6 +356,10 @@ __global__ void __launch_bounds__(WR_THREADS, 1) window_runs_kernel(WindowArgs a
     }
     if (!ok) {
         if (tid == 0 && a.err) *a.err = 1;
+        for (int i = tid; i < used * a.vdim; i += WR_THREADS) {
+            const int r = i / a.vdim;
+            a.out[((size_t)(row_base + r / grp) * a.H + g * grp + r % grp) * a.vdim + i % a.vdim] = __int_as_float(0x7fc00000);
+        }
     } else if (plain) {
         for (int r = warp; r < used; r += WR_WARPS) window_row(a, pt, row_base + r / grp, g * grp + r % grp, p_first + r / grp, lane);
     } else {
@@ -412,7 +416,9 @@ int launch_runs(const WindowArgs& a, const WindowTiles& tm, cudaStream_t stream)
 
 }  // namespace
 
-// heads of at most 128 channels and columns in whole 16-byte units, values beside the keys
+// Heads of at most 128 channels and columns in whole 16-byte units, values beside the keys; no size is too small.  The fp32 tile kernel / this one, us, four heads of 128: 33 new
+// tokens 25.5 / 16.1, 2 behind 600 cached ones 159 / 58, 500 new 153 / 54.  With all keys in its first half tile (32) the fp32 kernel is level: 16 heads of 128 in groups of
+// four 2 tokens 14.9 / 15.0, 9: 16.3 / 15.7, 17: 15.6 / 16.9; how many keys there are stands in device memory.
 bool window_tc_ok(const WindowArgs& a) {
     return a.dim <= 128 && a.vdim <= 128 && ((a.dim | a.vdim) & 3) == 0 && a.v_in_key < 0 && a.H / a.G <= WR_ROWS;
 }
