@@ -296,6 +296,28 @@ def test_first_tokens_and_long_decoding():
 
 
 # ------------------------------------------------------------------------------------------------ batches, pools
+@pytest.mark.parametrize("mixer", [memory(), space(), parallel()], ids=["memory", "space", "parallel"])
+def test_single_tokens_beside_long_portions(mixer):
+    """Decoding sessions beside portions of two whole runs of 128 tokens (and about): the rule takes each kind in a launch of its own."""
+    spec, w = make([layer(mixer, dense()), layer(mixer)], seed=17)
+    eng = engine(spec, w, max_batched_tokens=768, num_pages=40, debug_logit_rows=768)
+    try:
+        seqs = {n: tokens_of(spec, ln, 40 + i) for i, (n, ln) in enumerate([("a", 8), ("b", 35), ("c", 259), ("d", 300)])}
+        got = {n: [] for n in seqs}
+        at = {n: 0 for n in seqs}
+        for step in [{"a": 5, "b": 33, "d": 40}, {"a": 1, "b": 1, "c": 256, "d": 257}, {"a": 1, "b": 1, "c": 1, "d": 1}, {"a": 1, "c": 2, "d": 2}]:
+            out, o = eng.feed([(n, seqs[n][at[n]:at[n] + c], list(range(c))) for n, c in step.items()]), 0
+            for n, c in step.items():
+                got[n].append(out[o:o + c])
+                o += c
+                at[n] += c
+        for n, t in seqs.items():
+            assert at[n] == len(t)
+            assert rel(np.concatenate(got[n]), oracle_logits(spec, w, t)) < TOL, n
+    finally:
+        eng.close()
+
+
 def test_unequal_requests_in_one_batch_match_each_alone():
     spec, w = make(MIXED, seed=13)
     eng = engine(spec, w)
