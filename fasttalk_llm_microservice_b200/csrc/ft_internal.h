@@ -142,6 +142,7 @@ struct LinearArgs {
 int launch_linear(const LinearArgs& a, int rows_bound, int* err, cudaStream_t stream);
 // linear_stream.cu: a few rows per problem, the weights through shared memory
 bool linear_stream_ok(const LinearArgs& a);
+long long linear_stream_ctas(const LinearArgs& a);
 int launch_linear_stream(const LinearArgs& a, int* err, cudaStream_t stream);
 // ---- heads_tc.cu: a batched LinearArgs (seg, a_rows null) on tcgen05, fp32 activations as bf16 hi + lo planes; K and N whole
 // 32-column pieces.  err as for launch_paged16_tc

@@ -298,11 +298,20 @@ int launch_linear(const LinearArgs& a, int rows_bound, int* err, cudaStream_t st
     FT_REQUIRE(a.epi != LIN_SWIGLU_PAIR || (a.N & 1) == 0, "linear: the paired epilogue needs an even number of rows");
     // few rows per problem: one warp per output column, the weights stream once
     const bool few = a.seg ? rows_bound <= 4 * LROWS_MANY : rows_bound <= 2 * LROWS_MANY;
-    // The weights through shared memory where they are what counts: up to eight rows, or grouped problems of a row or so each or with two million
-    // weights and more.  Steps at width 2048, us by rows / through shared memory: Gedelorn of one session 412 / 309, four 518 / 372, eight
-    // 757 / 456; Vonedra 282 / 199, 342 / 238, 464 / 288; the experts of 16 sessions (32 pairs over 16 of 1024 x 2048 and 2048 x 1024) 56 / 38.
-    // Experts of 512 x 1024 and 1024 x 512 lose with the same pairs, whose groups of four rows wait for one another (a step 452 / 503).
-    if (few && linear_stream_ok(a) && (a.seg ? rows_bound <= a.P || (long long)a.N * a.K >= (1 << 21) : a.M <= 8)) return launch_linear_stream(a, err, stream);
+    // The weights through shared memory where they are what counts: up to eight rows, and grouped problems where their CTAs are few for the weights that each of them
+    // brings (an empty problem's CTAs cost as well, and many short ones keep the memory as busy in the kernel by rows, which is why one or two rows of many short
+    // weight rows stay there too).  Steps at width 2048, us by rows / through shared memory: Gedelorn of one session 412 / 309, four 518 / 372, eight 757 / 456; Vonedra 282 /
+    // 199, 342 / 238, 464 / 288; with a head of 128256 rows at width 512, one session: 60 / 87, two 74 / 92, four 104 / 101; at 1024: 87 / 94, 104 / 99, 141 / 111; 64 heads of
+    // 128 x 512 side by side, one row 14.9 / 16.7, two 19.0 / 20.0, four 27.5 / 26.6.
+    // Experts, rows x K of each, 1216 shapes measured, of which this rule takes seven (up to 17 %) wrongly: 16 of 2048 x 2048, 32 pairs: 26.2 / 19.2; 16 of 2048 x 1024, 32
+    // pairs: 24.9 / 22.8, 4 pairs: 8.8 / 9.1; 64 of 2048 x 1024, 24 pairs: 28.2 / 35.5; 32 of 512 x 512, 16 pairs: 6.2 / 7.3; a step of 128 of 2048 x 2048 and 2048 x 1024, 8
+    // pairs: 37 / 52.
+    auto stream_ahead = [&]() {
+        const double ctas = (double)linear_stream_ctas(a);
+        if (a.seg) return ctas * (2 * rows_bound >= a.P ? 1 : 2) <= (a.K >= 1024 ? 2.0 : 1.0) * a.K;
+        return a.M <= 8 && (a.M > 2 || a.K >= (a.M == 1 ? 2048 : 1024) || ctas <= (a.P > 1 ? 0.75 : a.M == 1 ? 1.5 : 2.0) * a.K);
+    };
+    if (few && linear_stream_ok(a) && stream_ahead()) return launch_linear_stream(a, err, stream);
     if (few) {
         const bool pair = a.epi == LIN_SWIGLU_PAIR;
         const int cols = pair ? a.N / 2 : a.N;

@@ -148,6 +148,7 @@ bool linear_stream_ok(const LinearArgs& a) {
     return a.K >= 512 && weight_rows(a.K) > 0 && (a.K & 7) == 0 && (a.ldw & 7) == 0 && (a.lda & 3) == 0 && (a.a_col_stride & 3) == 0 && (a.w_stride & 7) == 0 &&
            ((uintptr_t)a.A & 15) == 0 && ((uintptr_t)a.W & 15) == 0;
 }
+long long linear_stream_ctas(const LinearArgs& a) { return (long long)a.P * ((a.N + weight_rows(a.K) - 1) / weight_rows(a.K)); }
 int launch_linear_stream(const LinearArgs& a, int* err, cudaStream_t stream) {
     FT_REQUIRE(linear_stream_ok(a) && a.P <= 65535, "linear (few rows): K %d, row strides %d and %d do not fit", a.K, a.lda, a.ldw);
     const bool pair = a.epi == LIN_SWIGLU_PAIR;
