@@ -205,8 +205,9 @@ int launch_sandwich_joint(const SandwichArgs& a, int T, cudaStream_t stream) {
             attr.mark();
         }
     }
-    // Few rows: up to 4096 columns in registers (16 rows of 2048: 4.1 us, through shared memory 5.4).  Many rows want the other kernel's occupancy
-    // (2313 rows: 18.4 and 16.2 us).
+    // Few rows: up to 4096 columns in registers (16 rows of 2048: 4.1 us, through shared memory 5.4).  All joints of a step of two layers, shared memory / registers, by rows: 512 columns
+    // 16: 15.2 / 12.2, 296: 16.3 / 13.2; 2048 columns 20.2 / 16.3, 22.9 / 18.4; 4096 columns 28.3 / 22.4, 32.7 / 27.7: ahead at every size up to two rows per SM.  Many rows want
+    // the other kernel's occupancy (2313 rows of 2048: 16.2 us, in registers 18.4); between the two nothing was measured.
     const bool regs = v4 && T <= 2 * device_sms();
     if (regs && a.W <= 1024) sandwich_joint_regs_kernel<1><<<T, 256, 0, stream>>>(a);
     else if (regs && a.W <= 2048) sandwich_joint_regs_kernel<2><<<T, 256, 0, stream>>>(a);
