@@ -1,9 +1,9 @@
 #!/usr/bin/env python
-"""bench.py — streamed tok/s of the B200-native generation backend on BASELINE.json's metric.
+"""bench.py — streamed tok/s of the B200-native generation backend on the reference's headline metric.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
-Workload (BASELINE.json configs[1]): Llama-3.2-1B bf16, 64 concurrent sessions per GPU,
+Workload: Llama-3.2-1B bf16, 64 concurrent sessions per GPU,
 2k-token history, continuous batching.  A "step" is one decode step of the engine over the
 64-session batch at context ~2048 (one pass of the hot path over one batch).
 
@@ -46,7 +46,7 @@ if ROOT not in sys.path:
 MODEL = "llama-3.2-1b"
 SESSIONS = 64
 CTX = 2048
-TURN_NEW = 224          # new history tokens per turn (SURVEY.md §8d cfg 2)
+TURN_NEW = 224          # new history tokens per turn
 TURN_GEN = 32           # generated tokens per turn
 METRIC = "Llama-3.2-1B streamed tok/s at 64 sessions/GPU; p50 TTFT & inter-token latency"
 FALLBACK_HBM_GBS = 6650.0
@@ -67,7 +67,7 @@ class ClockSampler:
     """SM clock and clock-event reasons sampled DURING the timed region.
 
     In-process NVML (nvidia_ml_py) on a thread, one sample every 5 ms; the NVML calls release the GIL
-    and never touch the CUDA stream.  Round 1 spawned `nvidia-smi -lms 100` right before the timer:
+    and never touch the CUDA stream.  An earlier form spawned `nvidia-smi -lms 100` right before the timer:
     the tool's start-up (driver attach, ~0.3 s of host and PCIe activity) overlapped the whole 40 ms
     window of a 20-step run and only two samples ever landed.  start() is now called well before the
     timed region; mark()/unmark() bracket the region so only samples taken inside it are reported.
@@ -429,7 +429,7 @@ def run_native(args, rank, world, local_rank):
     e_steps = e1["steps"] - e0["steps"]
     e2e_value = world * n_out / e2e_s
 
-    # ---- cold TTFT: one 2048-token conversation nobody has cached, alone on the GPU (SURVEY.md §8d)
+    # ---- cold TTFT: one 2048-token conversation nobody has cached, alone on the GPU
     def ttft_once(key, toks):
         torch.cuda.synchronize()
         t0 = time.perf_counter()
@@ -522,7 +522,7 @@ def run_native(args, rank, world, local_rank):
     for i in range(SESSIONS):
         eng.close_session(f"h{i}")
 
-    # ---- WebSocket level (SURVEY.md §8d "two levels"): the reference's UNCHANGED WebSocketLLMServer from
+    # ---- WebSocket level: the reference's UNCHANGED WebSocketLLMServer from
     # baseline/_ref, uvicorn on 127.0.0.1, 64 `websockets` clients in their own process, two turns; turn 2 timed
     # client-side.  Rank 0 only, N = 1 only (one server per GPU in a deployment; the clients need host cores).
     ws_level = None
@@ -584,7 +584,7 @@ def run_native(args, rank, world, local_rank):
                          "ms_per_step_profiled": ms_prof / K},
             "step_roofline": {"bound": "hbm", "bytes_per_step": step_bytes, "achieved": step_achieved, "peak": peak,
                               "unit": "GB/s", "frac": step_achieved / peak,
-                              "note": "whole decode step: weights + KV bytes (SURVEY.md §8d) / device time"},
+                              "note": "whole decode step: weights + KV bytes / device time"},
             "cpu_baseline": cpu_base,
             "e2e": e2e_handler,
             "e2e_engine": {"value": e2e_value, "unit": "tok/s",

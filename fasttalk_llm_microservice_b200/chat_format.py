@@ -1,4 +1,4 @@
-"""OpenAI-wire message normalisation and Hermes tool-call parsing (boundary B, SURVEY.md §8b/§8f).
+"""OpenAI-wire message normalisation and Hermes tool-call parsing (boundary B).
 
 The reference starts vLLM with `--enable-auto-tool-choice --tool-call-parser hermes`
 (`docker-compose.vllm.yml:50-51`): tools are described to the model in a `<tools>` block of the

@@ -1,5 +1,5 @@
 """Load a Hugging Face Llama checkpoint directory (config.json + *.safetensors) into the engine's
-stacked weight layout (weights.py), and write one (SURVEY.md §8f-2).
+stacked weight layout (weights.py), and write one.
 
 The reference names models only by tag and lets the engine container fetch them
 (`app/utils/config.py:86`, `docker-compose.vllm.yml:39`); an in-process engine has to read the

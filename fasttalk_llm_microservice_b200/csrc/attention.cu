@@ -14,7 +14,7 @@
 // A (sequence, head) whose tiles span several CTAs is finished inside the same launch by the
 // last of those CTAs to arrive (per-segment arrival counters in the scratch buffer).
 // The math is mma.sync m16n8k16 with the GQA group (<= 8 q heads) in the M rows: decode
-// attention is HBM-bound (SURVEY.md §8a' a'5), tensor throughput is irrelevant here and
+// attention is HBM-bound, tensor throughput is irrelevant here and
 // tcgen05's minimum M of 64 would be 94 % padding.
 #include "common.cuh"
 #include "ft_internal.h"
@@ -113,7 +113,7 @@ __global__ void attn_decode_plan_kernel(const int* __restrict__ ctx_lens, int* _
 
 // Always-on per-CTA timeline of the most recent decode-attention launch (globaltimer ns):
 // [cta][0] entry, [1] first tile landed, [2] last tile consumed, [3] exit.  Read back with
-// ft_debug_attn_trace (tuning aid, scripts/trace_attn.py).
+// ft_debug_attn_trace (a tuning aid).
 constexpr int ATTN_TRACE_CTAS = 1024;
 __device__ unsigned long long g_attn_trace[ATTN_TRACE_CTAS * 4];
 __device__ __forceinline__ void attn_trace(int slot) {
@@ -167,7 +167,7 @@ attn_decode_kernel(const __half* __restrict__ q, const uint8_t* __restrict__ kv_
         waited = true;
     }
     // one coalesced read of the tile plan instead of a dependent global load per search step
-    // (the start-up chain was 3.3 us of idle HBM per launch, scripts/trace_attn.py)
+    // (the start-up chain was 3.3 us of idle HBM per launch)
     if (B <= ATTN_MAX_B_SMEM) {
         for (int i = threadIdx.x; i <= B; i += ATTN_THREADS) s_prefix[i] = tile_prefix[i];
         tile_prefix = s_prefix;

@@ -437,7 +437,7 @@ __device__ __forceinline__ uint32_t pack_f16_sat(float lo, float hi) {
 // as D / 64 sub-slabs of [64 tokens][64 dims] (128-byte rows), dims 0..63 first, and inside every sub-slab the eight
 // chunks of a row are XOR-swizzled with the row index.  That is (a) conflict-free for ldmatrix after a plain bulk copy
 // and (b) exactly the 128-byte-swizzled UMMA operand layout — K-major for K, MN-major for V — so the tcgen05 attention
-// consumes the cache in place (attention_tc.cu).  For D = 64 there is one sub-slab and this is the round-1 layout.
+// consumes the cache in place (attention_tc.cu).  For D = 64 there is one sub-slab.
 template <int D>
 __host__ __device__ __forceinline__ int kv_swizzled_chunk(int r, int c) {
     return (c >> 3) * (kKvTile * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4);

@@ -222,7 +222,7 @@ struct Layered {
     bool trail_on = false;
 };
 constexpr size_t kStepTimes = 4096;
-constexpr int kDefaultPrefillPlanes = 3;      // one fp16 plane x fp16 weight copies in the large prefill GEMMs (measured: DESIGN.md §2)
+constexpr int kDefaultPrefillPlanes = 3;      // one fp16 plane x fp16 weight copies in the large prefill GEMMs (measured)
 constexpr int kGemmTokenTile = 128;             // token tile of the multi-tile projections (gemm_pick_bn)
 constexpr int kDefaultDecodePrefillCap = 896;    // <= 128 decode rows + 896 -> 1024 rows: a 1B step of ~4.3 ms (1280 rows: 6.6 ms)
 

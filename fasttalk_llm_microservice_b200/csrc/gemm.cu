@@ -10,7 +10,7 @@
 // by the same weight tile into the same TMEM accumulator (D += W*hi; D += W*lo).  That keeps
 // ~16 mantissa bits of every activation through a pure bf16 x bf16 -> fp32 tensor-core product;
 // the weight tile is already in shared memory, so in the HBM-bound decode regime the second
-// product is free (DESIGN.md "precision").  lo may be absent (HILO = false).
+// product is free.  lo may be absent (HILO = false).
 //
 // Epilogue (8 warps): phase 1 moves the fp32 accumulator tile TMEM -> [token][row] staging
 // (shared memory, or — when K is split — this CTA's slab of an L2-resident scratch buffer);
@@ -56,7 +56,7 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
 }
 
 // Always-on, nearly free timeline of CTA (0,0,0) of the most recent GEMM launch (globaltimer ns):
-// read back with ft_debug_gemm_trace (tuning aid, scripts/trace_gemm.py).
+// read back with ft_debug_gemm_trace (a tuning aid).
 __device__ unsigned long long g_gemm_trace[16];
 // ... and of the last 256 launches (ft_debug_gemm_trace_hist): row = launch number mod 256.  Launches
 // overlap under PDL, so a launch's row index is fixed at entry and carried in shared memory.
@@ -105,7 +105,7 @@ __device__ __forceinline__ void store_f16x4(__half* p, size_t idx, float4 y) {
     *reinterpret_cast<uint2*>(p + idx) = h;
 }
 // explicit shared-memory loads: the staging / rstd pointers reach the epilogue as generic pointers, and
-// generic loads interleaved with global stores cost ~0.5 us per token row here (scripts/trace_decode_gemms.py)
+// generic loads interleaved with global stores cost ~0.5 us per token row here
 __device__ __forceinline__ float4 lds_f4(uint32_t a) {
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
@@ -200,7 +200,7 @@ __device__ __forceinline__ void gemm_epilogue_m(const ft_gemm_epilogue& ep, cons
     // ---- this CTA's share of the tile's tokens, and the global operands of the first token batch: residual
     // rows, or position -> RoPE angles / KV page.  They depend on nothing this launch computes, so they are
     // requested BEFORE the accumulator is touched and their L2 latency hides behind phases 1 and 2 (1.5 us of
-    // the 3.4 us a QKV tile's token loop took, scripts/trace_decode_gemms.py).  Tokens are taken U at a time
+    // the 3.4 us a QKV tile's token loop took).  Tokens are taken U at a time
     // per warp; later batches are requested while the current one is being finished.
     const int jbeg = reduce ? BN * split / n_split : col0;
     const int jend = reduce ? BN * (split + 1) / n_split : col0 + CB;
@@ -440,7 +440,7 @@ __device__ __forceinline__ void gemm_epilogue_m(const ft_gemm_epilogue& ep, cons
 // One specialised copy of the epilogue per mode, chosen once per tile: with the mode a run-time value
 // the token loop went through a jump table in constant memory on every row, and with ~0.7 KB of kernel
 // parameters re-read by uniform loads around it the loop ran at ~0.4 us per token row
-// (scripts/trace_decode_gemms.py: 3.4 us for 8 SwiGLU rows with no global access in them).
+// (3.4 us for 8 SwiGLU rows with no global access in them).
 template <int BN, int CB>
 __device__ __forceinline__ void gemm_epilogue(const ft_gemm_epilogue& ep, const EpiCtx& c, uint32_t tmem_acc,
                                               float* stage_f, const float* rstd_s, int col0) {
@@ -1311,7 +1311,7 @@ int launch_gemm(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap*
         // rounds the down and QKV projections lose more to the last, partly empty round than the shape gains)
         const long long work256 = (long long)(n_out / (2 * GEMM_BM)) * ((T + 255) / 256);
         // x_planes == 1: the multi-wave (prefill) tiles multiply the hi plane only — half the tensor work; the
-        // latency-bound decode tiles, where the second product is free, always use both (DESIGN.md §2)
+        // latency-bound decode tiles, where the second product is free, always use both
         const bool one = epi.x_planes == 1;
         if (epi.x_planes == 3) {      // ONE fp16 activation plane against fp16 weights (the caller passed those maps)
             // 256-token tiles also from two rounds on when K is long: the tile's epilogue then hides behind the next

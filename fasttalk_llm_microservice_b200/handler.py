@@ -1,4 +1,4 @@
-"""NativeHandler — the drop-in for the reference's backend handlers (boundary A, SURVEY.md §8b).
+"""NativeHandler — the drop-in for the reference's backend handlers (boundary A).
 
 Duck-types both `VLLMHandler` (`app/core/vllm_handler.py:24-338`) and `OllamaHandler`
 (`app/core/ollama_handler.py:24-458`): same constructor keywords, same
@@ -11,7 +11,7 @@ submits it to the in-process B200 engine and streams sampled tokens back.
 
 The continuous-batching loop runs on the engine's own native thread (`ft_engine_start`); one Python
 thread waits for its events (GIL released) and a second one detokenises and hands each event loop ONE
-wake-up carrying all of a step's tokens (SURVEY.md §7.3), so 64 sessions cost one
+wake-up carrying all of a step's tokens, so 64 sessions cost one
 `call_soon_threadsafe` per decode step rather than 64.  (Tensor-parallel leaders and
 `FASTTALK_NATIVE_LOOP=0` step from the Python thread instead.)
 """
@@ -597,7 +597,7 @@ class NativeHandler:
             raise LLMServiceError(f"native async generation error: {e}", category=ErrorCategory.PROCESSING,
                                   severity=ErrorSeverity.HIGH)
         finally:
-            # disconnects finalise the generator here (SURVEY.md §7.3): the batch slot is freed
+            # disconnects finalise the generator here: the batch slot is freed
             if sink is not None:
                 if sink.timer is not None:
                     sink.timer.cancel()
@@ -605,8 +605,8 @@ class NativeHandler:
 
 
 def install(into_vllm: bool = True, into_ollama: bool = True) -> None:
-    """Swap NativeHandler in for the reference's handler classes without editing the reference
-    (SURVEY.md §8b): `WebSocketLLMServer` imports `VLLMHandler` lazily
+    """Swap NativeHandler in for the reference's handler classes without editing the reference:
+    `WebSocketLLMServer` imports `VLLMHandler` lazily
     (websocket_server_vllm.py:113), the legacy server imports `OllamaHandler` at module top
     (websocket_server.py:22), so call this BEFORE importing `app.core.websocket_server*`."""
     if into_vllm:

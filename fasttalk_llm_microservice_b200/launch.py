@@ -1,4 +1,4 @@
-"""One engine process per GPU (SURVEY.md §8e: sessions are independent, replicas only, no
+"""One engine process per GPU (sessions are independent, replicas only, no
 collective).  Each replica is the OpenAI/Ollama-compatible server of openai_server.py bound to
 its own GPU and port; the reference's service instances (one per replica, unchanged) point
 `VLLM_BASE_URL` / `OLLAMA_BASE_URL` at them.  A conversation must keep going to the replica that

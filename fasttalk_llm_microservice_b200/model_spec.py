@@ -1,9 +1,9 @@
-"""Model dimensions for the three Llama configurations BASELINE.json names.
+"""Model dimensions for the three Llama configurations that are served.
 
 The reference (Berkay2002/fasttalk-llm-microservice) carries no model code: it
 names models only by tag (`app/utils/config.py:86` "llama3.2:1b",
 `docker-compose.vllm.yml:39`).  The dimensions below are the public HF configs
-of those models (SURVEY.md Appendix B).
+of those models.
 """
 from __future__ import annotations
 
@@ -60,15 +60,15 @@ class ModelSpec:
         return self.layers * per_layer + emb + head + self.hidden
 
     def weight_bytes(self) -> int:
-        """bf16 bytes streamed once per decode step (SURVEY.md §8d P_bytes)."""
+        """bf16 bytes streamed once per decode step."""
         return 2 * self.param_count()
 
     def kv_bytes_per_token(self) -> int:
-        """16-bit (fp16 in the cache, bf16 in SURVEY.md §8d: same size) K+V bytes one cached token occupies over all layers."""
+        """16-bit (fp16) K+V bytes one cached token occupies over all layers."""
         return 2 * self.layers * self.n_kv_heads * self.head_dim * 2
 
     def decode_step_bytes(self, ctx_lens) -> int:
-        """Algorithmic HBM bytes of one decode step (SURVEY.md §8d)."""
+        """Algorithmic HBM bytes of one decode step."""
         return self.weight_bytes() + int(sum(ctx_lens)) * self.kv_bytes_per_token()
 
     def to_dict(self) -> Dict:

@@ -1,4 +1,4 @@
-"""Ollama-compatible NDJSON routes over the in-process engine (SURVEY.md §8f-3).
+"""Ollama-compatible NDJSON routes over the in-process engine.
 
 With these routes listening where the reference expects Ollama (`OLLAMA_BASE_URL`), the unchanged
 `OllamaHandler` (`app/core/ollama_handler.py`) drives the B200 engine:

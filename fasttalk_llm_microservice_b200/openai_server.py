@@ -1,4 +1,4 @@
-"""OpenAI-compatible HTTP front over the in-process engine (boundary B, SURVEY.md §8b/§8f-1).
+"""OpenAI-compatible HTTP front over the in-process engine (boundary B).
 
 With this app listening where the reference expects vLLM, nothing in the reference is patched:
 `VLLM_BASE_URL=http://host:port/v1` and the unchanged `VLLMHandler`
@@ -244,7 +244,7 @@ def create_app(handler: NativeHandler, served_model: Optional[str] = None) -> St
         Route("/health", health, methods=["GET"]),
         Route("/v1/models", models, methods=["GET"]),
         Route("/v1/chat/completions", chat, methods=["POST"]),
-    ] + ollama_routes(handler, served, keys))     # the same process answers Ollama's wire (§8f-3)
+    ] + ollama_routes(handler, served, keys))     # the same process answers Ollama's wire
 
 
 def main(argv=None):

@@ -5,8 +5,8 @@ With Ollama / vLLM the reference never sees tokens (`app/core/vllm_handler.py:24
 
 * `HFTokenizer` wraps a real `tokenizer.json` (path in $FASTTALK_TOKENIZER_JSON) through the
   `tokenizers` package.
-* `ByteTokenizer` is the fallback when no vocabulary file is on the box (there is none here:
-  SURVEY.md Appendix D).  It is a bijection between text and ids: UTF-8 bytes are ids 0..255,
+* `ByteTokenizer` is the fallback when no vocabulary file is on the box (there is none
+  here).  It is a bijection between text and ids: UTF-8 bytes are ids 0..255,
   every other non-special id maps to one private-use code point, so text the model produced
   re-encodes to exactly the tokens it was generated from (the re-sent history then matches
   the session's cached KV prefix) and one token is one non-empty chunk.
@@ -18,7 +18,7 @@ import os
 import re
 from typing import Dict, Iterable, List, Optional, Sequence
 
-# Llama-3 special ids (public; SURVEY.md Appendix A)
+# Llama-3 special ids (public)
 BOS, EOT_TEXT, START_HEADER, END_HEADER, EOT = 128000, 128001, 128006, 128007, 128009
 
 

@@ -1,4 +1,4 @@
-"""Tensor parallelism over two GPUs for the 8B-class configuration (SURVEY.md §8e, §8a′12).
+"""Tensor parallelism over two GPUs for the 8B-class configuration.
 
 The reference gets this from vLLM's `--tensor-parallel-size` when one GPU is not enough
 (`docker-compose.vllm.yml:49`); here it is a latency optimisation: each GPU streams half of the

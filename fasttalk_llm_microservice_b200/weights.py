@@ -1,5 +1,5 @@
 """Deterministic random-init weights of the named architecture (no checkpoints on
-the box: BASELINE.json north_star, SURVEY.md §8d "Synthetic inputs").
+the box).
 
 Layout (all bf16, row-major, `[out_features, in_features]` like nn.Linear):
   embed      [V, h]

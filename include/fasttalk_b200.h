@@ -44,7 +44,7 @@ typedef struct {
     int eos_ids[4];          /* stop tokens (<|eot_id|> 128009, <|end_of_text|> 128001) */
     int use_pdl;             /* programmatic dependent launch between the step's kernels */
     int debug_logit_rows;    /* rows of the logits buffer (>= max_batch); more only for ft_debug_* */
-    /* Tensor parallelism (Llama-3.1-8B, TP=2 over NVLink).  tp_size 0/1 = off, 2 = this
+    /* Tensor parallelism.  tp_size 0/1 = off, 2 = this
      * engine is one of two ranks, one process per GPU.  n_q_heads, n_kv_heads and ffn are then this
      * rank's SHARE (half), vocab stays the full vocabulary, and the weights are the rank's slices:
      * wqkv rows (q | k | v of the local heads), wo columns of the local heads, wgu rows of the local
@@ -135,7 +135,7 @@ int ft_engine_step(ft_engine* e);
  * ft_engine_wait: blocks up to timeout_ms; returns the number of queued events (0 = timeout), or < 0 when the stepping
  * thread died on an error (ft_last_error has it) and nothing is left to drain, or when the engine is being destroyed
  * (ft_engine_destroy sends a thread that is still blocked here away before it frees anything).
- * No counterpart in the reference: its engines (Ollama, vLLM) are separate server processes (SURVEY.md §8b). */
+ * No counterpart in the reference: its engines (Ollama, vLLM) are separate server processes. */
 int ft_engine_start(ft_engine* e);
 int ft_engine_stop(ft_engine* e);
 int ft_engine_wait(ft_engine* e, int timeout_ms);

@@ -3,7 +3,7 @@
 Batched decode step of the oracle arithmetic (oracle/llama_oracle.py) on the host cores:
 the CPU stand-in for the reference's CPU path, which is Ollama/llama.cpp on host cores
 (`app/core/ollama_handler.py:142-177` with COMPUTE_DEVICE=cpu, docker-compose.cpu.yml:11) and
-cannot be installed here (BASELINE.md §2).  fp32 PyTorch, all host threads, weights read once
+cannot be installed here.  fp32 PyTorch, all host threads, weights read once
 per step for the whole batch (what any batching CPU engine does), per-sequence attention over
 a contiguous fp32 KV cache.  It is NOT llama.cpp: a quantised GGUF would be faster.
 """

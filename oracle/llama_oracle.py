@@ -2,8 +2,8 @@
 
 fp32 PyTorch restatement of the generation arithmetic the reference delegates to
 Ollama / vLLM (`app/core/ollama_handler.py:142-177`, `app/core/vllm_handler.py:177,271`).
-The reference holds no model code and no golden vectors for this path
-(SURVEY.md §4, §8c), and neither engine is installable here (Ollama: unpinned
+The reference holds no model code and no golden vectors for this path,
+and neither engine is installable here (Ollama: unpinned
 `ollama/ollama:latest`, docker-compose.cpu.yml:11; vLLM: unpinned
 `vllm/vllm-openai:latest`, docker-compose.vllm.yml:12), so against the reference
 itself **parity is unpinned**.  What pins this file instead: tests/test_oracle.py

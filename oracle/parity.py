@@ -1,8 +1,8 @@
 """Greedy-parity checker: TEST INFRASTRUCTURE (tests/, __graft_entry__.smoke(), never the product).
 
-north_star: "greedy token sequences must be identical for the first 64 tokens and logits must match
+The requirement: "greedy token sequences must be identical for the first 64 tokens and logits must match
 within 2e-2 relative".  On random-init weights the fp32 oracle itself meets top-1/top-2 near-ties that
-no 16-bit pipeline can resolve.  This checker therefore does what the round-1 verdict
+no 16-bit pipeline can resolve.  This checker therefore does what a review
 asked for instead of stopping at the first mismatch:
 
   * the engine generates greedily; at every step its logits are compared with the oracle's logits of
@@ -26,7 +26,7 @@ from typing import List, Optional, Sequence
 
 import torch
 
-LOGIT_TOL = 2e-2            # north_star: logits within 2e-2 relative (max|delta| / max|logit| per position)
+LOGIT_TOL = 2e-2            # logits within 2e-2 relative (max|delta| / max|logit| per position)
 WAIVER_FLOOR = 5e-4         # margins below this fraction of the logit scale are ties for any 16-bit path
 WAIVERS_PER_64 = 2
 

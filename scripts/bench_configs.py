@@ -1,5 +1,5 @@
-"""The other BASELINE.json configurations, measured like bench.py measures configs[1] (they are not
-bench lines; their numbers go into DESIGN.md §6 and profiles/):
+"""The other serving configurations, measured like bench.py measures its own (they are not
+bench lines; their numbers go into the design notes and profiles/):
 
   cfg1  Llama-3.2-1B, ONE session, 128-token prompt, 256 greedy tokens (the reference's CPU-runnable case)
   cfg3  Llama-3.2-3B, 256 sessions at a 2k history on one GPU, and the 32-sessions-per-GPU share of an 8-GPU node
@@ -118,7 +118,7 @@ def cfg5():
     th = threading.Thread(target=server.run, daemon=True); th.start()
     while not server.started:
         time.sleep(0.02)
-    # byte tokenizer: one ASCII character = one token, so text length = token count (SURVEY.md §8d)
+    # byte tokenizer: one ASCII character = one token, so text length = token count
     tools = [{"type": "function", "function": {"name": f"tool_{i}", "description": "d" * 40, "parameters": {
         "type": "object", "properties": {"q": {"type": "string"}}, "required": ["q"]}}} for i in range(2)]
     n_agents = 16

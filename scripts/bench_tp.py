@@ -4,7 +4,7 @@
         --master-port 29552 scripts/bench_tp.py [--model llama-3.1-8b] [--ctx 7936] [--steps 64]
 
 Rank 0 prints one JSON line: ms/step and tok/s for 1 and 8 sessions at ctx `--ctx`, TP=2 and TP=1
-side by side, with the HBM roofline of each (weights + KV bytes per GPU per step, SURVEY.md §8d)."""
+side by side, with the HBM roofline of each (weights + KV bytes per GPU per step)."""
 import argparse, json, os, sys, time
 import torch
 import torch.distributed as dist

@@ -1,4 +1,4 @@
-"""A/B of the tensor-parallel all-reduce (round-1 verdict, next #9): the row-parallel projection with the exchange
+"""A/B of the tensor-parallel all-reduce: the row-parallel projection with the exchange
 fused into its epilogue (P2P stores over NVLink + flags, csrc/gemm.cu) against the same projection followed by
 `ncclAllReduce` (torch.distributed, NCCL) on its output — Llama-3.1-8B's two row-parallel shapes at TP=2.
 

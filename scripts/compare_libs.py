@@ -1,4 +1,4 @@
-"""Same-box comparators at kernel level (round-1 verdict, next #7): the library kernels this image ships
+"""Same-box comparators at kernel level: the library kernels this image ships
 (FlashInfer 0.6, flash-attn 2.8, cuBLAS through torch.matmul) against this repository's own kernels,
 through the C ABI, at the shapes the engine runs.  Every pair is timed the same way: CUDA events over
 `iters` back-to-back launches on torch's current stream after a warm-up, rotating over enough copies of
@@ -148,7 +148,7 @@ def prefill_attention(rows):
                                                        N.ptr(out_lo), nq, nkv, d, q_rows, N.cur_stream()), "ft_attn_prefill")
         us = timed([ours(T)], iters=20)                  # tcgen05 / TMEM kernel
         hi_tc = out.float() + out_lo.float()
-        us_sync = timed([ours(0)], iters=20)             # the round-1 mma.sync kernel (q_rows = 0 selects it)
+        us_sync = timed([ours(0)], iters=20)             # the mma.sync kernel (q_rows = 0 selects it)
         hi_sync = out.float() + out_lo.float()
         row = {"section": f"prefill attention ({heads} heads: nq {nq}, nkv {nkv}, d {d})", "shape": label, "GFLOP": flops / 1e9, "ours_us": us,
                "ours": "attn_prefill_tc_kernel (tcgen05 / TMEM)", "ours_TFLOPs": flops / us / 1e6,
@@ -229,7 +229,7 @@ def projections(rows):
                             "ours_useful_TFLOPs": flops / us / 1e6, "ours_issued_TFLOPs": 2 * flops / us / 1e6,
                             "torch_TFLOPs": flops / us_t / 1e6, "torch_frac_tensor": flops / us_t / 1e6 / PEAK_TF,
                             "ours_issued_frac_tensor": 2 * flops / us / 1e6 / PEAK_TF})
-                # the form the engine's large prefill steps run since round 2: ONE fp16 plane against fp16 weight copies
+                # the form the engine's large prefill steps run: ONE fp16 plane against fp16 weight copies
                 # (CTA-pair kernels), here with a plain bf16 output like the library call, and the library on fp16 too
                 x16 = x32.half()
                 ws16 = [w.half() for w in ws]
@@ -252,7 +252,7 @@ def projections(rows):
 
 if __name__ == "__main__":
     ap = argparse.ArgumentParser()
-    ap.add_argument("--out", default=os.path.join(ROOT, "gpurun_out", "compare_libs.json"))
+    ap.add_argument("--out", default=os.path.join(ROOT, "compare_out", "compare_libs.json"))
     ap.add_argument("--only", default="", help="comma list of: decode, prefill, gemm")
     a = ap.parse_args()
     build.build()

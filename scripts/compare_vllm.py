@@ -1,4 +1,4 @@
-"""Engine-level comparator against what the reference actually delegates to (round-1 verdict, next #7 ii):
+"""Engine-level comparator against what the reference actually delegates to:
 vLLM (docker-compose.vllm.yml:12,38-53: `--dtype float16 --max-num-seqs .. --max-num-batched-tokens 8192`), the
 version this image ships, on the SAME random-init Llama-3.2-1B weights (exported with checkpoint.save_hf_checkpoint),
 the cfg-2 workload: 64 sessions x 2048-token histories (token ids), greedy, EOS ignored.
@@ -9,7 +9,7 @@ the cfg-2 workload: 64 sessions x 2048-token histories (token ids), greedy, EOS 
 
 Each engine runs in its own subprocess with a time limit; a failure is recorded as "unavailable: <why>".
 
-    python scripts/compare_vllm.py [--out gpurun_out/compare_vllm.json] [--limit-s 420]
+    python scripts/compare_vllm.py [--out compare_out/compare_vllm.json] [--limit-s 420]
 """
 import argparse
 import json
@@ -114,7 +114,7 @@ def run_hf(out_path, ckpt):
 
 if __name__ == "__main__":
     ap = argparse.ArgumentParser()
-    ap.add_argument("--out", default=os.path.join(ROOT, "gpurun_out", "compare_vllm.json"))
+    ap.add_argument("--out", default=os.path.join(ROOT, "compare_out", "compare_vllm.json"))
     ap.add_argument("--limit-s", type=int, default=420)
     ap.add_argument("--role", default="")
     ap.add_argument("--tmp", default="/tmp/ft_vllm_cmp")

@@ -2,7 +2,7 @@
 # Place the UNMODIFIED reference service (its `app` package) in git-ignored baseline/_ref so that the
 # boundary-A tests and bench.py's WebSocket-level run can drive the reference's own server
 # (app/core/websocket_server_vllm.py) on the GPU box, where /root/reference does not exist.
-# Used only by tests/ and bench.py — never by the product.  baseline/_ref is NOT gpurun-ignored: it travels.
+# Used only by tests/ and bench.py — never by the product.
 #
 #   scripts/install_reference.sh [/root/reference]
 #

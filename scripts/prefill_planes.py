@@ -1,8 +1,8 @@
-"""does prefill still need both activation planes now that attention is fp16?
+"""Does prefill still need both activation planes now that attention is fp16?
 
-For each model and for prefill_planes = 2 (hi + lo, round 1) and 1 (hi only in the multi-wave prefill GEMMs):
+For each model and for prefill_planes = 2 (hi + lo) and 1 (hi only in the multi-wave prefill GEMMs):
   * worst-position logit error of a 2048-token prompt prefilled in ONE 2048-token step (CTA-pair kernel) against
-    the fp32 oracle (max|delta| / max|logit| per position; north_star tolerance 2e-2),
+    the fp32 oracle (max|delta| / max|logit| per position; tolerance 2e-2),
   * teacher-forced decode error and greedy parity of 16 tokens generated AFTER that prefill (the KV cache the
     single-plane projections wrote is what decode then reads),
   * device time of a cold 8192-token prefill step (4 x 2048) and of the e2e-shaped mixed step.

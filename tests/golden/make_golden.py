@@ -3,8 +3,8 @@ authoring container; the GPU box only reads the committed vectors).
 
     python tests/golden/make_golden.py
 
-The reference repo has no model code or golden vectors for generation
-(SURVEY.md §4), so the public transformers implementation of the named
+The reference repo has no model code or golden vectors for generation,
+so the public transformers implementation of the named
 architecture is the pin for oracle/llama_oracle.py.
 """
 import os

@@ -1,4 +1,4 @@
-"""Real-model plumbing on CPU (SURVEY.md §8f-2): a checkpoint written by transformers'
+"""Real-model plumbing on CPU: a checkpoint written by transformers'
 `save_pretrained` loads into the stacked layout and the oracle reproduces transformers' logits on
 it; a real `tokenizer.json` (byte-level BPE built here) streams UTF-8 safely."""
 import json

@@ -1,7 +1,7 @@
 """Whole-path parity: the native engine (through the C ABI) against the fp32 oracle and the
 transformers-generated golden vectors.
 
-north_star tolerance: logits within 2e-2 relative in bf16 — measured here as
+Tolerance: logits within 2e-2 relative in bf16 — measured here as
 max|delta| / max|logit| per position — and greedy tokens identical to the fp32 reference.
 """
 import os
@@ -28,7 +28,7 @@ def make_engine(spec, w, **kw):
 
 
 def per_pos_rel(got, ref):
-    """north_star's "2e-2 relative": worst position of max|delta| / max|logit|."""
+    """The "2e-2 relative": worst position of max|delta| / max|logit|."""
     return ((got - ref).abs().amax(-1) / ref.abs().amax(-1)).max().item()
 
 
@@ -241,7 +241,7 @@ def llama1b():
 def test_llama1b_config1_greedy_and_logits(llama1b):
     """BASELINE config 1 shape: 128-token prompt, greedy decode, random-init Llama-3.2-1B.
     Teacher-forced logits over the prompt within 2e-2; the first 64 greedy tokens identical to
-    the fp32 oracle's.  On random-init weights greedy argmax can hit near-ties (SURVEY.md §7.3):
+    the fp32 oracle's.  On random-init weights greedy argmax can hit near-ties:
     a mismatch is waived only if the oracle's top-1/top-2 margin at that step is within 3x the logit error
     measured in this very run; the engine is then re-aligned to the oracle's token and all 64 positions are
     compared (oracle/parity.py)."""
@@ -704,7 +704,7 @@ def test_submit_cancel_and_close_while_a_step_is_on_the_gpu():
         eng.close()
 
 
-# ------------------------------------------------------------------ a real checkpoint directory (§8f-2)
+# ------------------------------------------------------------------ a real checkpoint directory
 def test_engine_generates_from_a_transformers_checkpoint(tmp_path):
     """transformers writes a Llama checkpoint (`save_pretrained`, sharded safetensors + config.json); checkpoint.py
     loads it into the engine's stacked layout on the GPU; the engine's logits and greedy tokens are compared with

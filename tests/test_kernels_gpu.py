@@ -88,7 +88,7 @@ def test_gemm_fused_swiglu(K, f, T, h):
     (16384, 1300, 2048, "swiglu", "gemm_pair_kernel<128> with a ragged last token tile"),
 ])
 def test_gemm_cta_pair_kernels(K, n_out, T, Kd, mode, what):
-    """The cta_group::2 prefill kernels at kernel level (round 1 only reached the 256-token instantiation through
+    """The cta_group::2 prefill kernels at kernel level (the engine's own sizes only reach the 256-token instantiation through
     the 8300-token engine test): integer-valued bf16 operands make the fp32 result exact, so every tile, the
     peer-CTA half of every activation tile and the ragged tail are checked bit for bit; then random data
     against fp32 torch."""
@@ -155,7 +155,7 @@ def test_gemm_fp16_single_plane_form(K, n_out, T, Kd, what):
 
 def test_attn_decode_empty_context_rows_are_zero(K):
     """A sequence with ctx_lens == 0 has no KV tile and so no CTA works on it: its output rows are defined
-    (zero) instead of left as whatever the buffer held (round-1 verdict, weak #11)."""
+    (zero) instead of left as whatever the buffer held."""
     g = torch.Generator(device=DEV).manual_seed(4)
     nq, nkv, d = 8, 2, 64
     kv = torch.randn(8, nkv, 2, 64, d, device=DEV, generator=g).half()
@@ -563,7 +563,7 @@ def test_attn_prefill_rows_without_a_request(K, before, after, as_given):
 @pytest.mark.parametrize("nq,nkv,d", [(8, 2, 64), (6, 2, 64), (32, 8, 64), (32, 8, 128), (24, 8, 128), (3, 1, 128)])
 def test_attn_prefill_tcgen05_against_mma_sync_and_oracle(K, nq, nkv, d):
     """The tcgen05 / TMEM prefill kernel (GQA groups of 3 and 4, head_dim 64 and 128 — the 1B, 3B and 8B shapes) on the
-    same inputs as the round-1 mma.sync kernel (`tensor_cores=False` selects it): cold and prefix-cached requests, ragged
+    same inputs as the mma.sync kernel (`tensor_cores=False` selects it): cold and prefix-cached requests, ragged
     query tiles, a single query, a context long enough for the lazy rescale and the ring to wrap several times.  Both
     against the fp32 oracle, and against each other."""
     reqs = [(0, 130), (700, 224), (64, 1), (5, 64), (1500, 33)]

@@ -1,6 +1,6 @@
-"""§8f-4 on the GPU: launch.py really starts one engine replica per GPU (separate processes, each seeing one device),
+"""launch.py really starts one engine replica per GPU (separate processes, each seeing one device),
 every replica answers the OpenAI wire, a conversation keeps landing on the replica that holds its KV, and the group
-goes down together on SIGTERM.  Uses every GPU the box has (one on the round-end box, 2/4/8 under `gpurun --gpus N`)."""
+goes down together on SIGTERM.  Uses every GPU the box has."""
 import os
 import signal
 import socket

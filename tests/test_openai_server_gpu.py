@@ -73,7 +73,7 @@ def test_openai_stream_equals_handler_stream_and_reuses_kv(served):
 
 
 def test_ollama_ndjson_wire_over_the_real_engine(served):
-    """§8f-3 on the GPU: the Ollama wire (`POST /api/chat`, NDJSON; ollama_handler.py:142-177, 268-296) answered by
+    """The Ollama wire on the GPU (`POST /api/chat`, NDJSON; ollama_handler.py:142-177, 268-296) answered by
     the same process over the real engine — raw NDJSON first, then, when the reference is on this box
     (baseline/_ref), the reference's UNCHANGED OllamaHandler as the client.  Both must give what NativeHandler
     yields for the conversation."""

@@ -1,5 +1,5 @@
 """The oracle against its pins: transformers-generated golden vectors (committed) and the
-model-size arithmetic SURVEY.md Appendix B quotes."""
+model-size arithmetic."""
 import os
 
 import numpy as np
@@ -24,7 +24,7 @@ def test_survey_byte_model():
     s = get_spec("llama3.2:1b")
     assert s.kv_bytes_per_token() == 32768
     assert abs(s.weight_bytes() / 1e9 - 2.472) < 1e-3
-    # SURVEY.md §8d worked target: 64 sessions x 2048 ctx = 6.767 GB / step
+    # worked target: 64 sessions x 2048 ctx = 6.767 GB / step
     assert abs(s.decode_step_bytes([2048] * 64) / 1e9 - 6.767) < 2e-3
     assert SPECS["llama-3.2-3b"].kv_bytes_per_token() == 114688
     assert SPECS["llama-3.1-8b"].kv_bytes_per_token() == 131072

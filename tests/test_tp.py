@@ -58,7 +58,7 @@ def test_weight_slices_recombine_to_the_full_model():
     assert s0["wgu"].shape == (2, 2 * loc.ffn, 256) and s0["wd"].shape == (2, 256, loc.ffn)
     assert s0["lm_head"].shape == (512, 256) and s0["embed"] is w["embed"]
     assert shard_weights(spec, w, 0, 1) is w and shard_spec(spec, 1) is spec
-    # the 8B configuration of BASELINE.json splits; shapes that cannot are refused
+    # the 8B configuration splits; shapes that cannot are refused
     l8 = shard_spec(LLAMA_3_1_8B, 2)
     assert (l8.n_q_heads, l8.n_kv_heads, l8.ffn) == (16, 4, 7168)
     for bad in ("tiny-d64", "tiny-d128"):           # one kv head per rank is not a whole 128-row tile / odd heads

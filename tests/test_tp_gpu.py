@@ -1,6 +1,6 @@
 """Two-GPU tensor parallelism: the row-parallel projections' all-reduce runs INSIDE the GEMM
 epilogue over NVLink peer memory (csrc/gemm.cu, ft_gemm_epilogue.tp_*).  Needs two GPUs in the
-box (`gpurun --gpus 2`); skipped on a single-GPU box."""
+box; skipped on a single-GPU box."""
 import os
 import socket
 import subprocess

@@ -1,4 +1,4 @@
-"""Boundary A on the GPU (round-1 verdict, missing #1): the reference's UNCHANGED WebSocketLLMServer
+"""Boundary A on the GPU: the reference's UNCHANGED WebSocketLLMServer
 (`app/core/websocket_server_vllm.py:111-123, 528-539`) with NativeHandler swapped in, over the REAL engine,
 64 concurrent `websockets` clients, byte tokenizer, DEFAULT_TEMPERATURE=0.0.  Every session's token frames
 must equal what the handler streams for the very conversation the server built.
@@ -14,7 +14,7 @@ import ws_harness as W
 
 pytestmark = [pytest.mark.gpu,
               pytest.mark.skipif(W.find_reference() is None,
-                                 reason="baseline/_ref missing: run scripts/install_reference.sh before gpurun")]
+                                 reason="baseline/_ref missing: run scripts/install_reference.sh first")]
 GOLD = os.path.join(os.path.dirname(__file__), "golden")
 
 

@@ -4,7 +4,7 @@
         --master-port 29551 tests/tp_worker.py [--model tiny-tp]
 
 Both ranks build the same full weights, keep their slices, swap buffer handles, then run the same
-prompts.  Checked on every rank: prefill logits vs the fp32 oracle (2e-2 relative, north_star),
+prompts.  Checked on every rank: prefill logits vs the fp32 oracle (2e-2 relative),
 greedy tokens vs the oracle's, bit-identical logits on the two ranks, and — rank 0 — that a
 TP=1 engine on the same GPU gives the same tokens."""
 import argparse
