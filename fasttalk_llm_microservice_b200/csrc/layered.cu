@@ -298,18 +298,25 @@ int launch_linear(const LinearArgs& a, int rows_bound, int* err, cudaStream_t st
     FT_REQUIRE(a.epi != LIN_SWIGLU_PAIR || (a.N & 1) == 0, "linear: the paired epilogue needs an even number of rows");
     // few rows per problem: one warp per output column, the weights stream once
     const bool few = a.seg ? rows_bound <= 4 * LROWS_MANY : rows_bound <= 2 * LROWS_MANY;
-    // The weights through shared memory where they are what counts: up to eight rows, and grouped problems where their CTAs are few for the weights that each of them
-    // brings (an empty problem's CTAs cost as well, and many short ones keep the memory as busy in the kernel by rows, which is why one or two rows of many short
-    // weight rows stay there too).  Steps at width 2048, us by rows / through shared memory: Gedelorn of one session 412 / 309, four 518 / 372, eight 757 / 456; Vonedra 282 /
-    // 199, 342 / 238, 464 / 288; with a head of 128256 rows at width 512, one session: 60 / 87, two 74 / 92, four 104 / 101; at 1024: 87 / 94, 104 / 99, 141 / 111; 64 heads of
-    // 128 x 512 side by side, one row 14.9 / 16.7, two 19.0 / 20.0, four 27.5 / 26.6.
-    // Experts, rows x K of each, 1216 shapes measured, of which this rule takes seven (up to 17 %) wrongly: 16 of 2048 x 2048, 32 pairs: 26.2 / 19.2; 16 of 2048 x 1024, 32
-    // pairs: 24.9 / 22.8, 4 pairs: 8.8 / 9.1; 64 of 2048 x 1024, 24 pairs: 28.2 / 35.5; 32 of 512 x 512, 16 pairs: 6.2 / 7.3; a step of 128 of 2048 x 2048 and 2048 x 1024, 8
-    // pairs: 37 / 52.
+    // The weights through shared memory where they are what counts, from 2400 shapes measured with both kernels (us by rows / through shared memory).  A CTA there takes its
+    // weights in one go, two to an SM: a round of them is ahead whatever the rows (one row of 2048: 4096 weight rows 8.3 / 5.4; as pairs of gate and up 7.5 / 6.5), more rounds are where
+    // rows and K are many (8192 x 2048, by rows of the input: one 8.8 / 11.2, two 10.7 / 12.1, four 14.3 / 14.1, eight 29.2 / 21.9; 128256 x 512, one: 41 / 71, four 75 / 82, eight
+    // 223 / 131; pairs of 8192 x 2048, one 8.5 / 11.5, four 13.0 / 14.4; of 16384 x 3072, one 31.7 / 24.6), because many short ones keep the memory busier by rows.
+    // Grouped problems by their CTAs, as an empty problem's cost too: 16 experts of 2048 x 2048, 32 pairs: 26.2 / 19.2; of 2048 x 1024, 32 pairs: 24.9 / 22.8, 4 pairs: 8.8 / 9.1; 64 of
+    // 2048 x 1024, 24 pairs: 28.2 / 35.5; 32 of 512 x 512, 16 pairs: 6.2 / 7.3.  Of all of them 12 go the slower way, seven experts by up to 17 %, the others by up to 4.
     auto stream_ahead = [&]() {
-        const double ctas = (double)linear_stream_ctas(a);
+        const double ctas = (double)linear_stream_ctas(a), sms = device_sms();
         if (a.seg) return ctas * (2 * rows_bound >= a.P ? 1 : 2) <= (a.K >= 1024 ? 2.0 : 1.0) * a.K;
-        return a.M <= 8 && (a.M > 2 || a.K >= (a.M == 1 ? 2048 : 1024) || ctas <= (a.P > 1 ? 0.75 : a.M == 1 ? 1.5 : 2.0) * a.K);
+        if (a.M > 8) return false;
+        if (ctas <= 2 * sms) return true;
+        if (a.epi == LIN_SWIGLU_PAIR) {
+            if (a.M >= 5) return a.K >= 4096 || (ctas > 4 * sms && (a.K >= 768 || a.M > 6 || ctas < 6 * sms));
+            return a.K >= 4096 || (ctas >= 6 * sms && a.K >= (a.M >= 3 ? 2048 : 3072));
+        }
+        if (a.K >= 4096 || a.M > 4) return true;
+        if (a.M == 4) return a.K >= 768 || ctas <= 12 * sms;
+        if (a.M == 3) return a.K >= 1024 ? ctas >= 6 * sms : ctas <= 4 * sms;
+        return a.K >= 2048 && ctas >= 12 * sms;
     };
     if (few && linear_stream_ok(a) && stream_ahead()) return launch_linear_stream(a, err, stream);
     if (few) {
