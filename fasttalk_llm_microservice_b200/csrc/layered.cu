@@ -303,10 +303,14 @@ int launch_linear(const LinearArgs& a, int rows_bound, int* err, cudaStream_t st
     // rows and K are many (8192 x 2048, by rows of the input: one 8.8 / 11.2, two 10.7 / 12.1, four 14.3 / 14.1, eight 29.2 / 21.9; 128256 x 512, one: 41 / 71, four 75 / 82, eight
     // 223 / 131; pairs of 8192 x 2048, one 8.5 / 11.5, four 13.0 / 14.4; of 16384 x 3072, one 31.7 / 24.6), because many short ones keep the memory busier by rows.
     // Grouped problems by their CTAs, as an empty problem's cost too: 16 experts of 2048 x 2048, 32 pairs: 26.2 / 19.2; of 2048 x 1024, 32 pairs: 24.9 / 22.8, 4 pairs: 8.8 / 9.1; 64 of
-    // 2048 x 1024, 24 pairs: 28.2 / 35.5; 32 of 512 x 512, 16 pairs: 6.2 / 7.3.  Of all of them 12 go the slower way, seven experts by up to 17 %, the others by up to 4.
+    // 2048 x 1024, 24 pairs: 28.2 / 35.5; 32 of 512 x 512, 16 pairs: 6.2 / 7.3; 16 of 1024 x 512, 2 pairs: 5.2 / 4.5.  Of all of them 12 go the slower way, seven experts by
+    // up to 9 %, the others by up to 4.
     auto stream_ahead = [&]() {
         const double ctas = (double)linear_stream_ctas(a), sms = device_sms();
-        if (a.seg) return ctas * (2 * rows_bound >= a.P ? 1 : 2) <= (a.K >= 1024 ? 2.0 : 1.0) * a.K;
+        if (a.seg) {
+            const double live = ctas / a.P * (rows_bound < a.P ? rows_bound : a.P);      // with a row, at most
+            return ctas * (2 * rows_bound >= a.P ? 1 : 2) <= (a.K >= 1024 ? 2.0 : 1.0) * a.K || (live <= 1.5 * sms && ctas <= 14 * sms);
+        }
         if (a.M > 8) return false;
         if (ctas <= 2 * sms) return true;
         if (a.epi == LIN_SWIGLU_PAIR) {
