@@ -1,4 +1,4 @@
-// K6 on tcgen05 / TMEM — causal chunked-prefill attention over the paged KV cache (head_dim 64, GQA group 4).
+// K6 on tcgen05 / TMEM — causal chunked-prefill attention over the paged KV cache (head_dim 64 or 128, GQA group of 3 or 4).
 //
 // One CTA = one (request, 64-query tile, KV head): the tile's 64 tokens x the 4 q heads of the group are 256
 // query rows, handled as two 128-row halves (32 tokens x 4 heads each, row = token * 4 + head) so that every
@@ -24,12 +24,15 @@
 // warp 1 = TMEM owner + MMA issuer (one elected thread), warps 2..5 = softmax / epilogue of half 0, warps 6..9 of
 // half 1 (warp w may touch TMEM lanes 32 * (w % 4) .. +31), one thread per query row.
 //
-// What bounds it (in-kernel clock64 timeline + ncu, profiles/r02_attn_prefill_tc.md): per 64-key tile the softmax
-// warps spend ~1200 clk in the exponentials — 64 x 256 of them at the SFU's 16 / clk / SM — and ~1300 clk in the
-// latency-bound rest (TMEM load ~450, row maximum, hand-over); both halves go through these phases in lock step, so
-// the SFU is busy half of the time and the tensor pipe 14 %.  Tried on top and not kept: two threads per row (16
-// softmax warps), prefetching the next tile's scores into a second register set, starting the halves half a tile
-// apart — each within 7 % either way.  The SFU bound itself is ~1024 clk per tile, i.e. about twice this speed.
+// What bounds it (in-kernel clock64 timelines, and this kernel with single parts left out): the hand-overs of a tile, load scores - maximum -
+// exponentials - store P - products - next scores, each a few hundred clocks of latency; 2100 clk per 64-key tile where the
+// exponentials alone take 1024 (the SFU's 16 / clk / SM) and the products 640 (d = 64) or 1280 (d = 128).  Without its
+// exponentials, or with a quarter of its products, it is no more than 15 % faster.  Tried and not kept (four prompts of 2k / 211
+// tokens over 5000, 1B / 8B shapes, us; this kernel 147 / 174): two threads per row 155 / 172 before the order below, one
+// persistent CTA per SM with 128-key tiles at d = 64 and an issuing warp per half 163 / 175, the same with the halves'
+// exponentials in turns 153 / 183 and with two threads per row 172 / 176, pages prefetched into L2 165 / 190.
+// What helped: the longest tiles first over all KV heads (163 -> 149; the last round of CTAs was 15 % of the time), and products whose
+// operands the compiler knows (149 -> 147, 179 -> 174).
 #include "common.cuh"
 #include "ft_internal.h"
 
@@ -43,6 +46,16 @@ constexpr int TC_TOK = 64;                   // query tokens per CTA
 constexpr int TC_SUB_BYTES = kKvTile * 128;  // one [64 tokens][64 dims] fp16 sub-slab = 8 KB; also 64 rows of a Q block
 constexpr int TC_QBLK_BYTES = TC_ROWS * 128; // one 128-row x 64-dim block of Q = 16 KB
 constexpr float TC_RESCALE_THRESHOLD = 8.f;  // log2 units
+
+template <int I>
+struct Int { static constexpr int value = I; };
+template <int N, int I = 0, class F>
+__device__ __forceinline__ void static_for(F&& f) {
+    if constexpr (I < N) {
+        f(Int<I>{});
+        static_for<N, I + 1>(f);
+    }
+}
 
 template <int D>
 struct TcCfg {
@@ -135,15 +148,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
     pdl_wait();
     pdl_launch_dependents();
 
-    // the engine lists a request's q tiles in order, so the LAST tiles see the most keys: take the list back to
-    // front, otherwise the longest CTAs start last and the grid ends in a long tail
-    const int tile_idx = (int)gridDim.x - 1 - (int)blockIdx.x;
+    // the LAST tiles of the list see the most keys where it is in that order: back to front, all KV heads of a tile side by side, or the
+    // longest CTAs would start last and the grid end in a long tail
+    const int tile_idx = (int)gridDim.x / nkv - 1 - (int)blockIdx.x / nkv;
     const int req = tile_req[tile_idx];
     const int q0 = tile_q0[tile_idx];
     const int q_row0 = req_q_start[req];
     const int q_len = req_q_start[req + 1] - q_row0;
     const int pos0 = req_pos0[req];
-    const int kvh = blockIdx.y;
+    const int kvh = (int)blockIdx.x % nkv;
     const int rows_here = q_len - q0 < TC_TOK ? q_len - q0 : TC_TOK;
     const int last_pos = pos0 + q0 + rows_here - 1;
     const int n_tiles = last_pos / kKvTile + 1;
@@ -180,58 +193,75 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
         if (elect_one()) {
             constexpr uint32_t idesc_qk = umma_idesc_f16(TC_ROWS, kKvTile, false);
             constexpr uint32_t idesc_pv = umma_idesc_f16(TC_ROWS, D, true);
-            const uint32_t q_addr = smem_u32(q_s);
-            auto issue_qk = [&](int h, int buf, uint32_t k_addr) {
+            const uint64_t q_desc = umma_desc_k128(smem_u32(q_s)), k_desc = umma_desc_k128(smem_u32(kv_s));
+            const uint64_t v_desc = umma_desc_mn128(smem_u32(kv_s) + KH * TC_SUB_BYTES);
+            // Half, buffer and stage are known to the compiler (the tile loop is unrolled over the ring): an operand put together at run time
+            // costs this thread ~150 clocks a product, four times what the tensor core takes for it.
+            auto issue_qk = [&](auto H, auto BUF, auto STAGE) {
+                constexpr int h = H.value, buf = BUF.value, stage = STAGE.value;
 #pragma unroll
-                for (int kh = 0; kh < KH; ++kh) {
-                    const uint64_t a = umma_desc_k128(q_addr + (h * KH + kh) * TC_QBLK_BYTES);
-                    const uint64_t b = umma_desc_k128(k_addr + kh * TC_SUB_BYTES);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        umma_bf16(tmem_base + C::COL_S + (2 * h + buf) * 64, a + 2 * k, b + 2 * k, idesc_qk, (kh | k) != 0);
-                }
+                for (int k = 0; k < 4 * KH; ++k)
+                    umma_bf16(tmem_base + C::COL_S + (2 * h + buf) * 64,
+                              q_desc + (((h * KH + (k >> 2)) * TC_QBLK_BYTES) >> 4) + 2 * (k & 3),
+                              k_desc + ((stage * C::TILE_BYTES + (k >> 2) * TC_SUB_BYTES) >> 4) + 2 * (k & 3), idesc_qk, k != 0);
                 umma_commit(&s_full[2 * h + buf]);
             };
-            auto stage_of = [&](int j) { return j % C::STAGES; };
-            auto k_addr_of = [&](int j) { return smem_u32(kv_s + (size_t)stage_of(j) * C::TILE_BYTES); };
+            auto issue_pv = [&](auto H, auto BUF, auto STAGE, auto FIRST) {
+                constexpr int h = H.value, buf = BUF.value, stage = STAGE.value;
+                const uint32_t p_tmem = tmem_base + C::COL_S + (2 * h + buf) * 64;        // 64 fp16 = 32 columns, over S
+#pragma unroll
+                for (int k = 0; k < kKvTile / 16; ++k)
+                    umma_f16_ts(tmem_base + C::COL_O + h * D, p_tmem + 8 * k, v_desc + ((stage * C::TILE_BYTES + k * 2048) >> 4), idesc_pv,
+                                !FIRST.value || k != 0);
+                umma_commit(&pv_done[2 * h + buf]);
+            };
             mbar_wait(q_full, 0);
             // scores run two tiles ahead of the softmax (two S buffers per half): tile j + 2 is issued as soon as the
             // product of tile j — which reads its P out of the same buffer — has been issued in front of it
-            for (int j = 0; j < 2 && j < n_tiles; ++j) {
-                mbar_wait(&kv_full[stage_of(j)], (j / C::STAGES) & 1);
-                tc_fence_after();
-                issue_qk(0, j & 1, k_addr_of(j));
-                if (!stagger_on) issue_qk(1, j & 1, k_addr_of(j));
-            }
+            static_for<2>([&](auto J) {
+                if (J.value < n_tiles) {
+                    mbar_wait(&kv_full[J.value], 0);
+                    tc_fence_after();
+                    issue_qk(Int<0>{}, J, J);
+                    if (!stagger_on) issue_qk(Int<1>{}, J, J);
+                }
+            });
             if (stagger_on) {        // half 1 starts when half 0 is about to enter its SFU-bound phase, so that the two halves'
                                      // exponentials do not fall on the SFU at the same time (profiles/r02_attn_prefill_tc.md)
                 mbar_wait(stagger, 0);
-                for (int j = 0; j < 2 && j < n_tiles; ++j) issue_qk(1, j & 1, k_addr_of(j));
+                static_for<2>([&](auto J) {
+                    if (J.value < n_tiles) issue_qk(Int<1>{}, J, J);
+                });
             }
-            for (int j = 0; j < n_tiles; ++j) {
-                const uint32_t v_addr = k_addr_of(j) + KH * TC_SUB_BYTES;
-                const bool more = j + 2 < n_tiles;
-                for (int h = 0; h < 2; ++h) {
-                    // Every hand-over has one barrier PER BUFFER (tile parity): the softmax of one half may run up to two
-                    // tiles ahead of what this thread has observed (it is busy with the other half), and a single barrier
-                    // completing two phases unobserved would look "not yet complete" again — a deadlock.
-                    mbar_wait(&p_full[2 * h + (j & 1)], (j >> 1) & 1);   // P_h(j) written, S_h(j) consumed, O_h rescaled if needed
-                    tc_fence_after();
-                    const uint32_t p_tmem = tmem_base + C::COL_S + (2 * h + (j & 1)) * 64;    // 64 fp16 = 32 columns, over S
-#pragma unroll
-                    for (int k = 0; k < kKvTile / 16; ++k)
-                        umma_f16_ts(tmem_base + C::COL_O + h * D, p_tmem + 8 * k, umma_desc_mn128(v_addr + k * 2048), idesc_pv,
-                                    (j | k) != 0);
-                    umma_commit(&pv_done[2 * h + (j & 1)]);
-                    if (h == 1) umma_commit(&kv_empty[stage_of(j)]);   // every product that reads this stage has been issued
-                    if (more) {
-                        if (h == 0) {
-                            mbar_wait(&kv_full[stage_of(j + 2)], ((j + 2) / C::STAGES) & 1);
+            uint32_t p_phase = 0, kv_phase = 0;      // p_full: every two tiles; kv_full: every round of the ring
+            for (int j0 = 0; j0 < n_tiles; j0 += C::STAGES) {
+                static_for<C::STAGES>([&](auto U) {
+                    constexpr int u = U.value, buf = u & 1, next = (u + 2) % C::STAGES;
+                    const int j = j0 + u;
+                    if (j < n_tiles) {
+                        const bool more = j + 2 < n_tiles;
+                        static_for<2>([&](auto H) {
+                            constexpr int h = H.value;
+                            // Every hand-over has one barrier PER BUFFER (tile parity): the softmax of one half may run up to two
+                            // tiles ahead of what this thread has observed (it is busy with the other half), and a single barrier
+                            // completing two phases unobserved would look "not yet complete" again — a deadlock.
+                            mbar_wait(&p_full[2 * h + buf], p_phase);    // P_h(j) written, S_h(j) consumed, O_h rescaled if needed
                             tc_fence_after();
-                        }
-                        issue_qk(h, j & 1, k_addr_of(j + 2));    // in order behind the product that read P out of this buffer
+                            if (u == 0 && j0 == 0) issue_pv(H, Int<buf>{}, U, Int<1>{});
+                            else issue_pv(H, Int<buf>{}, U, Int<0>{});
+                            if (h == 1) umma_commit(&kv_empty[u]);       // every product that reads this stage has been issued
+                            if (more) {
+                                if (h == 0) {
+                                    mbar_wait(&kv_full[next], u + 2 < C::STAGES ? kv_phase : kv_phase ^ 1);
+                                    tc_fence_after();
+                                }
+                                issue_qk(H, Int<buf>{}, Int<next>{});    // in order behind the product that read P out of this buffer
+                            }
+                        });
+                        if (buf == 1) p_phase ^= 1;
                     }
-                }
+                });
+                kv_phase ^= 1;
             }
         }
     } else {
@@ -377,7 +407,8 @@ static int launch_tc(const CUtensorMap& map, const void* kv_layer, const int* pa
     const float scale_log2 = 1.4426950408889634f / sqrtf((float)D);
     static const int stagger_on = getenv("FT_TC_STAGGER") ? atoi(getenv("FT_TC_STAGGER")) : 1;       // A/B switch; measured: 4–6 % at d = 64
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(n_tiles, nkv);
+    FT_REQUIRE((long long)n_tiles * nkv < (1ll << 31), "attn_prefill: %d tiles of %d KV heads", n_tiles, nkv);
+    cfg.gridDim = dim3(n_tiles * nkv);
     cfg.blockDim = dim3(TC_THREADS);
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = stream;

@@ -7,6 +7,7 @@
 #include "../../include/fasttalk_b200.h"
 
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <condition_variable>
 #include <deque>
@@ -1373,6 +1374,19 @@ static long long fill_batch(Engine* e, const std::vector<Portion>& dec, const st
         for (int q0 = 0; q0 < p.n; q0 += 64, ++tiles) {
             h[m.o_treq + tiles] = j;
             h[m.o_tq0 + tiles] = q0;
+        }
+    }
+    if (!e->lay && b.n_prefill_req > 1) {
+        // the attention kernel takes the list back to front: the tiles that see the most keys come last
+        std::vector<std::array<int, 3>> order(tiles);
+        for (int i = 0; i < tiles; ++i) {
+            const int j = h[m.o_treq + i], q0 = h[m.o_tq0 + i];
+            order[i] = {pre[j].pos0 + std::min(q0 + 64, pre[j].n), j, q0};
+        }
+        std::sort(order.begin(), order.end());
+        for (int i = 0; i < tiles; ++i) {
+            h[m.o_treq + i] = order[i][1];
+            h[m.o_tq0 + i] = order[i][2];
         }
     }
     h[m.o_xstart + b.n_req] = row;

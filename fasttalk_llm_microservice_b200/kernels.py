@@ -187,10 +187,13 @@ def attn_prefill(q: torch.Tensor, kv_layer: torch.Tensor, page_table: torch.Tens
     T, nq, d = q.shape
     nkv = kv_layer.shape[1]
     dev = q.device
-    tile_req, tile_q0 = [], []
+    # the kernel takes the list back to front: the tiles that see the most keys come last
+    tiles = []
     for r in range(len(req_slot)):
-        for q0 in range(0, req_q_start[r + 1] - req_q_start[r], 64):
-            tile_req.append(r); tile_q0.append(q0)
+        n, p0 = int(req_q_start[r + 1] - req_q_start[r]), int(req_pos0[r])
+        tiles += [(p0 + min(q0 + 64, n), r, q0) for q0 in range(0, n, 64)]
+    tiles.sort()
+    tile_req, tile_q0 = [t[1] for t in tiles], [t[2] for t in tiles]
     # The lists go up in one copy that the host does not wait for (five waiting ones cost 60 us of GPU time between calls).  While a
     # stream is captured the copy is an ordinary one, which capture refuses: a replay would read memory that is no longer this call's.
     i32 = lambda v: torch.tensor(v, device="cpu", dtype=torch.int32).reshape(-1)
