@@ -205,6 +205,100 @@ __global__ void __launch_bounds__(128) window_write_kernel(WindowArgs a) {
         row[nk + i] = v;
     }
 }
+// The same for heads of 16 * 2^n channels (up to 128) whose rows lie on 16 bytes, without a norm over all heads: a group of dim / 4 lanes takes a head, four channels
+// a lane, which stay in registers between the norm and the rotation (one channel per thread, two passes: 36 us for 2313 tokens of 16 + 4 + 4
+// heads of 128; now 15.6 us, the bytes take 9).  The heads of a token are dealt out to the groups of `gridDim.y` CTAs.
+__global__ void __launch_bounds__(128) window_write_rows_kernel(WindowArgs a, int lanes) {
+    extern __shared__ float trig[];
+    const int t = blockIdx.x, p = a.positions[t], half = a.rot_dims >> 1;
+    const float* pr = a.proj + (size_t)t * a.ldp;
+    for (int i = threadIdx.x; i < half; i += blockDim.x) {
+        float sn, cs;
+        sincosf((float)p * a.rot_freq[i], &sn, &cs);
+        trig[i] = cs * a.rot_mag;
+        trig[half + i] = sn * a.rot_mag;
+    }
+    const int nq = a.H * a.dim, nk = a.G * a.dim, nv = a.G * a.vdim;
+    const bool alias = a.v_in_key >= 0;
+    const int n_qk = a.H + (a.no_kv ? 0 : a.G), step = gridDim.y * 128 / lanes;
+    float* row = nullptr;
+    if (!a.no_kv) {
+        const int page = a.page_table[(size_t)a.seq_rows[t] * a.max_pages + (p >> 6)];
+        row = a.cache + ((size_t)page * 64 + (p & 63)) * (size_t)(alias ? nk : nk + nv);
+    }
+    const float qt = a.temp_every > 0 ? fmaf(a.temp_coef, logf((float)((p + 1) / a.temp_every + 1)), 1.f) : 1.f;
+    auto plus = [](float4 x, const float* b) {
+        const float4 y = load_f4(b);
+        return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+    };
+    const int c = (threadIdx.x & (lanes - 1)) * 4, group = (blockIdx.y * 128 + threadIdx.x) / lanes;
+    // rotation: four channels' own cosines, and sines with the sign of their partners'
+    const bool turns = c < a.rot_dims, second = a.rot_half && c >= half;
+    const int oc = second ? c - half : c + half;
+    __syncthreads();
+    float4 cs = make_float4(1.f, 1.f, 1.f, 1.f), sn = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (turns && a.rot_half) {
+        const int i0 = second ? c - half : c;
+        const float f = second ? 1.f : -1.f;
+        cs = make_float4(trig[i0], trig[i0 + 1], trig[i0 + 2], trig[i0 + 3]);
+        sn = make_float4(f * trig[half + i0], f * trig[half + i0 + 1], f * trig[half + i0 + 2], f * trig[half + i0 + 3]);
+    } else if (turns) {
+        const int i0 = c >> 1;
+        cs = make_float4(trig[i0], trig[i0], trig[i0 + 1], trig[i0 + 1]);
+        sn = make_float4(-trig[half + i0], trig[half + i0], -trig[half + i0 + 1], trig[half + i0 + 1]);
+    }
+    for (int u0 = group - (int)(threadIdx.x & 31) / lanes; u0 < n_qk; u0 += step) {      // the warp's first head: whole warps stay together for the sums
+        const int u = u0 + (int)(threadIdx.x & 31) / lanes;
+        const bool live = u < n_qk, isq = u < a.H;
+        const int h = !live ? 0 : isq ? u : u - a.H;
+        const float* src = pr + (isq || !live ? a.o_q : a.o_k) + h * a.dim;
+        const float* bias = isq || !live ? a.q_bias : a.k_bias;
+        const float* gain = isq || !live ? a.q_gain : a.k_gain;
+        float4 x = load_f4(src + c), y = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (bias) x = plus(x, bias + h * a.dim + c);
+        if (turns && a.rot_half) {
+            y = load_f4(src + oc);
+            if (bias) y = plus(y, bias + h * a.dim + oc);
+        }
+        float f = 1.f;
+        if (a.qk_norm) {
+            float ss = x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+            for (int o = lanes >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            f = 1.f / sqrtf(ss / (float)a.dim + a.eps);
+        }
+        x = make_float4(x.x * f, x.y * f, x.z * f, x.w * f);
+        y = make_float4(y.x * f, y.y * f, y.z * f, y.w * f);
+        if (gain) {
+            const float4 g = load_f4(gain + c);
+            x = make_float4(x.x * g.x, x.y * g.y, x.z * g.z, x.w * g.w);
+            if (turns && a.rot_half) {
+                const float4 o = load_f4(gain + oc);
+                y = make_float4(y.x * o.x, y.y * o.y, y.z * o.z, y.w * o.w);
+            }
+        }
+        if (turns) {
+            if (!a.rot_half) y = make_float4(x.y, x.x, x.w, x.z);
+            x = make_float4(x.x * cs.x + y.x * sn.x, x.y * cs.y + y.y * sn.y, x.z * cs.z + y.z * sn.z, x.w * cs.w + y.w * sn.w);
+        }
+        if (!live) continue;
+        if (isq) store_f4(a.q_out + (size_t)t * nq + h * a.dim + c, make_float4(qt * x.x, qt * x.y, qt * x.z, qt * x.w));
+        else store_f4(row + h * a.dim + c, x);
+    }
+    if (a.no_kv || alias) return;
+    const float lam = a.v_role == 2 ? a.v_mix[0] : 0.f;
+    for (int i = (blockIdx.y * 128 + threadIdx.x) * 4; i < nv; i += gridDim.y * 512) {
+        float4 v = load_f4(pr + (a.o_v >= 0 ? a.o_v : a.o_k) + i);
+        const float* bias = a.o_v >= 0 ? a.v_bias : a.k_bias;
+        if (bias) v = plus(v, bias + i);
+        if (a.v_role == 1) {
+            store_f4(a.v_first + (size_t)t * nv + i, v);
+        } else if (a.v_role == 2) {
+            const float4 w = load_f4(a.v_first + (size_t)t * nv + i);
+            v = make_float4((1.f - lam) * v.x + lam * w.x, (1.f - lam) * v.y + lam * w.y, (1.f - lam) * v.z + lam * w.z, (1.f - lam) * v.w + lam * w.w);
+        }
+        store_f4(row + nk + i, v);
+    }
+}
 
 // 16-byte asynchronous copy global -> shared of which only the first src_bytes (0 or 16) are read, the rest filled with zeros
 __device__ __forceinline__ void cp_async16_zfill(float* dst_smem, const float* src, int src_bytes) {
@@ -531,10 +625,16 @@ int launch_window_attention(const WindowArgs& a, int T, int n_single, const Wind
     FT_REQUIRE(a.keep_first >= 0 && (!a.rel || a.rel_n >= 1) && (a.v_role == 0 || (a.v_first && a.o_v >= 0)) &&
                    (a.v_role != 2 || a.v_mix),
                "window attention: incomplete options");
+    const int lanes = a.dim / 4;
+    const uintptr_t all = (uintptr_t)a.proj | (uintptr_t)a.q_bias | (uintptr_t)a.k_bias | (uintptr_t)a.v_bias | (uintptr_t)a.q_gain | (uintptr_t)a.k_gain |
+                          (uintptr_t)a.q_out | (uintptr_t)a.cache | (uintptr_t)a.v_first;
+    const bool rows16 = a.qk_norm != 2 && a.dim % 16 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && a.vdim % 4 == 0 && a.ldp % 4 == 0 &&
+                        ((a.o_q | a.o_k) & 3) == 0 && (a.o_v < 0 || a.o_v % 4 == 0) && a.rot_dims % (a.rot_half ? 8 : 4) == 0 && (all & 15) == 0;
     // parts per token: as many as give about two CTAs per SM
     int parts = 1;
     while (a.qk_norm != 2 && parts < a.H && T * parts < 256 && parts < 16) parts *= 2;
-    window_write_kernel<<<dim3(T, parts), 128, (size_t)((a.qk_norm ? a.H + a.G : 0) + a.rot_dims) * 4, stream>>>(a);
+    if (rows16) window_write_rows_kernel<<<dim3(T, parts), 128, (size_t)a.rot_dims * 4, stream>>>(a, lanes);
+    else window_write_kernel<<<dim3(T, parts), 128, (size_t)((a.qk_norm ? a.H + a.G : 0) + a.rot_dims) * 4, stream>>>(a);
     FT_CHECK_CUDA(cudaGetLastError());
     const int grp = a.H / a.G;
     FT_REQUIRE(a.v_in_key < 0 || (a.v_in_key + a.vdim <= a.dim && a.v_role == 0), "window attention: values inside the keys exceed them");
@@ -1083,6 +1183,59 @@ __global__ void __launch_bounds__(256) space_conv_kernel(SpaceArgs a, int T) {
         put(t, acc);
     }
 }
+// The same for blocks of eight tokens, rows on 16 bytes and four taps: a thread takes four channels (one: 27 us for 2313 tokens of 4352 channels; now
+// 25.2 us, the bytes take 12).
+__global__ void __launch_bounds__(128) space_conv_rows_kernel(SpaceArgs a, int T) {
+    constexpr int TB = 8;
+    const int t0 = blockIdx.x * TB, nt = min(TB, T - t0);
+    const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
+    if (blockIdx.y + 1 == gridDim.y)
+        for (int i = threadIdx.x; i < nt * a.heads; i += blockDim.x) {
+            const int t = t0 + i / a.heads, h = i % a.heads;
+            const float dt = softplus_f(a.proj[(size_t)t * a.ldp + a.o_dt + h] + a.dt_bias[h]);
+            a.ab[((size_t)t * a.heads + h) * 2] = expf(-expf(a.a_log[h]) * dt);
+            a.ab[((size_t)t * a.heads + h) * 2 + 1] = dt;
+        }
+    if (c >= a.channels) return;
+    const float4 bias = a.conv_b ? load_f4(a.conv_b + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 w[4];
+    load_taps4(a.conv_w + (size_t)c * 4, w);
+    auto put = [&](int t, float4 s) {
+        if (a.act) s = make_float4(silu_f(s.x), silu_f(s.y), silu_f(s.z), silu_f(s.w));
+        store_f4(a.xbc + (size_t)t * a.channels + c, s);
+    };
+    const int first = a.seq_rows[t0];
+    if (nt == TB && a.seq_rows[t0 + TB - 1] == first && t0 - a.req_start[first] >= 3) {
+        float4 v[TB + 3];
+        const float* row = a.proj + (size_t)(t0 - 3) * a.ldp + a.o_x + c;
+#pragma unroll
+        for (int i = 0; i < TB + 3; ++i) v[i] = load_f4(row + (size_t)i * (unsigned)a.ldp);
+#pragma unroll
+        for (int i = 0; i < TB; ++i) {
+            float4 acc = bias;
+#pragma unroll
+            for (int j = 3; j >= 0; --j) acc = fma_f4(w[j], v[i + j], acc);          // the current token's tap first, as above
+            put(t0 + i, acc);
+        }
+        return;
+    }
+    for (int t = t0; t < t0 + nt; ++t) {
+        const int r = a.seq_rows[t], k = t - a.req_start[r], pos0 = a.req_pos0[r];
+        const float* tail = a.state + (size_t)a.req_slot[r] * a.slot_stride + a.tail_off;
+        float4 acc = bias;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (k - j >= 0) u = load_f4(a.proj + (size_t)(t - j) * a.ldp + a.o_x + c);
+            else if (pos0 + k - j >= 0) {
+                const float* p = tail + (size_t)c * 3 + (k - j + 3);
+                u = make_float4(p[0], p[3], p[6], p[9]);
+            }
+            acc = fma_f4(w[3 - j], u, acc);
+        }
+        put(t, acc);
+    }
+}
 // The slot's tail after the step: the raw inputs of the last K-1 positions, from this step's rows or the old tail.
 constexpr int kMaxTaps = 16;
 __global__ void __launch_bounds__(256) space_tail_kernel(SpaceArgs a) {
@@ -1105,7 +1258,10 @@ __global__ void __launch_bounds__(256) space_tail_kernel(SpaceArgs a) {
 int launch_space_prep(const SpaceArgs& a, int T, int n_req, cudaStream_t stream) {
     FT_REQUIRE(a.taps >= 1 && a.taps <= kMaxTaps, "state space: 1 to %d convolution taps (got %d)", kMaxTaps, a.taps);
     const int groups = (a.channels + 255) / 256;
-    if (T > 64) space_conv_kernel<8><<<dim3((T + 7) / 8, groups), 256, 0, stream>>>(a, T);
+    const uintptr_t all = (uintptr_t)a.proj | (uintptr_t)a.conv_w | (uintptr_t)a.conv_b | (uintptr_t)a.xbc;
+    if (T > 64 && a.taps == 4 && a.channels % 4 == 0 && a.ldp % 4 == 0 && a.o_x % 4 == 0 && (all & 15) == 0)
+        space_conv_rows_kernel<<<dim3((T + 7) / 8, (a.channels / 4 + 127) / 128), 128, 0, stream>>>(a, T);
+    else if (T > 64) space_conv_kernel<8><<<dim3((T + 7) / 8, groups), 256, 0, stream>>>(a, T);
     else space_conv_kernel<1><<<dim3(T, groups), 256, 0, stream>>>(a, T);
     FT_CHECK_CUDA(cudaGetLastError());
     space_tail_kernel<<<dim3((a.channels + 255) / 256, n_req), 256, 0, stream>>>(a);
@@ -1157,6 +1313,56 @@ __global__ void __launch_bounds__(256) readout_kernel(ReadoutArgs a) {
             ((__nv_bfloat16*)a.out_lo)[at] = __float2bfloat16_rn(v - __bfloat162float(b));
         } else {
             a.out[at] = v;
+        }
+    }
+}
+// The same with a normaliser and a norm per head: a warp per (token, head), two columns per lane and step, all of a head's columns in registers, the
+// normaliser read once (a CTA per (token, head): 39 us for 2313 tokens of eight heads of 256; now 15.6 us, the bytes take 9).
+template <int NP>
+__global__ void __launch_bounds__(256) readout_heads_kernel(ReadoutArgs a, int n_pairs) {
+    const int id = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (id >= n_pairs) return;
+    const int t = id / a.heads, h = id % a.heads, n = a.vdim, c0 = h * n;
+    const float* orow = a.o + (size_t)t * a.ldo + (size_t)h * a.vd;
+    float2 v[NP], z[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        const int c = 2 * lane + 64 * i;
+        v[i] = c < n ? make_float2(orow[c], orow[c + 1]) : make_float2(0.f, 0.f);
+        z[i] = a.gate_kind && c < n ? *reinterpret_cast<const float2*>(a.gate + (size_t)t * a.ldg + c0 + c) : make_float2(0.f, 0.f);
+    }
+    const float den = fmaxf(fabsf(orow[n] * a.q_scale), a.floor[(size_t)t * a.heads + h]) + 1e-6f;
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        const int c = 2 * lane + 64 * i;
+        if (c >= n) continue;
+        v[i].x = v[i].x * a.q_scale / den;
+        v[i].y = v[i].y * a.q_scale / den;
+        if (a.skip) {
+            const float2 x = *reinterpret_cast<const float2*>(a.x + (size_t)t * a.ldx + c0 + c);
+            v[i].x = fmaf(a.skip[h], x.x, v[i].x);
+            v[i].y = fmaf(a.skip[h], x.y, v[i].y);
+        }
+        if (a.gate_kind == 1) { v[i].x *= silu_f(z[i].x); v[i].y *= silu_f(z[i].y); }
+        ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, ss));
+    }
+    const float rr = 1.f / sqrtf(warp_sum(ss) / (float)n + a.eps);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        const int c = 2 * lane + 64 * i;
+        if (c >= n) continue;
+        float x = v[i].x * rr, y = v[i].y * rr;
+        if (a.gain) { x *= a.gain[c0 + c]; y *= a.gain[c0 + c + 1]; }
+        if (a.gate_kind == 2) { x *= sigmoid_f(z[i].x); y *= sigmoid_f(z[i].y); }
+        else if (a.gate_kind == 3) { x *= silu_f(z[i].x); y *= silu_f(z[i].y); }
+        const size_t at = (size_t)t * a.heads * n + c0 + c;
+        if (a.out_hi) {
+            const uint32_t hi = pack_bf16(x, y);
+            *reinterpret_cast<uint32_t*>((__nv_bfloat16*)a.out_hi + at) = hi;
+            *reinterpret_cast<uint32_t*>((__nv_bfloat16*)a.out_lo + at) = pack_bf16(x - bf16_lo(hi), y - bf16_hi(hi));
+        } else {
+            *reinterpret_cast<float2*>(a.out + at) = make_float2(x, y);
         }
     }
 }
@@ -1229,6 +1435,15 @@ int launch_readout(const ReadoutArgs& a, int T, cudaStream_t stream) {
         else if (n <= 8 * th) readout_rows_kernel<2><<<T * a.norm_groups, th, 0, stream>>>(a);
         else if (n <= 16 * th) readout_rows_kernel<4><<<T * a.norm_groups, th, 0, stream>>>(a);
         else readout_rows_kernel<8><<<T * a.norm_groups, th, 0, stream>>>(a);
+        FT_CHECK_CUDA(cudaGetLastError());
+        return 0;
+    }
+    if (a.floor && a.norm_groups == a.heads && a.vdim % 2 == 0 && n <= 512 && (!a.gate_kind || a.ldg % 2 == 0) && (!a.skip || a.ldx % 2 == 0) &&
+        (((uintptr_t)a.out | (uintptr_t)a.gate | (uintptr_t)a.x) & 7) == 0 && (((uintptr_t)a.out_hi | (uintptr_t)a.out_lo) & 3) == 0) {
+        const int pairs = T * a.heads, grid = (pairs + 7) / 8;
+        if (n <= 128) readout_heads_kernel<2><<<grid, 256, 0, stream>>>(a, pairs);
+        else if (n <= 256) readout_heads_kernel<4><<<grid, 256, 0, stream>>>(a, pairs);
+        else readout_heads_kernel<8><<<grid, 256, 0, stream>>>(a, pairs);
         FT_CHECK_CUDA(cudaGetLastError());
         return 0;
     }

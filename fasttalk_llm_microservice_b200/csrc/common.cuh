@@ -78,6 +78,21 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     return r;
 }
 
+// rows of fp32 in groups of four columns on 16 bytes
+__device__ __forceinline__ float4 load_f4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void store_f4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+// taps of four neighbouring columns [column][4] -> w[tap] of the columns
+__device__ __forceinline__ void load_taps4(const float* p, float4* w) {
+    const float4 a = load_f4(p), b = load_f4(p + 4), c = load_f4(p + 8), d = load_f4(p + 12);
+    w[0] = make_float4(a.x, b.x, c.x, d.x);
+    w[1] = make_float4(a.y, b.y, c.y, d.y);
+    w[2] = make_float4(a.z, b.z, c.z, d.z);
+    w[3] = make_float4(a.w, b.w, c.w, d.w);
+}
+__device__ __forceinline__ float4 fma_f4(float4 a, float4 b, float4 c) {
+    return make_float4(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y), fmaf(a.z, b.z, c.z), fmaf(a.w, b.w, c.w));
+}
+
 // Programmatic dependent launch: let the next kernel's prologue start early / wait for
 // the producer grid's memory to be visible.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -112,12 +112,65 @@ __global__ void __launch_bounds__(256) canon_kernel(CanonArgs a, int T) {
         put(t, s);
     }
 }
+// The same for blocks of eight tokens, rows on 16 bytes and four taps: a thread takes four columns, so that a warp asks for 512 bytes of each of
+// eleven rows at once (one column per thread: 14.0 us for 2313 tokens of 2048 columns; now 12.1 us, the bytes take 8.7).
+__global__ void __launch_bounds__(128) canon_rows_kernel(CanonArgs a, int T) {
+    constexpr int TB = 8;
+    const int t0 = blockIdx.x * TB, nt = min(TB, T - t0), W = a.W;
+    const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
+    if (c >= W) return;
+    __nv_bfloat16 *hi = (__nv_bfloat16*)a.hi, *lo = (__nv_bfloat16*)a.lo;
+    auto put = [&](int t, float4 s) {
+        store_f4(a.hn + (size_t)t * W + c, s);
+        if (hi) {
+            const uint32_t h0 = pack_bf16(s.x, s.y), h1 = pack_bf16(s.z, s.w);
+            *reinterpret_cast<uint2*>(hi + (size_t)t * W + c) = make_uint2(h0, h1);
+            *reinterpret_cast<uint2*>(lo + (size_t)t * W + c) =
+                make_uint2(pack_bf16(s.x - bf16_lo(h0), s.y - bf16_hi(h0)), pack_bf16(s.z - bf16_lo(h1), s.w - bf16_hi(h1)));
+        }
+    };
+    auto plus = [](float4 x, float4 y) { return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w); };
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 w[4];
+    load_taps4(a.w + (size_t)c * 4, w);
+    const int first = a.seq_rows[t0];
+    if (nt == TB && a.seq_rows[t0 + TB - 1] == first && t0 - a.req_start[first] >= 3) {
+        float4 v[TB + 3];
+        const float* row = a.x + (size_t)(t0 - 3) * W + c;
+#pragma unroll
+        for (int i = 0; i < TB + 3; ++i) v[i] = load_f4(row + (size_t)i * (unsigned)W);
+#pragma unroll
+        for (int i = 0; i < TB; ++i) {
+            float4 acc = zero;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc = fma_f4(w[k], v[i + k], acc);
+            put(t0 + i, plus(v[i + 3], acc));
+        }
+        return;
+    }
+    for (int t = t0; t < t0 + nt; ++t) {
+        const int req = a.seq_rows[t], r = t - a.req_start[req], pos0 = a.req_pos0[req];
+        const float* ring = a.state + (size_t)a.req_slot[req] * a.slot_stride + a.tail_off;      // [3][W]
+        float4 acc = zero;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int back = 3 - i;
+            const float4 v = r - back >= 0 ? load_f4(a.x + (size_t)(t - back) * W + c)
+                                           : pos0 + r - back >= 0 ? load_f4(ring + (size_t)((pos0 + r - back) % 3) * W + c) : zero;
+            acc = fma_f4(w[i], v, acc);
+        }
+        put(t, plus(load_f4(a.x + (size_t)t * W + c), acc));
+    }
+}
 int launch_canon(const CanonArgs& a, int T, cudaStream_t stream) {
     FT_REQUIRE(a.x && a.hn && a.W >= 1, "input convolution: missing operands");
     FT_REQUIRE(!a.w || (a.taps >= 1 && a.taps <= kCanonMaxTaps && a.state), "input convolution: %d taps are beyond %d", a.taps,
                kCanonMaxTaps);
     const int cols = (a.W + 255) / 256;
-    if (T > 64) canon_kernel<8><<<dim3((T + 7) / 8, cols), 256, 0, stream>>>(a, T);
+    const uintptr_t all = (uintptr_t)a.x | (uintptr_t)a.w | (uintptr_t)a.hn | (uintptr_t)a.hi | (uintptr_t)a.lo | (uintptr_t)a.state | (uintptr_t)(a.slot_stride * 4) |
+                          (uintptr_t)(a.tail_off * 4);
+    if (T > 64 && a.w && a.taps == 4 && a.W % 4 == 0 && (all & 15) == 0) canon_rows_kernel<<<dim3((T + 7) / 8, (a.W / 4 + 127) / 128), 128, 0, stream>>>(a, T);
+    else if (T > 64) canon_kernel<8><<<dim3((T + 7) / 8, cols), 256, 0, stream>>>(a, T);
     else canon_kernel<1><<<dim3(T, cols), 256, 0, stream>>>(a, T);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;

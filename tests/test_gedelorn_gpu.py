@@ -800,3 +800,25 @@ def test_short_taps_do_not_reach_an_infinite_row_further_back():
         assert rel(got[clean], ref[clean]) < TOL
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("heads,dim,vdim,rot", [(3, 16, 2, 4), (2, 32, 66, 32), (1, 64, 130, 12), (2, 128, 256, 128), (1, 128, 510, 64)])
+def test_rows_by_four_channels(heads, dim, vdim, rot):
+    """Four taps and rows on 16 bytes: the state space's convolution, queries and cache rows and the matrix memory's read-out over their sizes.  Blocks of eight
+    tokens that hold one request, two, its first three tokens, a short last one; tokens whose taps reach into the state of an earlier step."""
+    spec, w = make([layer(space(heads=2 * heads, vdim=8, state=12, groups=heads, norm_groups=1), dense()), layer(memory(heads=heads, dim=dim, vdim=vdim)),
+                    layer(parallel(window(heads=2 * heads, kv_heads=heads, dim=dim, rot=(rot, 1e4), scale=dim ** -0.5)), dense())], width=84, seed=dim + vdim)
+    eng = engine(spec, w)
+    try:
+        seqs = {n: tokens_of(spec, ln, 40 + i) for i, (n, ln) in enumerate([("a", 203), ("b", 81), ("c", 142)])}
+        at, got = {n: 0 for n in seqs}, {n: [] for n in seqs}
+        for step in [{"a": 65}, {"a": 1, "b": 2, "c": 70}, {"a": 64, "b": 1, "c": 1}, {"a": 3, "b": 78, "c": 2}, {"a": 70, "c": 69}]:
+            out, o = eng.feed([(n, seqs[n][at[n]:at[n] + c], list(range(c))) for n, c in step.items()]), 0
+            for n, c in step.items():
+                got[n].append(out[o:o + c])
+                o += c
+                at[n] += c
+        for n in seqs:
+            assert rel(np.concatenate(got[n]), oracle_logits(spec, w, seqs[n])) < TOL, n
+    finally:
+        eng.close()

@@ -676,3 +676,33 @@ def test_delta_rule_sizes_with_a_decay_per_head(shape):
             at += len(t)
     finally:
         eng.close()
+
+
+def feed_plan(eng, seqs, plan):
+    """Steps of several sessions' portions (session -> tokens of the step); per session the logits of every position."""
+    at, got = {n: 0 for n in seqs}, {n: [] for n in seqs}
+    for step in plan:
+        entries = [(n, seqs[n][at[n]:at[n] + c], list(range(c))) for n, c in step.items()]
+        out, o = eng.feed(entries), 0
+        for n, c in step.items():
+            got[n].append(out[o:o + c])
+            o += c
+            at[n] += c
+    return {n: np.concatenate(g) for n, g in got.items()}
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(3, 1, 16, 4), (2, 2, 32, 36), (4, 2, 64, 64), (5, 5, 128, 12), (2, 1, 128, 128)])
+def test_rows_by_four_channels(heads, kv_heads, dim, vdim):
+    """Four taps and rows on 16 bytes: convolutions, norms and cache rows take four channels a thread and eight tokens a CTA.  Blocks that hold one
+    request, two, its first three tokens, a short last one; tokens whose taps reach into the state of an earlier step."""
+    spec, w = make([layer(attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, scale=dim ** -0.5), dense()),
+                    layer(delta(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim), dense()),
+                    layer(attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, scale=dim ** -0.5))], width=4 * (5 * heads + 1), seed=dim + heads, taps=4)
+    eng = engine(spec, w)
+    try:
+        seqs = {n: tokens_of(spec, ln, 40 + i) for i, (n, ln) in enumerate([("a", 203), ("b", 81), ("c", 142)])}
+        got = feed_plan(eng, seqs, [{"a": 65}, {"a": 1, "b": 2, "c": 70}, {"a": 64, "b": 1, "c": 1}, {"a": 3, "b": 78, "c": 2}, {"a": 70, "c": 69}])
+        for n in seqs:
+            assert rel(got[n], oracle_logits(spec, w, seqs[n])) < TOL, n
+    finally:
+        eng.close()
