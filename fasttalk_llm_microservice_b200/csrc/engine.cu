@@ -19,6 +19,7 @@
 #include <string>
 #include <thread>
 #include <unordered_map>
+#include <unistd.h>
 #include <vector>
 
 namespace ft {
@@ -2265,6 +2266,15 @@ static Session* session_for(Engine* e, unsigned long long key, const char* who) 
     return s;
 }
 
+// A caller's fresh array has no pages yet, and the copy into it would take their faults one by one behind the step (four rows of 128256 logits: @@).
+// They are taken here, while the GPU computes; the array's bytes stay as they are.
+static void fault_in(void* p, size_t bytes) {
+    static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    volatile char* c = static_cast<volatile char*>(p);
+    for (size_t i = 0; i < bytes; i += page) c[i] = c[i];
+    if (bytes) c[bytes - 1] = c[bytes - 1];
+}
+
 extern "C" int ft_engine_feed(ft_engine* h, int n_entries, const unsigned long long* keys, const int* counts,
                               const int* tokens, int n_want, const int* want_rows, float* logits_out) {
     Engine* e = reinterpret_cast<Engine*>(h);
@@ -2334,6 +2344,7 @@ extern "C" int ft_engine_feed(ft_engine* h, int n_entries, const unsigned long l
         b.logit_rows_identity = false;
         rc = upload_meta(e);
         if (!rc) rc = forward(e, b);
+        if (!rc && n_want > 0) fault_in(logits_out, (size_t)n_want * e->cfg.vocab * 4);
         if (!rc && n_want > 0 &&
             cudaMemcpyAsync(logits_out, e->logits, (size_t)n_want * e->cfg.vocab * 4, cudaMemcpyDeviceToHost, e->stream) != cudaSuccess) {
             set_last_error("ft_engine_feed: logits copy failed");
