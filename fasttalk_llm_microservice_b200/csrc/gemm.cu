@@ -151,6 +151,7 @@ struct EpiCtx {
     int n_out, T;
     bool has_acc;            // false: K range empty, the tile is all zeros
     int trace_base;          // row of the launch in the trace history, -1 = this CTA is not traced
+    int lo_cols = 0;       // columns from the hi plane's sums to the lo plane's, 0 where both share theirs
 };
 
 // per-token 1/rms of the activation's source (RMSNorm deferred past the projection), all BN tokens of the tile
@@ -262,6 +263,12 @@ __device__ __forceinline__ void gemm_epilogue_m(const ft_gemm_epilogue& ep, cons
             float v[16];
             if (c.has_acc) {
                 tmem_ld16(tmem_acc + ((uint32_t)(q * 32) << 16) + col0 + c0, v);
+                if (c.lo_cols) {                        // the lo plane's sums lie behind the hi plane's
+                    float low[16];
+                    tmem_ld16(tmem_acc + ((uint32_t)(q * 32) << 16) + c.lo_cols + col0 + c0, low);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] += low[j];
+                }
             } else {
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] = 0.f;
@@ -464,7 +471,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
     constexpr int B_PLANE = BN * GEMM_BK * 2;
     constexpr int B_BYTES = (HILO ? 2 : 1) * B_PLANE;
     constexpr int STAGE_BYTES = GEMM_A_BYTES + B_BYTES;
-    constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
+    // The two planes' tiles lie one after the other: ONE operand of 2 BN rows whose sums lie side by side and are added on the way out.  A product of 128
+    // weight rows takes 60 clk for 16 tokens and 77 for 128 (its 4 KB of weights out of shared memory 32 of them), so half as many of
+    // them halve what a chunk costs once its weights are there.
+    constexpr int N_MMA = (HILO ? 2 : 1) * BN;
+    static_assert(N_MMA <= 256, "one product's columns");
+    constexpr uint32_t TMEM_COLS = N_MMA < 32 ? 32 : N_MMA;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -570,7 +582,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
         }
     } else if (warp == 1) {
         if (elect_one()) {
-            constexpr uint32_t idesc = F16 ? umma_idesc_f16(GEMM_BM, BN) : umma_idesc_bf16(GEMM_BM, BN);
+            constexpr uint32_t idesc = F16 ? umma_idesc_f16(GEMM_BM, N_MMA) : umma_idesc_bf16(GEMM_BM, N_MMA);
             int s = 0;
             uint32_t ph = 0;
             for (int i = 0; i < n_iter; ++i) {
@@ -583,12 +595,6 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
 #pragma unroll
                 for (int k = 0; k < GEMM_BK / 16; ++k)   // UMMA K = 16 bf16 = 32 B -> +2 in addr>>4
                     umma_bf16(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, (i | k) != 0);
-                if (HILO) {
-                    const uint64_t l_desc = umma_desc_k128(a_addr + GEMM_A_BYTES + B_PLANE);
-#pragma unroll
-                    for (int k = 0; k < GEMM_BK / 16; ++k)
-                        umma_bf16(tmem_base, a_desc + 2 * k, l_desc + 2 * k, idesc, 1u);
-                }
                 umma_commit(&empty_bar[s]);               // frees the smem stage when MMAs retire
                 if (++s == stages) { s = 0; ph ^= 1; }
             }
@@ -604,6 +610,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
         c.cta_linear = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
         c.n_ctas = gridDim.x * gridDim.y * gridDim.z;
         c.n_out = n_out; c.T = T; c.has_acc = n_iter > 0; c.trace_base = s_trace_base;
+        c.lo_cols = HILO ? BN : 0;
         epilogue_rstd<BN>(ep, c, rstd_s);
         if (n_iter > 0) {
             mbar_wait(tmem_full_bar, 0);
