@@ -137,7 +137,7 @@ attn_decode_kernel(const __half* __restrict__ q, const uint8_t* __restrict__ kv_
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + (size_t)C::STAGES * C::TILE_BYTES);
     uint64_t* empty_bar = full_bar + C::STAGES;
     float* merge_buf = reinterpret_cast<float*>(empty_bar + C::STAGES);
-    __shared__ int s_last;
+    __shared__ int s_last, s_most;
     __shared__ int s_prefix[ATTN_MAX_B_SMEM + 1];     // tile plan, searched many times per CTA
     // `early` (engine, layers >= 1): the producer may start streaming KV tiles BEFORE the
     // programmatic-dependency wait, because everything it reads then — the tile plan, the page
@@ -168,10 +168,23 @@ attn_decode_kernel(const __half* __restrict__ q, const uint8_t* __restrict__ kv_
     }
     // one coalesced read of the tile plan instead of a dependent global load per search step
     // (the start-up chain was 3.3 us of idle HBM per launch)
-    if (B <= ATTN_MAX_B_SMEM) {
+    const bool one_each = B * nkv <= (int)gridDim.x;      // a CTA for every (sequence, head)
+    if (one_each) {
+        // 31 sequences a warp, the next one's place from the lane behind: the longest sequence too
+        if (threadIdx.x == 0) s_most = 0;
+        __syncthreads();
+        int most = 0;
+        for (int i0 = warp * 31; i0 < B; i0 += 31 * (ATTN_THREADS / 32)) {
+            const int i = min(i0 + lane, B), at = tile_prefix[i], next = __shfl_down_sync(0xffffffffu, at, 1);
+            if (B <= ATTN_MAX_B_SMEM) s_prefix[i] = at;
+            if (lane < 31) most = max(most, next - at);
+        }
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0 && most > 0) atomicMax(&s_most, most);
+    } else if (B <= ATTN_MAX_B_SMEM) {
         for (int i = threadIdx.x; i <= B; i += ATTN_THREADS) s_prefix[i] = tile_prefix[i];
-        tile_prefix = s_prefix;
     }
+    if (B <= ATTN_MAX_B_SMEM) tile_prefix = s_prefix;
     __syncthreads();
     if (!waited && !is_producer) {
         pdl_wait();
@@ -193,7 +206,20 @@ attn_decode_kernel(const __half* __restrict__ q, const uint8_t* __restrict__ kv_
     const long long per = (total + gridDim.x - 1) / gridDim.x;
     long long f = per * blockIdx.x;
     long long f_end = f + per < total ? f + per : total;
-    if (f >= total) {
+    // A CTA takes all of a (sequence, head) where there is one for each and that makes its walk longer by no more tiles than the merge of the parts costs
+    // (0.53 us a tile; the merge 2.5 to 4.5 us at head_dim 64, up to 6 at 128, by how the shares lie).  One call, plan included, us, by shares -> whole: head_dim 64,
+    // 4 sessions x 8 heads of 128 keys 7.5 -> 5.6, of 384 8.6 -> 7.8, of 512 8.7 and 8.8; 32 sessions of 512 14.0 -> 10.5; head_dim 128, 8 sessions
+    // of 320 12.8 -> 8.0, 4 of 512 9.6 -> 9.4, of 768 10.1 and 11.5.
+    if (one_each && s_most - (int)per <= (D == 64 ? (per == 1 ? 5 : 4) : 7)) {
+        const int b = blockIdx.x / nkv;
+        f = f_end = total;
+        if (b < B) {
+            const int first = tile_prefix[b], tiles = tile_prefix[b + 1] - first;
+            f = (long long)first * nkv + (long long)(blockIdx.x % nkv) * tiles;
+            f_end = f + tiles;
+        }
+    }
+    if (f >= f_end) {
         if (!waited) pdl_wait();
         return;
     }

@@ -47,16 +47,6 @@ constexpr int TC_SUB_BYTES = kKvTile * 128;  // one [64 tokens][64 dims] fp16 su
 constexpr int TC_QBLK_BYTES = TC_ROWS * 128; // one 128-row x 64-dim block of Q = 16 KB
 constexpr float TC_RESCALE_THRESHOLD = 8.f;  // log2 units
 
-template <int I>
-struct Int { static constexpr int value = I; };
-template <int N, int I = 0, class F>
-__device__ __forceinline__ void static_for(F&& f) {
-    if constexpr (I < N) {
-        f(Int<I>{});
-        static_for<N, I + 1>(f);
-    }
-}
-
 template <int D>
 struct TcCfg {
     static constexpr int KH = D / 64;                                   // 64-dim blocks of the head

@@ -78,6 +78,17 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     return r;
 }
 
+// whole numbers that the compiler knows, and loops over them
+template <int I>
+struct Int { static constexpr int value = I; };
+template <int N, int I = 0, class F>
+__device__ __forceinline__ void static_for(F&& f) {
+    if constexpr (I < N) {
+        f(Int<I>{});
+        static_for<N, I + 1>(f);
+    }
+}
+
 // rows of fp32 in groups of four columns on 16 bytes
 __device__ __forceinline__ float4 load_f4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void store_f4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
@@ -264,9 +275,9 @@ __device__ __forceinline__ unsigned peer_ld(const unsigned* p, int rank) {
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_addr(p, rank)) : "memory");
     return v;
 }
-__device__ __forceinline__ float peer_ld_at(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+__device__ __forceinline__ float4 peer_ld4_at(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
     return v;
 }
 // Tile load issued by EITHER CTA of the pair into its own shared memory; the bytes are counted on

@@ -38,6 +38,10 @@ def gemm_bf16(w: torch.Tensor, x: torch.Tensor, x_lo: Optional[torch.Tensor] = N
     if mode == "partials":
         if n_splits <= 0:
             n_splits = lib.ft_gemm_pick_splits(n_out, T, K, int(x_lo is not None))
+            # Few tokens and both planes: CTAs of a cluster share K and add their parts themselves.  Ahead of parts and a sum behind them up to 64 tokens
+            # (us, 2048 x 2048, parts + sum -> one: 4 tokens 7.9 -> 5.4, 64 tokens 9.5 -> 8.0), but for long K from 49 on (64 tokens of 2048 x 8192: 13.8, 14.0)
+            if x_lo is not None and (T <= 48 or (T <= 64 and K <= 4096)):
+                n_splits = 1
         out = torch.empty(n_splits, T, n_out, device=x.device, dtype=torch.float32)
         N.check(lib.ft_gemm_bf16(N.ptr(w), N.ptr(x), N.ptr(x_lo), N.ptr(out), 0, n_out, T, K, n_splits, 0, st),
                 "ft_gemm_bf16")
@@ -187,13 +191,14 @@ def attn_prefill(q: torch.Tensor, kv_layer: torch.Tensor, page_table: torch.Tens
     T, nq, d = q.shape
     nkv = kv_layer.shape[1]
     dev = q.device
-    # the kernel takes the list back to front: the tiles that see the most keys come last
-    tiles = []
+    tile_req, tile_q0 = [], []
     for r in range(len(req_slot)):
-        n, p0 = int(req_q_start[r + 1] - req_q_start[r]), int(req_pos0[r])
-        tiles += [(p0 + min(q0 + 64, n), r, q0) for q0 in range(0, n, 64)]
-    tiles.sort()
-    tile_req, tile_q0 = [t[1] for t in tiles], [t[2] for t in tiles]
+        for q0 in range(0, req_q_start[r + 1] - req_q_start[r], 64):
+            tile_req.append(r); tile_q0.append(q0)
+    if len(req_slot) > 1 and len(tile_req) * nkv > 128:      # more CTAs than run at once: the kernel takes the list back to front,
+        seen = [int(p) for p in req_pos0]                    # so the tiles that see the most keys come last
+        order = sorted(range(len(tile_req)), key=lambda i: seen[tile_req[i]] + tile_q0[i])
+        tile_req, tile_q0 = [tile_req[i] for i in order], [tile_q0[i] for i in order]
     # The lists go up in one copy that the host does not wait for (five waiting ones cost 60 us of GPU time between calls).  While a
     # stream is captured the copy is an ordinary one, which capture refuses: a replay would read memory that is no longer this call's.
     i32 = lambda v: torch.tensor(v, device="cpu", dtype=torch.int32).reshape(-1)
