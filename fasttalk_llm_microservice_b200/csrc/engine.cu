@@ -181,7 +181,24 @@ struct LayeredLayer {
     size_t canon_off[2] = {0, 0};      // post-norm layers: the tails [taps - 1][width] of the two input convolutions in a slot
     int lender_branch[2] = {0, 0};     // window attention over another layer's cache: which branch of that layer owns it
 };
+// A step of single tokens as a graph: its launches depend on the numbers of rows alone, everything else lies in the step's
+// uploaded block.
+struct StepGraph {
+    int T = 0, n_logit_rows = 0;
+    bool identity = false, refused = false;
+    cudaGraphExec_t exec = nullptr;    // null: seen once
+    long long launches = 0;
+    unsigned long long used = 0;       // of the model's counter: the least recent one gives way
+};
+constexpr size_t kStepGraphs = 16;
+
 struct Layered {
+    std::vector<StepGraph> graphs;     // at most kStepGraphs, used under the engine's step lock
+    unsigned long long graph_clock = 0;
+    ~Layered() {
+        for (StepGraph& g : graphs)
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+    }
     ft_layered_model m;
     std::vector<LayeredLayer> layers;
     float* lat_cache = nullptr;
@@ -412,8 +429,10 @@ static int run_gemm(Engine* e, const CUtensorMap& mw, const CUtensorMap* xmaps, 
 // `xn` planes always hold resid * gamma of the NEXT norm; `ssq` its per-row-tile sums of squares.
 static int forward_layered(Engine* e, const Batch& b);
 
+static int forward_layered_step(Engine* e, const Batch& b);
+
 static int forward(Engine* e, const Batch& b) {
-    if (e->lay) return forward_layered(e, b);
+    if (e->lay) return forward_layered_step(e, b);
     const ft_engine_config& c = e->cfg;
     StepMeta& m = e->meta;
     int* d = m.d;
@@ -1297,6 +1316,55 @@ static int forward_layered(Engine* e, const Batch& b) {
         }
         FT_TRY(dense(e, x, nullptr, nullptr, M.head, e->logits, b.n_logit_rows, M.vocab, W, M.logit_softcap));
     }
+    return 0;
+}
+
+// The same, single tokens out of a graph from the third step of a shape on: the second one records it.  A launch of a stream leaves 1 to 2.5 us between two short kernels, an
+// edge of a graph about half (Gedelorn, 46 launches a step of 16 sessions: 410 us, so 328).
+static int forward_layered_step(Engine* e, const Batch& b) {
+    Layered& L = *e->lay;
+    if (b.n_tiles > 0 || b.n_prefill_req > 0 || (L.trail_on && L.trail)) return forward_layered(e, b);
+    StepGraph* g = nullptr;
+    for (StepGraph& x : L.graphs)
+        if (x.T == b.T && x.n_logit_rows == b.n_logit_rows && x.identity == b.logit_rows_identity) g = &x;
+    if (!g) {
+        if (L.graphs.size() < kStepGraphs) {
+            g = &L.graphs.emplace_back();
+        } else {
+            g = &*std::min_element(L.graphs.begin(), L.graphs.end(), [](const StepGraph& x, const StepGraph& y) { return x.used < y.used; });
+            if (g->exec) cudaGraphExecDestroy(g->exec);
+            *g = StepGraph();
+        }
+        g->T = b.T;
+        g->n_logit_rows = b.n_logit_rows;
+        g->identity = b.logit_rows_identity;
+        g->used = ++L.graph_clock;
+        return forward_layered(e, b);
+    }
+    g->used = ++L.graph_clock;
+    if (g->refused) return forward_layered(e, b);
+    if (!g->exec) {
+        const long long before = e->st.kernel_launches;
+        cudaGraph_t graph = nullptr;
+        if (cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+            cudaGetLastError();
+            g->refused = true;
+            return forward_layered(e, b);
+        }
+        const int rc = forward_layered(e, b);
+        const cudaError_t end = cudaStreamEndCapture(e->stream, &graph);
+        g->launches = e->st.kernel_launches - before;
+        e->st.kernel_launches = before;
+        if (!rc && end == cudaSuccess && cudaGraphInstantiate(&g->exec, graph, 0) != cudaSuccess) g->exec = nullptr;
+        if (graph) cudaGraphDestroy(graph);
+        if (!g->exec) {                  // nothing of the step has run yet
+            cudaGetLastError();
+            g->refused = true;
+            return forward_layered(e, b);
+        }
+    }
+    FT_CHECK_CUDA(cudaGraphLaunch(g->exec, e->stream));
+    e->st.kernel_launches += g->launches;
     return 0;
 }
 

@@ -822,3 +822,41 @@ def test_rows_by_four_channels(heads, dim, vdim, rot):
             assert rel(np.concatenate(got[n]), oracle_logits(spec, w, seqs[n])) < TOL, n
     finally:
         eng.close()
+
+
+def test_steps_of_single_tokens_out_of_graphs():
+    """The same number of rows again and again (recorded at the second step, replayed from the third), other numbers in between, other sessions and other
+    wanted rows under the same number, portions beside, more shapes than are kept: all as the whole prompts give them."""
+    spec, w = make(MIXED, seed=29)
+    eng = engine(spec, w, max_batch=20, max_sessions=20, num_pages=24)
+    try:
+        names = [f"s{i}" for i in range(18)]
+        seqs = {n: tokens_of(spec, 60, 70 + i) for i, n in enumerate(names)}
+        ref = {n: oracle_logits(spec, w, t) for n, t in seqs.items()}
+        at = dict.fromkeys(names, 0)
+
+        def step(which, counts=None, wanted=None):
+            counts = counts or [1] * len(which)
+            entries = [(n, seqs[n][at[n]:at[n] + c], list(range(c)) if wanted is None or n in wanted else []) for n, c in zip(which, counts)]
+            out, o = eng.feed(entries), 0
+            for (n, t, rows) in entries:
+                for r in rows:
+                    assert rel(out[o], ref[n][at[n] + r]) < TOL, (n, at[n] + r)
+                    o += 1
+                at[n] += len(t)
+        step(names[:4], [3, 5, 2, 7])
+        step(names[4:], [2] * 14)
+        for k in range(5):
+            step(names[:4])
+        step(names[2:6])                       # the same shape, other sessions in other places
+        step(names[:4], wanted=names[1:2])     # fewer wanted rows
+        step(names[:4], wanted=names[2:3])
+        step(names[:4], wanted=names[3:4])
+        step(names[:5], [1, 1, 1, 1, 20])      # beside a portion
+        for n in range(1, 19):                 # shapes that push the first ones out
+            step(names[:n])
+            step(names[:n])
+        for k in range(3):
+            step(names[:4])
+    finally:
+        eng.close()
