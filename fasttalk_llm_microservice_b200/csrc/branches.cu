@@ -408,6 +408,179 @@ __global__ void __launch_bounds__(kWinWarps * 32) window_attn_kernel(WindowArgs 
     }
 }
 
+// The same for heads of up to 128 channels, up to four query heads per key head: one CTA per (token, key head), so that a key and a value row is read once for the
+// group and by neighbouring lanes.  A warp takes 16 keys at a time, all of their rows copied to its part of shared memory at once, the next ones' while it
+// works: scores by eight lanes a key, the softmax by a lane a key, the sums by four channels a lane.  Bound by the chain of a round of 128 keys: copies that
+// set out one step ahead, sums and maxima over lanes (3.8 us with four query heads, 2.2 with one).
+constexpr int kStepWarps = 8, kStepKeys = 16;
+template <int GRP>
+__global__ void __launch_bounds__(kStepWarps * 32) window_step_kernel(WindowArgs a) {
+    extern __shared__ __align__(16) float kv[];        // a warp's keys and values: [16][dim], [16][vdim]; at the end its sums [GRP][vdim]
+    __shared__ __align__(16) float ps[kStepWarps][kStepKeys][GRP];       // scores, then probabilities of a warp's keys
+    __shared__ float sm[kStepWarps][GRP], sl[kStepWarps][GRP];
+    const int t = blockIdx.x, g = blockIdx.y, grp = a.H / a.G, h0 = g * grp;
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & 7;
+    const int p = a.positions[t];
+    const int* pt = a.page_table + (size_t)a.seq_rows[t] * a.max_pages;
+    const int lo = a.window > 0 ? (a.chunked ? p - p % a.window : max(0, p - a.window + 1)) : 0;
+    const int nf = min(a.keep_first, lo);              // kept first positions that lie before the window
+    const int n = nf + p - lo + 1;                     // key idx < nf: position idx; otherwise position lo + idx - nf
+    const bool alias = a.v_in_key >= 0;
+    const size_t rowsz = (size_t)a.G * (alias ? a.dim : a.dim + a.vdim);
+    const float* k_at = a.cache + (size_t)g * a.dim;
+    const float* v_at = a.cache + (alias ? (size_t)g * a.dim + a.v_in_key : (size_t)a.G * a.dim + (size_t)g * a.vdim);
+    float* ks = kv + (size_t)wid * kStepKeys * (a.dim + a.vdim);
+    float* vs = ks + kStepKeys * a.dim;
+    constexpr int STEP = kStepWarps * kStepKeys;
+    // the place of key b0 + lane % 16 (behind the last one: of position p, whose weight is then 0)
+    auto place = [&](int b0) {
+        const int idx = b0 + (lane & 15), j = idx < n ? (idx < nf ? idx : lo + idx - nf) : p;
+        return pt[j >> 6] * 64 + (j & 63);
+    };
+    auto copy = [&](int row, const float* from, float* to, int width) {
+        const uint32_t dst = smem_u32(to) + lane * 16;
+#pragma unroll 4
+        for (int key = 0; key < kStepKeys; ++key) {
+            const int r = __shfl_sync(0xffffffffu, row, key);
+            if (4 * lane < width)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + key * width * 4), "l"(from + (size_t)r * rowsz + 4 * lane) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int b0 = wid * kStepKeys;
+    if (b0 < n) {
+        const int row = place(b0);
+        copy(row, k_at, ks, a.dim);
+        copy(row, v_at, vs, a.vdim);
+    }
+    float4 q[GRP][4];
+#pragma unroll
+    for (int h = 0; h < GRP; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int c = sub * 4 + 32 * i;
+            q[h][i] = h < grp && c < a.dim ? load_f4(a.q_out + ((size_t)t * a.H + h0 + h) * a.dim + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    float m[GRP], l[GRP];
+    float4 acc[GRP];
+#pragma unroll
+    for (int h = 0; h < GRP; ++h) {
+        m[h] = -INFINITY;
+        l[h] = 0.f;
+        acc[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const int c_out = lane * 4;
+    for (; b0 < n; b0 += STEP) {
+        const int idx = b0 + (lane & 15), j = idx < nf ? idx : lo + idx - nf;      // both halves of the warp hold the same key
+        const bool valid = idx < n, more = b0 + STEP < n;
+        const int row = more ? place(b0 + STEP) : 0;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");     // the keys (the values are the group behind them)
+        __syncwarp();
+#pragma unroll
+        for (int it = 0; it < kStepKeys / 4; ++it) {
+            const int key = 4 * it + (lane >> 3);
+            float s[GRP];
+#pragma unroll
+            for (int h = 0; h < GRP; ++h) s[h] = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int c = sub * 4 + 32 * i;
+                if (c >= a.dim) continue;
+                const float4 k = load_f4(ks + key * a.dim + c);
+#pragma unroll
+                for (int h = 0; h < GRP; ++h) s[h] = fmaf(q[h][i].x, k.x, fmaf(q[h][i].y, k.y, fmaf(q[h][i].z, k.z, fmaf(q[h][i].w, k.w, s[h]))));
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+                for (int h = 0; h < GRP; ++h) s[h] += __shfl_xor_sync(0xffffffffu, s[h], o);
+            if (sub == 0)
+#pragma unroll
+                for (int h = 0; h < GRP; ++h) ps[wid][key][h] = s[h];
+        }
+        __syncwarp();
+        if (more) copy(row, k_at, ks, a.dim);
+        float s[GRP], top[GRP], sum[GRP], corr[GRP];
+#pragma unroll
+        for (int h = 0; h < GRP; ++h) s[h] = ps[wid][lane & 15][h] * a.scale;
+        if (a.softcap > 0.f)
+#pragma unroll
+            for (int h = 0; h < GRP; ++h) s[h] = a.softcap * tanhf(s[h] / a.softcap);
+#pragma unroll
+        for (int h = 0; h < GRP; ++h) {
+            if (a.rel && valid && h < grp) s[h] += a.rel[(size_t)min(p - j, a.rel_n - 1) * a.H + h0 + h];
+            if (!valid || h >= grp) s[h] = -INFINITY;
+            top[h] = s[h];
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+            for (int h = 0; h < GRP; ++h) top[h] = fmaxf(top[h], __shfl_xor_sync(0xffffffffu, top[h], o));
+#pragma unroll
+        for (int h = 0; h < GRP; ++h) {
+            const float m_new = fmaxf(m[h], top[h]);
+            corr[h] = h < grp ? expf(m[h] - m_new) : 0.f;        // 0 on the first block (m = -inf)
+            sum[h] = valid && h < grp ? expf(s[h] - m_new) : 0.f;
+            m[h] = m_new;
+            ps[wid][lane & 15][h] = sum[h];
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+            for (int h = 0; h < GRP; ++h) sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], o);
+#pragma unroll
+        for (int h = 0; h < GRP; ++h) {
+            l[h] = l[h] * corr[h] + sum[h];
+            acc[h] = make_float4(acc[h].x * corr[h], acc[h].y * corr[h], acc[h].z * corr[h], acc[h].w * corr[h]);
+        }
+        if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        if (c_out < a.vdim)
+#pragma unroll
+            for (int u = 0; u < kStepKeys; ++u) {
+                const float4 v = load_f4(vs + u * a.vdim + c_out);
+#pragma unroll
+                for (int h = 0; h < GRP; ++h) {
+                    const float w = ps[wid][u][h];
+                    acc[h] = make_float4(fmaf(w, v.x, acc[h].x), fmaf(w, v.y, acc[h].y), fmaf(w, v.z, acc[h].z), fmaf(w, v.w, acc[h].w));
+                }
+            }
+        __syncwarp();
+        if (more) copy(row, v_at, vs, a.vdim);
+    }
+    if (lane == 0)
+#pragma unroll
+        for (int h = 0; h < GRP; ++h) {
+            sm[wid][h] = m[h];
+            sl[wid][h] = l[h];
+        }
+    if (c_out < a.vdim)
+#pragma unroll
+        for (int h = 0; h < GRP; ++h) store_f4(ks + h * a.vdim + c_out, acc[h]);        // (all copies have landed; four rows fit the warp's part)
+    __syncthreads();
+    for (int i = threadIdx.x; i < grp * a.vdim; i += kStepWarps * 32) {
+        const int h = i / a.vdim, c = i % a.vdim;
+        float mm = sm[0][h];
+#pragma unroll
+        for (int w = 1; w < kStepWarps; ++w) mm = fmaxf(mm, sm[w][h]);
+        float den = 0.f, num = 0.f;
+        if (a.sink) {
+            mm = fmaxf(mm, a.sink[h0 + h]);
+            den = expf(a.sink[h0 + h] - mm);
+        }
+#pragma unroll
+        for (int w = 0; w < kStepWarps; ++w) {
+            const float f = expf(sm[w][h] - mm);
+            den += sl[w][h] * f;
+            num += kv[(size_t)w * kStepKeys * (a.dim + a.vdim) + h * a.vdim + c] * f;
+        }
+        float r = num / den;
+        if (a.gate) r *= sigmoid_f(a.gate[(size_t)t * a.ldg + (h0 + h) * a.vdim + c]);
+        a.out[((size_t)t * a.H + h0 + h) * a.vdim + c] = r;
+    }
+}
+
 // Prompt portions: one CTA per (key head, run of QT consecutive tokens of one request), QT = 64 / (query heads per key head),
 // so that up to 64 query rows — the tokens of the run times the query heads of the group — share every key and value row
 // that is brought into shared memory.  Keys are taken 32 at a time from the first one the run's first token sees to the
@@ -662,6 +835,21 @@ int launch_window_attention(const WindowArgs& a, int T, int n_single, const Wind
     T = rows_each;
     const size_t smem = (size_t)(((a.dim + 3) & ~3) + 2 * kWinWarps + kWinWarps * a.vdim) * 4;
     const bool vec = (a.dim & 3) == 0 && (a.vdim & 3) == 0;      // every key row then starts on 16 bytes
+    const uintptr_t alias16 = (uintptr_t)a.cache | (uintptr_t)a.q_out | (a.v_in_key > 0 ? (uintptr_t)a.v_in_key * 4 : 0);
+    // One query head per key head, or long heads and some tokens (us, before -> window_step_kernel, behind 10 / 150 / 600 keys in a window of 512: 8 key heads
+    // of 64, one query head each, 4 tokens 4.5 / 9.2 / 16.9 -> 4.1 / 6.5 / 11.2; 4 key heads of 128 of four query heads, 16 tokens 6.5 / 15.2 / 31.9 -> 6.3 / 9.9 /
+    // 18.3, one token 5.3 / 11.4 / 22.5 -> 5.9 / 9.5 / 17.6; one key head of 64 of four 5.0 / 9.5 / 17.1 -> 5.6 / 8.7 / 16.4, of 32 of three 4.3 / 8.4 / 14.9 -> 5.5 / 8.8 / 16.4).
+    if (vec && a.dim <= 128 && a.vdim <= 128 && (grp == 1 || (grp <= 4 && a.dim + a.vdim >= 192 && T >= 4)) && a.G <= 65535 && (alias16 & 15) == 0) {
+        const size_t rows = (size_t)kStepWarps * kStepKeys * (a.dim + a.vdim) * 4;
+        auto step = [&](auto kernel) -> int {
+            if (rows > 40 * 1024) FT_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows));
+            kernel<<<dim3(T, a.G), kStepWarps * 32, rows, stream>>>(a);
+            return 0;
+        };
+        if (int r = grp <= 1 ? step(window_step_kernel<1>) : grp <= 2 ? step(window_step_kernel<2>) : step(window_step_kernel<4>)) return r;
+        FT_CHECK_CUDA(cudaGetLastError());
+        return 0;
+    }
     dim3 grid(T, a.H);
     const int vpl = (a.vdim + 31) / 32;
 #define FT_WIN(V)                                                                                   \

@@ -706,3 +706,20 @@ def test_rows_by_four_channels(heads, kv_heads, dim, vdim):
             assert rel(got[n], oracle_logits(spec, w, seqs[n])) < TOL, n
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 4, 64, 64), (3, 3, 20, 128), (8, 2, 128, 128), (6, 2, 96, 100), (4, 2, 128, 64)])
+@pytest.mark.parametrize("size,keep_first", [(5, 0), (127, 3), (128, 0), (400, 2)])
+def test_attention_of_single_tokens_by_group_and_window(heads, kv_heads, dim, vdim, size, keep_first):
+    """Five sessions' single tokens at once, behind histories around whole rounds of 16 and 128 keys, windows shorter and longer than they are."""
+    spec, w = make([layer(attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, size=size, keep_first=keep_first, scale=dim ** -0.5, rows=9)),
+                    layer(attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, size=size, keep_first=keep_first, scale=dim ** -0.5))], width=64, seed=size + dim)
+    eng = engine(spec, w, max_batch=5, max_sessions=5, max_batched_tokens=1024, num_pages=24, debug_logit_rows=1024)
+    try:
+        seqs = {n: tokens_of(spec, ln + 5, 60 + ln) for n, ln in (("a", 14), ("b", 30), ("c", 126), ("d", 255), ("e", 381))}
+        plan = [{n: len(t) - 5 for n, t in seqs.items()}] + [dict.fromkeys(seqs, 1)] * 5
+        got = feed_plan(eng, seqs, plan)
+        for n in seqs:
+            assert rel(got[n], oracle_logits(spec, w, seqs[n])) < TOL, n
+    finally:
+        eng.close()
