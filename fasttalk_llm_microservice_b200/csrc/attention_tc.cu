@@ -28,14 +28,15 @@
 // exponentials - store P - products - next scores, each a few hundred clocks of latency; 2100 clk per 64-key tile where the
 // exponentials alone take 1024 (the SFU's 16 / clk / SM) and the products 640 (d = 64) or 1280 (d = 128).  Without its
 // exponentials, or with a quarter of its products, it is no more than 15 % faster.  Tried and not kept (four prompts of 2k / 211
-// tokens over 5000, 1B / 8B shapes, us; this kernel 147 / 174): two threads per row 155 / 172 before the order below, one
+// tokens over 5000, 1B / 8B shapes, us; 147 / 174 at that point): two threads per row 155 / 172 before the order below, one
 // persistent CTA per SM with 128-key tiles at d = 64 and an issuing warp per half 163 / 175, the same with the halves'
 // exponentials in turns 153 / 183 and with two threads per row 172 / 176, pages prefetched into L2 165 / 190.
-// What helped: the longest tiles first over all KV heads (163 -> 149; the last round of CTAs was 15 % of the time), and products whose
-// operands the compiler knows (149 -> 147, 179 -> 174).
+// What helped: the longest tiles first over all KV heads (163 -> 149; the last round of CTAs was 15 % of the time), and keys shared by the halves where
+// the queries fill one only (17 tokens over 5000 keys 74 -> 36 at d = 64, 79 -> 51 at d = 128; six requests of 211 174 -> 145).
 #include "common.cuh"
 #include "ft_internal.h"
 
+#include <algorithm>
 #include <mutex>
 
 namespace ft {
@@ -45,6 +46,8 @@ constexpr int TC_ROWS = 128;                 // rows per half (UMMA M); 32 token
 constexpr int TC_TOK = 64;                   // query tokens per CTA
 constexpr int TC_SUB_BYTES = kKvTile * 128;  // one [64 tokens][64 dims] fp16 sub-slab = 8 KB; also 64 rows of a Q block
 constexpr int TC_QBLK_BYTES = TC_ROWS * 128; // one 128-row x 64-dim block of Q = 16 KB
+constexpr int TC_GRID_Y = 65535;             // query tiles along y
+constexpr int TC_SPLIT_TILES = 4;            // key tiles from which a tile of few queries shares them between the halves
 constexpr float TC_RESCALE_THRESHOLD = 8.f;  // log2 units
 
 template <int D>
@@ -53,7 +56,7 @@ struct TcCfg {
     static constexpr int TILE_BYTES = 2 * KH * TC_SUB_BYTES;             // K slab + V slab: 16 KB (d 64) / 32 KB (d 128)
     static constexpr int STAGES = D == 64 ? 6 : 4;
     static constexpr int Q_BYTES = 2 * KH * TC_QBLK_BYTES;               // both halves
-    static constexpr size_t SMEM = 1024 + Q_BYTES + (size_t)STAGES * TILE_BYTES + 512;
+    static constexpr size_t SMEM = 1024 + Q_BYTES + (size_t)STAGES * TILE_BYTES + 512;      // (d = 128: the largest that leaves 60 KB of L1; beyond it every launch takes 1 us longer)
     // TMEM columns: S, two buffers per half, 64 fp32 columns each; P (fp16, 32 columns) is written over the first half
     // of the S buffer it was computed from; O of the two halves behind them
     static constexpr int COL_S = 0, COL_O = 256, COLS = 512;
@@ -77,12 +80,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t* __restrict__ kv_layer,
                        const int* __restrict__ page_table, int max_pages, const int* __restrict__ req_q_start,
                        const int* __restrict__ req_slot, const int* __restrict__ req_pos0,
-                       const int* __restrict__ tile_req, const int* __restrict__ tile_q0,
+                       const int* __restrict__ tile_req, const int* __restrict__ tile_q0, int n_q_tiles,
                        __nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ out_lo, int nq, int nkv,
                        float scale_log2, int stagger_on) {
     using C = TcCfg<D>;
     constexpr int KH = C::KH;
     constexpr int R = 32 * G;                                 // real rows of a half (row = token * G + head)
+    // the LAST tiles of the list see the most keys where it is in that order: back to front, all KV heads of a tile side by side, or the
+    // longest CTAs would start last and the grid end in a long tail
+    const int tile_idx = n_q_tiles - 1 - (int)(blockIdx.z * TC_GRID_Y + blockIdx.y);
+    if (tile_idx < 0) return;                                // (the last layer of a grid of more than 65535 tiles)
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* q_s = smem;                                     // [2 halves][KH dim blocks][128 rows][128 B]
@@ -138,25 +145,25 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
     pdl_wait();
     pdl_launch_dependents();
 
-    // the LAST tiles of the list see the most keys where it is in that order: back to front, all KV heads of a tile side by side, or the
-    // longest CTAs would start last and the grid end in a long tail
-    const int tile_idx = (int)gridDim.x / nkv - 1 - (int)blockIdx.x / nkv;
     const int req = tile_req[tile_idx];
     const int q0 = tile_q0[tile_idx];
     const int q_row0 = req_q_start[req];
     const int q_len = req_q_start[req + 1] - q_row0;
     const int pos0 = req_pos0[req];
-    const int kvh = (int)blockIdx.x % nkv;
+    const int kvh = blockIdx.x;
     const int rows_here = q_len - q0 < TC_TOK ? q_len - q0 : TC_TOK;
     const int last_pos = pos0 + q0 + rows_here - 1;
     const int n_tiles = last_pos / kKvTile + 1;
+    // Up to 32 tokens would leave the second half idle: both take the same queries then, every other tile of keys each (tile j: half j & 1), and their
+    // results are put together at the end (about a microsecond).
+    const bool split = rows_here <= TC_TOK / 2 && n_tiles >= TC_SPLIT_TILES;
     const int* pt = page_table + (size_t)req_slot[req] * max_pages;
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
         if (lane == 0) {
-            mbar_expect_tx(q_full, 2 * KH * R * 128);
-            for (int h = 0; h < 2; ++h)
+            mbar_expect_tx(q_full, (split ? 1 : 2) * KH * R * 128);
+            for (int h = 0; h < (split ? 1 : 2); ++h)
                 for (int kh = 0; kh < KH; ++kh)
                     tma_tile_3d(q_s + (size_t)(h * KH + kh) * TC_QBLK_BYTES, &map_q, kh * 64, kvh * G, q_row0 + q0 + 32 * h, q_full);
         }
@@ -185,73 +192,77 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
             constexpr uint32_t idesc_pv = umma_idesc_f16(TC_ROWS, D, true);
             const uint64_t q_desc = umma_desc_k128(smem_u32(q_s)), k_desc = umma_desc_k128(smem_u32(kv_s));
             const uint64_t v_desc = umma_desc_mn128(smem_u32(kv_s) + KH * TC_SUB_BYTES);
-            // Half, buffer and stage are known to the compiler (the tile loop is unrolled over the ring): an operand put together at run time
-            // costs this thread ~150 clocks a product, four times what the tensor core takes for it.
-            auto issue_qk = [&](auto H, auto BUF, auto STAGE) {
-                constexpr int h = H.value, buf = BUF.value, stage = STAGE.value;
+            // An operand is a base of the half, buffer or stage, put together once, plus what the compiler knows: put together whole for every product it costs
+            // this thread twice what the tensor core takes for it (unrolled over the ring, with the bases known too, it is no faster)
+            auto issue_qk = [&](int h, int buf, int stage, int qh) {
+                const uint64_t a = q_desc + qh * ((KH * TC_QBLK_BYTES) >> 4), b = k_desc + stage * (C::TILE_BYTES >> 4);
+                const uint32_t d = tmem_base + C::COL_S + (2 * h + buf) * 64;
 #pragma unroll
                 for (int k = 0; k < 4 * KH; ++k)
-                    umma_bf16(tmem_base + C::COL_S + (2 * h + buf) * 64,
-                              q_desc + (((h * KH + (k >> 2)) * TC_QBLK_BYTES) >> 4) + 2 * (k & 3),
-                              k_desc + ((stage * C::TILE_BYTES + (k >> 2) * TC_SUB_BYTES) >> 4) + 2 * (k & 3), idesc_qk, k != 0);
+                    umma_bf16(d, a + (((k >> 2) * TC_QBLK_BYTES) >> 4) + 2 * (k & 3), b + (((k >> 2) * TC_SUB_BYTES) >> 4) + 2 * (k & 3), idesc_qk, k != 0);
                 umma_commit(&s_full[2 * h + buf]);
             };
-            auto issue_pv = [&](auto H, auto BUF, auto STAGE, auto FIRST) {
-                constexpr int h = H.value, buf = BUF.value, stage = STAGE.value;
-                const uint32_t p_tmem = tmem_base + C::COL_S + (2 * h + buf) * 64;        // 64 fp16 = 32 columns, over S
+            auto issue_pv = [&](int h, int buf, int stage, bool first) {
+                const uint32_t p = tmem_base + C::COL_S + (2 * h + buf) * 64, d = tmem_base + C::COL_O + h * D;        // 64 fp16 = 32 columns, over S
+                const uint64_t b = v_desc + stage * (C::TILE_BYTES >> 4);
 #pragma unroll
-                for (int k = 0; k < kKvTile / 16; ++k)
-                    umma_f16_ts(tmem_base + C::COL_O + h * D, p_tmem + 8 * k, v_desc + ((stage * C::TILE_BYTES + k * 2048) >> 4), idesc_pv,
-                                !FIRST.value || k != 0);
+                for (int k = 0; k < kKvTile / 16; ++k) umma_f16_ts(d, p + 8 * k, b + ((k * 2048) >> 4), idesc_pv, k != 0 || !first);
                 umma_commit(&pv_done[2 * h + buf]);
             };
+            auto keys_here = [&](int j) {
+                mbar_wait(&kv_full[j % C::STAGES], (j / C::STAGES) & 1);
+                tc_fence_after();
+            };
             mbar_wait(q_full, 0);
-            // scores run two tiles ahead of the softmax (two S buffers per half): tile j + 2 is issued as soon as the
-            // product of tile j — which reads its P out of the same buffer — has been issued in front of it
-            static_for<2>([&](auto J) {
-                if (J.value < n_tiles) {
-                    mbar_wait(&kv_full[J.value], 0);
-                    tc_fence_after();
-                    issue_qk(Int<0>{}, J, J);
-                    if (!stagger_on) issue_qk(Int<1>{}, J, J);
-                }
-            });
-            if (stagger_on) {        // half 1 starts when half 0 is about to enter its SFU-bound phase, so that the two halves'
-                                     // exponentials do not fall on the SFU at the same time (profiles/r02_attn_prefill_tc.md)
-                mbar_wait(stagger, 0);
-                static_for<2>([&](auto J) {
-                    if (J.value < n_tiles) issue_qk(Int<1>{}, J, J);
-                });
-            }
-            uint32_t p_phase = 0, kv_phase = 0;      // p_full: every two tiles; kv_full: every round of the ring
-            for (int j0 = 0; j0 < n_tiles; j0 += C::STAGES) {
-                static_for<C::STAGES>([&](auto U) {
-                    constexpr int u = U.value, buf = u & 1, next = (u + 2) % C::STAGES;
-                    const int j = j0 + u;
-                    if (j < n_tiles) {
-                        const bool more = j + 2 < n_tiles;
-                        static_for<2>([&](auto H) {
-                            constexpr int h = H.value;
-                            // Every hand-over has one barrier PER BUFFER (tile parity): the softmax of one half may run up to two
-                            // tiles ahead of what this thread has observed (it is busy with the other half), and a single barrier
-                            // completing two phases unobserved would look "not yet complete" again — a deadlock.
-                            mbar_wait(&p_full[2 * h + buf], p_phase);    // P_h(j) written, S_h(j) consumed, O_h rescaled if needed
-                            tc_fence_after();
-                            if (u == 0 && j0 == 0) issue_pv(H, Int<buf>{}, U, Int<1>{});
-                            else issue_pv(H, Int<buf>{}, U, Int<0>{});
-                            if (h == 1) umma_commit(&kv_empty[u]);       // every product that reads this stage has been issued
-                            if (more) {
-                                if (h == 0) {
-                                    mbar_wait(&kv_full[next], u + 2 < C::STAGES ? kv_phase : kv_phase ^ 1);
-                                    tc_fence_after();
-                                }
-                                issue_qk(H, Int<buf>{}, Int<next>{});    // in order behind the product that read P out of this buffer
-                            }
-                        });
-                        if (buf == 1) p_phase ^= 1;
+            if (split) {
+                // Scores run AHEAD tiles of the list ahead: three where the ring is deep enough that their keys set out three tiles ago, else two (the half's next
+                // tile).  The product that read P out of their buffer was issued one or two tiles ago.  (Tile j is its half's (j / 2)-th and the
+                // (j / 4)-th in its buffer.)
+                constexpr int AHEAD = C::STAGES >= 6 ? 3 : 2;
+#pragma unroll 1
+                for (int j = -AHEAD; j < n_tiles; ++j) {
+                    if (j >= 0) {
+                        mbar_wait(&p_full[2 * (j & 1) + (j >> 1 & 1)], (j >> 2) & 1);
+                        tc_fence_after();
+                        issue_pv(j & 1, j >> 1 & 1, j % C::STAGES, j < 2);
+                        umma_commit(&kv_empty[j % C::STAGES]);
                     }
-                });
-                kv_phase ^= 1;
+                    const int a = j + AHEAD;
+                    if (a < n_tiles) {
+                        keys_here(a);
+                        issue_qk(a & 1, a >> 1 & 1, a % C::STAGES, 0);
+                    }
+                }
+            } else {
+                // scores run two tiles ahead of the softmax (two S buffers per half): tile j + 2 is issued as soon as the
+                // product of tile j — which reads its P out of the same buffer — has been issued in front of it
+                for (int j = 0; j < 2 && j < n_tiles; ++j) {
+                    keys_here(j);
+                    issue_qk(0, j, j, 0);
+                    if (!stagger_on) issue_qk(1, j, j, 1);
+                }
+                if (stagger_on) {        // half 1 starts when half 0 is about to enter its SFU-bound phase, so that the two halves'
+                                         // exponentials do not fall on the SFU at the same time (profiles/r02_attn_prefill_tc.md)
+                    mbar_wait(stagger, 0);
+                    for (int j = 0; j < 2 && j < n_tiles; ++j) issue_qk(1, j, j, 1);
+                }
+#pragma unroll 1
+                for (int j = 0; j < n_tiles; ++j) {
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h) {
+                        // Every hand-over has one barrier PER BUFFER (tile parity): the softmax of one half may run up to two
+                        // tiles ahead of what this thread has observed (it is busy with the other half), and a single barrier
+                        // completing two phases unobserved would look "not yet complete" again — a deadlock.
+                        mbar_wait(&p_full[2 * h + (j & 1)], (j >> 1) & 1);   // P_h(j) written, S_h(j) consumed, O_h rescaled if needed
+                        tc_fence_after();
+                        issue_pv(h, j & 1, j % C::STAGES, j == 0);
+                        if (h == 1) umma_commit(&kv_empty[j % C::STAGES]);   // every product that reads this stage has been issued
+                        if (j + 2 < n_tiles) {
+                            if (h == 0) keys_here(j + 2);
+                            issue_qk(h, j & 1, (j + 2) % C::STAGES, h);      // in order behind the product that read P out of this buffer
+                        }
+                    }
+                }
             }
         }
     } else {
@@ -259,17 +270,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
         const int h = (warp - 2) >> 2;
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;                     // TMEM lane == row of the half
-        const int tok = h * 32 + row / G;                        // query token within the CTA's 64
+        const int tok = (split ? 0 : h * 32) + row / G;          // query token within the CTA's 64
         const int head = kvh * G + row % G;
         const int pos = pos0 + q0 + tok;                         // absolute position of this row's query
         const bool valid = row < R && q0 + tok < q_len;
         const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
         const uint32_t s_taddr0 = lane_base + C::COL_S + 2 * h * 64, o_taddr = lane_base + C::COL_O + h * D;
         float m_ref = -INFINITY, l_run = 0.f;                    // m_ref in scaled (log2) units
-        for (int j = 0; j < n_tiles; ++j) {
-            mbar_wait(&s_full[2 * h + (j & 1)], (j >> 1) & 1);
+        const int mine = split ? (n_tiles - h + 1) / 2 : n_tiles;
+        for (int i = 0; i < mine; ++i) {
+            const int j = split ? h + 2 * i : i;                 // tile of the list, the half's i-th
+            mbar_wait(&s_full[2 * h + (i & 1)], (i >> 1) & 1);
             tc_fence_after();
-            const uint32_t s_taddr = s_taddr0 + (j & 1) * 64;
+            const uint32_t s_taddr = s_taddr0 + (i & 1) * 64;
             uint32_t sr[64];
 #pragma unroll
             for (int c = 0; c < 4; ++c) tmem_ld16_nowait(s_taddr + 16 * c, sr + 16 * c);
@@ -288,18 +301,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
                 for (int c = 0; c < 64; ++c) t4[c & 3] = fmaxf(t4[c & 3], __uint_as_float(sr[c]));
             }
             const float tmax = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3]));
-            if (stagger_on && j == 0 && h == 0) {
+            if (stagger_on && i == 0 && h == 0) {
                 __syncwarp();
                 if (lane == 0) mbar_arrive(stagger);
             }
             const float m_new = fmaxf(m_ref, tmax * scale_log2);
-            const bool grow = m_new > m_ref + TC_RESCALE_THRESHOLD;
-            if (j == 0) {
+            // rows without a query of this request say nothing: a row's rounding depends on its own request alone
+            const bool grow = valid && m_new > m_ref + TC_RESCALE_THRESHOLD;
+            if (i == 0) {
                 m_ref = m_new;
             } else if (__any_sync(0xffffffffu, grow)) {          // tcgen05.ld / st are warp-wide: rescale all 32 rows
-                mbar_wait(&pv_done[2 * h + ((j - 1) & 1)], ((j - 1) >> 1) & 1);     // O_h complete up to tile j - 1
+                mbar_wait(&pv_done[2 * h + ((i - 1) & 1)], ((i - 1) >> 1) & 1);     // O_h complete up to the half's tile i - 1
                 tc_fence_after();
-                const float alpha = exp2f(m_ref - m_new);        // rows that did not grow: m_new >= m_ref, alpha <= 1
+                const float alpha = m_new == -INFINITY ? 1.f : exp2f(m_ref - m_new);        // rows that did not grow: m_new >= m_ref, alpha <= 1
                 l_run *= alpha;
                 m_ref = m_new;
 #pragma unroll
@@ -333,33 +347,70 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
             l_run += (ps[0] + ps[1]) + (ps[2] + ps[3]);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&p_full[2 * h + (j & 1)]);
+            if (lane == 0) mbar_arrive(&p_full[2 * h + (i & 1)]);
         }
         // ---- epilogue: O / l -> bf16 hi + lo planes
-        mbar_wait(&pv_done[2 * h + ((n_tiles - 1) & 1)], ((n_tiles - 1) >> 1) & 1);
+        mbar_wait(&pv_done[2 * h + ((mine - 1) & 1)], ((mine - 1) >> 1) & 1);
         tc_fence_after();
-        const float inv = 1.f / l_run;
-        const size_t off = ((size_t)(q_row0 + q0 + tok) * nq + head) * D;
-#pragma unroll
-        for (int c = 0; c < D / 16; ++c) {
-            uint32_t orr[16];
-            tmem_ld16_nowait(o_taddr + 16 * c, orr);
+        float inv = 1.f / l_run, inv_other = 0.f;
+        if (split) {                                             // each half forms half of the channels' results
+            // maximum and sum by way of the scores' columns, which have all been read
+            uint32_t ml[16] = {__float_as_uint(m_ref), __float_as_uint(l_run)};
+            tmem_st16(s_taddr0, ml);
+            tmem_st_wait();
+            tc_fence_before();
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            tc_fence_after();
+            tmem_ld16_nowait(lane_base + C::COL_S + 2 * (1 - h) * 64, ml);
             tmem_ld_wait();
-            if (valid) {
-                uint32_t hi[8], lo[8];
+            const float2 o = make_float2(__uint_as_float(ml[0]), __uint_as_float(ml[1]));
+            const float m = fmaxf(m_ref, o.x), w = m_ref == -INFINITY ? 0.f : exp2f(m_ref - m), wo = o.x == -INFINITY ? 0.f : exp2f(o.x - m);
+            const float r = 1.f / (h == 0 ? l_run * w + o.y * wo : o.y * wo + l_run * w);
+            inv = w * r;
+            inv_other = wo * r;
+        }
+        const size_t off = ((size_t)(q_row0 + q0 + tok) * nq + head) * D;
+        auto put = [&](int c, const uint32_t* v) {               // 16 channels of the row
+            uint32_t hi[8], lo[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const float x = __uint_as_float(orr[2 * k]) * inv, y = __uint_as_float(orr[2 * k + 1]) * inv;
-                    hi[k] = pack_bf16(x, y);
-                    lo[k] = pack_bf16(x - bf16_lo(hi[k]), y - bf16_hi(hi[k]));
+            for (int k = 0; k < 8; ++k) {
+                const float x = __uint_as_float(v[2 * k]), y = __uint_as_float(v[2 * k + 1]);
+                hi[k] = pack_bf16(x, y);
+                lo[k] = pack_bf16(x - bf16_lo(hi[k]), y - bf16_hi(hi[k]));
+            }
+            uint4* dst = reinterpret_cast<uint4*>(out + off + 16 * c);
+            dst[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            dst[1] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+            if (out_lo) {
+                uint4* dl = reinterpret_cast<uint4*>(out_lo + off + 16 * c);
+                dl[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                dl[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+            }
+        };
+        if (!split) {
+#pragma unroll
+            for (int c = 0; c < D / 16; ++c) {
+                uint32_t orr[16];
+                tmem_ld16_nowait(o_taddr + 16 * c, orr);
+                tmem_ld_wait();
+                if (valid) {
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) orr[k] = __float_as_uint(__uint_as_float(orr[k]) * inv);
+                    put(c, orr);
                 }
-                uint4* dst = reinterpret_cast<uint4*>(out + off + 16 * c);
-                dst[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                dst[1] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
-                if (out_lo) {
-                    uint4* dl = reinterpret_cast<uint4*>(out_lo + off + 16 * c);
-                    dl[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-                    dl[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+            }
+        } else {
+#pragma unroll 1
+            for (int i = 0; i < D / 32; ++i) {
+                const int c = D / 32 * h + i;
+                uint32_t orr[16], x[16];
+                tmem_ld16_nowait(o_taddr + 16 * c, orr);
+                tmem_ld16_nowait(lane_base + C::COL_O + (1 - h) * D + 16 * c, x);
+                tmem_ld_wait();
+                if (valid) {
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) orr[k] = __float_as_uint(fmaf(__uint_as_float(x[k]), inv_other, __uint_as_float(orr[k]) * inv));
+                    put(c, orr);
                 }
             }
         }
@@ -397,8 +448,7 @@ static int launch_tc(const CUtensorMap& map, const void* kv_layer, const int* pa
     const float scale_log2 = 1.4426950408889634f / sqrtf((float)D);
     static const int stagger_on = getenv("FT_TC_STAGGER") ? atoi(getenv("FT_TC_STAGGER")) : 1;       // A/B switch; measured: 4–6 % at d = 64
     cudaLaunchConfig_t cfg = {};
-    FT_REQUIRE((long long)n_tiles * nkv < (1ll << 31), "attn_prefill: %d tiles of %d KV heads", n_tiles, nkv);
-    cfg.gridDim = dim3(n_tiles * nkv);
+    cfg.gridDim = dim3(nkv, std::min(n_tiles, TC_GRID_Y), (n_tiles + TC_GRID_Y - 1) / TC_GRID_Y);
     cfg.blockDim = dim3(TC_THREADS);
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = stream;
@@ -408,7 +458,7 @@ static int launch_tc(const CUtensorMap& map, const void* kv_layer, const int* pa
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
     FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_prefill_tc_kernel<D, G>, map, (const uint8_t*)kv_layer, page_table, max_pages,
-                                     req_q_start, req_slot, req_pos0, tile_req, tile_q0, (__nv_bfloat16*)out,
+                                     req_q_start, req_slot, req_pos0, tile_req, tile_q0, n_tiles, (__nv_bfloat16*)out,
                                      (__nv_bfloat16*)out_lo, nq, nkv, scale_log2, stagger_on));
     return 0;
 }

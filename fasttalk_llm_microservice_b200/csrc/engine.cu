@@ -1446,11 +1446,11 @@ static long long fill_batch(Engine* e, const std::vector<Portion>& dec, const st
         }
     }
     if (!e->lay && b.n_prefill_req > 1) {
-        // the attention kernel takes the list back to front: the tiles that see the most keys come last
+        // the attention kernel takes the list back to front: the tiles that take longest come last (up to 32 tokens: half as long)
         std::vector<std::array<int, 3>> order(tiles);
         for (int i = 0; i < tiles; ++i) {
             const int j = h[m.o_treq + i], q0 = h[m.o_tq0 + i];
-            order[i] = {pre[j].pos0 + std::min(q0 + 64, pre[j].n), j, q0};
+            order[i] = {(pre[j].pos0 + q0 + 64) * (pre[j].n - q0 > 32 ? 2 : 1), j, q0};
         }
         std::sort(order.begin(), order.end());
         for (int i = 0; i < tiles; ++i) {

@@ -196,8 +196,9 @@ def attn_prefill(q: torch.Tensor, kv_layer: torch.Tensor, page_table: torch.Tens
         for q0 in range(0, req_q_start[r + 1] - req_q_start[r], 64):
             tile_req.append(r); tile_q0.append(q0)
     if len(req_slot) > 1 and len(tile_req) * nkv > 128:      # more CTAs than run at once: the kernel takes the list back to front,
-        seen = [int(p) for p in req_pos0]                    # so the tiles that see the most keys come last
-        order = sorted(range(len(tile_req)), key=lambda i: seen[tile_req[i]] + tile_q0[i])
+        seen = [int(p) for p in req_pos0]                    # so the tiles that take longest come last (up to 32 tokens: half as long)
+        ends = [int(req_q_start[r + 1] - req_q_start[r]) for r in range(len(req_slot))]
+        order = sorted(range(len(tile_req)), key=lambda i: (seen[tile_req[i]] + tile_q0[i] + 64) * (1 + (ends[tile_req[i]] - tile_q0[i] > 32)))
         tile_req, tile_q0 = [tile_req[i] for i in order], [tile_q0[i] for i in order]
     # The lists go up in one copy that the host does not wait for (five waiting ones cost 60 us of GPU time between calls).  While a
     # stream is captured the copy is an ordinary one, which capture refuses: a replay would read memory that is no longer this call's.

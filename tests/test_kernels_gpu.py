@@ -513,6 +513,23 @@ def test_attn_prefill_few_tiles_over_many_keys(K, nq, nkv, d, reqs):
         assert rel_err(tc[q_start[r]:q_start[r + 1]], ref) < 2e-3, r
 
 
+@pytest.mark.parametrize("nq,nkv,d", [(4, 1, 64), (6, 2, 64), (8, 2, 128), (3, 1, 128)])
+@pytest.mark.parametrize("tiles", [1, 2, 3, 4, 5, 6, 7, 8, 13])
+@pytest.mark.parametrize("n", [1, 31, 32, 33])
+def test_attn_prefill_tiles_of_few_queries_by_keys(K, nq, nkv, d, tiles, n):
+    """Up to 32 queries of a tile share its keys between the halves from four key tiles on: every count of tiles around that and around whole rounds of the rings,
+    one behind another request's 64 queries."""
+    g = torch.Generator(device=DEV).manual_seed(nq * 17 + d + tiles)
+    reqs = [(0, 64), (max(0, tiles * 64 - n - 3), min(n, tiles * 64 - 3))]
+    kv, pt, ks, vs = build_paged_kv(K, [p + m for p, m in reqs], nkv, d, g)
+    q_start = [0, 64, 64 + reqs[1][1]]
+    q = (torch.randn(q_start[-1], nq, d, device=DEV, generator=g) * 1.5).half()
+    got = hilo(*K.attn_prefill(q, kv, pt, q_start, [0, 1], [p for p, _ in reqs]))
+    for r, (p0, _) in enumerate(reqs):
+        ref = O.attention(q[q_start[r]:q_start[r + 1]].float(), ks[r].float(), vs[r].float(), p0)
+        assert rel_err(got[q_start[r]:q_start[r + 1]], ref) < 2e-3, r
+
+
 @pytest.mark.parametrize("nq,nkv,d", [(32, 8, 64), (32, 8, 128), (6, 2, 128)])
 @pytest.mark.parametrize("p0,n", [(1472, 21), (5 * 64, 64), (0, 300)])
 def test_attn_prefill_rows_depend_on_nothing_else(K, nq, nkv, d, p0, n):
