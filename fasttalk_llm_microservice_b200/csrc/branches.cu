@@ -1561,23 +1561,40 @@ __global__ void __launch_bounds__(256) readout_rows_kernel(ReadoutArgs a) {
     __shared__ float red[33];
     const int t = blockIdx.x / a.norm_groups, g = blockIdx.x % a.norm_groups;
     const int n = a.heads * a.vdim / a.norm_groups, c0 = g * n;
-    float4 v[NV];
+    // Everything that a long row needs is asked for before the first number is used (4096 columns, 16 rows 8.9 us, so 6.7; 2313 rows 38, so 33); short rows want
+    // the registers for more CTAs instead (2313 rows of 2048: 12.5 us, 14.1 that way).
+    constexpr bool FIRST = NV > 2;
+    float4 v[NV], x[FIRST ? NV : 1], z[FIRST ? NV : 1];
+    float k[FIRST ? NV : 1];
     float ss = 0.f;
-    auto gate4 = [&](int c) { return *reinterpret_cast<const float4*>(a.gate + (size_t)t * a.ldg + c); };
+    auto gate4 = [&](int c) { return load_f4(a.gate + (size_t)t * a.ldg + c); };
+    if (FIRST)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int c = 4 * ((int)threadIdx.x + (int)blockDim.x * i);
+            if (c < n) {
+                v[i] = load_f4(a.o + (size_t)t * a.ldo + c0 + c);
+                if (a.gate_kind) z[FIRST ? i : 0] = gate4(c0 + c);
+                if (a.skip) {
+                    x[FIRST ? i : 0] = load_f4(a.x + (size_t)t * a.ldx + c0 + c);
+                    k[FIRST ? i : 0] = a.skip[(c0 + c) / a.vdim];
+                }
+            }
+        }
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const int c = 4 * ((int)threadIdx.x + (int)blockDim.x * i);
         if (c >= n) continue;
-        float4 o = *reinterpret_cast<const float4*>(a.o + (size_t)t * a.ldo + c0 + c);
+        float4 o = FIRST ? v[i] : load_f4(a.o + (size_t)t * a.ldo + c0 + c);
         o.x *= a.q_scale; o.y *= a.q_scale; o.z *= a.q_scale; o.w *= a.q_scale;
         if (a.skip) {
-            const float k = a.skip[(c0 + c) / a.vdim];
-            const float4 x = *reinterpret_cast<const float4*>(a.x + (size_t)t * a.ldx + c0 + c);
-            o.x = fmaf(k, x.x, o.x); o.y = fmaf(k, x.y, o.y); o.z = fmaf(k, x.z, o.z); o.w = fmaf(k, x.w, o.w);
+            const float f = FIRST ? k[FIRST ? i : 0] : a.skip[(c0 + c) / a.vdim];
+            const float4 u = FIRST ? x[FIRST ? i : 0] : load_f4(a.x + (size_t)t * a.ldx + c0 + c);
+            o.x = fmaf(f, u.x, o.x); o.y = fmaf(f, u.y, o.y); o.z = fmaf(f, u.z, o.z); o.w = fmaf(f, u.w, o.w);
         }
         if (a.gate_kind == 1) {
-            const float4 z = gate4(c0 + c);
-            o.x *= silu_f(z.x); o.y *= silu_f(z.y); o.z *= silu_f(z.z); o.w *= silu_f(z.w);
+            const float4 g = FIRST ? z[FIRST ? i : 0] : gate4(c0 + c);
+            o.x *= silu_f(g.x); o.y *= silu_f(g.y); o.z *= silu_f(g.z); o.w *= silu_f(g.w);
         }
         v[i] = o;
         ss += o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w;
@@ -1594,9 +1611,9 @@ __global__ void __launch_bounds__(256) readout_rows_kernel(ReadoutArgs a) {
             o.x *= w.x; o.y *= w.y; o.z *= w.z; o.w *= w.w;
         }
         if (a.gate_kind >= 2) {
-            const float4 z = gate4(c0 + c);
-            if (a.gate_kind == 2) { o.x *= sigmoid_f(z.x); o.y *= sigmoid_f(z.y); o.z *= sigmoid_f(z.z); o.w *= sigmoid_f(z.w); }
-            else { o.x *= silu_f(z.x); o.y *= silu_f(z.y); o.z *= silu_f(z.z); o.w *= silu_f(z.w); }
+            const float4 g = FIRST ? z[FIRST ? i : 0] : gate4(c0 + c);
+            if (a.gate_kind == 2) { o.x *= sigmoid_f(g.x); o.y *= sigmoid_f(g.y); o.z *= sigmoid_f(g.z); o.w *= sigmoid_f(g.w); }
+            else { o.x *= silu_f(g.x); o.y *= silu_f(g.y); o.z *= silu_f(g.z); o.w *= silu_f(g.w); }
         }
         const size_t at = (size_t)t * a.heads * a.vdim + c0 + c;
         if (a.out_hi) {                               // as the bf16 planes that the output projection reads
