@@ -46,6 +46,7 @@ __device__ __forceinline__ float cta_sum(float v, float* red) {      // red: >= 
 // x[t][c0 .. c0 + n) <- silu(x) in place, rows of stride ld; V columns (16 bytes or one) per thread
 template <int V>
 __global__ void __launch_bounds__(256) silu_cols_kernel(float* __restrict__ x, int ld, int c0, int n) {
+    pdl_wait();
     const int c = (blockIdx.y * 256 + threadIdx.x) * V;
     if (c >= n) return;
     float* r = x + (size_t)blockIdx.x * ld + c0 + c;
@@ -61,12 +62,13 @@ int launch_silu_cols(float* x, int ld, int c0, int n, int T, cudaStream_t stream
     const bool v4 = ld % 4 == 0 && c0 % 4 == 0 && n % 4 == 0 && ((uintptr_t)x & 15) == 0;
     const int per = 256 * (v4 ? 4 : 1);
     const dim3 grid(T, (n + per - 1) / per);
-    if (v4) silu_cols_kernel<4><<<grid, 256, 0, stream>>>(x, ld, c0, n);
-    else silu_cols_kernel<1><<<grid, 256, 0, stream>>>(x, ld, c0, n);
+    if (v4) launch_after(silu_cols_kernel<4>, grid, 256, 0, stream, x, ld, c0, n);
+    else launch_after(silu_cols_kernel<1>, grid, 256, 0, stream, x, ld, c0, n);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 __global__ void turn_qk_kernel(TurnArgs a) {
+    pdl_wait();
     const int t = blockIdx.x, half = a.rot_dims >> 1, per = half + a.dim - a.rot_dims;      // pairs, then single coordinates of a head
     const float pos = (float)a.positions[t];
     for (int i = threadIdx.x; i < (a.heads + a.kv_heads) * per; i += blockDim.x) {
@@ -88,18 +90,19 @@ __global__ void turn_qk_kernel(TurnArgs a) {
 int launch_turn_qk(const TurnArgs& a, int T, cudaStream_t stream) {
     FT_REQUIRE(a.rot_dims >= 0 && a.rot_dims <= a.dim && (a.rot_dims & 1) == 0 && (a.rot_dims == 0 || a.rot_freq),
                "rotation: bad sizes (dim %d, rotated %d)", a.dim, a.rot_dims);
-    turn_qk_kernel<<<T, 256, 0, stream>>>(a);
+    launch_after(turn_qk_kernel, T, 256, 0, stream, a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 // ab[t][h] = (decay[h], 1)
 __global__ void const_decay_kernel(const float* __restrict__ decay, float* __restrict__ ab, int heads, int n) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) { ab[2 * (size_t)i] = decay[i % heads]; ab[2 * (size_t)i + 1] = 1.f; }
 }
 int launch_const_decay(const float* decay, float* ab, int heads, int T, cudaStream_t stream) {
     const int n = T * heads;
-    const_decay_kernel<<<(n + 255) / 256, 256, 0, stream>>>(decay, ab, heads, n);
+    launch_after(const_decay_kernel, (n + 255) / 256, 256, 0, stream, decay, ab, heads, n);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -130,6 +133,7 @@ __device__ __forceinline__ float rotated(const float* __restrict__ src, const fl
 // CTA (token x, part y): the heads whose number is y modulo the parts — a step of few tokens is cut by heads so that more than a CTA
 // per token runs (one root mean square over all heads, qk_norm 2, keeps to one part).
 __global__ void __launch_bounds__(128) window_write_kernel(WindowArgs a) {
+    pdl_wait();
     extern __shared__ float inv[];             // qk_norm: 1 / rms of every query head, then of every key head; then the pairs' trig
     const int t = blockIdx.x, part = blockIdx.y, parts = gridDim.y;
     const float* pr = a.proj + (size_t)t * a.ldp;
@@ -209,6 +213,7 @@ __global__ void __launch_bounds__(128) window_write_kernel(WindowArgs a) {
 // a lane, which stay in registers between the norm and the rotation (one channel per thread, two passes: 36 us for 2313 tokens of 16 + 4 + 4
 // heads of 128; now 15.6 us, the bytes take 9).  The heads of a token are dealt out to the groups of `gridDim.y` CTAs.
 __global__ void __launch_bounds__(128) window_write_rows_kernel(WindowArgs a, int lanes) {
+    pdl_wait();
     extern __shared__ float trig[];
     const int t = blockIdx.x, p = a.positions[t], half = a.rot_dims >> 1;
     const float* pr = a.proj + (size_t)t * a.ldp;
@@ -308,6 +313,7 @@ __device__ __forceinline__ void cp_async16_zfill(float* dst_smem, const float* s
 constexpr int kWinWarps = 4;
 template <int VPL, bool VEC>
 __global__ void __launch_bounds__(kWinWarps * 32) window_attn_kernel(WindowArgs a) {
+    pdl_wait();
     extern __shared__ float sh[];
     float* sq = sh;                                    // [dim]
     float* sm = sq + ((a.dim + 3) & ~3);               // [warps] running maxima
@@ -415,6 +421,7 @@ __global__ void __launch_bounds__(kWinWarps * 32) window_attn_kernel(WindowArgs 
 constexpr int kStepWarps = 8, kStepKeys = 16;
 template <int GRP>
 __global__ void __launch_bounds__(kStepWarps * 32) window_step_kernel(WindowArgs a) {
+    pdl_wait();
     extern __shared__ __align__(16) float kv[];        // a warp's keys and values: [16][dim], [16][vdim]; at the end its sums [GRP][vdim]
     __shared__ __align__(16) float ps[kStepWarps][kStepKeys][GRP];       // scores, then probabilities of a warp's keys
     __shared__ float sm[kStepWarps][GRP], sl[kStepWarps][GRP];
@@ -590,6 +597,7 @@ __global__ void __launch_bounds__(kStepWarps * 32) window_step_kernel(WindowArgs
 constexpr int WT_ROWS = 64, WT_KEYS = 32, WT_THREADS = 256;
 template <int VK>
 __global__ void __launch_bounds__(WT_THREADS) window_tile_kernel(WindowArgs a, WindowTiles tm, int QT, int subs) {
+    pdl_wait();
     extern __shared__ __align__(16) float wsh[];
     const bool alias = a.v_in_key >= 0;       // the values are columns v_in_key.. of the key rows: no value tile of their own
     const int ldq = a.dim + 4, ldv = alias ? ldq : a.vdim, ldp = WT_KEYS + 1;
@@ -806,8 +814,8 @@ int launch_window_attention(const WindowArgs& a, int T, int n_single, const Wind
     // parts per token: as many as give about two CTAs per SM
     int parts = 1;
     while (a.qk_norm != 2 && parts < a.H && T * parts < 256 && parts < 16) parts *= 2;
-    if (rows16) window_write_rows_kernel<<<dim3(T, parts), 128, (size_t)a.rot_dims * 4, stream>>>(a, lanes);
-    else window_write_kernel<<<dim3(T, parts), 128, (size_t)((a.qk_norm ? a.H + a.G : 0) + a.rot_dims) * 4, stream>>>(a);
+    if (rows16) launch_after(window_write_rows_kernel, dim3(T, parts), 128, (size_t)a.rot_dims * 4, stream, a, lanes);
+    else launch_after(window_write_kernel, dim3(T, parts), 128, (size_t)((a.qk_norm ? a.H + a.G : 0) + a.rot_dims) * 4, stream, a);
     FT_CHECK_CUDA(cudaGetLastError());
     const int grp = a.H / a.G;
     FT_REQUIRE(a.v_in_key < 0 || (a.v_in_key + a.vdim <= a.dim && a.v_role == 0), "window attention: values inside the keys exceed them");
@@ -824,10 +832,10 @@ int launch_window_attention(const WindowArgs& a, int T, int n_single, const Wind
         dim3 grid(tm.n_tiles * subs, a.G);
         if (a.vdim <= 128) {
             FT_CHECK_CUDA(cudaFuncSetAttribute(window_tile_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
-            window_tile_kernel<1><<<grid, WT_THREADS, tsm, stream>>>(a, tm, QT, subs);
+            launch_after(window_tile_kernel<1>, grid, WT_THREADS, tsm, stream, a, tm, QT, subs);
         } else {
             FT_CHECK_CUDA(cudaFuncSetAttribute(window_tile_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
-            window_tile_kernel<2><<<grid, WT_THREADS, tsm, stream>>>(a, tm, QT, subs);
+            launch_after(window_tile_kernel<2>, grid, WT_THREADS, tsm, stream, a, tm, QT, subs);
         }
         FT_CHECK_CUDA(cudaGetLastError());
     }
@@ -843,7 +851,7 @@ int launch_window_attention(const WindowArgs& a, int T, int n_single, const Wind
         const size_t rows = (size_t)kStepWarps * kStepKeys * (a.dim + a.vdim) * 4;
         auto step = [&](auto kernel) -> int {
             if (rows > 40 * 1024) FT_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows));
-            kernel<<<dim3(T, a.G), kStepWarps * 32, rows, stream>>>(a);
+            launch_after(kernel, dim3(T, a.G), kStepWarps * 32, rows, stream, a);
             return 0;
         };
         if (int r = grp <= 1 ? step(window_step_kernel<1>) : grp <= 2 ? step(window_step_kernel<2>) : step(window_step_kernel<4>)) return r;
@@ -854,8 +862,8 @@ int launch_window_attention(const WindowArgs& a, int T, int n_single, const Wind
     const int vpl = (a.vdim + 31) / 32;
 #define FT_WIN(V)                                                                                   \
     do {                                                                                            \
-        if (vec) window_attn_kernel<V, true><<<grid, kWinWarps * 32, smem, stream>>>(a);            \
-        else window_attn_kernel<V, false><<<grid, kWinWarps * 32, smem, stream>>>(a);               \
+        if (vec) launch_after(window_attn_kernel<V, true>, grid, kWinWarps * 32, smem, stream, a);            \
+        else launch_after(window_attn_kernel<V, false>, grid, kWinWarps * 32, smem, stream, a);               \
     } while (0)
     if (vpl <= 1) FT_WIN(1);
     else if (vpl <= 2) FT_WIN(2);
@@ -894,6 +902,7 @@ __device__ __forceinline__ void cp_async_f32x4(float* dst_smem, const float* src
 // other half, afterwards every lane holds one column and the tree goes on as usual.
 template <int LPC, int DPT, int CPT, bool VEC>
 __global__ void __launch_bounds__(RTHREADS) decay_rule_kernel(RecurArgs a) {
+    pdl_wait();
     constexpr int VB = RTHREADS / LPC * CPT, RUN = DPT + 4, DP = LPC * RUN;
     constexpr int BUF = 2 * RCH * DP + RCH * VB + RCH * 2;      // floats of one staged chunk: keys | queries | values | (a, b)
     constexpr int NST = rule_stages(DP);
@@ -1085,6 +1094,7 @@ __global__ void __launch_bounds__(RTHREADS) decay_rule_kernel(RecurArgs a) {
 // one a decode step of three such layers takes 40 us less.
 template <int V>
 __global__ void __launch_bounds__(256) decay_step_kernel(RecurArgs a, int TX) {
+    pdl_wait();
     extern __shared__ __align__(16) float sh[];
     float* part = sh;                                 // [256][V]
     float *sk = sh + 256 * V, *sq = sk + a.dim;
@@ -1169,8 +1179,8 @@ static int launch_decay_step(const RecurArgs& a, int n_req, const StepPlan& p, c
     const int TX = p.TX;
     const dim3 grid(n_req, a.heads, ((wide ? a.vd / 4 : a.vd) + TX - 1) / TX);
     const size_t smem = (size_t)(256 * (wide ? 4 : 1) + 2 * a.dim) * 4;
-    if (wide) decay_step_kernel<4><<<grid, 256, smem, stream>>>(a, TX);
-    else decay_step_kernel<1><<<grid, 256, smem, stream>>>(a, TX);
+    if (wide) launch_after(decay_step_kernel<4>, grid, 256, smem, stream, a, TX);
+    else launch_after(decay_step_kernel<1>, grid, 256, smem, stream, a, TX);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1185,8 +1195,8 @@ static int launch_decay_rule_t(const RecurArgs& a, int n_req, cudaStream_t strea
         FT_CHECK_CUDA(cudaFuncSetAttribute(decay_rule_kernel<LPC, DPT, CPT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     }
     dim3 grid((a.vd + VB - 1) / VB, a.heads, n_req);
-    if (vec) decay_rule_kernel<LPC, DPT, CPT, true><<<grid, RTHREADS, smem, stream>>>(a);
-    else decay_rule_kernel<LPC, DPT, CPT, false><<<grid, RTHREADS, smem, stream>>>(a);
+    if (vec) launch_after(decay_rule_kernel<LPC, DPT, CPT, true>, grid, RTHREADS, smem, stream, a);
+    else launch_after(decay_rule_kernel<LPC, DPT, CPT, false>, grid, RTHREADS, smem, stream, a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1257,6 +1267,7 @@ extern "C" int ft_decay_rule(const float* q, const float* k, const float* v, con
 // Per token: values with a column of ones appended (the normaliser rides along as one more state column), and the log
 // gates i = cap tanh((z_i + b_i) / cap), f = logsigmoid(cap tanh((z_f + b_f) / cap)).
 __global__ void __launch_bounds__(128) memory_prep_kernel(MemoryArgs a) {
+    pdl_wait();
     const int t = blockIdx.x, h = blockIdx.y;
     const float* pr = a.proj + (size_t)t * a.ldp;
     const int ve = a.vdim + 1;
@@ -1275,6 +1286,7 @@ __global__ void __launch_bounds__(128) memory_prep_kernel(MemoryArgs a) {
 // m_t = max(F_t + m_in, G_t).  Then a = exp(f + m_(t-1) - m_t), b = exp(i - m_t), floor[t] = exp(-m_t), the lower bound of the
 // read-out's denominator.  m lives in the state slot, 0 at a sequence's start.
 __global__ void __launch_bounds__(128) memory_scan_kernel(MemoryArgs a, int n_units) {
+    pdl_wait();
     const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (unit >= n_units) return;
     const int r = unit / a.heads, h = unit % a.heads;
@@ -1307,10 +1319,10 @@ __global__ void __launch_bounds__(128) memory_scan_kernel(MemoryArgs a, int n_un
 }
 int launch_memory_prep(const MemoryArgs& a, int T, int n_req, cudaStream_t stream) {
     FT_REQUIRE(a.heads >= 1 && a.cap > 0.f, "matrix memory: bad head count or gate cap");
-    memory_prep_kernel<<<dim3(T, a.heads), 128, 0, stream>>>(a);
+    launch_after(memory_prep_kernel, dim3(T, a.heads), 128, 0, stream, a);
     FT_CHECK_CUDA(cudaGetLastError());
     const int units = n_req * a.heads;
-    memory_scan_kernel<<<(units + 3) / 4, 128, 0, stream>>>(a, units);
+    launch_after(memory_scan_kernel, (units + 3) / 4, 128, 0, stream, a, units);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1322,6 +1334,7 @@ int launch_memory_prep(const MemoryArgs& a, int T, int n_req, cudaStream_t strea
 // whose inputs are all rows of this step and of one request are read once for the block.
 template <int TB>
 __global__ void __launch_bounds__(256) space_conv_kernel(SpaceArgs a, int T) {
+    pdl_wait();
     const int t0 = blockIdx.x * TB, nt = min(TB, T - t0), K = a.taps;
     const int c = blockIdx.y * 256 + threadIdx.x;
     if (blockIdx.y + 1 == gridDim.y)
@@ -1374,6 +1387,7 @@ __global__ void __launch_bounds__(256) space_conv_kernel(SpaceArgs a, int T) {
 // The same for blocks of eight tokens, rows on 16 bytes and four taps: a thread takes four channels (one: 27 us for 2313 tokens of 4352 channels; now
 // 25.2 us, the bytes take 12).
 __global__ void __launch_bounds__(128) space_conv_rows_kernel(SpaceArgs a, int T) {
+    pdl_wait();
     constexpr int TB = 8;
     const int t0 = blockIdx.x * TB, nt = min(TB, T - t0);
     const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
@@ -1427,6 +1441,7 @@ __global__ void __launch_bounds__(128) space_conv_rows_kernel(SpaceArgs a, int T
 // The slot's tail after the step: the raw inputs of the last K-1 positions, from this step's rows or the old tail.
 constexpr int kMaxTaps = 16;
 __global__ void __launch_bounds__(256) space_tail_kernel(SpaceArgs a) {
+    pdl_wait();
     const int r = blockIdx.y;
     const int start = a.req_start[r], n = a.req_start[r + 1] - start, pos0 = a.req_pos0[r], K = a.taps;
     if (n <= 0 || K <= 1) return;
@@ -1448,11 +1463,11 @@ int launch_space_prep(const SpaceArgs& a, int T, int n_req, cudaStream_t stream)
     const int groups = (a.channels + 255) / 256;
     const uintptr_t all = (uintptr_t)a.proj | (uintptr_t)a.conv_w | (uintptr_t)a.conv_b | (uintptr_t)a.xbc;
     if (T > 64 && a.taps == 4 && a.channels % 4 == 0 && a.ldp % 4 == 0 && a.o_x % 4 == 0 && (all & 15) == 0)
-        space_conv_rows_kernel<<<dim3((T + 7) / 8, (a.channels / 4 + 127) / 128), 128, 0, stream>>>(a, T);
-    else if (T > 64) space_conv_kernel<8><<<dim3((T + 7) / 8, groups), 256, 0, stream>>>(a, T);
-    else space_conv_kernel<1><<<dim3(T, groups), 256, 0, stream>>>(a, T);
+        launch_after(space_conv_rows_kernel, dim3((T + 7) / 8, (a.channels / 4 + 127) / 128), 128, 0, stream, a, T);
+    else if (T > 64) launch_after(space_conv_kernel<8>, dim3((T + 7) / 8, groups), 256, 0, stream, a, T);
+    else launch_after(space_conv_kernel<1>, dim3(T, groups), 256, 0, stream, a, T);
     FT_CHECK_CUDA(cudaGetLastError());
-    space_tail_kernel<<<dim3((a.channels + 255) / 256, n_req), 256, 0, stream>>>(a);
+    launch_after(space_tail_kernel, dim3((a.channels + 255) / 256, n_req), 256, 0, stream, a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1475,6 +1490,7 @@ __device__ __forceinline__ float readout_value(const ReadoutArgs& a, int t, int 
 }
 constexpr int kReadoutKeep = 8;      // values a thread keeps in registers between the two passes
 __global__ void __launch_bounds__(256) readout_kernel(ReadoutArgs a) {
+    pdl_wait();
     __shared__ float red[33];
     const int t = blockIdx.x / a.norm_groups, g = blockIdx.x % a.norm_groups;
     const int n = a.heads * a.vdim / a.norm_groups, c0 = g * n;
@@ -1508,6 +1524,7 @@ __global__ void __launch_bounds__(256) readout_kernel(ReadoutArgs a) {
 // normaliser read once (a CTA per (token, head): 39 us for 2313 tokens of eight heads of 256; now 15.6 us, the bytes take 9).
 template <int NP>
 __global__ void __launch_bounds__(256) readout_heads_kernel(ReadoutArgs a, int n_pairs) {
+    pdl_wait();
     const int id = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (id >= n_pairs) return;
     const int t = id / a.heads, h = id % a.heads, n = a.vdim, c0 = h * n;
@@ -1558,6 +1575,7 @@ __global__ void __launch_bounds__(256) readout_heads_kernel(ReadoutArgs a, int n
 // group's columns in registers between the two passes (one column at a time: 91 us for 2313 tokens of 4096 gated columns; now 36 us).
 template <int NV>
 __global__ void __launch_bounds__(256) readout_rows_kernel(ReadoutArgs a) {
+    pdl_wait();
     __shared__ float red[33];
     const int t = blockIdx.x / a.norm_groups, g = blockIdx.x % a.norm_groups;
     const int n = a.heads * a.vdim / a.norm_groups, c0 = g * n;
@@ -1636,24 +1654,24 @@ int launch_readout(const ReadoutArgs& a, int T, cudaStream_t stream) {
     if (!a.floor && a.vd == a.vdim && a.vdim % 4 == 0 && n % 4 == 0 && n <= 8192 && a.ldo % 4 == 0 && (!a.gate || a.ldg % 4 == 0) && (!a.skip || a.ldx % 4 == 0) &&
         (all & 15) == 0) {
         const int th = n <= 128 ? 32 : n <= 256 ? 64 : n <= 512 ? 128 : 256;
-        if (n <= 4 * th) readout_rows_kernel<1><<<T * a.norm_groups, th, 0, stream>>>(a);
-        else if (n <= 8 * th) readout_rows_kernel<2><<<T * a.norm_groups, th, 0, stream>>>(a);
-        else if (n <= 16 * th) readout_rows_kernel<4><<<T * a.norm_groups, th, 0, stream>>>(a);
-        else readout_rows_kernel<8><<<T * a.norm_groups, th, 0, stream>>>(a);
+        if (n <= 4 * th) launch_after(readout_rows_kernel<1>, T * a.norm_groups, th, 0, stream, a);
+        else if (n <= 8 * th) launch_after(readout_rows_kernel<2>, T * a.norm_groups, th, 0, stream, a);
+        else if (n <= 16 * th) launch_after(readout_rows_kernel<4>, T * a.norm_groups, th, 0, stream, a);
+        else launch_after(readout_rows_kernel<8>, T * a.norm_groups, th, 0, stream, a);
         FT_CHECK_CUDA(cudaGetLastError());
         return 0;
     }
     if (a.floor && a.norm_groups == a.heads && a.vdim % 2 == 0 && n <= 512 && (!a.gate_kind || a.ldg % 2 == 0) && (!a.skip || a.ldx % 2 == 0) &&
         (((uintptr_t)a.out | (uintptr_t)a.gate | (uintptr_t)a.x) & 7) == 0 && (((uintptr_t)a.out_hi | (uintptr_t)a.out_lo) & 3) == 0) {
         const int pairs = T * a.heads, grid = (pairs + 7) / 8;
-        if (n <= 128) readout_heads_kernel<2><<<grid, 256, 0, stream>>>(a, pairs);
-        else if (n <= 256) readout_heads_kernel<4><<<grid, 256, 0, stream>>>(a, pairs);
-        else readout_heads_kernel<8><<<grid, 256, 0, stream>>>(a, pairs);
+        if (n <= 128) launch_after(readout_heads_kernel<2>, grid, 256, 0, stream, a, pairs);
+        else if (n <= 256) launch_after(readout_heads_kernel<4>, grid, 256, 0, stream, a, pairs);
+        else launch_after(readout_heads_kernel<8>, grid, 256, 0, stream, a, pairs);
         FT_CHECK_CUDA(cudaGetLastError());
         return 0;
     }
     const int threads = n <= 64 ? 32 : n <= 256 ? 64 : n <= 1024 ? 128 : 256;
-    readout_kernel<<<T * a.norm_groups, threads, 0, stream>>>(a);
+    launch_after(readout_kernel, T * a.norm_groups, threads, 0, stream, a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -77,6 +77,7 @@ __device__ __forceinline__ void hold(f32x2* x) {
 }
 template <bool VEC, int DB>
 __global__ void __launch_bounds__(DR_THREADS, 1) decay_runs_kernel(RecurArgs a, int* err) {
+    pdl_wait();
     extern __shared__ uint8_t dr_raw[];
     __shared__ Two pref[DR_RUN], suff[DR_RUN], full[8];      // products of decays inside a block of 16 tokens: up to and with i, behind j, all
     __shared__ Two mid[8][8], tail[8], head[9];          // of whole blocks: between two, behind one, before one (head[8]: of the run)
@@ -561,7 +562,7 @@ int launch_runs(const RecurArgs& a, dim3 grid, cudaStream_t stream) {
         FT_CHECK_CUDA(cudaFuncSetAttribute(decay_runs_kernel<VEC, DB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DR_SMEM));
         attr.mark();
     }
-    decay_runs_kernel<VEC, DB><<<grid, DR_THREADS, DR_SMEM, stream>>>(a, a.err);
+    launch_after(decay_runs_kernel<VEC, DB>, grid, DR_THREADS, DR_SMEM, stream, a, a.err);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -33,6 +33,7 @@ template <int KIND>
 __global__ void __launch_bounds__(XT_THREADS, 2)
 experts_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
                   ExpertsKernelArgs a) {
+    pdl_wait();
     extern __shared__ uint8_t xt_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(xt_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint64_t full[XT_STAGES], empty[XT_STAGES], acc_full, drain;
@@ -219,9 +220,9 @@ int launch_experts_tc(const ExpertsTcArgs& t, cudaStream_t stream) {
     const int tiles = t.pairs / XT_N + (t.E < t.pairs ? t.E : t.pairs);      // an upper bound: every expert may end with a partial tile
     FT_REQUIRE(tiles <= 65535, "experts (tcgen05): %d pairs are too many", t.pairs);
     const dim3 grid(t.n_rows / XT_M, tiles);
-    if (t.out) experts_tc_kernel<XT_ROWS><<<grid, XT_THREADS, XT_SMEM, stream>>>(mw, mh, ml, a);
-    else if (t.act == FT_ACT_RELU2) experts_tc_kernel<XT_RELU2><<<grid, XT_THREADS, XT_SMEM, stream>>>(mw, mh, ml, a);
-    else experts_tc_kernel<XT_GLU><<<grid, XT_THREADS, XT_SMEM, stream>>>(mw, mh, ml, a);
+    if (t.out) launch_after(experts_tc_kernel<XT_ROWS>, grid, XT_THREADS, XT_SMEM, stream, mw, mh, ml, a);
+    else if (t.act == FT_ACT_RELU2) launch_after(experts_tc_kernel<XT_RELU2>, grid, XT_THREADS, XT_SMEM, stream, mw, mh, ml, a);
+    else launch_after(experts_tc_kernel<XT_GLU>, grid, XT_THREADS, XT_SMEM, stream, mw, mh, ml, a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

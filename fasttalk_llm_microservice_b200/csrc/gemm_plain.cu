@@ -58,6 +58,7 @@ gemm_plain_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     cluster_sync_all();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    pdl_wait();
     if (warp == 0) {
         if (elect_one()) {
             // weights are read again by every token tile; a launch of one token tile streams them
@@ -178,6 +179,7 @@ gemm_plain_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    pdl_wait();
     if (warp == 0) {
         if (elect_one()) {
             const uint64_t pol_w = policy_evict_first(), pol_x = policy_evict_last();
@@ -346,11 +348,13 @@ int launch_few(const CUtensorMap& mw, const CUtensorMap& mh, const CUtensorMap& 
     cfg.blockDim = dim3(PF_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = S; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_plain_few_kernel<BN>, mw, mh, ml, out, n_out, T, kc, stages));
     return 0;
 }
@@ -421,7 +425,7 @@ int launch_gemm_plain(const void* w, const void* hi, const void* lo, float* out,
     if (stages > PL_MAX_STAGES) stages = PL_MAX_STAGES;
     // the whole ring's memory, also where the stages take less: a pair's CTA holds all columns while it waits for its partner, so no
     // other kernel with columns of its own may have room beside it
-    gemm_plain_pair_kernel<<<2 * (units < clusters ? units : clusters), PL_THREADS, PL_RING + 1024, stream>>>(mw, mh, ml, out, n_out, T, K / PL_BK, stages, bn);
+    launch_after(gemm_plain_pair_kernel, 2 * (units < clusters ? units : clusters), PL_THREADS, PL_RING + 1024, stream, mw, mh, ml, out, n_out, T, K / PL_BK, stages, bn);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -30,6 +30,7 @@ __device__ __forceinline__ void ht_copy16(uint32_t dst_smem, const void* src) {
 
 template <int NT>
 __global__ void __launch_bounds__(HT_THREADS) linear_heads_kernel(LinearArgs a, int* err) {
+    pdl_wait();
     constexpr int W_BYTES = HT_ROWS * 128, X_BYTES = NT * 128, STAGE = W_BYTES + 2 * X_BYTES;
     constexpr int COLS = NT < 32 ? 32 : NT;
     constexpr int PIECES = (NT * 8 + HT_THREADS - 1) / HT_THREADS;      // (token row, 8 columns) pieces per thread and block
@@ -179,7 +180,7 @@ int launch_nt(const LinearArgs& a, int* err, cudaStream_t stream) {
         attr.mark();
     }
     const dim3 grid((a.N + HT_ROWS - 1) / HT_ROWS, (a.M + NT - 1) / NT, a.P);
-    linear_heads_kernel<NT><<<grid, HT_THREADS, SMEM, stream>>>(a, err);
+    launch_after(linear_heads_kernel<NT>, grid, HT_THREADS, SMEM, stream, a, err);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

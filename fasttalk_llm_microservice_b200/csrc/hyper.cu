@@ -28,6 +28,7 @@ constexpr int kMaxStreams = 16;
 // the width is a multiple of four and every row starts on 16 bytes)
 template <int MS, int V>
 __global__ void __launch_bounds__(256) hyper_joint_kernel(HyperArgs a) {
+    pdl_wait();
     __shared__ float red[33];
     __shared__ float smix[kMaxStreams * kMaxStreams], sout[kMaxStreams], sin_[kMaxStreams];
     extern __shared__ __align__(16) float row[];  // [W]: the row the next norm reads
@@ -182,6 +183,7 @@ __global__ void __launch_bounds__(256) hyper_joint_kernel(HyperArgs a) {
 __global__ void __launch_bounds__(256) scaled_rows_kernel(const float* __restrict__ src, const float* __restrict__ wt,
                                                           const int* __restrict__ slot_pos, int top, float* __restrict__ dst,
                                                           __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, int W) {
+    pdl_wait();
     const int i = blockIdx.x;
     const float w = wt[i];
     const float* s = src + (size_t)(i / top) * W;
@@ -228,6 +230,7 @@ __device__ __forceinline__ float ex2_h(float x) {
 // without guards beyond n < N and the shared-memory reads of a token get constant offsets.
 template <int PHASE, int LPC, int KEEP>
 __global__ void __launch_bounds__(kScanThreads, 4) selective_scan_kernel(ScanArgs a, int seg_len) {
+    pdl_wait();
     constexpr int lpc = LPC;
     extern __shared__ __align__(16) float ssm[];
     const int r = blockIdx.y, seg = blockIdx.z + PHASE;
@@ -388,13 +391,13 @@ int launch_hyper_joint(const HyperArgs& a, int T, cudaStream_t stream) {
     const bool v4 = a.W % 4 == 0 && al(a.X, 16) && al(a.y0, 16) && al(a.y1, 16) && al(a.g0, 16) && al(a.g1, 16) && al(a.eout, 16) &&
                     al(a.nw, 16) && al(a.nb, 16) && al(a.hn, 16) && al(a.sum_out, 16) && al(a.embed, 8) && al(a.hi, 8) && al(a.lo, 8);
     if (v4) {
-        if (a.S <= 4) hyper_joint_kernel<4, 4><<<T, 256, smem, stream>>>(a);
-        else if (a.S <= 8) hyper_joint_kernel<8, 4><<<T, 256, smem, stream>>>(a);
-        else hyper_joint_kernel<kMaxStreams, 1><<<T, 256, smem, stream>>>(a);
+        if (a.S <= 4) launch_after(hyper_joint_kernel<4, 4>, T, 256, smem, stream, a);
+        else if (a.S <= 8) launch_after(hyper_joint_kernel<8, 4>, T, 256, smem, stream, a);
+        else launch_after(hyper_joint_kernel<kMaxStreams, 1>, T, 256, smem, stream, a);
     } else {
-        if (a.S <= 4) hyper_joint_kernel<4, 1><<<T, 256, smem, stream>>>(a);
-        else if (a.S <= 8) hyper_joint_kernel<8, 1><<<T, 256, smem, stream>>>(a);
-        else hyper_joint_kernel<kMaxStreams, 1><<<T, 256, smem, stream>>>(a);
+        if (a.S <= 4) launch_after(hyper_joint_kernel<4, 1>, T, 256, smem, stream, a);
+        else if (a.S <= 8) launch_after(hyper_joint_kernel<8, 1>, T, 256, smem, stream, a);
+        else launch_after(hyper_joint_kernel<kMaxStreams, 1>, T, 256, smem, stream, a);
     }
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
@@ -404,7 +407,7 @@ int launch_scaled_rows(const float* src, const float* wt, const int* slot_pos, i
                        int W, cudaStream_t stream) {
     FT_REQUIRE(src && wt && slot_pos && top >= 1 && (dst || (hi && lo)), "scaled rows: missing operands");
     if (pairs <= 0) return 0;
-    scaled_rows_kernel<<<pairs, 256, 0, stream>>>(src, wt, slot_pos, top, dst, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, W);
+    launch_after(scaled_rows_kernel, pairs, 256, 0, stream, src, wt, slot_pos, top, dst, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, W);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -436,8 +439,8 @@ int launch_selective_scan(const ScanArgs& a, int n_req, cudaStream_t stream) {
             FT_CHECK_CUDA(cudaFuncSetAttribute(selective_scan_kernel<0, L, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
             FT_CHECK_CUDA(cudaFuncSetAttribute(selective_scan_kernel<1, L, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
         }                                                                                                             \
-        selective_scan_kernel<0, L, K><<<g0, kScanThreads, smem, stream>>>(a, seg_len);                               \
-        if (n_seg > 1) selective_scan_kernel<1, L, K><<<g1, kScanThreads, smem, stream>>>(a, seg_len);                \
+        launch_after(selective_scan_kernel<0, L, K>, g0, kScanThreads, smem, stream, a, seg_len);                               \
+        if (n_seg > 1) launch_after(selective_scan_kernel<1, L, K>, g1, kScanThreads, smem, stream, a, seg_len);                \
     } while (0)
 #define FT_SCAN(L)                                \
     do {                                          \

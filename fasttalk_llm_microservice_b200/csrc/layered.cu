@@ -58,6 +58,7 @@ constexpr int LBM = 64, LBN = 64, LBK = 16, LTHREADS = 256;
 
 template <bool VEC>
 __global__ void __launch_bounds__(LTHREADS) linear_tile_kernel(LinearArgs a) {
+    pdl_wait();
     __shared__ float sA[LBK][LBM + 4];
     __shared__ float sW[LBK][LBN + 4];
     __shared__ int s_info[3];
@@ -186,6 +187,7 @@ constexpr int LWARPS = 8, LROWS_MANY = 16, LROWS_FEW = 4, LSTAGE = 8192;
 
 template <bool PAIR, bool VEC, int LROWS>
 __global__ void __launch_bounds__(LWARPS * 32) linear_rows_kernel(LinearArgs a) {
+    pdl_wait();
     constexpr int LKC = LSTAGE / LROWS;
     constexpr int CPW = PAIR ? 2 : 4;                 // output columns per warp
     constexpr int WR = PAIR ? 2 * CPW : CPW;          // weight rows per warp
@@ -334,8 +336,8 @@ int launch_linear(const LinearArgs& a, int rows_bound, int* err, cudaStream_t st
         const bool handful = a.seg ? rows_bound <= 3 * a.P : a.M <= LROWS_FEW;
 #define FT_ROWS(PAIR_, VEC_)                                                                                             \
     do {                                                                                                                 \
-        if (handful) linear_rows_kernel<PAIR_, VEC_, LROWS_FEW><<<grid, LWARPS * 32, 0, stream>>>(a);                    \
-        else linear_rows_kernel<PAIR_, VEC_, LROWS_MANY><<<grid, LWARPS * 32, 0, stream>>>(a);                           \
+        if (handful) launch_after(linear_rows_kernel<PAIR_, VEC_, LROWS_FEW>, grid, LWARPS * 32, 0, stream, a);                    \
+        else launch_after(linear_rows_kernel<PAIR_, VEC_, LROWS_MANY>, grid, LWARPS * 32, 0, stream, a);                           \
     } while (0)
         if (pair) {
             if (v8) FT_ROWS(true, true);
@@ -353,8 +355,8 @@ int launch_linear(const LinearArgs& a, int rows_bound, int* err, cudaStream_t st
     dim3 grid((a.N + LBN - 1) / LBN, 1, 1);
     if (a.seg) grid.y = (rows_bound + LBM - 1) / LBM + a.P;
     else { grid.y = (a.M + LBM - 1) / LBM; grid.z = a.P; }
-    if (vec) linear_tile_kernel<true><<<grid, LTHREADS, 0, stream>>>(a);
-    else linear_tile_kernel<false><<<grid, LTHREADS, 0, stream>>>(a);
+    if (vec) launch_after(linear_tile_kernel<true>, grid, LTHREADS, 0, stream, a);
+    else launch_after(linear_tile_kernel<false>, grid, LTHREADS, 0, stream, a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -370,11 +372,13 @@ __device__ __forceinline__ void store_planes(__nv_bfloat16* hi, __nv_bfloat16* l
 
 __global__ void to_planes_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
                                  size_t n) {
+    pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         store_planes(hi, lo, i, x[i]);
 }
 
 __global__ void softcap_kernel(float* __restrict__ x, size_t n, float cap) {
+    pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         x[i] = cap * tanhf(x[i] / cap);
 }
@@ -382,6 +386,7 @@ __global__ void softcap_kernel(float* __restrict__ x, size_t n, float cap) {
 // planes of the rows an index list names: out row i = planes(src[idx[i]])
 __global__ void gather_planes_kernel2(const float* __restrict__ src, const int* __restrict__ idx, __nv_bfloat16* __restrict__ hi,
                                       __nv_bfloat16* __restrict__ lo, int W) {
+    pdl_wait();
     const size_t i = blockIdx.x;
     const float* r = src + (size_t)idx[i] * W;
     for (int c = threadIdx.x; c < W; c += blockDim.x) store_planes(hi, lo, i * W + c, r[c]);
@@ -390,6 +395,7 @@ __global__ void gather_planes_kernel2(const float* __restrict__ src, const int* 
 // gu [rows][2 ff] with columns (2j, 2j+1) = (gate_j, up_j)  ->  planes of their gated product (GluSpec), [rows][ff]
 __global__ void glu_planes_kernel(const float* __restrict__ gu, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, size_t n,
                                   int ff, GluSpec glu) {
+    pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const float2 v = reinterpret_cast<const float2*>(gu)[i];
         store_planes(hi, lo, i, glu_value(glu, v.x, v.y, glu.bias ? (int)(i % ff) : 0));
@@ -399,6 +405,7 @@ __global__ void glu_planes_kernel(const float* __restrict__ gu, __nv_bfloat16* _
 // u [rows][ff]  ->  planes of relu(u)^2
 __global__ void relu2_planes_kernel(const float* __restrict__ u, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
                                     size_t n) {
+    pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const float v = fmaxf(u[i], 0.f);
         store_planes(hi, lo, i, v * v);
@@ -406,28 +413,28 @@ __global__ void relu2_planes_kernel(const float* __restrict__ u, __nv_bfloat16* 
 }
 
 int launch_gather_planes_rows(const float* src, const int* idx, void* hi, void* lo, int n, int W, cudaStream_t stream) {
-    gather_planes_kernel2<<<n, 256, 0, stream>>>(src, idx, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, W);
+    launch_after(gather_planes_kernel2, n, 256, 0, stream, src, idx, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, W);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 int launch_act_planes(const float* gu, void* hi, void* lo, int rows, int ff, int act, const GluSpec& glu, cudaStream_t stream) {
     const size_t n = (size_t)rows * ff;
     const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-    if (act == FT_ACT_RELU2) relu2_planes_kernel<<<blocks, 256, 0, stream>>>(gu, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n);
-    else glu_planes_kernel<<<blocks, 256, 0, stream>>>(gu, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n, ff, glu);
+    if (act == FT_ACT_RELU2) launch_after(relu2_planes_kernel, blocks, 256, 0, stream, gu, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n);
+    else launch_after(glu_planes_kernel, blocks, 256, 0, stream, gu, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n, ff, glu);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 
 int launch_to_planes(const float* x, void* hi, void* lo, size_t n, cudaStream_t stream) {
     const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-    to_planes_kernel<<<blocks, 256, 0, stream>>>(x, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n);
+    launch_after(to_planes_kernel, blocks, 256, 0, stream, x, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 int launch_softcap(float* x, size_t n, float cap, cudaStream_t stream) {
     const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-    softcap_kernel<<<blocks, 256, 0, stream>>>(x, n, cap);
+    launch_after(softcap_kernel, blocks, 256, 0, stream, x, n, cap);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -438,6 +445,7 @@ __global__ void __launch_bounds__(256)
 embed_norm_kernel(const int* __restrict__ tokens, const __nv_bfloat16* __restrict__ embed, float* __restrict__ x,
                   float* __restrict__ hn, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, int W, float eps,
                   float gain, const float* __restrict__ gain_w) {
+    pdl_wait();
     __shared__ float red[33];
     const int t = blockIdx.x;
     const __nv_bfloat16* e = embed + (size_t)tokens[t] * W;
@@ -464,6 +472,7 @@ combine_norm_kernel(float* __restrict__ x, float* __restrict__ hn, const float* 
                     int o_rg2, const float* __restrict__ rg_bias, const float* __restrict__ mix,
                     const float* __restrict__ eout, const float* __restrict__ wt, const int* __restrict__ slot_pos,
                     int top, int W, float eps, float gain, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
+    pdl_wait();
     __shared__ float red[33];
     extern __shared__ float row[];
     const int t = blockIdx.x;
@@ -493,6 +502,7 @@ combine_norm_kernel(float* __restrict__ x, float* __restrict__ hn, const float* 
 
 // rows of the normed stream that the head reads: out[i] = hn[idx[i]]
 __global__ void gather_rows_kernel(const float* __restrict__ src, const int* __restrict__ idx, float* __restrict__ dst, int W) {
+    pdl_wait();
     const int i = blockIdx.x;
     const float* s = src + (size_t)idx[i] * W;
     for (int c = threadIdx.x; c < W; c += blockDim.x) dst[(size_t)i * W + c] = s[c];
@@ -500,7 +510,7 @@ __global__ void gather_rows_kernel(const float* __restrict__ src, const int* __r
 
 int launch_embed_norm(const int* tokens, const void* embed, float* x, float* hn, void* hi, void* lo, int T, int W, float eps,
                       float gain, const float* gain_w, cudaStream_t stream) {
-    embed_norm_kernel<<<T, 256, 0, stream>>>(tokens, (const __nv_bfloat16*)embed, x, hn, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo,
+    launch_after(embed_norm_kernel, T, 256, 0, stream, tokens, (const __nv_bfloat16*)embed, x, hn, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo,
                                              W, eps, gain_w ? 1.f : gain, gain_w);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
@@ -508,13 +518,13 @@ int launch_embed_norm(const int* tokens, const void* embed, float* x, float* hn,
 int launch_combine_norm(float* x, float* hn, const float* proj, int ldp, int o_rg1, int o_rg2, const float* rg_bias,
                         const float* mix, const float* eout, const float* wt, const int* slot_pos, int top, int T, int W,
                         float eps, float gain, void* hi, void* lo, cudaStream_t stream) {
-    combine_norm_kernel<<<T, 256, (size_t)W * 4, stream>>>(x, hn, proj, ldp, o_rg1, o_rg2, rg_bias, mix, eout, wt, slot_pos,
+    launch_after(combine_norm_kernel, T, 256, (size_t)W * 4, stream, x, hn, proj, ldp, o_rg1, o_rg2, rg_bias, mix, eout, wt, slot_pos,
                                                           top, W, eps, gain, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
 int launch_gather_rows(const float* src, const int* idx, float* dst, int n, int W, cudaStream_t stream) {
-    gather_rows_kernel<<<n, 256, 0, stream>>>(src, idx, dst, W);
+    launch_after(gather_rows_kernel, n, 256, 0, stream, src, idx, dst, W);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -524,6 +534,7 @@ int launch_gather_rows(const float* src, const int* idx, float* dst, int n, int 
 // pos % 64 of the layer's caches ([page][64][rank + rot] fp32; bf16 as latent_chunk16 lays a page out); the rotated part
 // of every query head goes to qlat.  Pairs (i, i + rot / 2); the angle's sine and cosine are formed once per token.
 __global__ void __launch_bounds__(128) latent_prep_kernel(LatentArgs a, int row16) {
+    pdl_wait();
     __shared__ float red[33];
     extern __shared__ float trig[];                        // [rot / 2] cosines, [rot / 2] sines
     const int t = blockIdx.x, rank = a.rank, rot = a.rot, half = rot >> 1;
@@ -594,6 +605,7 @@ __device__ __forceinline__ float latent_finish(float m, float l, const LatentArg
 
 template <int NR, int KB>
 __global__ void __launch_bounds__(128) latent_attn_kernel(LatentArgs a, int n_pairs, int n_split) {
+    pdl_wait();
     const int pair = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int split = blockIdx.y;
     if (pair >= n_pairs) return;
@@ -681,7 +693,7 @@ __global__ void __launch_bounds__(128) latent_attn_kernel(LatentArgs a, int n_pa
 int launch_latent_prep(const LatentArgs& a, int T, cudaStream_t stream) {
     FT_REQUIRE(a.proj && a.norm_w && (a.cache || a.cache16) && (a.rot == 0 || (a.rot_freq && (a.qlat || a.qlat16) && a.rot % 2 == 0)),
                "latent prep: missing operands");
-    latent_prep_kernel<<<T, 128, (size_t)a.rot * 4, stream>>>(a, latent_row16(a.rank, a.rot));
+    launch_after(latent_prep_kernel, T, 128, (size_t)a.rot * 4, stream, a, latent_row16(a.rank, a.rot));
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -714,7 +726,7 @@ int launch_latent_attn(const LatentArgs& a, int T, cudaStream_t stream) {
         FT_REQUIRE(a.cache && a.qlat, "latent attention: no fp32 cache or queries");
         const int kd = a.rank + a.rot;
         const dim3 grid((n_pairs + 3) / 4, n_split);
-#define FT_LAT(NR_, KB_) latent_attn_kernel<NR_, KB_><<<grid, 128, 0, stream>>>(a, n_pairs, n_split)
+#define FT_LAT(NR_, KB_) launch_after(latent_attn_kernel<NR_, KB_>, grid, 128, 0, stream, a, n_pairs, n_split)
         if (kd <= 32) FT_LAT(1, 8);
         else if (kd <= 64) FT_LAT(2, 8);
         else if (kd <= 128) FT_LAT(4, 8);
@@ -754,6 +766,7 @@ __device__ __forceinline__ void delta_decays(const DeltaArgs& a, int t0, int nt,
 template <int TB>
 __global__ void __launch_bounds__(128)
 delta_prep_kernel(DeltaArgs a, int T) {
+    pdl_wait();
     __shared__ float red[3][TB][4];
     const int t0 = blockIdx.x * TB, nt = min(TB, T - t0), g = blockIdx.y;
     const int qk = a.kvh * a.dim, ch = 2 * qk + a.heads * a.vdim, hd = a.heads * a.dim;
@@ -877,6 +890,7 @@ delta_prep_kernel(DeltaArgs a, int T) {
 // head, whose sums need no shared memory (one channel per thread: 73 us for 2313 tokens of 6144 channels; now 48.5 us, the bytes take 17).
 template <int TB>
 __global__ void __launch_bounds__(128) delta_prep_rows_kernel(DeltaArgs a, int T, int qk_groups, int v_groups) {
+    pdl_wait();
     const int t0 = blockIdx.x * TB, nt = min(TB, T - t0), g = blockIdx.y;
     const int qk = a.kvh * a.dim, ch = 2 * qk + a.heads * a.vdim, hd = a.heads * a.dim;
     if (g >= qk_groups + v_groups) {
@@ -967,6 +981,7 @@ __global__ void __launch_bounds__(128) delta_prep_rows_kernel(DeltaArgs a, int T
 
 // New tail of raw convolution inputs per (request, channel): the last taps-1 entries of (old tail ++ this step's inputs).
 __global__ void delta_tail_kernel(DeltaArgs a, int n_req) {
+    pdl_wait();
     const int req = blockIdx.y;
     const int ch = 2 * a.kvh * a.dim + a.heads * a.vdim;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -999,6 +1014,7 @@ constexpr int DCHUNK = 16, DLANES = 16, DCPT = 2;
 template <int DPT, bool HD, bool VEC>
 __global__ void __launch_bounds__(128)
 delta_rule_kernel(DeltaArgs a) {
+    pdl_wait();
     extern __shared__ __align__(16) float sh[];
     constexpr int DP = DLANES * DPT;
     const int cols = blockDim.x / DLANES * DCPT, per = (HD ? 2 : 3) * DP + cols + 4;      // floats of a staged token: q | k | (g) | v | beta, kq, (g)
@@ -1179,7 +1195,7 @@ static int launch_delta_rule_t(const DeltaArgs& a, int n_req, cudaStream_t strea
     const size_t smem = (size_t)2 * DCHUNK * ((HD ? 2 : 3) * DLANES * DPT + threads / DLANES * DCPT + 4) * 4;
     if (smem > 48 * 1024)
         FT_CHECK_CUDA(cudaFuncSetAttribute(delta_rule_kernel<DPT, HD, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    delta_rule_kernel<DPT, HD, VEC><<<grid_of(threads), threads, smem, stream>>>(a);
+    launch_after(delta_rule_kernel<DPT, HD, VEC>, grid_of(threads), threads, smem, stream, a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1196,6 +1212,7 @@ static int launch_delta_rule(const DeltaArgs& a, int n_req, cudaStream_t stream)
 __global__ void __launch_bounds__(128)
 delta_out_kernel(float* __restrict__ o, const float* __restrict__ gate, const float* __restrict__ w, int vdim, float eps,
                  int n_pairs, int heads, int ldg, int gate_act) {
+    pdl_wait();
     const int pair = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (pair >= n_pairs) return;
     float* p = o + (size_t)pair * vdim;
@@ -1219,20 +1236,20 @@ int launch_delta(const DeltaArgs& a, const float* gate, const float* out_norm, f
     if (T > 64 && a.taps == 4 && a.dim % 16 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && a.heads * a.vdim % 4 == 0 && a.ldp % 4 == 0 && a.o_q % 4 == 0 &&
         (all & 15) == 0) {
         const int qg = (a.kvh * lanes + 127) / 128, vg = (a.heads * a.vdim / 4 + 127) / 128;
-        delta_prep_rows_kernel<8><<<dim3((T + 7) / 8, qg + vg + (a.head_decay ? 1 : a.heads)), 128, 0, stream>>>(a, T, qg, vg);
+        launch_after(delta_prep_rows_kernel<8>, dim3((T + 7) / 8, qg + vg + (a.head_decay ? 1 : a.heads)), 128, 0, stream, a, T, qg, vg);
     }
-    else if (T > 64) delta_prep_kernel<8><<<dim3((T + 7) / 8, groups), 128, 0, stream>>>(a, T);
-    else delta_prep_kernel<1><<<dim3(T, groups), 128, 0, stream>>>(a, T);
+    else if (T > 64) launch_after(delta_prep_kernel<8>, dim3((T + 7) / 8, groups), 128, 0, stream, a, T);
+    else launch_after(delta_prep_kernel<1>, dim3(T, groups), 128, 0, stream, a, T);
     FT_CHECK_CUDA(cudaGetLastError());
     if (a.taps > 1) {
-        delta_tail_kernel<<<dim3((ch + 127) / 128, n_req), 128, 0, stream>>>(a, n_req);
+        launch_after(delta_tail_kernel, dim3((ch + 127) / 128, n_req), 128, 0, stream, a, n_req);
         FT_CHECK_CUDA(cudaGetLastError());
     }
     if (a.dim <= 64) { if (int r = launch_delta_rule<4>(a, n_req, stream)) return r; }
     else if (a.dim <= 128) { if (int r = launch_delta_rule<8>(a, n_req, stream)) return r; }
     else { if (int r = launch_delta_rule<16>(a, n_req, stream)) return r; }
     const int n_pairs = T * a.heads;
-    delta_out_kernel<<<(n_pairs + 3) / 4, 128, 0, stream>>>(a.o, gate, out_norm, a.vdim, eps, n_pairs, a.heads,
+    launch_after(delta_out_kernel, (n_pairs + 3) / 4, 128, 0, stream, a.o, gate, out_norm, a.vdim, eps, n_pairs, a.heads,
                                                             ldg > 0 ? ldg : a.heads * a.vdim, gate_act);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
@@ -1245,6 +1262,7 @@ int launch_delta(const DeltaArgs& a, const float* gate, const float* out_norm, f
 __global__ void __launch_bounds__(128)
 route_kernel(const float* __restrict__ proj, int ldp, int o_router, int E, int top, int groups, int keep, int* __restrict__ ids,
              float* __restrict__ wts, int T, int sigmoid_scores, int normalise, float scale, const float* __restrict__ bias) {
+    pdl_wait();
     extern __shared__ float sh[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + wid;
@@ -1322,6 +1340,7 @@ route_kernel(const float* __restrict__ proj, int ldp, int o_router, int E, int t
 __global__ void __launch_bounds__(1024)
 route_sort_kernel(const int* __restrict__ ids, int n_pairs, int top, int E, int* __restrict__ seg, int* __restrict__ slot_token,
                   int* __restrict__ slot_pos) {
+    pdl_wait();
     extern __shared__ int shi[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     int* cnt = shi;                    // [warps][E]: a warp's pairs per expert, then where its next one goes
@@ -1376,14 +1395,14 @@ int launch_route(const float* proj, int ldp, int o_router, int E, int top, int g
                "router: %d experts, %d groups, keep %d, top %d do not fit together", E, groups, keep, top);
     const size_t smem = (size_t)4 * (E + groups) * 4;
     FT_REQUIRE(smem <= 48 * 1024 && (size_t)(2 * E + 1) * 4 <= 48 * 1024, "router: %d experts are too many", E);
-    route_kernel<<<(T + 3) / 4, 128, smem, stream>>>(proj, ldp, o_router, E, top, groups, keep, ids, wts, T,
+    launch_after(route_kernel, (T + 3) / 4, 128, smem, stream, proj, ldp, o_router, E, top, groups, keep, ids, wts, T,
                                                      route_kind == FT_ROUTE_SIGMOID, normalise, scale > 0.f ? scale : 1.f, bias);
     FT_CHECK_CUDA(cudaGetLastError());
     // Every expert's thread walks the warps' counts, so few pairs take few warps (one token's two choices of 16 experts: all 32
     // took a microsecond more); fewer, too, where the counts of so many would not fit.
     int warps = 32;
     while (warps > 1 && (warps * 16 >= std::max(T * top, E) || (size_t)(warps * E + E + 1) * 4 > 48 * 1024)) warps /= 2;
-    route_sort_kernel<<<1, warps * 32, (size_t)(warps * E + E + 1) * 4, stream>>>(ids, T * top, top, E, seg, slot_token, slot_pos);
+    launch_after(route_sort_kernel, 1, warps * 32, (size_t)(warps * E + E + 1) * 4, stream, ids, T * top, top, E, seg, slot_token, slot_pos);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

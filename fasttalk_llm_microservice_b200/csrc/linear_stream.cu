@@ -33,6 +33,7 @@ __device__ __forceinline__ float transpose_sum(float (&v)[32], int lane) {
 
 template <bool PAIR, int NC>
 __global__ void __launch_bounds__(LS_WARPS * 32) linear_stream_kernel(LinearArgs a, int* err) {
+    pdl_wait();
     constexpr int HALVES = NC / 8;                           // groups of eight weight rows
     extern __shared__ __align__(128) uint8_t ls_w[];
     __shared__ float red[LS_WARPS][32];
@@ -136,7 +137,7 @@ int launch(const LinearArgs& a, int* err, cudaStream_t stream) {
         FT_CHECK_CUDA(cudaFuncSetAttribute(linear_stream_kernel<PAIR, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, LS_MAX_BYTES));
         attr.mark();
     }
-    linear_stream_kernel<PAIR, NC><<<dim3((a.N + NC - 1) / NC, a.P), LS_WARPS * 32, (size_t)NC * a.K * 2, stream>>>(a, err);
+    launch_after(linear_stream_kernel<PAIR, NC>, dim3((a.N + NC - 1) / NC, a.P), LS_WARPS * 32, (size_t)NC * a.K * 2, stream, a, err);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -16,6 +16,7 @@ __device__ __forceinline__ float sigmoid_full(float z) { return 1.f / (1.f + exp
 constexpr int PW_WARPS = 4;
 __global__ void __launch_bounds__(PW_WARPS * 32) paged16_write_kernel(WindowArgs a, __nv_bfloat16* __restrict__ q16, __nv_bfloat16* __restrict__ cache,
                                                                       int key_blocks, int v_blocks, int row_floats) {
+    pdl_wait();
     extern __shared__ __align__(16) float pw_rows[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x;
     const int hh = blockIdx.y * PW_WARPS + wid;
@@ -84,6 +85,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32) paged16_write_kernel(WindowArgs
 template <int NV, int NH>
 __global__ void __launch_bounds__(PW_WARPS * 32) paged16_write_rows_kernel(WindowArgs a, __nv_bfloat16* __restrict__ q16,
                                                                            __nv_bfloat16* __restrict__ cache, int key_blocks, int v_blocks) {
+    pdl_wait();
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x;
     const int hh0 = (blockIdx.y * PW_WARPS + wid) * NH, n_heads = a.H + 2 * a.G;
     if (hh0 >= n_heads) return;
@@ -176,6 +178,7 @@ __device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_
 
 template <int VC>
 __global__ void __launch_bounds__(128) paged16_mma_kernel(Paged16Args a, int kp, int vc, int row_groups, int v_groups, int n_split) {
+    pdl_wait();
     const bool apart = a.v_block > 0;
     const int grp = a.H / a.G;
     const int g = blockIdx.z / (row_groups * v_groups), rest = blockIdx.z % (row_groups * v_groups);
@@ -342,6 +345,7 @@ __global__ void __launch_bounds__(128) paged16_mma_kernel(Paged16Args a, int kp,
 
 // The shares of one (token, head) put together: one CTA each.
 __global__ void __launch_bounds__(128) paged16_merge_kernel(Paged16Args a, int n_split) {
+    pdl_wait();
     __shared__ float share[kAttnMaxSplits];                // what a share's sums count in the result
     const int pair = blockIdx.x, n = a.vdim, t = pair / a.H, h = pair % a.H;
     const float* p = a.part + (size_t)pair * n_split * (n + 2);
@@ -392,8 +396,8 @@ int launch_paged16_write(const WindowArgs& a, __nv_bfloat16* q16, void* cache, i
         const dim3 grid(T, (a.H + 2 * a.G + PW_WARPS * nh - 1) / (PW_WARPS * nh));
 #define FT_P16W(NV_)                                                                                                                      \
     do {                                                                                                                                  \
-        if (nh == 2) paged16_write_rows_kernel<NV_, 2><<<grid, PW_WARPS * 32, 0, stream>>>(a, q16, (__nv_bfloat16*)cache, kb, vb);        \
-        else paged16_write_rows_kernel<NV_, 1><<<grid, PW_WARPS * 32, 0, stream>>>(a, q16, (__nv_bfloat16*)cache, kb, vb);                \
+        if (nh == 2) launch_after(paged16_write_rows_kernel<NV_, 2>, grid, PW_WARPS * 32, 0, stream, a, q16, (__nv_bfloat16*)cache, kb, vb);        \
+        else launch_after(paged16_write_rows_kernel<NV_, 1>, grid, PW_WARPS * 32, 0, stream, a, q16, (__nv_bfloat16*)cache, kb, vb);                \
     } while (0)
         if (row <= 128) FT_P16W(1);
         else if (row <= 256) FT_P16W(2);
@@ -405,7 +409,7 @@ int launch_paged16_write(const WindowArgs& a, __nv_bfloat16* q16, void* cache, i
     const size_t smem = (size_t)PW_WARPS * row * 4;
     FT_REQUIRE(smem <= 48 * 1024, "paged bf16 cache: head sizes %d / %d are too large", a.dim, a.vdim);
     const dim3 grid(T, (a.H + 2 * a.G + PW_WARPS - 1) / PW_WARPS);
-    paged16_write_kernel<<<grid, PW_WARPS * 32, smem, stream>>>(a, q16, (__nv_bfloat16*)cache, kb, vb, row);
+    launch_after(paged16_write_kernel, grid, PW_WARPS * 32, smem, stream, a, q16, (__nv_bfloat16*)cache, kb, vb, row);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -415,7 +419,7 @@ bool paged16_mma_ok(const Paged16Args& a) {
 }
 
 int launch_paged16_merge(const Paged16Args& a, int n_pairs, int n_split, cudaStream_t stream) {
-    paged16_merge_kernel<<<n_pairs, 128, 0, stream>>>(a, n_split);
+    launch_after(paged16_merge_kernel, n_pairs, 128, 0, stream, a, n_split);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -438,7 +442,7 @@ int launch_paged16_mma(const Paged16Args& a, int T, cudaStream_t stream) {
             FT_CHECK_CUDA(cudaFuncSetAttribute(paged16_mma_kernel<VC_>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024)); \
             attr.mark();                                                                                                    \
         }                                                                                                                   \
-        paged16_mma_kernel<VC_><<<grid, 128, c.smem, stream>>>(a, c.kp, c.vc, rg, c.v_groups, n_split);                     \
+        launch_after(paged16_mma_kernel<VC_>, grid, 128, c.smem, stream, a, c.kp, c.vc, rg, c.v_groups, n_split);                     \
         break;                                                                                                              \
     }
     switch (c.per) {

@@ -71,6 +71,7 @@ bool paged_tc_cfg(const Paged16Args& a, PagedTcCfg& c) {
 template <int PER_SM>
 __global__ void __launch_bounds__(LT_THREADS, PER_SM)
 paged16_tc_kernel(Paged16Args a, WindowTiles tm, PagedTcCfg cfg, int subs, int* err) {
+    pdl_wait();
     using TM = LtTmem<PER_SM>;
     constexpr int NBUF = TM::NBUF;                                     // score buffers
     extern __shared__ uint8_t smem_raw[];
@@ -443,8 +444,8 @@ int launch_paged16_tc(const Paged16Args& a, const WindowTiles& tm, int* err, cud
     }
     const int subs = (c.span * c.grp + LT_ROWS - 1) / LT_ROWS;
     const dim3 grid(tm.n_tiles * subs * a.G, c.groups);
-    if (c.per_sm == 2) paged16_tc_kernel<2><<<grid, LT_THREADS, c.smem, stream>>>(a, tm, c, subs, err);
-    else paged16_tc_kernel<1><<<grid, LT_THREADS, c.smem, stream>>>(a, tm, c, subs, err);
+    if (c.per_sm == 2) launch_after(paged16_tc_kernel<2>, grid, LT_THREADS, c.smem, stream, a, tm, c, subs, err);
+    else launch_after(paged16_tc_kernel<1>, grid, LT_THREADS, c.smem, stream, a, tm, c, subs, err);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -37,6 +37,7 @@ __device__ __forceinline__ void planes_put(__nv_bfloat16* hi, __nv_bfloat16* lo,
 __global__ void __launch_bounds__(256)
 embed_scale_kernel(const int* __restrict__ tokens, const __nv_bfloat16* __restrict__ embed, float scale, float* __restrict__ x,
                    float* __restrict__ hist, int W) {
+    pdl_wait();
     const int t = blockIdx.x;
     const __nv_bfloat16* e = embed + (size_t)tokens[t] * W;
     for (int c = threadIdx.x; c < W; c += blockDim.x) {
@@ -46,7 +47,7 @@ embed_scale_kernel(const int* __restrict__ tokens, const __nv_bfloat16* __restri
     }
 }
 int launch_embed_scale(const int* tokens, const void* embed, float scale, float* x, float* hist, int T, int W, cudaStream_t stream) {
-    embed_scale_kernel<<<T, 256, 0, stream>>>(tokens, (const __nv_bfloat16*)embed, scale, x, hist, W);
+    launch_after(embed_scale_kernel, T, 256, 0, stream, tokens, (const __nv_bfloat16*)embed, scale, x, hist, W);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -61,6 +62,7 @@ constexpr int kCanonMaxTaps = 17;
 // request are read once for the block (2313 tokens of 2048 columns, one CTA per token: 31 us; now 15 us).
 template <int TB>
 __global__ void __launch_bounds__(256) canon_kernel(CanonArgs a, int T) {
+    pdl_wait();
     const int t0 = blockIdx.x * TB, nt = min(TB, T - t0), W = a.W, taps = a.taps, keep = taps - 1;
     const int c = blockIdx.y * 256 + threadIdx.x;
     if (c >= W) return;
@@ -115,6 +117,7 @@ __global__ void __launch_bounds__(256) canon_kernel(CanonArgs a, int T) {
 // The same for blocks of eight tokens, rows on 16 bytes and four taps: a thread takes four columns, so that a warp asks for 512 bytes of each of
 // eleven rows at once (one column per thread: 14.0 us for 2313 tokens of 2048 columns; now 12.1 us, the bytes take 8.7).
 __global__ void __launch_bounds__(128) canon_rows_kernel(CanonArgs a, int T) {
+    pdl_wait();
     constexpr int TB = 8;
     const int t0 = blockIdx.x * TB, nt = min(TB, T - t0), W = a.W;
     const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
@@ -169,9 +172,9 @@ int launch_canon(const CanonArgs& a, int T, cudaStream_t stream) {
     const int cols = (a.W + 255) / 256;
     const uintptr_t all = (uintptr_t)a.x | (uintptr_t)a.w | (uintptr_t)a.hn | (uintptr_t)a.hi | (uintptr_t)a.lo | (uintptr_t)a.state | (uintptr_t)(a.slot_stride * 4) |
                           (uintptr_t)(a.tail_off * 4);
-    if (T > 64 && a.w && a.taps == 4 && a.W % 4 == 0 && (all & 15) == 0) canon_rows_kernel<<<dim3((T + 7) / 8, (a.W / 4 + 127) / 128), 128, 0, stream>>>(a, T);
-    else if (T > 64) canon_kernel<8><<<dim3((T + 7) / 8, cols), 256, 0, stream>>>(a, T);
-    else canon_kernel<1><<<dim3(T, cols), 256, 0, stream>>>(a, T);
+    if (T > 64 && a.w && a.taps == 4 && a.W % 4 == 0 && (all & 15) == 0) launch_after(canon_rows_kernel, dim3((T + 7) / 8, (a.W / 4 + 127) / 128), 128, 0, stream, a, T);
+    else if (T > 64) launch_after(canon_kernel<8>, dim3((T + 7) / 8, cols), 256, 0, stream, a, T);
+    else launch_after(canon_kernel<1>, dim3(T, cols), 256, 0, stream, a, T);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -192,6 +195,7 @@ __device__ __forceinline__ float post_y(const PostNormArgs& a, size_t i, int c) 
     return y;
 }
 __global__ void __launch_bounds__(256) postnorm_kernel(PostNormArgs a) {
+    pdl_wait();
     __shared__ float red[33];
     extern __shared__ float sm[];
     const int t = blockIdx.x, W = a.W;
@@ -260,6 +264,7 @@ __global__ void __launch_bounds__(256) postnorm_kernel(PostNormArgs a) {
 // sum and the result (one column at a time through shared memory: 41 us for 2313 rows of 2048, the mean of a layer's two joints; now 17 us).
 template <int NV>
 __global__ void __launch_bounds__(256) postnorm_rows_kernel(PostNormArgs a) {
+    pdl_wait();
     __shared__ float red[33];
     const int t = blockIdx.x, n4 = a.W >> 2;
     int r = 0, pos0 = 0, n = 1;
@@ -326,12 +331,12 @@ int launch_postnorm(const PostNormArgs& a, int T, cudaStream_t stream) {
     const uintptr_t all = (uintptr_t)a.x | (uintptr_t)a.x_out | (uintptr_t)a.y0 | (uintptr_t)a.y1 | (uintptr_t)a.b0 | (uintptr_t)a.b1 | (uintptr_t)a.post_w |
                           (uintptr_t)a.hist | (a.save_off >= 0 ? (uintptr_t)a.state | (uintptr_t)(a.slot_stride * 4) | (uintptr_t)(a.save_off * 4) : 0);
     if (!a.cw && a.W % 4 == 0 && a.W <= 8192 && (all & 15) == 0) {
-        if (a.W <= 1024) postnorm_rows_kernel<1><<<T, 256, 0, stream>>>(a);
-        else if (a.W <= 2048) postnorm_rows_kernel<2><<<T, 256, 0, stream>>>(a);
-        else if (a.W <= 4096) postnorm_rows_kernel<4><<<T, 256, 0, stream>>>(a);
-        else postnorm_rows_kernel<8><<<T, 256, 0, stream>>>(a);
+        if (a.W <= 1024) launch_after(postnorm_rows_kernel<1>, T, 256, 0, stream, a);
+        else if (a.W <= 2048) launch_after(postnorm_rows_kernel<2>, T, 256, 0, stream, a);
+        else if (a.W <= 4096) launch_after(postnorm_rows_kernel<4>, T, 256, 0, stream, a);
+        else launch_after(postnorm_rows_kernel<8>, T, 256, 0, stream, a);
     } else {
-        postnorm_kernel<<<T, 256, (size_t)a.W * 8, stream>>>(a);
+        launch_after(postnorm_kernel, T, 256, (size_t)a.W * 8, stream, a);
     }
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
@@ -341,6 +346,7 @@ int launch_postnorm(const PostNormArgs& a, int T, cudaStream_t stream) {
 __global__ void __launch_bounds__(256)
 rms_rows_kernel(const float* __restrict__ x, const int* __restrict__ rows, const float* __restrict__ w, float gain,
                 float* __restrict__ out, int W, float eps) {
+    pdl_wait();
     __shared__ float red[33];
     const float* src = x + (size_t)(rows ? rows[blockIdx.x] : blockIdx.x) * W;
     float ss = 0.f;
@@ -351,7 +357,7 @@ rms_rows_kernel(const float* __restrict__ x, const int* __restrict__ rows, const
 }
 int launch_rms_rows(const float* x, const int* rows, const float* w, float gain, float* out, int n, int W, float eps,
                     cudaStream_t stream) {
-    rms_rows_kernel<<<n, 256, 0, stream>>>(x, rows, w, gain, out, W, eps);
+    launch_after(rms_rows_kernel, n, 256, 0, stream, x, rows, w, gain, out, W, eps);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -359,6 +365,7 @@ int launch_rms_rows(const float* x, const int* rows, const float* w, float gain,
 __global__ void __launch_bounds__(128)
 rms_cols_kernel(const float* __restrict__ src, int lds, int src_off, const float* __restrict__ w, float* __restrict__ dst, int ldd,
                 int dst_off, int n, float eps) {
+    pdl_wait();
     __shared__ float red[33];
     const float* s = src + (size_t)blockIdx.x * lds + src_off;
     float* d = dst + (size_t)blockIdx.x * ldd + dst_off;
@@ -370,7 +377,7 @@ rms_cols_kernel(const float* __restrict__ src, int lds, int src_off, const float
 }
 int launch_rms_cols(const float* src, int lds, int src_off, const float* w, float* dst, int ldd, int dst_off, int n, float eps,
                     int T, cudaStream_t stream) {
-    rms_cols_kernel<<<T, 128, 0, stream>>>(src, lds, src_off, w, dst, ldd, dst_off, n, eps);
+    launch_after(rms_cols_kernel, T, 128, 0, stream, src, lds, src_off, w, dst, ldd, dst_off, n, eps);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -381,6 +388,7 @@ int launch_rms_cols(const float* src, int lds, int src_off, const float* w, floa
 __global__ void __launch_bounds__(128)
 latent_stage_kernel(const float* __restrict__ q, int heads, int dim, int rot, const float* __restrict__ proj, int ldp, int o_k,
                     int rank, const float* __restrict__ w, float eps, float* __restrict__ stage, int lds) {
+    pdl_wait();
     __shared__ float red[33];
     const int t = blockIdx.x, kd = rot + rank;
     float* st = stage + (size_t)t * lds;
@@ -403,7 +411,7 @@ latent_stage_kernel(const float* __restrict__ q, int heads, int dim, int rot, co
 }
 int launch_latent_stage(const float* q, int heads, int dim, int rot, const float* proj, int ldp, int o_k, int rank, const float* w,
                         float eps, float* stage, int lds, int T, cudaStream_t stream) {
-    latent_stage_kernel<<<T, 128, 0, stream>>>(q, heads, dim, rot, proj, ldp, o_k, rank, w, eps, stage, lds);
+    launch_after(latent_stage_kernel, T, 128, 0, stream, q, heads, dim, rot, proj, ldp, o_k, rank, w, eps, stage, lds);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -28,6 +28,7 @@ __device__ __forceinline__ void add_embedding(float (&x)[V], const PreNormArgs& 
 
 template <int V>
 __global__ void __launch_bounds__(256) prenorm_joint_kernel(PreNormArgs a) {
+    pdl_wait();
     __shared__ float red[33];
     extern __shared__ __align__(16) float row[];          // [W]: the new row of the stream
     const int t = blockIdx.x, W = a.W;
@@ -112,8 +113,8 @@ int launch_prenorm_joint(const PreNormArgs& a, int T, cudaStream_t stream) {
             attr.mark();
         }
     }
-    if (v4) prenorm_joint_kernel<4><<<T, 256, smem, stream>>>(a);
-    else prenorm_joint_kernel<1><<<T, 256, smem, stream>>>(a);
+    if (v4) launch_after(prenorm_joint_kernel<4>, T, 256, smem, stream, a);
+    else launch_after(prenorm_joint_kernel<1>, T, 256, smem, stream, a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

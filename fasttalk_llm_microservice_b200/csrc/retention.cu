@@ -49,6 +49,7 @@ __device__ __forceinline__ float turned(const float* __restrict__ x, int c, int 
 // ------------------------------------------------------------------ one token per request
 template <int CV>
 __global__ void __launch_bounds__(RT_THREADS) retention_step_kernel(RetentionArgs a) {
+    pdl_wait();
     extern __shared__ __align__(16) float rs_smem[];
     const int D = a.dim, V = a.vdim, h = blockIdx.x, r = blockIdx.y, t = a.req_start[r], tid = threadIdx.x;
     float* sq = rs_smem;                                 // [D]
@@ -136,6 +137,7 @@ __global__ void __launch_bounds__(RT_THREADS) retention_step_kernel(RetentionArg
 // ------------------------------------------------------------------ portions: bf16 rows
 // q16, k16 [row][heads][Dp], v16 [row][heads][Vp] of the step's rows from `row0` on (row index counted from there)
 __global__ void __launch_bounds__(256) retention_pack_kernel(RetentionArgs a, int row0, int Dp, int Vp) {
+    pdl_wait();
     extern __shared__ float trig[];
     const int t = row0 + blockIdx.x, H = a.heads, D = a.dim, V = a.vdim, half = a.rot_dims >> 1;
     const float* pr = a.proj + (size_t)t * a.ldp;
@@ -252,6 +254,7 @@ __device__ __forceinline__ void tile_out(float* tile, int ld, uint32_t tmem, int
 // ------------------------------------------------------------------ what a run adds to the state
 // D[d][v] (TMEM, M = 128 key channels, N = up to 128 value columns) = Kd^T V over the run's tokens; both operands MN-major.
 __global__ void __launch_bounds__(RT_THREADS) retention_gain_kernel(RetentionArgs a, WindowTiles tm, int Dp, int Vp, int* err) {
+    pdl_wait();
     extern __shared__ uint8_t rg_raw[];
     __shared__ float pw[RT_RUN];
     __shared__ uint64_t done;
@@ -351,6 +354,7 @@ __global__ void __launch_bounds__(RT_THREADS) retention_gain_kernel(RetentionArg
 // ws of a run: what it adds -> what it starts from.  CV numbers per thread.
 template <int CV>
 __global__ void __launch_bounds__(256) retention_carry_kernel(RetentionArgs a, WindowTiles tm, int first_req) {
+    pdl_wait();
     const int j = blockIdx.z, h = blockIdx.y, e = (blockIdx.x * blockDim.x + threadIdx.x) * CV, DV = a.dim * a.vdim;
     if (e >= DV) return;
     const int len = tm.req_q_start[j + 1] - tm.req_q_start[j], n_runs = (len + RT_RUN - 1) / RT_RUN;
@@ -389,6 +393,7 @@ __global__ void __launch_bounds__(256) retention_carry_kernel(RetentionArgs a, W
 // its lo plane that of v once the run's part is.
 constexpr int RT_COL_S = 0, RT_COL_PH = 0, RT_COL_PL = 64, RT_COL_O1 = 0, RT_COL_O2 = 128;
 __global__ void __launch_bounds__(RT_THREADS, 2) retention_runs_kernel(RetentionArgs a, WindowTiles tm, int Dp, int Vp, int raw, int first_req, int* err) {
+    pdl_wait();
     extern __shared__ uint8_t rr_raw[];
     __shared__ float pw[RT_RUN + 1];
     __shared__ uint64_t done[3];
@@ -666,8 +671,8 @@ int launch_retention_step(const RetentionArgs& a, int n_req, cudaStream_t stream
     const size_t smem = (size_t)(((2 * a.dim + a.rot_dims + 33 + 3) & ~3) + 2 * ((a.vdim + 3) & ~3) + RT_THREADS * cv) * 4;
     FT_REQUIRE(smem <= 48 * 1024, "retention step: head sizes %d / %d are too large", a.dim, a.vdim);
     const dim3 grid(a.heads, n_req);
-    if (v4) retention_step_kernel<4><<<grid, RT_THREADS, smem, stream>>>(a);
-    else retention_step_kernel<1><<<grid, RT_THREADS, smem, stream>>>(a);
+    if (v4) launch_after(retention_step_kernel<4>, grid, RT_THREADS, smem, stream, a);
+    else launch_after(retention_step_kernel<1>, grid, RT_THREADS, smem, stream, a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
@@ -681,17 +686,17 @@ int launch_retention_tc(const RetentionArgs& a, const WindowTiles& tm, int first
         FT_CHECK_CUDA(cudaFuncSetAttribute(retention_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
         attr.mark();
     }
-    retention_pack_kernel<<<rows, 256, (size_t)a.rot_dims * 4, stream>>>(a, row0, Dp, Vp);
+    launch_after(retention_pack_kernel, rows, 256, (size_t)a.rot_dims * 4, stream, a, row0, Dp, Vp);
     FT_CHECK_CUDA(cudaGetLastError());
     const dim3 grid(tm.n_tiles, a.heads, groups);
-    retention_gain_kernel<<<grid, RT_THREADS, RT_GAIN_SMEM, stream>>>(a, tm, Dp, Vp, err);
+    launch_after(retention_gain_kernel, grid, RT_THREADS, RT_GAIN_SMEM, stream, a, tm, Dp, Vp, err);
     FT_CHECK_CUDA(cudaGetLastError());
     const int dv = a.dim * a.vdim;
     const bool v4 = a.vdim % 4 == 0 && a.slot_stride % 4 == 0 && a.s_off % 4 == 0 && ((uintptr_t)a.state & 15) == 0;
-    if (v4) retention_carry_kernel<4><<<dim3((dv / 4 + 255) / 256, a.heads, portions), 256, 0, stream>>>(a, tm, first_req);
-    else retention_carry_kernel<1><<<dim3((dv + 255) / 256, a.heads, portions), 256, 0, stream>>>(a, tm, first_req);
+    if (v4) launch_after(retention_carry_kernel<4>, dim3((dv / 4 + 255) / 256, a.heads, portions), 256, 0, stream, a, tm, first_req);
+    else launch_after(retention_carry_kernel<1>, dim3((dv + 255) / 256, a.heads, portions), 256, 0, stream, a, tm, first_req);
     FT_CHECK_CUDA(cudaGetLastError());
-    retention_runs_kernel<<<grid, RT_THREADS, runs_smem(a.dim, a.vdim), stream>>>(a, tm, Dp, Vp, !retention_one_pass(a.vdim), first_req, err);
+    launch_after(retention_runs_kernel, grid, RT_THREADS, runs_smem(a.dim, a.vdim), stream, a, tm, Dp, Vp, !retention_one_pass(a.vdim), first_req, err);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -19,6 +19,7 @@ __device__ __forceinline__ void put_row(float* f32, void* hi, void* lo, size_t a
 
 template <int V>
 __global__ void __launch_bounds__(256) sandwich_joint_kernel(SandwichArgs a) {
+    pdl_wait();
     __shared__ float red[33];
     extern __shared__ __align__(16) float row[];          // [W]: the sublayer's result, then the new row of the stream
     const int t = blockIdx.x, W = a.W;
@@ -98,6 +99,7 @@ __global__ void __launch_bounds__(256) sandwich_joint_kernel(SandwichArgs a) {
 // The same with a row's numbers in registers, N passes of them: every load is on the way before the first sum, two barriers in all.
 template <int N>
 __global__ void __launch_bounds__(256) sandwich_joint_regs_kernel(SandwichArgs a) {
+    pdl_wait();
     __shared__ float red[2][8];
     const int t = blockIdx.x, W = a.W, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool sub = a.y0 || a.y1 || a.top > 0;
@@ -209,11 +211,11 @@ int launch_sandwich_joint(const SandwichArgs& a, int T, cudaStream_t stream) {
     // 16: 15.2 / 12.2, 296: 16.3 / 13.2; 2048 columns 20.2 / 16.3, 22.9 / 18.4; 4096 columns 28.3 / 22.4, 32.7 / 27.7: ahead at every size up to two rows per SM.  Many rows want
     // the other kernel's occupancy (2313 rows of 2048: 16.2 us, in registers 18.4); between the two nothing was measured.
     const bool regs = v4 && T <= 2 * device_sms();
-    if (regs && a.W <= 1024) sandwich_joint_regs_kernel<1><<<T, 256, 0, stream>>>(a);
-    else if (regs && a.W <= 2048) sandwich_joint_regs_kernel<2><<<T, 256, 0, stream>>>(a);
-    else if (regs && a.W <= 4096) sandwich_joint_regs_kernel<4><<<T, 256, 0, stream>>>(a);
-    else if (v4) sandwich_joint_kernel<4><<<T, 256, smem, stream>>>(a);
-    else sandwich_joint_kernel<1><<<T, 256, smem, stream>>>(a);
+    if (regs && a.W <= 1024) launch_after(sandwich_joint_regs_kernel<1>, T, 256, 0, stream, a);
+    else if (regs && a.W <= 2048) launch_after(sandwich_joint_regs_kernel<2>, T, 256, 0, stream, a);
+    else if (regs && a.W <= 4096) launch_after(sandwich_joint_regs_kernel<4>, T, 256, 0, stream, a);
+    else if (v4) launch_after(sandwich_joint_kernel<4>, T, 256, smem, stream, a);
+    else launch_after(sandwich_joint_kernel<1>, T, 256, smem, stream, a);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

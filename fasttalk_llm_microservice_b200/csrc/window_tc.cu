@@ -98,6 +98,7 @@ __device__ __noinline__ void window_row(const WindowArgs& a, const int* pt, int 
 
 template <int DB, int VB>
 __global__ void __launch_bounds__(WR_THREADS, 1) window_runs_kernel(WindowArgs a, WindowTiles tm, int QT, int subs) {
+    pdl_wait();
     extern __shared__ uint8_t wr_raw[];
     __shared__ float part_max[4][WR_ROWS], part_sum[4][WR_ROWS];
     __shared__ uint64_t done[2];                         // scores, sums
@@ -409,7 +410,7 @@ int launch_runs(const WindowArgs& a, const WindowTiles& tm, cudaStream_t stream)
         attr.mark();
     }
     const int QT = std::min(64, WR_ROWS / (a.H / a.G)), subs = (64 + QT - 1) / QT;
-    window_runs_kernel<DB, VB><<<dim3(tm.n_tiles * subs, a.G), WR_THREADS, window_smem<DB, VB>(), stream>>>(a, tm, QT, subs);
+    launch_after(window_runs_kernel<DB, VB>, dim3(tm.n_tiles * subs, a.G), WR_THREADS, window_smem<DB, VB>(), stream, a, tm, QT, subs);
     FT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }
