@@ -124,7 +124,8 @@ __device__ __forceinline__ void attn_trace(int slot) {
     }
 }
 
-template <int D>
+// EACH: the grid has a CTA for every (sequence, head).  A kernel of its own, so that the larger batches pay nothing for the choice below.
+template <int D, bool EACH>
 __global__ void __launch_bounds__(ATTN_THREADS)
 attn_decode_kernel(const __half* __restrict__ q, const uint8_t* __restrict__ kv_layer,
                    const int* __restrict__ page_table, int max_pages, const int* __restrict__ ctx_lens,
@@ -137,7 +138,7 @@ attn_decode_kernel(const __half* __restrict__ q, const uint8_t* __restrict__ kv_
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + (size_t)C::STAGES * C::TILE_BYTES);
     uint64_t* empty_bar = full_bar + C::STAGES;
     float* merge_buf = reinterpret_cast<float*>(empty_bar + C::STAGES);
-    __shared__ int s_last, s_most;
+    __shared__ int s_last;
     __shared__ int s_prefix[ATTN_MAX_B_SMEM + 1];     // tile plan, searched many times per CTA
     // `early` (engine, layers >= 1): the producer may start streaming KV tiles BEFORE the
     // programmatic-dependency wait, because everything it reads then — the tile plan, the page
@@ -168,19 +169,16 @@ attn_decode_kernel(const __half* __restrict__ q, const uint8_t* __restrict__ kv_
     }
     // one coalesced read of the tile plan instead of a dependent global load per search step
     // (the start-up chain was 3.3 us of idle HBM per launch)
-    const bool one_each = B * nkv <= (int)gridDim.x;      // a CTA for every (sequence, head)
-    if (one_each) {
-        // 31 sequences a warp, the next one's place from the lane behind: the longest sequence too
-        if (threadIdx.x == 0) s_most = 0;
-        __syncthreads();
-        int most = 0;
-        for (int i0 = warp * 31; i0 < B; i0 += 31 * (ATTN_THREADS / 32)) {
-            const int i = min(i0 + lane, B), at = tile_prefix[i], next = __shfl_down_sync(0xffffffffu, at, 1);
-            if (B <= ATTN_MAX_B_SMEM) s_prefix[i] = at;
-            if (lane < 31) most = max(most, next - at);
+    int most = 0;                                         // tiles of the longest sequence
+    if constexpr (EACH) {
+        // every warp for itself, 64 sequences at a time so that the loads of a pass are in flight together
+        for (int i = lane; i < B + lane; i += 64) {
+            const int i1 = min(i + 1, B), i2 = min(i + 32, B), i3 = min(i + 33, B), i0 = min(i, B);
+            const int a0 = tile_prefix[i0], a1 = tile_prefix[i1], a2 = tile_prefix[i2], a3 = tile_prefix[i3];
+            most = max(most, max(a1 - a0, a3 - a2));
+            if (warp == 0 && B <= ATTN_MAX_B_SMEM) s_prefix[i0] = a0, s_prefix[i2] = a2, s_prefix[i3] = a3;
         }
         most = __reduce_max_sync(0xffffffffu, most);
-        if (lane == 0 && most > 0) atomicMax(&s_most, most);
     } else if (B <= ATTN_MAX_B_SMEM) {
         for (int i = threadIdx.x; i <= B; i += ATTN_THREADS) s_prefix[i] = tile_prefix[i];
     }
@@ -208,9 +206,10 @@ attn_decode_kernel(const __half* __restrict__ q, const uint8_t* __restrict__ kv_
     long long f_end = f + per < total ? f + per : total;
     // A CTA takes all of a (sequence, head) where there is one for each and that makes its walk longer by no more tiles than the merge of the parts costs
     // (0.53 us a tile; the merge 2.5 to 4.5 us at head_dim 64, up to 6 at 128, by how the shares lie).  One call, plan included, us, by shares -> whole: head_dim 64,
-    // 4 sessions x 8 heads of 128 keys 7.5 -> 5.6, of 384 8.6 -> 7.8, of 512 8.7 and 8.8; 32 sessions of 512 14.0 -> 10.5; head_dim 128, 8 sessions
-    // of 320 12.8 -> 8.0, 4 of 512 9.6 -> 9.4, of 768 10.1 and 11.5.
-    if (one_each && s_most - (int)per <= (D == 64 ? (per == 1 ? 5 : 4) : 7)) {
+    // 4 sessions x 8 heads of 256 keys 7.3 -> 5.9, of 512 8.5 -> 8.4; 16 of 512 9.5 -> 8.6; 37 of 1024 15.3 -> 13.9; head_dim 128, 8 sessions
+    // of 256 9.5 -> 7.6, one of 512 9.2 -> 8.8; 16 of 1024 18.8 -> 13.8, of 2048 28.8 -> 24.4.  Longer walks stay in shares: 4 of 512 (24 query heads) 8.8 by shares, 9.2 whole.
+    const bool whole_each = EACH && most - (int)per <= (D == 64 ? (per == 1 ? 5 : 4) : (per == 1 ? 7 : 5));
+    if (whole_each) {
         const int b = blockIdx.x / nkv;
         f = f_end = total;
         if (b < B) {
@@ -280,8 +279,34 @@ attn_decode_kernel(const __half* __restrict__ q, const uint8_t* __restrict__ kv_
 #pragma unroll
         for (int nt = 0; nt < D / 8; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.f;
         float m_run = -INFINITY, l_run = 0.f;
+        // A walk that takes a sequence whole starts its running maximum again half a share and adds those parts up in fp32 here: its probabilities then
+        // round no more than those of the shares that it stands for.  (One running maximum for the whole walk: 5 to 10 % more error against 64 bits, 9.7e-5 -> 1.05e-4.)
+        float o_all[EACH ? D / 8 : 1][2] = {}, m_all = -INFINITY, l_all = 0.f;
+        auto add_part = [&]() {
+            const float m = fmaxf(m_all, m_run), m_use = m == -INFINITY ? 0.f : m;
+            const float wa = exp2f(m_all - m_use), wr = exp2f(m_run - m_use);
+            l_all = fmaf(l_run, wr, l_all * wa);
+#pragma unroll
+            for (int nt = 0; nt < (EACH ? D / 8 : 0); ++nt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    o_all[nt][e] = fmaf(o[nt][e], wr, o_all[nt][e] * wa);
+                    o[nt][e] = 0.f;
+                }
+            m_all = m;
+            m_run = -INFINITY;
+            l_run = 0.f;
+        };
+        const int part_tiles = whole_each ? (int)(per + 1) / 2 : INT_MAX;
+        int part_left = part_tiles;
 
         for (int tile = seg.tile_begin; tile < seg.tile_end; ++tile) {
+            if constexpr (EACH) {
+                if (part_left-- == 0) {
+                    add_part();
+                    part_left = part_tiles - 1;
+                }
+            }
             mbar_wait(&full_bar[stage], phase);
             if (threadIdx.x == 0 && blockIdx.x < ATTN_TRACE_CTAS && g_attn_trace[blockIdx.x * 4 + 1] == 0) attn_trace(1);
             const uint32_t kbase = smem_u32(smem + (size_t)stage * C::TILE_BYTES);
@@ -345,6 +370,16 @@ attn_decode_kernel(const __half* __restrict__ q, const uint8_t* __restrict__ kv_
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty_bar[stage]);
             if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
+        }
+
+        if constexpr (EACH) {
+            if (seg.tile_end - seg.tile_begin > part_tiles) {
+                add_part();
+#pragma unroll
+                for (int nt = 0; nt < D / 8; ++nt) o[nt][0] = o_all[nt][0], o[nt][1] = o_all[nt][1];
+                m_run = m_all;
+                l_run = l_all;
+            }
         }
 
         if (threadIdx.x == 0) attn_trace(2);
@@ -643,10 +678,10 @@ size_t attn_decode_scratch_floats(int B, int nkv, int group, int d, int n_ctas) 
 template <int D>
 static int decode_ctas_per_sm_d() {
     using C = AttnCfg<D>;
-    FT_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    FT_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)C::SMEM));
     int n = 0;
-    FT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_kernel<D>, ATTN_THREADS,
+    FT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_kernel<D, false>, ATTN_THREADS,
                                                                 C::SMEM));
     return n;
 }
@@ -688,7 +723,9 @@ static int launch_attn_decode_d(const void* q, const void* kv_layer, const int* 
     using C = AttnCfg<D>;
     static PerDeviceFlag attr_set;
     if (!attr_set.done()) {
-        FT_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        FT_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)C::SMEM));
+        FT_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)C::SMEM));
         attr_set.mark();
     }
@@ -697,7 +734,7 @@ static int launch_attn_decode_d(const void* q, const void* kv_layer, const int* 
     cudaLaunchAttribute attr[1];
     fill_cfg(cfg, attr, dim3(n_ctas), dim3(ATTN_THREADS), C::SMEM, pdl && !ev0, stream);
     if (ev0) FT_CHECK_CUDA(cudaEventRecord(ev0, stream));
-    FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_decode_kernel<D>, (const __half*)q,
+    FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, B * nkv <= n_ctas ? attn_decode_kernel<D, true> : attn_decode_kernel<D, false>, (const __half*)q,
                                      (const uint8_t*)kv_layer, page_table, max_pages, ctx_lens, tile_prefix,
                                      (__nv_bfloat16*)out, (__nv_bfloat16*)out_lo, reinterpret_cast<int*>(scratch),
                                      scratch + counter_floats(B, nkv), B, nq, nkv, scale_log2,

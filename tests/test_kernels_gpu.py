@@ -441,6 +441,38 @@ def test_attn_decode(K, nq, nkv, d, ctx_lens, n_ctas):
     assert torch.equal(again, out)
 
 
+@pytest.mark.parametrize("nq,nkv,d", [(4, 1, 64), (32, 8, 64), (6, 2, 128), (32, 8, 128)])
+@pytest.mark.parametrize("ctx_lens", [[64 * 5], [64 * 6 + 1], [64 * 8 - 1, 64 * 8 + 1], [1, 64, 65, 0, 300], [64 * 7, 0, 0, 64 * 7 + 5], [700, 10], [33] * 18, [200, 450, 130] * 6,
+                                      [64 * 2 + 7 * i for i in range(40)], [5 * i for i in range(70)]])
+def test_attn_decode_whole_sequences_and_shares(K, nq, nkv, d, ctx_lens):
+    """Around the length at which a CTA takes all of a (sequence, head): one tile more than that, ragged and empty sequences beside long ones, more (sequence, head)s than
+    CTAs, and few CTAs, which then share what one each would take whole."""
+    g = torch.Generator(device=DEV).manual_seed(sum(ctx_lens) + nq + d)
+    kv, pt, ks, vs = build_paged_kv(K, [max(1, c) for c in ctx_lens], nkv, d, g)
+    q = torch.randn(len(ctx_lens), nq, d, device=DEV, generator=g).half()
+    ctx = torch.tensor(ctx_lens, device=DEV, dtype=torch.int32)
+    for n_ctas in (0, 7):
+        out = hilo(*K.attn_decode(q, kv, pt, ctx, n_ctas=n_ctas))
+        for b, n in enumerate(ctx_lens):
+            ref = O.attention(q[b:b + 1].float(), ks[b].float(), vs[b].float(), n - 1) if n else torch.zeros_like(out[b:b + 1])
+            assert (rel_err(out[b:b + 1], ref) < 2e-3) if n else out[b].abs().max().item() == 0, (n_ctas, b)
+
+
+@pytest.mark.parametrize("n_out,Kd", [(256, 64), (384, 1024), (2048, 4096), (1024, 4160)])
+@pytest.mark.parametrize("T", [1, 3, 16, 17, 47, 48, 49, 64, 65])
+def test_gemm_few_tokens_as_one_result_or_parts(K, n_out, Kd, T):
+    """Both planes, the count of parts left to the library: one result up to 48 tokens, or 64 of not too long a K; rows that the CTAs of a cluster add four at a time."""
+    g = torch.Generator(device=DEV).manual_seed(n_out + T + Kd)
+    w = (torch.randn(n_out, Kd, device=DEV, generator=g) * 0.05).bfloat16()
+    xf = torch.randn(T, Kd, device=DEV, generator=g)
+    x, x_lo = K.split_hi_lo(xf)
+    part = K.gemm_bf16(w, x, x_lo)
+    if T <= 48 or (T <= 64 and Kd <= 4096):
+        assert part.shape == (1, T, n_out)
+    # the planes' own numbers: what is left are 32-bit sums, a unit of the last place (of a partial sum, cut off) for every 16 columns of K
+    assert rel_err(part.sum(0), hilo(x, x_lo).double() @ w.double().T) < 1e-6 + Kd / 16 * 2.0 ** -23
+
+
 def test_attn_decode_cfg2_shape(K):
     """BASELINE config 2 shape: 64 sequences x 2048 context, Llama-3.2-1B heads.  Checked by a
     size-independent property as well: softmax weights sum to 1, so with V == const the
