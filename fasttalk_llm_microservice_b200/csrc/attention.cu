@@ -20,6 +20,7 @@
 #include "ft_internal.h"
 
 #include <mutex>
+#include <new>
 
 namespace ft {
 
@@ -831,6 +832,17 @@ extern "C" int ft_attn_decode(const void* q, const void* kv_layer, const int* pa
     if (int r = ft::launch_attn_decode_plan(ctx_lens, tile_prefix, B, nkv, scratch, false, st)) return r;
     return ft::launch_attn_decode(q, kv_layer, page_table, max_pages, ctx_lens, tile_prefix, out, out_lo,
                                   scratch, B, nq, nkv, d, n_ctas, true, st, nullptr, nullptr, false);      // its start runs beside the plan
+}
+
+extern "C" int ft_attn_prefill_order_tiles(const int* req_q_start, const int* req_pos0, int* tile_req, int* tile_q0, int n_tiles, int nq, int nkv,
+                                           int d, int q_rows) {
+    FT_REQUIRE(n_tiles >= 0 && (n_tiles == 0 || (req_q_start && req_pos0 && tile_req && tile_q0)), "ft_attn_prefill_order_tiles: bad arguments");
+    try {
+        ft::order_query_tiles(req_q_start, req_pos0, tile_req, tile_q0, n_tiles, nq, nkv, d, q_rows);
+    } catch (const std::bad_alloc&) {
+        FT_REQUIRE(false, "ft_attn_prefill_order_tiles: out of host memory (%d tiles)", n_tiles);
+    }
+    return 0;
 }
 
 extern "C" int ft_attn_prefill(const void* q, const void* kv_layer, const int* page_table, int max_pages,

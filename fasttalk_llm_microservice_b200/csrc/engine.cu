@@ -7,7 +7,6 @@
 #include "../../include/fasttalk_b200.h"
 
 #include <algorithm>
-#include <array>
 #include <chrono>
 #include <condition_variable>
 #include <deque>
@@ -1445,19 +1444,8 @@ static long long fill_batch(Engine* e, const std::vector<Portion>& dec, const st
             h[m.o_tq0 + tiles] = q0;
         }
     }
-    if (!e->lay && b.n_prefill_req > 1) {
-        // the attention kernel takes the list back to front: the tiles that take longest come last (up to 32 tokens: half as long)
-        std::vector<std::array<int, 3>> order(tiles);
-        for (int i = 0; i < tiles; ++i) {
-            const int j = h[m.o_treq + i], q0 = h[m.o_tq0 + i];
-            order[i] = {(pre[j].pos0 + q0 + 64) * (pre[j].n - q0 > 32 ? 2 : 1), j, q0};
-        }
-        std::sort(order.begin(), order.end());
-        for (int i = 0; i < tiles; ++i) {
-            h[m.o_treq + i] = order[i][1];
-            h[m.o_tq0 + i] = order[i][2];
-        }
-    }
+    if (!e->lay)
+        order_query_tiles(h + m.o_qstart, h + m.o_rpos0, h + m.o_treq, h + m.o_tq0, tiles, e->cfg.n_q_heads, e->cfg.n_kv_heads, e->cfg.head_dim, e->t_max);
     h[m.o_xstart + b.n_req] = row;
     b.T = row;
     b.n_tiles = tiles;

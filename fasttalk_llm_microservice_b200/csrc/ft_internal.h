@@ -85,6 +85,9 @@ int launch_attn_prefill(const void* q, const void* kv_layer, const int* page_tab
                         const int* tile_req, const int* tile_q0, int n_tiles, void* out, void* out_lo, int nq,
                         int nkv, int d, bool pdl, cudaStream_t stream, int q_rows = 0);
 
+// Puts a list of query tiles (host arrays) in the order that the kernel for these sizes wants: attention_tc.cu
+void order_query_tiles(const int* q_start, const int* pos0, int* tile_req, int* tile_q0, int n_tiles, int nq, int nkv, int d, int q_rows);
+
 // ---- attention_tc.cu (tcgen05 / TMEM prefill attention: head_dim 64 / 128, GQA group 3 / 4)
 bool attn_prefill_tc_supported(int nq, int nkv, int d);
 int launch_attn_prefill_tc(const void* q, int q_rows, const void* kv_layer, const int* page_table, int max_pages,

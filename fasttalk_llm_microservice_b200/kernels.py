@@ -195,15 +195,15 @@ def attn_prefill(q: torch.Tensor, kv_layer: torch.Tensor, page_table: torch.Tens
     for r in range(len(req_slot)):
         for q0 in range(0, req_q_start[r + 1] - req_q_start[r], 64):
             tile_req.append(r); tile_q0.append(q0)
-    if len(req_slot) > 1 and len(tile_req) * nkv > 128:      # more CTAs than run at once: the kernel takes the list back to front,
-        seen = [int(p) for p in req_pos0]                    # so the tiles that take longest come last (up to 32 tokens: half as long)
-        ends = [int(req_q_start[r + 1] - req_q_start[r]) for r in range(len(req_slot))]
-        order = sorted(range(len(tile_req)), key=lambda i: (seen[tile_req[i]] + tile_q0[i] + 64) * (1 + (ends[tile_req[i]] - tile_q0[i] > 32)))
-        tile_req, tile_q0 = [tile_req[i] for i in order], [tile_q0[i] for i in order]
     # The lists go up in one copy that the host does not wait for (five waiting ones cost 60 us of GPU time between calls).  While a
     # stream is captured the copy is an ordinary one, which capture refuses: a replay would read memory that is no longer this call's.
     i32 = lambda v: torch.tensor(v, device="cpu", dtype=torch.int32).reshape(-1)
     parts = [i32(v) for v in (req_q_start, req_slot, req_pos0, tile_req, tile_q0)]
+    assert parts[2].numel() >= len(req_slot), "req_pos0: a position for every request"
+    rows = T if tensor_cores else 0
+    lib = N.load()
+    N.check(lib.ft_attn_prefill_order_tiles(N.ptr(parts[0]), N.ptr(parts[2]), N.ptr(parts[3]), N.ptr(parts[4]), len(tile_req), nq, nkv, d, rows),
+            "ft_attn_prefill_order_tiles")
     lists = torch.cat(parts)
     waits = dev.index != torch.cuda.current_device() or torch.cuda.is_current_stream_capturing()
     lists = lists.to(dev) if waits else lists.pin_memory().to(dev, non_blocking=True)
@@ -213,10 +213,9 @@ def attn_prefill(q: torch.Tensor, kv_layer: torch.Tensor, page_table: torch.Tens
     owned = bool(starts) and starts[0] == 0 and starts[-1] == T and all(x <= y for x, y in zip(starts, starts[1:]))
     out = (torch.empty if owned else torch.zeros)(T, nq * d, device=dev, dtype=torch.bfloat16)
     out_lo = torch.empty_like(out) if owned else torch.zeros_like(out)
-    N.check(N.load().ft_attn_prefill(N.ptr(q), N.ptr(kv_layer), N.ptr(page_table), page_table.shape[1],
-                                     N.ptr(t_qs), N.ptr(t_slot), N.ptr(t_pos0), N.ptr(t_treq), N.ptr(t_tq0),
-                                     len(tile_req), N.ptr(out), N.ptr(out_lo), nq, nkv, d, T if tensor_cores else 0,
-                                     N.cur_stream()),
+    N.check(lib.ft_attn_prefill(N.ptr(q), N.ptr(kv_layer), N.ptr(page_table), page_table.shape[1],
+                                N.ptr(t_qs), N.ptr(t_slot), N.ptr(t_pos0), N.ptr(t_treq), N.ptr(t_tq0),
+                                len(tile_req), N.ptr(out), N.ptr(out_lo), nq, nkv, d, rows, N.cur_stream()),
             "ft_attn_prefill")
     return out, out_lo
 

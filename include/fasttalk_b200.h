@@ -638,7 +638,13 @@ int ft_attn_decode_noalloc(const void* q, const void* kv_layer, const int* page_
  * q_rows = number of rows (tokens) the q and out buffers hold.  With a GQA group of 3 or 4 (Llama-3.2-1B / 3B,
  * Llama-3.1-8B), head_dim 64 or 128 and q_rows > 0 this runs on tcgen05 / TMEM (one CTA per 64 queries x KV head, S, P
  * and O in tensor memory, K/V slabs consumed as UMMA operands exactly as they lie in the cache); other shapes, or
- * q_rows <= 0, run the mma.sync kernel. */
+ * q_rows <= 0, run the mma.sync kernel.
+ * The order of the tiles changes no result.  The tcgen05 kernel takes the list back to front, all KV heads of a tile side by side, and is fastest where tiles
+ * that see many more keys than others stand at its end (a tile of up to 32 queries takes half as long as its keys say); the mma.sync kernel takes it front to
+ * back, head by head.  ft_attn_prefill_order_tiles puts HOST copies of the lists in that order, in place (with the sizes and q_rows of the call to come; it
+ * leaves the list as it is for the mma.sync kernel). */
+int ft_attn_prefill_order_tiles(const int* req_q_start, const int* req_pos0, int* tile_req, int* tile_q0, int n_tiles, int nq, int nkv, int d,
+                                int q_rows);
 int ft_attn_prefill(const void* q, const void* kv_layer, const int* page_table, int max_pages,
                     const int* req_q_start, const int* req_slot, const int* req_pos0, const int* tile_req,
                     const int* tile_q0, int n_tiles, void* out, void* out_lo, int nq, int nkv, int d,
