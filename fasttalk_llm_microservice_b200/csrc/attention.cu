@@ -786,13 +786,13 @@ static int launch_attn_prefill_d(const void* q, const void* kv_layer, const int*
 int launch_attn_prefill(const void* q, const void* kv_layer, const int* page_table, int max_pages,
                         const int* req_q_start, const int* req_slot, const int* req_pos0,
                         const int* tile_req, const int* tile_q0, int n_tiles, void* out, void* out_lo, int nq,
-                        int nkv, int d, bool pdl, cudaStream_t stream, int q_rows) {
+                        int nkv, int d, bool pdl, cudaStream_t stream, int q_rows, bool few) {
     FT_REQUIRE(d == 64 || d == 128, "attn_prefill: head_dim %d not supported (64 or 128)", d);
     FT_REQUIRE(nq % nkv == 0, "attn_prefill: nq %% nkv != 0");
     FT_REQUIRE(n_tiles >= 1, "attn_prefill: no tiles");
     if (q_rows > 0 && attn_prefill_tc_supported(nq, nkv, d))        // tcgen05 / TMEM kernel (attention_tc.cu)
         return launch_attn_prefill_tc(q, q_rows, kv_layer, page_table, max_pages, req_q_start, req_slot, req_pos0,
-                                      tile_req, tile_q0, n_tiles, out, out_lo, nq, nkv, d, pdl, stream);
+                                      tile_req, tile_q0, n_tiles, out, out_lo, nq, nkv, d, few, pdl, stream);
     if (d == 64)
         return launch_attn_prefill_d<64>(q, kv_layer, page_table, max_pages, req_q_start, req_slot, req_pos0,
                                          tile_req, tile_q0, n_tiles, out, out_lo, nq, nkv, pdl, stream);
@@ -838,20 +838,27 @@ extern "C" int ft_attn_prefill_order_tiles(const int* req_q_start, const int* re
                                            int d, int q_rows) {
     FT_REQUIRE(n_tiles >= 0 && (n_tiles == 0 || (req_q_start && req_pos0 && tile_req && tile_q0)), "ft_attn_prefill_order_tiles: bad arguments");
     try {
-        ft::order_query_tiles(req_q_start, req_pos0, tile_req, tile_q0, n_tiles, nq, nkv, d, q_rows);
+        return ft::order_query_tiles(req_q_start, req_pos0, tile_req, tile_q0, n_tiles, nq, nkv, d, q_rows) ? 1 : 0;
     } catch (const std::bad_alloc&) {
         FT_REQUIRE(false, "ft_attn_prefill_order_tiles: out of host memory (%d tiles)", n_tiles);
     }
-    return 0;
+}
+
+extern "C" int ft_attn_prefill_ordered(const void* q, const void* kv_layer, const int* page_table, int max_pages,
+                                       const int* req_q_start, const int* req_slot, const int* req_pos0,
+                                       const int* tile_req, const int* tile_q0, int n_tiles, void* out, void* out_lo,
+                                       int nq, int nkv, int d, int q_rows, int few, void* stream) {
+    return ft::launch_attn_prefill(q, kv_layer, page_table, max_pages, req_q_start, req_slot, req_pos0,
+                                   tile_req, tile_q0, n_tiles, out, out_lo, nq, nkv, d, false,
+                                   static_cast<cudaStream_t>(stream), q_rows, few != 0);
 }
 
 extern "C" int ft_attn_prefill(const void* q, const void* kv_layer, const int* page_table, int max_pages,
                                const int* req_q_start, const int* req_slot, const int* req_pos0,
                                const int* tile_req, const int* tile_q0, int n_tiles, void* out, void* out_lo,
                                int nq, int nkv, int d, int q_rows, void* stream) {
-    return ft::launch_attn_prefill(q, kv_layer, page_table, max_pages, req_q_start, req_slot, req_pos0,
-                                   tile_req, tile_q0, n_tiles, out, out_lo, nq, nkv, d, false,
-                                   static_cast<cudaStream_t>(stream), q_rows);
+    return ft_attn_prefill_ordered(q, kv_layer, page_table, max_pages, req_q_start, req_slot, req_pos0,
+                                   tile_req, tile_q0, n_tiles, out, out_lo, nq, nkv, d, q_rows, 1, stream);
 }
 
 // ------------------------------------------------------------------ decode attention without allocations

@@ -1,26 +1,26 @@
 // K6 on tcgen05 / TMEM — causal chunked-prefill attention over the paged KV cache (head_dim 64 or 128, GQA group of 3 or 4).
 //
-// One CTA = one (request, 64-query tile, KV head): the tile's 64 tokens x the 4 q heads of the group are 256
-// query rows, handled as two 128-row halves (32 tokens x 4 heads each, row = token * 4 + head) so that every
-// K/V tile that reaches shared memory feeds 256 rows of tensor-core work (the mma.sync kernel re-fetched each
-// tile per q head).  Per KV tile of 64 keys and per half:
+// One CTA = one (request, 64-query tile, KV head): the tile's 64 tokens x the G q heads of the group are 64 G query rows, handled as two
+// halves of 32 tokens (row = token * G + head; 128 rows, of which a group of 3 leaves 32 unused), so that every K/V tile that reaches shared
+// memory feeds both (the mma.sync kernel re-fetched each tile per q head).  Up to 32 tokens that see four key tiles or more are one half only: both
+// halves then take the same queries and every other key tile each, and their results are put together at the end.  Per KV tile of 64 keys and per half:
 //
-//   S  = Q K^T   tcgen05.mma  M128 N64 K64   A = Q half (TMA 3-D box -> 128-byte-swizzled rows in smem),
+//   S  = Q K^T   tcgen05.mma  M128 N64 K=D   A = Q half (TMA 3-D box -> 128-byte-swizzled rows in smem),
 //                                           B = the K slab exactly as it lies in the cache: [64 keys][64 d] fp16
 //                                           with chunk ^ (row & 7) IS the K-major SWIZZLE_128B operand layout
 //   softmax      4 warps, one thread per row: tcgen05.ld of the row's 64 scores, running max / sum in fp32,
 //                exp2, P -> fp16 -> TENSOR MEMORY (tcgen05.st, row = lane: the A operand of the next product)
-//   O += P V     tcgen05.mma  M128 N64 K64   B = the V slab as it lies in the cache: [64 keys][64 d] is the
+//   O += P V     tcgen05.mma  M128 N=D K64   B = the V slab as it lies in the cache: [64 keys][64 d] is the
 //                                           MN-major SWIZZLE_128B layout (d contiguous, 8-key groups 1 KB apart)
 //
-// S (two buffers per half, so the scores of tile j + 1 are ready before the softmax of tile j ends) and O live in
-// TMEM together with two P buffers per half (all 512 columns: S 4 x 64, O 2 x 64, P 4 x 32).  O is rescaled lazily: the row maximum used for scaling only moves when
+// S (two buffers per half, so the scores of tile j + 1 are ready before the softmax of tile j ends) and O live in TMEM, P over the first half of
+// the scores that it came from (S 4 x 64 columns, O 2 x D).  O is rescaled lazily: the row maximum used for scaling only moves when
 // the running maximum exceeds it by more than 2^8 (P stays far inside fp16 range, the accumulation is fp32, the
 // final normalisation uses the same reference — exact arithmetic, not an approximation), so the TMEM round trip
 // of a rescale happens on the first tiles only.  The two halves ping-pong: while the softmax warps of one half
 // work on their scores, the tensor core runs the other half's products.
 //
-// Warp roles (320 threads): warp 0 = TMA producer (Q once, then a ring of 16 KB K|V tiles, one bulk copy each),
+// Warp roles (320 threads): warp 0 = TMA producer (Q once, then a ring of K|V tiles of 16 KB (D = 64) or 32 KB, one bulk copy each),
 // warp 1 = TMEM owner + MMA issuer (one elected thread), warps 2..5 = softmax / epilogue of half 0, warps 6..9 of
 // half 1 (warp w may touch TMEM lanes 32 * (w % 4) .. +31), one thread per query row.
 //
@@ -47,7 +47,7 @@ constexpr int TC_ROWS = 128;                 // rows per half (UMMA M); 32 token
 constexpr int TC_TOK = 64;                   // query tokens per CTA
 constexpr int TC_SUB_BYTES = kKvTile * 128;  // one [64 tokens][64 dims] fp16 sub-slab = 8 KB; also 64 rows of a Q block
 constexpr int TC_QBLK_BYTES = TC_ROWS * 128; // one 128-row x 64-dim block of Q = 16 KB
-constexpr int TC_GRID_Y = 65535;             // query tiles along y
+constexpr int TC_GRID_Y = 65535;             // query tiles of one launch
 constexpr int TC_SPLIT_TILES = 4;            // key tiles from which a tile of few queries shares them between the halves
 constexpr float TC_RESCALE_THRESHOLD = 8.f;  // log2 units
 
@@ -76,12 +76,16 @@ __device__ __forceinline__ void mbar_wait_sleep(uint64_t* bar, uint32_t parity) 
     while (!mbar_try_wait(bar, parity)) __nanosleep(20);
 }
 
-template <int D, int G>
+// FEW: the list has tiles whose keys the halves share.  A kernel of its own for the lists without one: the second way in the same kernel costs every CTA 0.1 to
+// 0.25 us, also those that don't take it (64 requests of 30 tokens behind 100, 32 heads of 64 / 128: 27.2 / 36.3 us, without it 26.6 / 35.1; 16 of
+// 64 behind 100 9.1 / 13.1, 8.9 / 12.6), and in there one copy of the rescale loop, which is rare, leaves its instructions for the rest (six of 211 behind 5000, in the
+// caller's order 151 / 172 -> 138 / 168).
+template <int D, int G, bool FEW>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t* __restrict__ kv_layer,
                        const int* __restrict__ page_table, int max_pages, const int* __restrict__ req_q_start,
                        const int* __restrict__ req_slot, const int* __restrict__ req_pos0,
-                       const int* __restrict__ tile_req, const int* __restrict__ tile_q0, int n_q_tiles,
+                       const int* __restrict__ tile_req, const int* __restrict__ tile_q0,
                        __nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ out_lo, int nq, int nkv,
                        float scale_log2, int stagger_on) {
     using C = TcCfg<D>;
@@ -89,8 +93,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
     constexpr int R = 32 * G;                                 // real rows of a half (row = token * G + head)
     // the LAST tiles of the list see the most keys where it is in that order: back to front, all KV heads of a tile side by side, or the
     // longest CTAs would start last and the grid end in a long tail
-    const int tile_idx = n_q_tiles - 1 - (int)(blockIdx.z * TC_GRID_Y + blockIdx.y);
-    if (tile_idx < 0) return;                                // (the last layer of a grid of more than 65535 tiles)
+    const int tile_idx = (int)gridDim.y - 1 - (int)blockIdx.y;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* q_s = smem;                                     // [2 halves][KH dim blocks][128 rows][128 B]
@@ -157,7 +160,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
     const int n_tiles = last_pos / kKvTile + 1;
     // Up to 32 tokens would leave the second half idle: both take the same queries then, every other tile of keys each (tile j: half j & 1), and their
     // results are put together at the end (about a microsecond).
-    const bool split = rows_here <= TC_TOK / 2 && n_tiles >= TC_SPLIT_TILES;
+    const bool split = FEW && rows_here <= TC_TOK / 2 && n_tiles >= TC_SPLIT_TILES;
     const int* pt = page_table + (size_t)req_slot[req] * max_pages;
 
     if (warp == 0) {
@@ -191,27 +194,29 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
         if (elect_one()) {
             constexpr uint32_t idesc_qk = umma_idesc_f16(TC_ROWS, kKvTile, false);
             constexpr uint32_t idesc_pv = umma_idesc_f16(TC_ROWS, D, true);
-            const uint64_t q_desc = umma_desc_k128(smem_u32(q_s)), k_desc = umma_desc_k128(smem_u32(kv_s));
-            const uint64_t v_desc = umma_desc_mn128(smem_u32(kv_s) + KH * TC_SUB_BYTES);
-            // An operand is a base of the half, buffer or stage, put together once, plus what the compiler knows: put together whole for every product it costs
-            // this thread twice what the tensor core takes for it (unrolled over the ring, with the bases known too, it is no faster)
-            auto issue_qk = [&](int h, int buf, int stage, int qh) {
-                const uint64_t a = q_desc + qh * ((KH * TC_QBLK_BYTES) >> 4), b = k_desc + stage * (C::TILE_BYTES >> 4);
-                const uint32_t d = tmem_base + C::COL_S + (2 * h + buf) * 64;
+            const uint32_t q_addr = smem_u32(q_s);
+            auto issue_qk = [&](int h, int buf, uint32_t k_addr, int qh) {
 #pragma unroll
-                for (int k = 0; k < 4 * KH; ++k)
-                    umma_bf16(d, a + (((k >> 2) * TC_QBLK_BYTES) >> 4) + 2 * (k & 3), b + (((k >> 2) * TC_SUB_BYTES) >> 4) + 2 * (k & 3), idesc_qk, k != 0);
+                for (int kh = 0; kh < KH; ++kh) {
+                    const uint64_t a = umma_desc_k128(q_addr + (qh * KH + kh) * TC_QBLK_BYTES);
+                    const uint64_t b = umma_desc_k128(k_addr + kh * TC_SUB_BYTES);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        umma_bf16(tmem_base + C::COL_S + (2 * h + buf) * 64, a + 2 * k, b + 2 * k, idesc_qk, (kh | k) != 0);
+                }
                 umma_commit(&s_full[2 * h + buf]);
             };
-            auto issue_pv = [&](int h, int buf, int stage, bool first) {
-                const uint32_t p = tmem_base + C::COL_S + (2 * h + buf) * 64, d = tmem_base + C::COL_O + h * D;        // 64 fp16 = 32 columns, over S
-                const uint64_t b = v_desc + stage * (C::TILE_BYTES >> 4);
+            auto issue_pv = [&](int h, int buf, uint32_t v_addr, bool first) {
+                const uint32_t p_tmem = tmem_base + C::COL_S + (2 * h + buf) * 64;    // 64 fp16 = 32 columns, over S
 #pragma unroll
-                for (int k = 0; k < kKvTile / 16; ++k) umma_f16_ts(d, p + 8 * k, b + ((k * 2048) >> 4), idesc_pv, k != 0 || !first);
+                for (int k = 0; k < kKvTile / 16; ++k)
+                    umma_f16_ts(tmem_base + C::COL_O + h * D, p_tmem + 8 * k, umma_desc_mn128(v_addr + k * 2048), idesc_pv, k != 0 || !first);
                 umma_commit(&pv_done[2 * h + buf]);
             };
+            auto stage_of = [&](int j) { return j % C::STAGES; };
+            auto k_addr_of = [&](int j) { return smem_u32(kv_s + (size_t)stage_of(j) * C::TILE_BYTES); };
             auto keys_here = [&](int j) {
-                mbar_wait(&kv_full[j % C::STAGES], (j / C::STAGES) & 1);
+                mbar_wait(&kv_full[stage_of(j)], (j / C::STAGES) & 1);
                 tc_fence_after();
             };
             mbar_wait(q_full, 0);
@@ -225,13 +230,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
                     if (j >= 0) {
                         mbar_wait(&p_full[2 * (j & 1) + (j >> 1 & 1)], (j >> 2) & 1);
                         tc_fence_after();
-                        issue_pv(j & 1, j >> 1 & 1, j % C::STAGES, j < 2);
-                        umma_commit(&kv_empty[j % C::STAGES]);
+                        issue_pv(j & 1, j >> 1 & 1, k_addr_of(j) + KH * TC_SUB_BYTES, j < 2);
+                        umma_commit(&kv_empty[stage_of(j)]);
                     }
                     const int a = j + AHEAD;
                     if (a < n_tiles) {
                         keys_here(a);
-                        issue_qk(a & 1, a >> 1 & 1, a % C::STAGES, 0);
+                        issue_qk(a & 1, a >> 1 & 1, k_addr_of(a), 0);
                     }
                 }
             } else {
@@ -239,28 +244,26 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
                 // product of tile j — which reads its P out of the same buffer — has been issued in front of it
                 for (int j = 0; j < 2 && j < n_tiles; ++j) {
                     keys_here(j);
-                    issue_qk(0, j, j, 0);
-                    if (!stagger_on) issue_qk(1, j, j, 1);
+                    issue_qk(0, j & 1, k_addr_of(j), 0);
+                    if (!stagger_on) issue_qk(1, j & 1, k_addr_of(j), 1);
                 }
                 if (stagger_on) {        // half 1 starts when half 0 is about to enter its SFU-bound phase, so that the two halves'
                                          // exponentials do not fall on the SFU at the same time (profiles/r02_attn_prefill_tc.md)
                     mbar_wait(stagger, 0);
-                    for (int j = 0; j < 2 && j < n_tiles; ++j) issue_qk(1, j, j, 1);
+                    for (int j = 0; j < 2 && j < n_tiles; ++j) issue_qk(1, j & 1, k_addr_of(j), 1);
                 }
-#pragma unroll 1
                 for (int j = 0; j < n_tiles; ++j) {
-#pragma unroll 1
                     for (int h = 0; h < 2; ++h) {
                         // Every hand-over has one barrier PER BUFFER (tile parity): the softmax of one half may run up to two
                         // tiles ahead of what this thread has observed (it is busy with the other half), and a single barrier
                         // completing two phases unobserved would look "not yet complete" again — a deadlock.
                         mbar_wait(&p_full[2 * h + (j & 1)], (j >> 1) & 1);   // P_h(j) written, S_h(j) consumed, O_h rescaled if needed
                         tc_fence_after();
-                        issue_pv(h, j & 1, j % C::STAGES, j == 0);
-                        if (h == 1) umma_commit(&kv_empty[j % C::STAGES]);   // every product that reads this stage has been issued
+                        issue_pv(h, j & 1, k_addr_of(j) + KH * TC_SUB_BYTES, j == 0);
+                        if (h == 1) umma_commit(&kv_empty[stage_of(j)]);   // every product that reads this stage has been issued
                         if (j + 2 < n_tiles) {
                             if (h == 0) keys_here(j + 2);
-                            issue_qk(h, j & 1, (j + 2) % C::STAGES, h);      // in order behind the product that read P out of this buffer
+                            issue_qk(h, j & 1, k_addr_of(j + 2), h);      // in order behind the product that read P out of this buffer
                         }
                     }
                 }
@@ -317,7 +320,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const uint8_t*
                 const float alpha = m_new == -INFINITY ? 1.f : exp2f(m_ref - m_new);        // rows that did not grow: m_new >= m_ref, alpha <= 1
                 l_run *= alpha;
                 m_ref = m_new;
-#pragma unroll
+#pragma unroll(FEW ? 1 : D / 16)
                 for (int c = 0; c < D / 16; ++c) {
                     uint32_t orr[16];
                     tmem_ld16_nowait(o_taddr + 16 * c, orr);
@@ -436,17 +439,19 @@ bool attn_prefill_tc_supported(int nq, int nkv, int d) {
 // 500 tokens 70 / 75, 74 / 82, 71 / 77; four of 2048 174 / 186, 170 / 181, 170 / 179; six of 211 behind 5000 170 / 172, 142 / 144, 142 / 145; 128 of 100 behind 100
 // 153 / 164, 159 / 170, 153 / 164).  The mma.sync kernel takes any list front to back, head by head; it stays as it is (sorted: six requests
 // of 17 to 2048 tokens, 8 heads of 64, 85 -> 91 us).
-void order_query_tiles(const int* q_start, const int* pos0, int* tile_req, int* tile_q0, int n_tiles, int nq, int nkv, int d, int q_rows) {
-    if (q_rows <= 0 || n_tiles < 2 || !attn_prefill_tc_supported(nq, nkv, d)) return;
+bool order_query_tiles(const int* q_start, const int* pos0, int* tile_req, int* tile_q0, int n_tiles, int nq, int nkv, int d, int q_rows) {
+    if (q_rows <= 0 || !attn_prefill_tc_supported(nq, nkv, d)) return false;
     struct Tile { long long work; int req, q0; };
     std::vector<Tile> t(n_tiles);
     long long all = 0;
+    bool few = false;
     for (int i = 0; i < n_tiles; ++i) {
         const int r = tile_req[i], q0 = tile_q0[i], left = q_start[r + 1] - q_start[r] - q0, rows = std::min(left, TC_TOK);
         const int keys = (pos0[r] + q0 + rows - 1) / kKvTile + 1;
         const bool shared = rows <= TC_TOK / 2 && keys >= TC_SPLIT_TILES;                  // by the halves: half as many
         t[i] = {(shared ? (keys + 1) / 2 + 1 : keys) + 5, r, q0};                          // start and end of a CTA: five key tiles' time
         all += t[i].work;
+        few |= shared;
     }
     const long long width = std::max(4LL, all * nkv / device_sms() / 8);
     std::stable_sort(t.begin(), t.end(), [&](const Tile& a, const Tile& b) { return a.work / width < b.work / width; });
@@ -454,6 +459,7 @@ void order_query_tiles(const int* q_start, const int* pos0, int* tile_req, int* 
         tile_req[i] = t[i].req;
         tile_q0[i] = t[i].q0;
     }
+    return few;
 }
 
 // q tensor maps are cached per (device, pointer, rows, heads, head_dim, group): the engine's q buffer never moves
@@ -462,20 +468,19 @@ static std::mutex g_qmap_mu;
 static QMapEntry g_qmaps[16];
 static int g_qmap_n = 0, g_qmap_next = 0;
 
-template <int D, int G>
+template <int D, int G, bool FEW>
 static int launch_tc(const CUtensorMap& map, const void* kv_layer, const int* page_table, int max_pages,
                      const int* req_q_start, const int* req_slot, const int* req_pos0, const int* tile_req,
                      const int* tile_q0, int n_tiles, void* out, void* out_lo, int nq, int nkv, bool pdl, cudaStream_t stream) {
     using C = TcCfg<D>;
     static PerDeviceFlag attr_set;
     if (!attr_set.done()) {
-        FT_CHECK_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel<D, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
+        FT_CHECK_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel<D, G, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
         attr_set.mark();
     }
     const float scale_log2 = 1.4426950408889634f / sqrtf((float)D);
     static const int stagger_on = getenv("FT_TC_STAGGER") ? atoi(getenv("FT_TC_STAGGER")) : 1;       // A/B switch; measured: 4–6 % at d = 64
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nkv, std::min(n_tiles, TC_GRID_Y), (n_tiles + TC_GRID_Y - 1) / TC_GRID_Y);
     cfg.blockDim = dim3(TC_THREADS);
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = stream;
@@ -484,15 +489,20 @@ static int launch_tc(const CUtensorMap& map, const void* kv_layer, const int* pa
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_prefill_tc_kernel<D, G>, map, (const uint8_t*)kv_layer, page_table, max_pages,
-                                     req_q_start, req_slot, req_pos0, tile_req, tile_q0, n_tiles, (__nv_bfloat16*)out,
-                                     (__nv_bfloat16*)out_lo, nq, nkv, scale_log2, stagger_on));
+    for (int left = n_tiles; left > 0;) {                        // the end of the list first
+        const int n = std::min(left, TC_GRID_Y);
+        left -= n;
+        cfg.gridDim = dim3(nkv, n);
+        FT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_prefill_tc_kernel<D, G, FEW>, map, (const uint8_t*)kv_layer, page_table, max_pages,
+                                         req_q_start, req_slot, req_pos0, tile_req + left, tile_q0 + left, (__nv_bfloat16*)out,
+                                         (__nv_bfloat16*)out_lo, nq, nkv, scale_log2, stagger_on));
+    }
     return 0;
 }
 
 int launch_attn_prefill_tc(const void* q, int q_rows, const void* kv_layer, const int* page_table, int max_pages,
                            const int* req_q_start, const int* req_slot, const int* req_pos0, const int* tile_req,
-                           const int* tile_q0, int n_tiles, void* out, void* out_lo, int nq, int nkv, int d, bool pdl,
+                           const int* tile_q0, int n_tiles, void* out, void* out_lo, int nq, int nkv, int d, bool few, bool pdl,
                            cudaStream_t stream) {
     FT_REQUIRE(q_rows >= 1, "attn_prefill (tcgen05): the q buffer's row count is needed for its tensor map");
     const int g = nq / nkv;
@@ -515,10 +525,11 @@ int launch_attn_prefill_tc(const void* q, int q_rows, const void* kv_layer, cons
         }
         map = hit->map;
     }
-#define FT_TC_CASE(D_, G_)                                                                                        \
-    if (d == D_ && g == G_)                                                                                       \
-        return launch_tc<D_, G_>(map, kv_layer, page_table, max_pages, req_q_start, req_slot, req_pos0, tile_req,  \
-                                 tile_q0, n_tiles, out, out_lo, nq, nkv, pdl, stream);
+#define FT_TC_CASE(D_, G_)                                                                                               \
+    if (d == D_ && g == G_)                                                                                              \
+        return (few ? launch_tc<D_, G_, true> : launch_tc<D_, G_, false>)(map, kv_layer, page_table, max_pages,          \
+                                                                          req_q_start, req_slot, req_pos0, tile_req,     \
+                                                                          tile_q0, n_tiles, out, out_lo, nq, nkv, pdl, stream);
     FT_TC_CASE(64, 4)
     FT_TC_CASE(64, 3)
     FT_TC_CASE(128, 4)

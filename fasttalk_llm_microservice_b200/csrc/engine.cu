@@ -362,6 +362,7 @@ struct Batch {
     int n_req = 0;                    // page-table rows (decode first, then prefill requests)
     int n_prefill_req = 0;
     int n_tiles = 0;                  // prefill attention q tiles
+    bool few_tiles = false;           // some of them with few queries over many keys
     int n_logit_rows = 0;
     bool logit_rows_identity = false; // logits wanted for rows 0..n_logit_rows-1 exactly (no gather)
 };
@@ -500,7 +501,7 @@ static int forward(Engine* e, const Batch& b) {
             FT_TRY(launch_attn_prefill(e->q, kv_l, d + m.o_pt, e->max_pages, d + m.o_qstart, d + m.o_rslot,
                                        d + m.o_rpos0, d + m.o_treq, d + m.o_tq0, b.n_tiles, e->attn_out,
                                        e->attn_out_lo, c.n_q_heads, c.n_kv_heads, c.head_dim, e->pdl,
-                                       e->stream, e->t_max));
+                                       e->stream, e->t_max, b.few_tiles));
             e->st.kernel_launches++;
         }
         {
@@ -1445,7 +1446,7 @@ static long long fill_batch(Engine* e, const std::vector<Portion>& dec, const st
         }
     }
     if (!e->lay)
-        order_query_tiles(h + m.o_qstart, h + m.o_rpos0, h + m.o_treq, h + m.o_tq0, tiles, e->cfg.n_q_heads, e->cfg.n_kv_heads, e->cfg.head_dim, e->t_max);
+        b.few_tiles = order_query_tiles(h + m.o_qstart, h + m.o_rpos0, h + m.o_treq, h + m.o_tq0, tiles, e->cfg.n_q_heads, e->cfg.n_kv_heads, e->cfg.head_dim, e->t_max);
     h[m.o_xstart + b.n_req] = row;
     b.T = row;
     b.n_tiles = tiles;

@@ -79,20 +79,21 @@ int launch_attn_decode(const void* q, const void* kv_layer, const int* page_tabl
                        int B, int nq, int nkv, int d, int n_ctas, bool pdl, cudaStream_t stream,
                        cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, bool early = false);
 // q_rows: rows (tokens) the q / out buffers hold — the tcgen05 kernel builds a tensor map over q; <= 0 = unknown,
-// which selects the mma.sync kernel
+// which selects the mma.sync kernel.  few: there may be tiles whose keys the tcgen05 kernel's halves share (false: none is)
 int launch_attn_prefill(const void* q, const void* kv_layer, const int* page_table, int max_pages,
                         const int* req_q_start, const int* req_slot, const int* req_pos0,
                         const int* tile_req, const int* tile_q0, int n_tiles, void* out, void* out_lo, int nq,
-                        int nkv, int d, bool pdl, cudaStream_t stream, int q_rows = 0);
+                        int nkv, int d, bool pdl, cudaStream_t stream, int q_rows = 0, bool few = true);
 
-// Puts a list of query tiles (host arrays) in the order that the kernel for these sizes wants: attention_tc.cu
-void order_query_tiles(const int* q_start, const int* pos0, int* tile_req, int* tile_q0, int n_tiles, int nq, int nkv, int d, int q_rows);
+// Puts a list of query tiles (host arrays) in the order that the kernel for these sizes wants; tells whether it has tiles whose keys the tcgen05
+// kernel's halves share: attention_tc.cu
+bool order_query_tiles(const int* q_start, const int* pos0, int* tile_req, int* tile_q0, int n_tiles, int nq, int nkv, int d, int q_rows);
 
 // ---- attention_tc.cu (tcgen05 / TMEM prefill attention: head_dim 64 / 128, GQA group 3 / 4)
 bool attn_prefill_tc_supported(int nq, int nkv, int d);
 int launch_attn_prefill_tc(const void* q, int q_rows, const void* kv_layer, const int* page_table, int max_pages,
                            const int* req_q_start, const int* req_slot, const int* req_pos0, const int* tile_req,
-                           const int* tile_q0, int n_tiles, void* out, void* out_lo, int nq, int nkv, int d, bool pdl,
+                           const int* tile_q0, int n_tiles, void* out, void* out_lo, int nq, int nkv, int d, bool few, bool pdl,
                            cudaStream_t stream);
 
 // ---- layered.cu (the layered model family: every size is a run-time value, activations fp32, weights bf16)

@@ -202,8 +202,8 @@ def attn_prefill(q: torch.Tensor, kv_layer: torch.Tensor, page_table: torch.Tens
     assert parts[2].numel() >= len(req_slot), "req_pos0: a position for every request"
     rows = T if tensor_cores else 0
     lib = N.load()
-    N.check(lib.ft_attn_prefill_order_tiles(N.ptr(parts[0]), N.ptr(parts[2]), N.ptr(parts[3]), N.ptr(parts[4]), len(tile_req), nq, nkv, d, rows),
-            "ft_attn_prefill_order_tiles")
+    few = N.check(lib.ft_attn_prefill_order_tiles(N.ptr(parts[0]), N.ptr(parts[2]), N.ptr(parts[3]), N.ptr(parts[4]), len(tile_req), nq, nkv, d, rows),
+                  "ft_attn_prefill_order_tiles")
     lists = torch.cat(parts)
     waits = dev.index != torch.cuda.current_device() or torch.cuda.is_current_stream_capturing()
     lists = lists.to(dev) if waits else lists.pin_memory().to(dev, non_blocking=True)
@@ -213,9 +213,9 @@ def attn_prefill(q: torch.Tensor, kv_layer: torch.Tensor, page_table: torch.Tens
     owned = bool(starts) and starts[0] == 0 and starts[-1] == T and all(x <= y for x, y in zip(starts, starts[1:]))
     out = (torch.empty if owned else torch.zeros)(T, nq * d, device=dev, dtype=torch.bfloat16)
     out_lo = torch.empty_like(out) if owned else torch.zeros_like(out)
-    N.check(lib.ft_attn_prefill(N.ptr(q), N.ptr(kv_layer), N.ptr(page_table), page_table.shape[1],
-                                N.ptr(t_qs), N.ptr(t_slot), N.ptr(t_pos0), N.ptr(t_treq), N.ptr(t_tq0),
-                                len(tile_req), N.ptr(out), N.ptr(out_lo), nq, nkv, d, rows, N.cur_stream()),
+    N.check(lib.ft_attn_prefill_ordered(N.ptr(q), N.ptr(kv_layer), N.ptr(page_table), page_table.shape[1],
+                                        N.ptr(t_qs), N.ptr(t_slot), N.ptr(t_pos0), N.ptr(t_treq), N.ptr(t_tq0),
+                                        len(tile_req), N.ptr(out), N.ptr(out_lo), nq, nkv, d, rows, few, N.cur_stream()),
             "ft_attn_prefill")
     return out, out_lo
 

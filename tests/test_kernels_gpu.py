@@ -562,6 +562,43 @@ def test_attn_prefill_tiles_of_few_queries_by_keys(K, nq, nkv, d, tiles, n):
         assert rel_err(got[q_start[r]:q_start[r + 1]], ref) < 2e-3, r
 
 
+@pytest.mark.parametrize("nq,nkv,d", [(4, 1, 64), (6, 2, 64), (32, 8, 128), (3, 1, 128)])
+@pytest.mark.parametrize("reqs", [[(0, 64)], [(100, 33), (0, 300), (3000, 64)], [(120, 40)] * 20, [(500, 7), (0, 300), (0, 8)]])
+def test_attn_prefill_with_and_without_the_shared_way(K, nq, nkv, d, reqs):
+    """The two kernels of a list: without tiles of few queries over many keys they give the same bits; with one (the last list) both are right."""
+    from fasttalk_llm_microservice_b200 import native as N
+    g = torch.Generator(device=DEV).manual_seed(nq + d + len(reqs))
+    kv, pt, ks, vs = build_paged_kv(K, [p + n for p, n in reqs], nkv, d, g)
+    start = [sum(n for _, n in reqs[:i]) for i in range(len(reqs) + 1)]
+    q = (torch.randn(start[-1], nq, d, device=DEV, generator=g) * 1.5).half()
+    i32 = lambda v: torch.tensor(v, device=DEV, dtype=torch.int32)
+    tiles = [(r, q0) for r, (_, n) in enumerate(reqs) for q0 in range(0, n, 64)]
+    lists = [i32(start), i32(range(len(reqs))), i32([p for p, _ in reqs]), i32([r for r, _ in tiles]), i32([q0 for _, q0 in tiles])]
+    got = []
+    for few in (0, 1):
+        out = torch.empty(start[-1], nq * d, device=DEV, dtype=torch.bfloat16)
+        lo = torch.empty_like(out)
+        N.check(N.load().ft_attn_prefill_ordered(N.ptr(q), N.ptr(kv), N.ptr(pt), pt.shape[1], *map(N.ptr, lists), len(tiles), N.ptr(out), N.ptr(lo),
+                                                 nq, nkv, d, start[-1], few, N.cur_stream()), "ft_attn_prefill_ordered")
+        got.append(hilo(out, lo))
+    assert reqs[-1] == (0, 8) or torch.equal(got[0], got[1])
+    for x in got:
+        for r, (p0, _) in enumerate(reqs):
+            ref = O.attention(q[start[r]:start[r + 1]].float(), ks[r].float(), vs[r].float(), p0)
+            assert rel_err(x[start[r]:start[r + 1]], ref) < 2e-3, r
+
+
+def test_attn_prefill_more_tiles_than_one_launch_takes(K):
+    """70000 requests of one token at position 0, all on one page: each sees its one key, so its row is that key's value."""
+    n, nq, d = 70000, 4, 64
+    g = torch.Generator(device=DEV).manual_seed(1)
+    kv, pt, ks, vs = build_paged_kv(K, [1], 1, d, g)
+    q = torch.randn(n, nq, d, device=DEV, generator=g).half()
+    out = hilo(*K.attn_prefill(q, kv, pt, list(range(n + 1)), [0] * n, [0] * n))
+    # the only probability is 2^(a score's rounding): 2^-24 of a score of up to 16
+    assert torch.allclose(out.view(n, nq, d), vs[0][0, 0].float().expand(n, nq, d), rtol=2e-6, atol=0)
+
+
 @pytest.mark.parametrize("nq,nkv,d", [(32, 8, 64), (32, 8, 128), (6, 2, 128)])
 @pytest.mark.parametrize("p0,n", [(1472, 21), (5 * 64, 64), (0, 300)])
 def test_attn_prefill_rows_depend_on_nothing_else(K, nq, nkv, d, p0, n):
