@@ -15,7 +15,8 @@ def ordered(lens, pos0, nq, nkv, d, rows=None):
     req, q0 = (np.array([t[i] for t in tiles], np.int32) for i in (0, 1))
     rc = N.load().ft_attn_prefill_order_tiles(starts.ctypes.data, pos.ctypes.data, req.ctypes.data, q0.ctypes.data, len(tiles), nq, nkv, d,
                                               int(starts[-1]) if rows is None else rows)
-    assert rc == 0
+    tc = (nq // nkv in (3, 4)) and d in (64, 128) and (rows is None or rows > 0)
+    assert rc == int(tc and any(min(64, lens[r] - q) <= 32 and (pos0[r] + min(lens[r], q + 64) - 1) // 64 + 1 >= 4 for r, q in tiles))
     return tiles, list(zip(req.tolist(), q0.tolist()))
 
 
