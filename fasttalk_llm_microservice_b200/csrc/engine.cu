@@ -185,17 +185,25 @@ struct LayeredLayer {
 struct StepGraph {
     int T = 0, n_logit_rows = 0;
     bool identity = false, refused = false;
-    cudaGraphExec_t exec = nullptr;    // null: seen once
+    cudaGraphExec_t exec = nullptr;    // null: not recorded
     long long launches = 0;
-    unsigned long long used = 0;       // of the model's counter: the least recent one gives way
+    long long uses = 0;                // plain steps of the shape, then replays of its graph
+    long long last = 0;                // the model's step that used it last
 };
-constexpr size_t kStepGraphs = 16;
+// A replay gains 5 to 20 us on a step of 80 to 480, recording one costs 130 to 320 (Gedelorn, Vonedra and Fedutar of 1024 and 2048 columns, 1 to 16 sessions): what
+// kGraphCost replays gain.  So recordings are paid for: by replays, by an advance of one, and by plain steps, half a replay's worth each, which bounds what
+// shapes that never come again can cost to 3 % of their steps.  A shape is recorded at its third step at the earliest.  kStepGraphs are kept; one gives
+// way only when it has not come for kGraphIdle steps, and where it had not earned its recording the next ones cost twice as much.  (Recorded at the second
+// step, the least recent of sixteen giving way: twenty shapes, each two steps running, 275 us a step without graphs, 402; now 284, of 1024 columns 215, 315, 217.)
+constexpr int kStepShapes = 64, kStepGraphs = 16, kGraphCost = 16, kGraphIdle = 1024;
 
 struct Layered {
-    std::vector<StepGraph> graphs;     // at most kStepGraphs, used under the engine's step lock
-    unsigned long long graph_clock = 0;
+    std::vector<StepGraph> shapes;     // at most kStepShapes, used under the engine's step lock
+    long long graph_steps = 0, graph_cost = kGraphCost;
+    double graph_credit = kGraphCost;  // in replays
+    long long graphs_recorded = 0, graphs_replayed = 0, graphs_refused = 0;
     ~Layered() {
-        for (StepGraph& g : graphs)
+        for (StepGraph& g : shapes)
             if (g.exec) cudaGraphExecDestroy(g.exec);
     }
     ft_layered_model m;
@@ -1319,51 +1327,74 @@ static int forward_layered(Engine* e, const Batch& b) {
     return 0;
 }
 
-// The same, single tokens out of a graph from the third step of a shape on: the second one records it.  A launch of a stream leaves 1 to 2.5 us between two short kernels, an
-// edge of a graph about half (Gedelorn, 46 launches a step of 16 sessions: 410 us, so 328).
+// Room for one more graph: is there, or made where one has not come for long.
+static bool step_graph_room(Layered& L) {
+    int n = 0;
+    StepGraph* idle = nullptr;
+    for (StepGraph& x : L.shapes) {
+        if (!x.exec) continue;
+        ++n;
+        if (L.graph_steps - x.last > kGraphIdle && (!idle || x.last < idle->last)) idle = &x;
+    }
+    if (n < kStepGraphs) return true;
+    if (!idle) return false;
+    cudaGraphExecDestroy(idle->exec);
+    if (idle->uses < kGraphCost) L.graph_cost = std::min<long long>(2 * L.graph_cost, 1 << 20);
+    idle->exec = nullptr;
+    idle->uses = 0;
+    return true;
+}
+
+// The same, steps of single tokens whose shape comes again out of a graph.  A launch of a stream leaves up to a microsecond between two short kernels,
+// an edge of a graph about a third of that less (16 sessions, a step: Gedelorn of 1024 columns 268 us, so 252, Vonedra 321 and 300; of 2048 columns 318 and 314).
 static int forward_layered_step(Engine* e, const Batch& b) {
     Layered& L = *e->lay;
     if (b.n_tiles > 0 || b.n_prefill_req > 0 || (L.trail_on && L.trail)) return forward_layered(e, b);
+    ++L.graph_steps;
     StepGraph* g = nullptr;
-    for (StepGraph& x : L.graphs)
+    for (StepGraph& x : L.shapes)
         if (x.T == b.T && x.n_logit_rows == b.n_logit_rows && x.identity == b.logit_rows_identity) g = &x;
     if (!g) {
-        if (L.graphs.size() < kStepGraphs) {
-            g = &L.graphs.emplace_back();
-        } else {
-            g = &*std::min_element(L.graphs.begin(), L.graphs.end(), [](const StepGraph& x, const StepGraph& y) { return x.used < y.used; });
-            if (g->exec) cudaGraphExecDestroy(g->exec);
+        if ((int)L.shapes.size() < kStepShapes) {
+            g = &L.shapes.emplace_back();
+        } else {                             // the shape without a graph that has not come for longest
+            for (StepGraph& x : L.shapes)
+                if (!x.exec && (!g || x.last < g->last)) g = &x;
             *g = StepGraph();
         }
         g->T = b.T;
         g->n_logit_rows = b.n_logit_rows;
         g->identity = b.logit_rows_identity;
-        g->used = ++L.graph_clock;
-        return forward_layered(e, b);
     }
-    g->used = ++L.graph_clock;
-    if (g->refused) return forward_layered(e, b);
+    g->last = L.graph_steps;
+    ++g->uses;
     if (!g->exec) {
+        L.graph_credit = std::min(L.graph_credit + 0.5, (double)kStepGraphs * L.graph_cost);
+        if (g->refused || g->uses < 3 || L.graph_credit < (double)L.graph_cost || !step_graph_room(L)) return forward_layered(e, b);
         const long long before = e->st.kernel_launches;
         cudaGraph_t graph = nullptr;
-        if (cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-            cudaGetLastError();
-            g->refused = true;
-            return forward_layered(e, b);
+        int rc = -1;
+        if (cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+            rc = forward_layered(e, b);
+            if (cudaStreamEndCapture(e->stream, &graph) != cudaSuccess) rc = -1;
         }
-        const int rc = forward_layered(e, b);
-        const cudaError_t end = cudaStreamEndCapture(e->stream, &graph);
         g->launches = e->st.kernel_launches - before;
         e->st.kernel_launches = before;
-        if (!rc && end == cudaSuccess && cudaGraphInstantiate(&g->exec, graph, 0) != cudaSuccess) g->exec = nullptr;
+        if (!rc && cudaGraphInstantiate(&g->exec, graph, 0) != cudaSuccess) g->exec = nullptr;
         if (graph) cudaGraphDestroy(graph);
-        if (!g->exec) {                  // nothing of the step has run yet
+        if (!g->exec) {                      // nothing of the step has run yet
             cudaGetLastError();
             g->refused = true;
+            ++L.graphs_refused;
             return forward_layered(e, b);
         }
+        ++L.graphs_recorded;
+        L.graph_credit -= (double)L.graph_cost;
+        g->uses = 0;
     }
+    L.graph_credit = std::min(L.graph_credit + 1.0, (double)kStepGraphs * L.graph_cost);
     FT_CHECK_CUDA(cudaGraphLaunch(g->exec, e->stream));
+    ++L.graphs_replayed;
     e->st.kernel_launches += g->launches;
     return 0;
 }
@@ -2740,6 +2771,19 @@ extern "C" int ft_engine_stats_get(ft_engine* h, ft_engine_stats* out) {
     e->st.live_sessions = (int)e->sessions.size();
     e->st.free_pages = (int)e->free_pages.size();
     *out = e->st;
+    return 0;
+}
+
+extern "C" int ft_engine_step_graphs(ft_engine* h, long long* out4) {
+    Engine* e = reinterpret_cast<Engine*>(h);
+    FT_REQUIRE(e && out4, "ft_engine_step_graphs: bad arguments");
+    std::lock_guard<std::mutex> sk(e->step_mu);
+    out4[0] = out4[1] = out4[2] = out4[3] = 0;
+    if (!e->lay) return 0;
+    for (const StepGraph& g : e->lay->shapes) out4[0] += g.exec != nullptr;
+    out4[1] = e->lay->graphs_recorded;
+    out4[2] = e->lay->graphs_replayed;
+    out4[3] = e->lay->graphs_refused;
     return 0;
 }
 

@@ -269,6 +269,12 @@ class Engine:
                                         out.ctypes.data if len(want) else None), "ft_engine_feed")
         return out
 
+    def step_graphs(self) -> Dict:
+        """Layered models: graphs of single-token steps kept now, recorded, steps run out of one, shapes that could not be recorded."""
+        out = (C.c_longlong * 4)()
+        N.check(self.lib.ft_engine_step_graphs(self._h, out), "ft_engine_step_graphs")
+        return dict(zip(("kept", "recorded", "replayed", "refused"), out))
+
     def debug_trail(self, on: bool = True):
         N.check(self.lib.ft_engine_debug_trail(self._h, int(on)), "ft_engine_debug_trail")
 

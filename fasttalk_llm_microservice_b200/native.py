@@ -90,6 +90,7 @@ SIGNATURES = {
     "ft_engine_drain": (_I, [_VP, _VP, _VP, _VP, _I]),
     "ft_engine_cancel": (_I, [_VP, _LL]),
     "ft_engine_session_close": (_I, [_VP, _ULL]),
+    "ft_engine_step_graphs": (_I, [_VP, _VP]),
     "ft_engine_stats_get": (_I, [_VP, C.POINTER(EngineStats)]),
     "ft_engine_get_logits": (_I, [_VP, _LL, _VP]),
     "ft_engine_timer": (_I, [_VP, _I, _VP]),

@@ -151,6 +151,9 @@ int ft_engine_cancel(ft_engine* e, long long req);
 /* Forget a session and free its KV pages (session end / disconnect). */
 int ft_engine_session_close(ft_engine* e, unsigned long long session_key);
 int ft_engine_stats_get(ft_engine* e, ft_engine_stats* out);
+/* Layered models: steps of single tokens whose numbers of rows come again and again run out of recorded graphs -> HOST long long [4]: graphs kept now,
+ * recorded, steps run out of one, shapes that could not be recorded (all 0 for other models). */
+int ft_engine_step_graphs(ft_engine* e, long long* out4);
 /* Change ft_engine_config.decode_prefill_cap of a live engine (same encoding: 0 default, < 0 uncapped);
  * takes effect at the next step. */
 int ft_engine_set_decode_prefill_cap(ft_engine* e, int cap);

@@ -825,13 +825,13 @@ def test_rows_by_four_channels(heads, dim, vdim, rot):
 
 
 def test_steps_of_single_tokens_out_of_graphs():
-    """The same number of rows again and again (recorded at the second step, replayed from the third), other numbers in between, other sessions and other
-    wanted rows under the same number, portions beside, more shapes than are kept: all as the whole prompts give them."""
+    """Steps of single tokens with the same numbers of rows are recorded at the third and replayed; other numbers in between, other sessions and other wanted
+    rows under the same number, portions beside: all as the whole prompts give them."""
     spec, w = make(MIXED, seed=29)
     eng = engine(spec, w, max_batch=20, max_sessions=20, num_pages=24)
     try:
         names = [f"s{i}" for i in range(18)]
-        seqs = {n: tokens_of(spec, 60, 70 + i) for i, n in enumerate(names)}
+        seqs = {n: tokens_of(spec, 90 if i < 6 else 60, 70 + i) for i, n in enumerate(names)}
         ref = {n: oracle_logits(spec, w, t) for n, t in seqs.items()}
         at = dict.fromkeys(names, 0)
 
@@ -846,17 +846,69 @@ def test_steps_of_single_tokens_out_of_graphs():
                 at[n] += len(t)
         step(names[:4], [3, 5, 2, 7])
         step(names[4:], [2] * 14)
-        for k in range(5):
+        for k in range(6):
             step(names[:4])
+        assert eng.step_graphs() == {"kept": 1, "recorded": 1, "replayed": 4, "refused": 0}
         step(names[2:6])                       # the same shape, other sessions in other places
+        assert eng.step_graphs()["replayed"] == 5
         step(names[:4], wanted=names[1:2])     # fewer wanted rows
         step(names[:4], wanted=names[2:3])
         step(names[:4], wanted=names[3:4])
         step(names[:5], [1, 1, 1, 1, 20])      # beside a portion
-        for n in range(1, 19):                 # shapes that push the first ones out
+        for n in range(1, 19):                 # many shapes, none of them often: none is worth a recording
             step(names[:n])
             step(names[:n])
+        got = eng.step_graphs()
+        assert got["recorded"] == 1 and got["refused"] == 0
         for k in range(3):
             step(names[:4])
+        assert eng.step_graphs()["replayed"] == got["replayed"] + 3
     finally:
         eng.close()
+
+
+def test_step_graphs_are_kept_replaced_and_left_for_the_trail():
+    """Against an engine that records nothing (its trail is on), bit by bit: more shapes than are kept, one that takes the place of one which has not come for long,
+    the trail turned on and off between replays."""
+    spec, w = make([layer(space(), dense()), layer(parallel())], seed=30)
+    kw = dict(max_batch=6, max_sessions=6, max_context=4096, num_pages=300)
+    eng, plain = engine(spec, w, **kw), engine(spec, w, **kw)
+    try:
+        plain.debug_trail(True)
+        rng = np.random.default_rng(5)
+
+        def step(n, wanted):
+            entries = [(s, [int(rng.integers(spec.vocab))], [0] if s < wanted else []) for s in range(n)]
+            a, b = eng.feed(entries), plain.feed(entries)
+            assert np.array_equal(a, b), (n, wanted)
+
+        for e in (eng, plain):
+            e.feed([(s, list(range(s + 2)), []) for s in range(6)])
+        for k in range(10):
+            step(3, 3)
+        assert eng.step_graphs() == {"kept": 1, "recorded": 1, "replayed": 8, "refused": 0}
+        eng.debug_trail(True)
+        step(3, 3)
+        assert np.array_equal(eng.read_trail(3), plain.read_trail(3))
+        eng.debug_trail(False)
+        step(3, 3)
+        assert eng.step_graphs()["replayed"] == 9
+        shapes = [(n, w) for n in range(1, 7) for w in range(1, n + 1)][:20]
+        for n, w in shapes:
+            step(n, w), step(n, w)
+        assert eng.step_graphs()["recorded"] == 1
+        for n, w in shapes:
+            for k in range(36):
+                step(n, w)
+        got = eng.step_graphs()
+        assert got["kept"] == got["recorded"] == 16 and got["refused"] == 0
+        for k in range(1025):
+            step(2, 2)
+        for k in range(3):                     # a shape that came often enough before, without a place then
+            step(*shapes[-1])
+        got = eng.step_graphs()
+        assert got["kept"] == 16 and got["recorded"] == 17 and got["refused"] == 0
+        assert plain.step_graphs() == {"kept": 0, "recorded": 0, "replayed": 0, "refused": 0}
+    finally:
+        eng.close()
+        plain.close()
