@@ -415,16 +415,17 @@ __global__ void __launch_bounds__(kWinWarps * 32) window_attn_kernel(WindowArgs 
 }
 
 // The same for heads of up to 128 channels, up to four query heads per key head: one CTA per (token, key head), so that a key and a value row is read once for the
-// group and by neighbouring lanes.  A warp takes 16 keys at a time, all of their rows copied to its part of shared memory at once, the next ones' while it
-// works: scores by eight lanes a key, the softmax by a lane a key, the sums by four channels a lane.  Bound by the chain of a round of 128 keys: copies that
-// set out one step ahead, sums and maxima over lanes (3.8 us with four query heads, 2.2 with one).
-constexpr int kStepWarps = 8, kStepKeys = 16;
-template <int GRP>
-__global__ void __launch_bounds__(kStepWarps * 32) window_step_kernel(WindowArgs a) {
+// group and by neighbouring lanes.  A warp takes KEYS keys at a time, all of their rows copied to its part of shared memory at once, the next ones' while it
+// works: scores by eight lanes a key, the softmax by a lane a key, the sums by four channels a lane.  Bound by the chain of a round of WARPS * KEYS keys: copies that
+// set out one step ahead, sums and maxima over lanes (3.8 us for 128 keys with four query heads, 2.2 with one).  Eight warps of 16 keys are the shortest chain while
+// every CTA runs at once; beyond that four of eight, of which four to eight times as many fit an SM.
+constexpr int step_ctas(int grp, int warps) { return warps == 8 ? (grp == 1 ? 3 : grp == 2 ? 2 : 1) : (grp == 1 ? 8 : grp == 2 ? 5 : 3); }      // that an SM's registers hold
+template <int GRP, int WARPS, int KEYS>
+__global__ void __launch_bounds__(WARPS * 32, step_ctas(GRP, WARPS)) window_step_kernel(WindowArgs a) {
     pdl_wait();
-    extern __shared__ __align__(16) float kv[];        // a warp's keys and values: [16][dim], [16][vdim]; at the end its sums [GRP][vdim]
-    __shared__ __align__(16) float ps[kStepWarps][kStepKeys][GRP];       // scores, then probabilities of a warp's keys
-    __shared__ float sm[kStepWarps][GRP], sl[kStepWarps][GRP];
+    extern __shared__ __align__(16) float kv[];        // a warp's keys and values: [KEYS][dim], [KEYS][vdim]; at the end its sums [GRP][vdim]
+    __shared__ __align__(16) float ps[WARPS][KEYS][GRP];       // scores, then probabilities of a warp's keys
+    __shared__ float sm[WARPS][GRP], sl[WARPS][GRP];
     const int t = blockIdx.x, g = blockIdx.y, grp = a.H / a.G, h0 = g * grp;
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & 7;
     const int p = a.positions[t];
@@ -436,25 +437,25 @@ __global__ void __launch_bounds__(kStepWarps * 32) window_step_kernel(WindowArgs
     const size_t rowsz = (size_t)a.G * (alias ? a.dim : a.dim + a.vdim);
     const float* k_at = a.cache + (size_t)g * a.dim;
     const float* v_at = a.cache + (alias ? (size_t)g * a.dim + a.v_in_key : (size_t)a.G * a.dim + (size_t)g * a.vdim);
-    float* ks = kv + (size_t)wid * kStepKeys * (a.dim + a.vdim);
-    float* vs = ks + kStepKeys * a.dim;
-    constexpr int STEP = kStepWarps * kStepKeys;
-    // the place of key b0 + lane % 16 (behind the last one: of position p, whose weight is then 0)
+    float* ks = kv + (size_t)wid * KEYS * (a.dim + a.vdim);
+    float* vs = ks + KEYS * a.dim;
+    constexpr int STEP = WARPS * KEYS;
+    // the place of key b0 + lane % KEYS (behind the last one: of position p, whose weight is then 0)
     auto place = [&](int b0) {
-        const int idx = b0 + (lane & 15), j = idx < n ? (idx < nf ? idx : lo + idx - nf) : p;
+        const int idx = b0 + (lane & (KEYS - 1)), j = idx < n ? (idx < nf ? idx : lo + idx - nf) : p;
         return pt[j >> 6] * 64 + (j & 63);
     };
     auto copy = [&](int row, const float* from, float* to, int width) {
         const uint32_t dst = smem_u32(to) + lane * 16;
 #pragma unroll 4
-        for (int key = 0; key < kStepKeys; ++key) {
+        for (int key = 0; key < KEYS; ++key) {
             const int r = __shfl_sync(0xffffffffu, row, key);
             if (4 * lane < width)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + key * width * 4), "l"(from + (size_t)r * rowsz + 4 * lane) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    int b0 = wid * kStepKeys;
+    int b0 = wid * KEYS;
     if (b0 < n) {
         const int row = place(b0);
         copy(row, k_at, ks, a.dim);
@@ -478,13 +479,13 @@ __global__ void __launch_bounds__(kStepWarps * 32) window_step_kernel(WindowArgs
     }
     const int c_out = lane * 4;
     for (; b0 < n; b0 += STEP) {
-        const int idx = b0 + (lane & 15), j = idx < nf ? idx : lo + idx - nf;      // both halves of the warp hold the same key
+        const int idx = b0 + (lane & (KEYS - 1)), j = idx < nf ? idx : lo + idx - nf;      // every KEYS lanes hold the same keys
         const bool valid = idx < n, more = b0 + STEP < n;
         const int row = more ? place(b0 + STEP) : 0;
         asm volatile("cp.async.wait_group 1;" ::: "memory");     // the keys (the values are the group behind them)
         __syncwarp();
 #pragma unroll
-        for (int it = 0; it < kStepKeys / 4; ++it) {
+        for (int it = 0; it < KEYS / 4; ++it) {
             const int key = 4 * it + (lane >> 3);
             float s[GRP];
 #pragma unroll
@@ -509,7 +510,7 @@ __global__ void __launch_bounds__(kStepWarps * 32) window_step_kernel(WindowArgs
         if (more) copy(row, k_at, ks, a.dim);
         float s[GRP], top[GRP], sum[GRP], corr[GRP];
 #pragma unroll
-        for (int h = 0; h < GRP; ++h) s[h] = ps[wid][lane & 15][h] * a.scale;
+        for (int h = 0; h < GRP; ++h) s[h] = ps[wid][lane & (KEYS - 1)][h] * a.scale;
         if (a.softcap > 0.f)
 #pragma unroll
             for (int h = 0; h < GRP; ++h) s[h] = a.softcap * tanhf(s[h] / a.softcap);
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(kStepWarps * 32) window_step_kernel(WindowArgs
             top[h] = s[h];
         }
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1)
+        for (int o = KEYS / 2; o > 0; o >>= 1)
 #pragma unroll
             for (int h = 0; h < GRP; ++h) top[h] = fmaxf(top[h], __shfl_xor_sync(0xffffffffu, top[h], o));
 #pragma unroll
@@ -529,10 +530,10 @@ __global__ void __launch_bounds__(kStepWarps * 32) window_step_kernel(WindowArgs
             corr[h] = h < grp ? expf(m[h] - m_new) : 0.f;        // 0 on the first block (m = -inf)
             sum[h] = valid && h < grp ? expf(s[h] - m_new) : 0.f;
             m[h] = m_new;
-            ps[wid][lane & 15][h] = sum[h];
+            ps[wid][lane & (KEYS - 1)][h] = sum[h];
         }
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1)
+        for (int o = KEYS / 2; o > 0; o >>= 1)
 #pragma unroll
             for (int h = 0; h < GRP; ++h) sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], o);
 #pragma unroll
@@ -545,7 +546,7 @@ __global__ void __launch_bounds__(kStepWarps * 32) window_step_kernel(WindowArgs
         __syncwarp();
         if (c_out < a.vdim)
 #pragma unroll
-            for (int u = 0; u < kStepKeys; ++u) {
+            for (int u = 0; u < KEYS; ++u) {
                 const float4 v = load_f4(vs + u * a.vdim + c_out);
 #pragma unroll
                 for (int h = 0; h < GRP; ++h) {
@@ -566,21 +567,21 @@ __global__ void __launch_bounds__(kStepWarps * 32) window_step_kernel(WindowArgs
 #pragma unroll
         for (int h = 0; h < GRP; ++h) store_f4(ks + h * a.vdim + c_out, acc[h]);        // (all copies have landed; four rows fit the warp's part)
     __syncthreads();
-    for (int i = threadIdx.x; i < grp * a.vdim; i += kStepWarps * 32) {
+    for (int i = threadIdx.x; i < grp * a.vdim; i += WARPS * 32) {
         const int h = i / a.vdim, c = i % a.vdim;
         float mm = sm[0][h];
 #pragma unroll
-        for (int w = 1; w < kStepWarps; ++w) mm = fmaxf(mm, sm[w][h]);
+        for (int w = 1; w < WARPS; ++w) mm = fmaxf(mm, sm[w][h]);
         float den = 0.f, num = 0.f;
         if (a.sink) {
             mm = fmaxf(mm, a.sink[h0 + h]);
             den = expf(a.sink[h0 + h] - mm);
         }
 #pragma unroll
-        for (int w = 0; w < kStepWarps; ++w) {
+        for (int w = 0; w < WARPS; ++w) {
             const float f = expf(sm[w][h] - mm);
             den += sl[w][h] * f;
-            num += kv[(size_t)w * kStepKeys * (a.dim + a.vdim) + h * a.vdim + c] * f;
+            num += kv[(size_t)w * KEYS * (a.dim + a.vdim) + h * a.vdim + c] * f;
         }
         float r = num / den;
         if (a.gate) r *= sigmoid_f(a.gate[(size_t)t * a.ldg + (h0 + h) * a.vdim + c]);
@@ -847,16 +848,23 @@ int launch_window_attention(const WindowArgs& a, int T, int n_single, const Wind
     // One query head per key head, or long heads and some tokens (us, before -> window_step_kernel, behind 10 / 150 / 600 keys in a window of 512: 8 key heads
     // of 64, one query head each, 4 tokens 4.5 / 9.2 / 16.9 -> 4.1 / 6.5 / 11.2; 4 key heads of 128 of four query heads, 16 tokens 6.5 / 15.2 / 31.9 -> 6.3 / 9.9 /
     // 18.3, one token 5.3 / 11.4 / 22.5 -> 5.9 / 9.5 / 17.6; one key head of 64 of four 5.0 / 9.5 / 17.1 -> 5.6 / 8.7 / 16.4, of 32 of three 4.3 / 8.4 / 14.9 -> 5.5 / 8.8 / 16.4).
+    // Where more CTAs come than run at once, the small ones, but for heads shorter than 64 (before, eight warps, four, behind 10 / 40 / 150 / 600 keys: 16 key heads of 128, one
+    // query head each, 32 tokens 6.8 / 8.9 / 28 / 68, 14 / 14 / 25 / 53, 4.4 / 6.7 / 13 / 46; of 64 64 tokens 5.9 / 8.6 / 23 / 63, 12 / 13 / 22 / 49, 5.0 / 8.2 / 19 / 51; 8 of 128 of
+    // four query heads, 64 tokens 13 / 24 / 69 / 179, 23 / 23 / 39 / 77, 11 / 16 / 32 / 82; 32 of 32 of one, 32 tokens 5.1 / 7.0 / 14 / 44, 11 / 12 / 21 / 45, 4.9 / 8.1 / 18 / 50).
     if (vec && a.dim <= 128 && a.vdim <= 128 && (grp == 1 || (grp <= 4 && a.dim + a.vdim >= 192 && T >= 4)) && a.G <= 65535 && (alias16 & 15) == 0) {
-        const size_t rows = (size_t)kStepWarps * kStepKeys * (a.dim + a.vdim) * 4;
-        auto step = [&](auto kernel) -> int {
-            if (rows > 40 * 1024) FT_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows));
-            launch_after(kernel, dim3(T, a.G), kStepWarps * 32, rows, stream, a);
+        const int g = grp <= 2 ? grp : 4, row = (a.dim + a.vdim) * 4;
+        const size_t rows = (size_t)8 * 16 * row;
+        const int fit = (int)std::min<size_t>(step_ctas(g, 8), 227 * 1024 / (rows + 8 * 16 * g * 4 + 8 * g * 8 + 1024));      // the copies, the block's own, the system's
+        const bool once = (long long)T * a.G <= (long long)device_sms() * fit;
+        auto step = [&](auto kernel, int warps, size_t bytes) -> int {
+            if (bytes > 40 * 1024) FT_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+            launch_after(kernel, dim3(T, a.G), warps * 32, bytes, stream, a);
+            FT_CHECK_CUDA(cudaGetLastError());
             return 0;
         };
-        if (int r = grp <= 1 ? step(window_step_kernel<1>) : grp <= 2 ? step(window_step_kernel<2>) : step(window_step_kernel<4>)) return r;
-        FT_CHECK_CUDA(cudaGetLastError());
-        return 0;
+        if (once) return g == 1 ? step(window_step_kernel<1, 8, 16>, 8, rows) : g == 2 ? step(window_step_kernel<2, 8, 16>, 8, rows) : step(window_step_kernel<4, 8, 16>, 8, rows);
+        const size_t few = (size_t)4 * 8 * row;
+        if (row >= 512) return g == 1 ? step(window_step_kernel<1, 4, 8>, 4, few) : g == 2 ? step(window_step_kernel<2, 4, 8>, 4, few) : step(window_step_kernel<4, 4, 8>, 4, few);
     }
     dim3 grid(T, a.H);
     const int vpl = (a.vdim + 31) / 32;

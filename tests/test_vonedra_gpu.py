@@ -723,3 +723,21 @@ def test_attention_of_single_tokens_by_group_and_window(heads, kv_heads, dim, vd
             assert rel(got[n], oracle_logits(spec, w, seqs[n])) < TOL, n
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,tokens", [(8, 8, 128, 128, 19), (40, 40, 64, 64, 12), (20, 20, 96, 100, 16), (16, 8, 128, 128, 19), (30, 10, 96, 100, 15), (32, 8, 128, 64, 19),
+                                                            (40, 40, 32, 32, 12)])
+@pytest.mark.parametrize("size,keep_first", [(33, 3), (400, 0)])
+def test_attention_of_more_single_tokens_than_run_at_once(heads, kv_heads, dim, vdim, tokens, size, keep_first):
+    """One CTA a (token, key head) and more of them than an SM each: histories around whole rounds of 8 and 32 keys, two layers."""
+    spec, w = make([layer(attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, size=size, keep_first=keep_first, scale=dim ** -0.5, rows=9)),
+                    layer(attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, size=size, keep_first=keep_first, scale=dim ** -0.5))], width=64, seed=size + dim)
+    eng = engine(spec, w, max_batch=tokens, max_sessions=tokens, max_batched_tokens=2048, num_pages=4 * tokens, debug_logit_rows=2048)
+    try:
+        lengths = [1, 5, 6, 7, 8, 13, 29, 30, 31, 32, 33, 61, 93, 94, 95, 125, 157, 190, 2][:tokens]
+        seqs = {f"s{i}": tokens_of(spec, n + 4, 60 + i) for i, n in enumerate(lengths)}
+        got = feed_plan(eng, seqs, [{n: len(t) - 4 for n, t in seqs.items()}] + [dict.fromkeys(seqs, 1)] * 4)
+        for n in seqs:
+            assert rel(got[n], oracle_logits(spec, w, seqs[n])) < TOL, n
+    finally:
+        eng.close()
