@@ -38,10 +38,6 @@ def gemm_bf16(w: torch.Tensor, x: torch.Tensor, x_lo: Optional[torch.Tensor] = N
     if mode == "partials":
         if n_splits <= 0:
             n_splits = lib.ft_gemm_pick_splits(n_out, T, K, int(x_lo is not None))
-            # Few tokens and both planes: CTAs of a cluster share K and add their parts themselves.  Ahead of parts and a sum behind them up to 64 tokens
-            # (us, 2048 x 2048, parts + sum -> one: 4 tokens 7.9 -> 5.4, 64 tokens 9.5 -> 8.0), but for long K from 49 on (64 tokens of 2048 x 8192: 13.8, 14.0)
-            if x_lo is not None and (T <= 48 or (T <= 64 and K <= 4096)):
-                n_splits = 1
         out = torch.empty(n_splits, T, n_out, device=x.device, dtype=torch.float32)
         N.check(lib.ft_gemm_bf16(N.ptr(w), N.ptr(x), N.ptr(x_lo), N.ptr(out), 0, n_out, T, K, n_splits, 0, st),
                 "ft_gemm_bf16")
