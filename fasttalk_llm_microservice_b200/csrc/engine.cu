@@ -2356,8 +2356,15 @@ static Session* session_for(Engine* e, unsigned long long key, const char* who) 
 
 // A caller's fresh array has no pages yet, and the copy into it would take their faults one by one behind the step (turn of four Llama sessions, 128256 logits a row: 38.5 ms, so 31.5, where
 // a fault is dear; level where the arrays' memory is used again).
-// They are taken here, while the GPU computes; the array's bytes stay as they are.
+// They are taken here, while the GPU computes; the array's bytes stay as they are.  Only memory that CUDA does not know is touched: pinned pages are there, and a
+// device address, which is not the host's to read, is for the copy to take or to refuse.
 static void fault_in(void* p, size_t bytes) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return;
     static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
     volatile char* c = static_cast<volatile char*>(p);
     for (size_t i = 0; i < bytes; i += page) c[i] = c[i];

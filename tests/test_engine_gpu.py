@@ -161,6 +161,33 @@ def test_stop_cancel_and_limits(tiny):
     assert eng.stats()["free_pages"] > free
 
 
+def test_fed_logits_into_memory_of_any_kind(tiny):
+    """A caller's place for the logits may be ordinary or page-locked memory; a device address comes back filled or refused and is never read by the host."""
+    from fasttalk_llm_microservice_b200 import native as N
+    from fasttalk_llm_microservice_b200.engine import session_key
+    spec, w = tiny[:2]
+    eng = make_engine(spec, w, debug_logit_rows=8)
+    toks, want, count = np.array([3, 1, 4, 1, 5], np.int32), np.array([0, 4], np.int32), np.array([5], np.int32)
+
+    def feed(name, at):
+        key = np.array([session_key(name)], np.uint64)
+        return eng.lib.ft_engine_feed(eng._h, 1, key.ctypes.data, count.ctypes.data, toks.ctypes.data, 2, want.ctypes.data, at)
+    try:
+        plain, again = np.empty((2, spec.vocab), np.float32), np.empty((2, spec.vocab), np.float32)
+        assert feed("a", plain.ctypes.data) == 0
+        pinned = torch.empty(2, spec.vocab, pin_memory=True)
+        assert feed("b", pinned.data_ptr()) == 0
+        assert np.array_equal(pinned.numpy(), plain)
+        device = torch.zeros(2, spec.vocab, device="cuda")
+        rc = feed("c", device.data_ptr())
+        torch.cuda.synchronize()
+        assert (rc == 0 and np.array_equal(device.cpu().numpy(), plain)) or (rc < 0 and "logits copy" in N.last_error())
+        assert feed("d", again.ctypes.data) == 0
+        assert np.array_equal(again, plain)
+    finally:
+        eng.close()
+
+
 def test_eos_stops():
     from fasttalk_llm_microservice_b200.model_spec import SPECS
     from fasttalk_llm_microservice_b200.weights import init_weights
