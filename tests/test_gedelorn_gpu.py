@@ -912,3 +912,18 @@ def test_step_graphs_are_kept_replaced_and_left_for_the_trail():
     finally:
         eng.close()
         plain.close()
+
+
+@pytest.mark.parametrize("heads,vdim,groups", [(27, 76, 1), (54, 76, 2), (32, 128, 1), (41, 100, 1), (64, 64, 1), (64, 128, 1)])
+@pytest.mark.parametrize("exact", [True, False], ids=["rows", "planes"])
+def test_read_out_of_long_rows(heads, vdim, groups, exact):
+    """Norm groups of more than 2048 columns, 2052 to 8192: with a gate before the norm and a skip (state space), with a gate behind the norm (decay attention); as fp32
+    rows and, where the projection behind takes them, as the bf16 planes of long portions."""
+    spec, w = make([layer(space(heads=heads, vdim=vdim, state=6, groups=1, norm_groups=groups)),
+                    layer(parallel(right=decaying(heads=heads, dim=4, vdim=vdim, decay=[0.5 + 0.49 * h / heads for h in range(heads)])))], width=128, seed=heads + vdim)
+    eng = engine(spec, w, exact_f32=exact)
+    try:
+        toks = tokens_of(spec, 47, heads)
+        assert rel(feed_cut(eng, "s", toks, [40, 1, 1, 5]), oracle_logits(spec, w, toks)) < (TOL if exact else 4e-4)
+    finally:
+        eng.close()
