@@ -79,16 +79,9 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     return r;
 }
 
-// whole numbers that the compiler knows, and loops over them
+// a whole number that the compiler knows
 template <int I>
 struct Int { static constexpr int value = I; };
-template <int N, int I = 0, class F>
-__device__ __forceinline__ void static_for(F&& f) {
-    if constexpr (I < N) {
-        f(Int<I>{});
-        static_for<N, I + 1>(f);
-    }
-}
 
 // rows of fp32 in groups of four columns on 16 bytes
 __device__ __forceinline__ float4 load_f4(const float* p) { return *reinterpret_cast<const float4*>(p); }

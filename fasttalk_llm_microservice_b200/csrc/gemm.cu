@@ -6,11 +6,10 @@
 // through a ring of TMA stages exactly once (measured ~6 TB/s in steady state).  Split-K over
 // gridDim.z gives one full wave of CTAs when n_out/128 is small.
 //
-// Activations come as TWO bf16 planes, hi = bf16(x) and lo = bf16(x - hi): both are multiplied
-// by the same weight tile into the same TMEM accumulator (D += W*hi; D += W*lo).  That keeps
-// ~16 mantissa bits of every activation through a pure bf16 x bf16 -> fp32 tensor-core product;
-// the weight tile is already in shared memory, so in the HBM-bound decode regime the second
-// product is free.  lo may be absent (HILO = false).
+// Activations come as TWO bf16 planes, hi = bf16(x) and lo = bf16(x - hi), both multiplied by the same weight tile, which keeps ~16 mantissa bits of every
+// activation through a pure bf16 x bf16 -> fp32 tensor-core product.  The kernel of a tile per CTA lays the planes one behind the other as ONE operand of twice
+// the tokens: the two sums lie side by side in TMEM and are added on the way out.  The persistent and the CTA-pair kernels add both into the same
+// accumulator (D += W*hi; D += W*lo).  The weight tile is in shared memory for both, so in the HBM-bound decode regime lo is free.  lo may be absent (HILO = false).
 //
 // Epilogue (8 warps): phase 1 moves the fp32 accumulator tile TMEM -> [token][row] staging
 // (shared memory, or — when K is split — this CTA's slab of an L2-resident scratch buffer);
