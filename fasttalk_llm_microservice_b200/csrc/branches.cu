@@ -526,9 +526,9 @@ __global__ void __launch_bounds__(WARPS * 32, step_ctas(GRP, WARPS)) window_step
             for (int h = 0; h < GRP; ++h) top[h] = fmaxf(top[h], __shfl_xor_sync(0xffffffffu, top[h], o));
 #pragma unroll
         for (int h = 0; h < GRP; ++h) {
-            const float m_new = fmaxf(m[h], top[h]);
-            corr[h] = h < grp ? expf(m[h] - m_new) : 0.f;        // 0 on the first block (m = -inf)
-            sum[h] = valid && h < grp ? expf(s[h] - m_new) : 0.f;
+            const float m_new = fmaxf(m[h], top[h]), base = m_new == -INFINITY ? 0.f : m_new;      // (scores may all be -inf so far: their weights are 0)
+            corr[h] = h < grp ? expf(m[h] - base) : 0.f;         // 0 on the first block (m = -inf)
+            sum[h] = valid && h < grp ? expf(s[h] - base) : 0.f;
             m[h] = m_new;
             ps[wid][lane & (KEYS - 1)][h] = sum[h];
         }

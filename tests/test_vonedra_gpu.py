@@ -741,3 +741,21 @@ def test_attention_of_more_single_tokens_than_run_at_once(heads, kv_heads, dim, 
             assert rel(got[n], oracle_logits(spec, w, seqs[n])) < TOL, n
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("heads,kv_heads,tokens", [(2, 2, 1), (8, 2, 5), (40, 40, 12)])
+def test_attention_of_single_tokens_with_keys_that_the_bias_hides(heads, kv_heads, tokens):
+    """The bias of far keys is minus infinity: a warp's keys may all be hidden, which leaves the sums of the others as they are."""
+    def hide(w):
+        w["l0.mix.rel"][-1] = float("-inf")
+    spec, w = make([layer(attention(heads=heads, kv_heads=kv_heads, dim=128 if heads == 8 else 64, vdim=64, size=400, keep_first=0, rows=7, bias_max=7, scale=0.1))], width=64, seed=heads,
+                   tweak=hide)
+    eng = engine(spec, w, max_batch=tokens, max_sessions=tokens)
+    try:
+        seqs = {f"s{i}": tokens_of(spec, 18 + i, i) for i in range(tokens)}
+        got = feed_plan(eng, seqs, [{n: len(t) - 3 for n, t in seqs.items()}] + [dict.fromkeys(seqs, 1)] * 3)
+        for n in seqs:
+            ref = oracle_logits(spec, w, seqs[n])
+            assert np.isfinite(ref).all() and rel(got[n], ref) < TOL, n
+    finally:
+        eng.close()
