@@ -1102,12 +1102,12 @@ int gemm_pick_splits(int n_out, int T, int K, int num_sms, bool hilo) {
     return s < 1 ? 1 : s;
 }
 
-// The same for fp32 results that the caller adds up.  Few tokens from both planes come as ONE result, K shared by up to eight CTAs of a cluster that add their
+// Parts of an fp32 result that the caller adds up, so that the sum is there soonest.  Few tokens from both planes come as ONE result, K shared by up to eight CTAs of a cluster that add their
 // parts themselves (gemm_plain.cu), unless K is so long for the row tiles that the sixteen shares a split may have are ahead with their sum behind them.  us, parts and
 // sum against one result, weights out of HBM: 2048 x 2048 of 4 tokens 8.4, 5.5; of 64 9.7, 8.1; 8192 columns of 48: 128 rows 10.3, 10.1, 512 10.3, 10.5, 2048 13.5,
 // 13.2; of 64: 10.3, 10.4, 10.5, 10.8, 13.7, 13.9, but 3072 rows 16.2, 15.9; 14336 columns of 16: 128 rows 9.8, 10.3, 256 10.2, 10.2, 512 11.0, 10.5; of 32: 512 11.2, 12.4,
 // 1024 12.9, 13.1, 1536 14.5, 14.4; of 48: 2048 16.9, 18.2, 3072 22.0, 20.7.
-static int gemm_partial_splits(int n_out, int T, int K, int num_sms, bool hilo) {
+static int gemm_pick_parts(int n_out, int T, int K, int num_sms, bool hilo) {
     if (hilo && T <= 64) {
         const int bn = gemm_pick_bn(T, true);
         if (K <= (T <= 48 ? 8192 : 4096) || n_out >= (bn == 16 ? 512 : 48 * bn)) return 1;
@@ -1402,7 +1402,7 @@ extern "C" int ft_gemm_fused(const void* w, const void* x, const void* x_lo, int
     const bool staged = epi->mode == FT_EPI_RESID || epi->mode == FT_EPI_QKV_ROPE;
     const int bn = gemm_pick_bn(T, hilo);
     if (n_splits <= 0)
-        n_splits = epi->mode == FT_EPI_PARTIAL ? gemm_partial_splits(n_out, T, K, sms, hilo) : staged ? gemm_pick_splits(n_out, T, K, sms, hilo) : 1;
+        n_splits = epi->mode == FT_EPI_PARTIAL || staged ? gemm_pick_splits(n_out, T, K, sms, hilo) : 1;
     if (hilo && epi->mode == FT_EPI_PARTIAL && n_splits == 1)      // one unsplit fp32 result: the kernels made for it
         return launch_gemm_plain(w, x, x_lo, reinterpret_cast<float*>(epi->out), n_out, T, K, static_cast<cudaStream_t>(stream));
     CUtensorMap mw, mx, mxl;
@@ -1457,5 +1457,9 @@ extern "C" long long ft_gemm_scratch_bytes(int n_out, int T, int K, int n_splits
 }
 
 extern "C" int ft_gemm_pick_splits(int n_out, int T, int K, int hilo) {
-    return ft::gemm_partial_splits(n_out, T, K, ft::device_sms(), hilo != 0);
+    return ft::gemm_pick_splits(n_out, T, K, ft::device_sms(), hilo != 0);
+}
+
+extern "C" int ft_gemm_pick_parts(int n_out, int T, int K, int hilo) {
+    return ft::gemm_pick_parts(n_out, T, K, ft::device_sms(), hilo != 0);
 }

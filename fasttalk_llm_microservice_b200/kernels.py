@@ -37,7 +37,7 @@ def gemm_bf16(w: torch.Tensor, x: torch.Tensor, x_lo: Optional[torch.Tensor] = N
     st = N.cur_stream()
     if mode == "partials":
         if n_splits <= 0:
-            n_splits = lib.ft_gemm_pick_splits(n_out, T, K, int(x_lo is not None))
+            n_splits = lib.ft_gemm_pick_parts(n_out, T, K, int(x_lo is not None))
         out = torch.empty(n_splits, T, n_out, device=x.device, dtype=torch.float32)
         N.check(lib.ft_gemm_bf16(N.ptr(w), N.ptr(x), N.ptr(x_lo), N.ptr(out), 0, n_out, T, K, n_splits, 0, st),
                 "ft_gemm_bf16")

@@ -105,6 +105,7 @@ SIGNATURES = {
     "ft_ipc_close": (_I, [_VP]),
     "ft_gemm_bf16": (_I, [_VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _VP]),
     "ft_gemm_pick_splits": (_I, [_I, _I, _I, _I]),
+    "ft_gemm_pick_parts": (_I, [_I, _I, _I, _I]),
     "ft_debug_gemm_trace": (_I, [_VP]),
     "ft_debug_gemm_trace_hist": (_I, [_VP, _I]),
     "ft_gemm_scratch_bytes": (_LL, [_I, _I, _I, _I]),

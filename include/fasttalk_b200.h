@@ -480,6 +480,9 @@ int ft_engine_debug_read_trail(ft_engine* e, float* host_out, int rows);
 int ft_gemm_bf16(const void* w, const void* x, const void* x_lo, void* out, void* out_lo, int n_out, int T,
                  int K, int n_splits, int out_mode, void* stream);
 int ft_gemm_pick_splits(int n_out, int T, int K, int hilo);
+/* The n_splits with which the SUM over the partial results of out_mode 0 is there soonest: 1 for few tokens of both planes, whose CTAs add their shares
+ * of K up themselves, where that is ahead of parts and a sum behind them; else as ft_gemm_pick_splits. */
+int ft_gemm_pick_parts(int n_out, int T, int K, int hilo);
 /* Tuning aid: globaltimer (ns) timeline of CTA (0,0,0) of the most recent GEMM launch -> HOST
  * uint64[16]: 0 entry, 1 set-up done, 2 weights requested, 3 dependency wait passed, 4 first stage
  * landed, 5 last MMA issued, 6 accumulator ready, 7 epilogue stores issued, 8 reduce done, 9 exit. */

@@ -91,8 +91,8 @@ def test_a_c_host_links_and_runs(tmp_path):
 
 def test_parts_of_few_token_projections():
     """One result where its cluster form is ahead of parts and a sum behind them, parts where K is long for the row tiles, for one plane and for many tokens."""
-    pick = native.load().ft_gemm_pick_splits
+    pick, splits = native.load().ft_gemm_pick_parts, native.load().ft_gemm_pick_splits
     for n_out, T, K, one in [(2048, 1, 2048, True), (128, 48, 8192, True), (512, 64, 4096, True), (512, 64, 4160, False), (3072, 64, 14336, True), (512, 16, 14336, True),
                              (256, 16, 14336, False), (1024, 32, 14336, False), (1536, 32, 14336, True), (2048, 48, 14336, False), (3072, 48, 14336, True), (1024, 65, 1024, False)]:
         assert (pick(n_out, T, K, 1) == 1) == one, (n_out, T, K)
-        assert pick(n_out, T, K, 0) > 1
+        assert pick(n_out, T, K, 0) == splits(n_out, T, K, 0) > 1 and splits(n_out, T, K, 1) > 1

@@ -474,17 +474,19 @@ def test_gemm_few_tokens_as_one_result_or_parts(K, n_out, Kd, T):
 
 
 @pytest.mark.parametrize("n_out,T,Kd", [(256, 4, 512), (512, 16, 8256), (384, 16, 8256), (1024, 40, 8192), (1024, 40, 8256), (512, 49, 4096), (512, 64, 4160), (3072, 64, 4160)])
-def test_gemm_parts_left_to_the_library(K, n_out, T, Kd):
-    """A C caller that leaves the count of parts to the library gets what ft_gemm_pick_splits names, the same as the Python call."""
+def test_gemm_parts_that_the_library_names(K, n_out, T, Kd):
+    """A C caller that asks for the parts gets what the Python call takes; one that leaves their count out gets what ft_gemm_pick_splits names, as ever."""
     from fasttalk_llm_microservice_b200 import native as N
     g = torch.Generator(device=DEV).manual_seed(n_out + T)
     w = (torch.randn(n_out, Kd, device=DEV, generator=g) * 0.05).bfloat16()
     x, x_lo = K.split_hi_lo(torch.randn(T, Kd, device=DEV, generator=g))
-    lib = N.load()
-    out = torch.empty(lib.ft_gemm_pick_splits(n_out, T, Kd, 1), T, n_out, device=DEV, dtype=torch.float32)
-    N.check(lib.ft_gemm_bf16(N.ptr(w), N.ptr(x), N.ptr(x_lo), N.ptr(out), 0, n_out, T, Kd, 0, 0, N.cur_stream()), "ft_gemm_bf16")
-    assert torch.equal(out, K.gemm_bf16(w, x, x_lo))
-    assert rel_err(out.sum(0), hilo(x, x_lo).double() @ w.double().T) < 1e-6 + Kd / 16 * 2.0 ** -23
+    lib, tol = N.load(), 1e-6 + Kd / 16 * 2.0 ** -23
+    ref = hilo(x, x_lo).double() @ w.double().T
+    for count, given in ((lib.ft_gemm_pick_parts(n_out, T, Kd, 1), True), (lib.ft_gemm_pick_splits(n_out, T, Kd, 1), False)):
+        out = torch.empty(count, T, n_out, device=DEV, dtype=torch.float32)
+        N.check(lib.ft_gemm_bf16(N.ptr(w), N.ptr(x), N.ptr(x_lo), N.ptr(out), 0, n_out, T, Kd, count if given else 0, 0, N.cur_stream()), "ft_gemm_bf16")
+        assert not given or torch.equal(out, K.gemm_bf16(w, x, x_lo))
+        assert rel_err(out.sum(0), ref) < tol
 
 
 def test_attn_decode_cfg2_shape(K):
