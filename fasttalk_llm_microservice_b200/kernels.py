@@ -194,16 +194,17 @@ def attn_prefill(q: torch.Tensor, kv_layer: torch.Tensor, page_table: torch.Tens
     # The lists go up in one copy that the host does not wait for (five waiting ones cost 60 us of GPU time between calls).  While a
     # stream is captured the copy is an ordinary one, which capture refuses: a replay would read memory that is no longer this call's.
     i32 = lambda v: torch.tensor(v, device="cpu", dtype=torch.int32).reshape(-1)
-    parts = [i32(v) for v in (req_q_start, req_slot, req_pos0, tile_req, tile_q0)]
+    n = len(tile_req)
+    parts = [i32(v) for v in (req_q_start, req_slot, req_pos0, tile_req + tile_q0)]
     assert parts[2].numel() >= len(req_slot), "req_pos0: a position for every request"
     rows = T if tensor_cores else 0
     lib = N.load()
-    few = N.check(lib.ft_attn_prefill_order_tiles(N.ptr(parts[0]), N.ptr(parts[2]), N.ptr(parts[3]), N.ptr(parts[4]), len(tile_req), nq, nkv, d, rows),
-                  "ft_attn_prefill_order_tiles")
+    tiles = N.ptr(parts[3])
+    few = N.check(lib.ft_attn_prefill_order_tiles(N.ptr(parts[0]), N.ptr(parts[2]), tiles, tiles + 4 * n, n, nq, nkv, d, rows), "ft_attn_prefill_order_tiles")
     lists = torch.cat(parts)
     waits = dev.index != torch.cuda.current_device() or torch.cuda.is_current_stream_capturing()
     lists = lists.to(dev) if waits else lists.pin_memory().to(dev, non_blocking=True)
-    t_qs, t_slot, t_pos0, t_treq, t_tq0 = lists.split([p.numel() for p in parts])
+    t_qs, t_slot, t_pos0, t_treq, t_tq0 = lists.split([p.numel() for p in parts[:3]] + [n, n])
     # rows that no request owns are zeros
     starts = parts[0].tolist()[:len(req_slot) + 1]
     owned = bool(starts) and starts[0] == 0 and starts[-1] == T and all(x <= y for x, y in zip(starts, starts[1:]))
@@ -211,7 +212,7 @@ def attn_prefill(q: torch.Tensor, kv_layer: torch.Tensor, page_table: torch.Tens
     out_lo = torch.empty_like(out) if owned else torch.zeros_like(out)
     N.check(lib.ft_attn_prefill_ordered(N.ptr(q), N.ptr(kv_layer), N.ptr(page_table), page_table.shape[1],
                                         N.ptr(t_qs), N.ptr(t_slot), N.ptr(t_pos0), N.ptr(t_treq), N.ptr(t_tq0),
-                                        len(tile_req), N.ptr(out), N.ptr(out_lo), nq, nkv, d, rows, few, N.cur_stream()),
+                                        n, N.ptr(out), N.ptr(out_lo), nq, nkv, d, rows, few, N.cur_stream()),
             "ft_attn_prefill")
     return out, out_lo
 
